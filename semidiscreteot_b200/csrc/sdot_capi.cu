@@ -14,6 +14,7 @@
 
 #include "sdot_device.cuh"
 #include "sdot_internal.h"
+#include "sdot_lattice_host.h"
 
 using namespace sdot;
 
@@ -203,6 +204,7 @@ size_t device_bytes(const sdot_ctx *c)
 {
     return c->x.bytes() + c->rho.bytes() + c->jxw.bytes() + c->w.bytes() + c->cell_ctr.bytes() +
            c->sblk_sph.bytes() + c->sblk_sph32.bytes() + c->sblk_cell.bytes() + c->tblk_off.bytes() +
+           c->lat_x.bytes() + c->lat_q.bytes() +
            c->tblk_sph32.bytes() + c->part.bytes() + c->fwd_t.bytes() + c->pmask.bytes() + c->pmpre.bytes() +
            c->inv_b.bytes() + c->fwd2inv.bytes() + c->inv_tmpb.bytes() + c->inv_tmpk.bytes() + c->inv_off.bytes() +
            c->y.bytes() + c->nu.bytes() + c->perm.bytes() +
@@ -233,7 +235,7 @@ sdot_status ensure_eval_buffers(sdot_ctx *c)
     CK(c->grad.alloc(nt), "alloc grad");
     CK(c->tpack.alloc(nt * TPACK), "alloc tpack");
     CK(c->Lq.alloc(nq), "alloc Lq");
-    CK(c->gpart.alloc(nt * dense_grad_slices(INT64_MAX / 2, nt)), "alloc gpart");
+    CK(c->gpart.alloc(std::max<size_t>(nt * dense_grad_slices(INT64_MAX / 2, nt), dense_gpart_need(c))), "alloc gpart");
     CK(c->blkpart.alloc(4 * nval), "alloc blkpart");
     CK(c->redpart.alloc(148 * 8), "alloc redpart");
     CK(c->scal.alloc(SC_COUNT), "alloc scal");
@@ -450,7 +452,7 @@ void sdot_destroy(sdot_ctx *c)
         c->y.release(); c->nu.release();
         c->perm.release(); c->tblk_sph.release(); c->psi.release(); c->grad.release(); c->tpack.release();
         c->Lq.release(); c->gpart.release(); c->blkpart.release(); c->scal.release(); c->redpart.release();
-        c->vpart.release();
+        c->vpart.release(); c->lat_x.release(); c->lat_q.release();
         c->io_a.release(); c->io_b.release(); c->x0.release(); c->pdir.release(); c->sk.release(); c->yk.release();
         c->hist_s.release(); c->hist_y.release(); c->gtmp.release();
         if (c->scal_host) cudaFreeHost(c->scal_host);
@@ -609,6 +611,24 @@ sdot_status sdot_set_source(sdot_ctx *c, int dim, int64_t n_q, const double *x, 
     CK(cudaMemcpy(c->cell_ctr.p, hc.data(), hc.size() * 8, cudaMemcpyHostToDevice), "copy cells");
     CK(cudaMemcpy(c->sblk_sph.p, ssph.data(), ssph.size() * 8, cudaMemcpyHostToDevice), "copy spheres");
     CK(cudaMemcpy(c->sblk_cell.p, bounds.data(), bounds.size() * 8, cudaMemcpyHostToDevice), "copy blocks");
+    // tensor lattice of the points, for the untruncated sweeps
+    c->lat_ok = false;
+    Lattice lat;
+    find_lattice(hx.data(), n_q, dim, lat);
+    if (lat.ok) {
+        CK(c->lat_x.alloc(lat.X.size()), "alloc lattice");
+        CK(c->lat_q.alloc(n_q), "alloc lattice");
+        CK(cudaMemcpy(c->lat_x.p, lat.X.data(), lat.X.size() * 8, cudaMemcpyHostToDevice), "copy lattice");
+        CK(cudaMemcpy(c->lat_q.p, lat.q.data(), lat.q.size() * sizeof(int), cudaMemcpyHostToDevice), "copy lattice");
+        for (int d = 0; d < 3; ++d) {
+            c->lat_n[d] = lat.n[d];
+            c->lat_xo[d] = lat.xo[d];
+            c->lat_period[d] = lat.period[d];
+            c->lat_step[d] = lat.step[d];
+        }
+        c->lat_X = lat.X;
+        c->lat_ok = true;
+    }
     c->src_sph_host = ssph;
     c->covering_radius = 0.0;  // reference: recomputed by the next solve
     c->nq = n_q;
@@ -619,6 +639,7 @@ sdot_status sdot_set_source(sdot_ctx *c, int dim, int64_t n_q, const double *x, 
         c->ncells = 0;
         return cuda_error(c, eg, "set_source: block spheres");
     }
+    ++c->geometry_id;
     return SDOT_OK;
 }
 
@@ -682,6 +703,7 @@ sdot_status sdot_set_target(sdot_ctx *c, int64_t n, const double *y, const doubl
         c->nt = 0;
         return cuda_error(c, eg, "set_target: block spheres");
     }
+    ++c->geometry_id;
     return SDOT_OK;
 }
 

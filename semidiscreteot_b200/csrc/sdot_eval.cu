@@ -32,6 +32,8 @@
 #include "sdot_dense.cuh"
 #include "sdot_device.cuh"
 #include "sdot_internal.h"
+#include "sdot_lattice.cuh"
+#include "sdot_lattice_host.h"
 
 namespace sdot {
 
@@ -108,24 +110,98 @@ __global__ void k_minmax(const double *v, int64_t n, double *out)
 
 // tpack[j] = {A_j, B_j(DIM), nu_j, y_j(DIM)}: scaled exponent coefficients.
 template <int DIM>
+__device__ __forceinline__ void target_prep_one(int64_t j, const double *__restrict__ y, const double *__restrict__ nu,
+                                                const double *__restrict__ psi, const EvalArgs &a,
+                                                double *__restrict__ tpack)
+{
+    double yt[3], ysq = 0.0;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+        yt[d] = y[j * DIM + d] - a.o[d];
+        ysq += yt[d] * yt[d];
+    }
+    double *t = tpack + j * TPACK;
+    t[0] = a.s * psi[j] - a.halfs * ysq;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) t[1 + d] = a.s * yt[d];
+    t[1 + DIM] = nu[j];
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) t[2 + DIM + d] = y[j * DIM + d];
+}
+
+template <int DIM>
 __global__ void k_target_prep(int64_t nt, const double *__restrict__ y, const double *__restrict__ nu,
                               const double *__restrict__ psi, EvalArgs a, double *__restrict__ tpack)
 {
-    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < nt; j += (int64_t)gridDim.x * blockDim.x) {
-        double yt[3], ysq = 0.0;
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) {
-            yt[d] = y[j * DIM + d] - a.o[d];
-            ysq += yt[d] * yt[d];
-        }
-        double *t = tpack + j * TPACK;
-        t[0] = a.s * psi[j] - a.halfs * ysq;
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) t[1 + d] = a.s * yt[d];
-        t[1 + DIM] = nu[j];
-#pragma unroll
-        for (int d = 0; d < DIM; ++d) t[2 + DIM + d] = y[j * DIM + d];
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < nt; j += (int64_t)gridDim.x * blockDim.x)
+        target_prep_one<DIM>(j, y, nu, psi, a, tpack);
+}
+
+// Target packing (with the target blocks' largest s psi and the targets' step
+// factors, to full precision: a run multiplies up to seven of them) and the lattice
+// tiles' shifts in one launch: the first npb CTAs pack the targets, warp <->
+// target block, the others take one tile each.
+constexpr int LAT_PREP_THREADS = 512;
+template <int DIM>
+__global__ void __launch_bounds__(LAT_PREP_THREADS)
+k_lat_prep(const double *__restrict__ y, const double *__restrict__ nu, const double *__restrict__ psi, EvalArgs a,
+           LatArgs L, const int64_t *__restrict__ tblk_off, int ntb, int npb, double *__restrict__ tpack,
+           double *__restrict__ top, double *__restrict__ shift, double *__restrict__ step)
+{
+    if ((int)blockIdx.x >= npb) {
+        lat_shift_block<DIM, LAT_PREP_THREADS>(L, a, blockIdx.x - npb, y, psi, shift);
+        return;
     }
+    constexpr int NW = LAT_PREP_THREADS / 32;
+    const int lane = threadIdx.x & 31;
+    for (int b = blockIdx.x * NW + (threadIdx.x >> 5); b < ntb; b += npb * NW) {
+        const int64_t j = tblk_off[b] + lane;
+        double v = -CUDART_INF;
+        if (j < tblk_off[b + 1]) {
+            target_prep_one<DIM>(j, y, nu, psi, a, tpack);
+            v = a.s * psi[j];
+            if (L.runs > 0) {
+#pragma unroll
+                for (int d = 0; d < DIM; ++d) step[j * DIM + d] = exp2(tpack[j * TPACK + 1 + d] * L.step16[d]);
+            }
+        }
+        v = warp_max(v);
+        if (lane == 0) top[b] = v;
+    }
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(LAT_THREADS, 2)
+k_lat_value(LatArgs L, EvalArgs a, const double *__restrict__ tpack, const double *__restrict__ shift,
+            const double *__restrict__ step, int64_t tslice, double *__restrict__ ms)
+{
+    extern __shared__ __align__(16) unsigned char lat_smem[];
+    const int64_t t0 = blockIdx.y * tslice;
+    const int64_t t1 = min(a.nt, t0 + tslice);
+    lat_value_block<DIM>(lat_smem, L, a, tpack, shift, step, blockIdx.x, t0, t1,
+                         ms + ((int64_t)blockIdx.y * L.ntiles + blockIdx.x) * LAT_TILE);
+}
+
+template <int DIM, bool WT>
+__global__ void __launch_bounds__(LAT_THREADS)
+k_lat_merge(LatArgs L, EvalArgs a, LatBlocks K, int nslice, double *__restrict__ ms, const double *__restrict__ shift,
+            const double *__restrict__ tpack, const double *__restrict__ rho, const double *__restrict__ jxw, double *__restrict__ Lq,
+            double *__restrict__ part)
+{
+    constexpr int PER = LAT_TILE / LAT_THREADS;
+    lat_merge_block<DIM, WT>(L, a, K, blockIdx.x / PER, blockIdx.x % PER, nslice, ms, shift, tpack, rho, jxw, Lq,
+                             part + (int64_t)blockIdx.x * 4);
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(LAT_THREADS, 2)
+k_lat_grad(LatArgs L, EvalArgs a, const double *__restrict__ tpack, const double *__restrict__ shift,
+           const double *__restrict__ step, const double *__restrict__ wt, int tslice, double *__restrict__ gpart)
+{
+    extern __shared__ __align__(16) unsigned char lat_smem[];
+    const int ta = blockIdx.y * tslice;
+    lat_grad_block<DIM>(lat_smem, L, a, tpack, shift, step, wt, blockIdx.x * (int64_t)LAT_GT, ta, min(L.ntiles, ta + tslice),
+                        gpart + blockIdx.y * a.nt);
 }
 
 // truncated-path layout: {y(3), nu, log2 nu, kappa psi / eps}
@@ -893,6 +969,11 @@ double host_threshold(sdot_ctx *c, double maxpsi, double minpsi)
 // points) the value sweep runs over cells (k_value_dense_tensor): ncb cell
 // blocks x nvs target slices (about six CTAs per SM in all, at least 32
 // targets per slice, at most 64 slices), always merged per point.
+//
+// Sources whose points form a tensor lattice run the lattice sweeps instead
+// (lat: sdot_lattice.cuh; the value sweep always, the gradient sweep in FP64):
+// ntiles x nvs CTAs of the value sweep (at least 16 targets per slice), and
+// target blocks x gts tile groups of the gradient sweep.
 struct DenseShape {
     int64_t nval, tb;
     int nks;
@@ -900,6 +981,16 @@ struct DenseShape {
     int64_t tslice;   // targets per value slice
     int tm;           // > 0: the cell-based tensor value sweep with tm points per dimension
     int64_t ncb;      // its cell blocks
+    LatTiling lat;    // cap > 0: the lattice sweeps
+    bool lat_grad;    // the gradient sweep too
+    int gts;          // tiles per CTA of the lattice gradient sweep (nks groups)
+    // doubles of the value sweep's partials and of the gradient partials
+    size_t vpart_need(int64_t nq, int64_t nt, int64_t ntblk) const
+    {
+        if (lat.cap > 0) return (size_t)lat.ntiles * ((size_t)nvs * LAT_TILE + 2) + (size_t)(3 * nt + ntblk);
+        return (nvs > 1 || tm > 0) ? (size_t)2 * nvs * nq : 0;
+    }
+    size_t gpart_need(int64_t nt) const { return (size_t)nks * nt; }
 };
 // The tensor value sweep applies to the euclidean untruncated evaluation of
 // cells whose points form a symmetric tensor grid of at most 9 points, with
@@ -936,6 +1027,114 @@ static DenseShape dense_shape(int64_t nq, int64_t nt, int tm = 0, int64_t ncells
         d.tslice = (nt + d.nvs - 1) / d.nvs;
     }
     return d;
+}
+
+// dense_shape for an evaluation of the context's problem at eps (every dense
+// evaluation path takes its shape from here).
+static DenseShape dense_shape_of(const sdot_ctx *c, double eps, bool fp64)
+{
+    const double s = KAPPA / eps;
+    DenseShape d = dense_shape(c->nq, c->nt, dense_tensor_m(c, s), c->ncells);
+    if (!c->lat_ok || c->distance != 0) return d;
+    double reach[3];
+    for (int k = 0; k < 3; ++k)
+        reach[k] = std::max(std::fabs(c->tgt_lo[k] - c->origin[k]), std::fabs(c->tgt_hi[k] - c->origin[k]));
+    d.lat = lat_tiling(c->lat_n, c->lat_xo, c->lat_X.data(), c->dim, s, reach, LAT_BITS);
+    if (d.lat.cap == 0) return d;
+    constexpr int SLOTS = 148 * 2;
+    d.nvs = lat_slices(d.lat.ntiles, (c->nt + 15) / 16, SLOTS);
+    d.tslice = (c->nt + d.nvs - 1) / d.nvs;
+    d.nvs = (int)((c->nt + d.tslice - 1) / d.tslice);
+    d.nval = (int64_t)d.lat.ntiles * (LAT_TILE / LAT_THREADS);
+    d.lat_grad = fp64;
+    if (fp64) {
+        const int g = lat_slices((c->nt + LAT_GT - 1) / LAT_GT, d.lat.ntiles, SLOTS);
+        d.gts = (d.lat.ntiles + g - 1) / g;
+        d.nks = (d.lat.ntiles + d.gts - 1) / d.gts;
+    }
+    return d;
+}
+
+size_t dense_gpart_need(const sdot_ctx *c)
+{
+    if (c->prm.tau > 0 || c->prm.threshold_type != SDOT_THRESH_POINTWISE || !(c->prm.epsilon > 0)) return 0;
+    return dense_shape_of(c, c->prm.epsilon, c->precision == SDOT_PREC_FP64).gpart_need(c->nt);
+}
+
+static LatArgs lat_args(const sdot_ctx *c, const LatTiling &t)
+{
+    LatArgs L{};
+    L.X = c->lat_x.p;
+    L.q = c->lat_q.p;
+    for (int d = 0; d < 3; ++d) {
+        L.n[d] = c->lat_n[d];
+        L.nt[d] = t.nt[d];
+        L.xo[d] = c->lat_xo[d];
+    }
+    L.cap = t.cap;
+    L.ntiles = t.ntiles;
+    lat_runs(c->lat_period, c->lat_step, c->dim, L);
+    return L;
+}
+
+template <class K>
+static void lat_smem_limit(K k, size_t bytes)
+{
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
+// Launches of the lattice sweeps; vpart holds vpart_need doubles (the slices'
+// partials, then the tile shifts, the targets' step factors and the target
+// blocks' largest s psi).
+struct LatScratch {
+    double *shift, *step, *top;
+    LatScratch(const DenseShape &ds, double *vpart, int64_t nt, int dim)
+        : shift(vpart + (size_t)ds.lat.ntiles * ds.nvs * LAT_TILE), step(shift + 2 * ds.lat.ntiles), top(step + nt * dim)
+    {
+    }
+};
+
+template <int DIM>
+static void launch_lat_prep(const sdot_ctx *c, const DenseShape &ds, const double *psi, const EvalArgs &a,
+                            double *tpack, double *vpart, cudaStream_t st)
+{
+    constexpr int NW = LAT_PREP_THREADS / 32;
+    const int npb = (int)std::min<int64_t>((c->ntblk + NW - 1) / NW, 148);
+    const LatScratch S(ds, vpart, a.nt, DIM);
+    k_lat_prep<DIM><<<(unsigned)(npb + ds.lat.ntiles), LAT_PREP_THREADS, 0, st>>>(
+        c->y.p, c->nu.p, psi, a, lat_args(c, ds.lat), c->tblk_off.p, (int)c->ntblk, npb, tpack, S.top, S.shift,
+        S.step);
+}
+
+template <int DIM>
+static void launch_lat_value(const sdot_ctx *c, const DenseShape &ds, const double *tpack, const EvalArgs &a,
+                             double *vpart, double *Lq, double *blkpart, cudaStream_t st)
+{
+    const LatArgs L = lat_args(c, ds.lat);
+    const LatScratch S(ds, vpart, a.nt, DIM);
+    const LatBlocks K{c->tblk_off.p, c->tblk_sph.p, S.top, (int)c->ntblk};
+    const size_t smem = sizeof(LatValueSmem<DIM>);
+    lat_smem_limit(k_lat_value<DIM>, smem);
+    k_lat_value<DIM><<<dim3((unsigned)L.ntiles, (unsigned)ds.nvs), LAT_THREADS, smem, st>>>(
+        L, a, tpack, S.shift, S.step, ds.tslice, vpart);
+    auto merge = [&](auto kern) {
+        kern<<<(unsigned)ds.nval, LAT_THREADS, 0, st>>>(L, a, K, ds.nvs, vpart, S.shift, tpack, c->rho.p, c->jxw.p,
+                                                        Lq, blkpart);
+    };
+    if (ds.lat_grad) merge(k_lat_merge<DIM, true>);
+    else merge(k_lat_merge<DIM, false>);
+}
+
+template <int DIM>
+static void launch_lat_grad(const sdot_ctx *c, const DenseShape &ds, const double *tpack, const EvalArgs &a,
+                            double *vpart, double *gpart, cudaStream_t st)
+{
+    const LatArgs L = lat_args(c, ds.lat);
+    const LatScratch S(ds, vpart, a.nt, DIM);
+    const size_t smem = sizeof(LatGradSmem<DIM>);
+    lat_smem_limit(k_lat_grad<DIM>, smem);
+    k_lat_grad<DIM><<<dim3((unsigned)((a.nt + LAT_GT - 1) / LAT_GT), (unsigned)ds.nks), LAT_THREADS, smem, st>>>(
+        L, a, tpack, S.shift, S.step, vpart, ds.gts, gpart);
 }
 
 template <int DIM>
@@ -1010,7 +1209,17 @@ static sdot_status run_eval(sdot_ctx *c, const EvalArgs &a, bool dense, const do
         if (c->profiling) cudaEventRecord(c->pev[i], st);
     };
     mark(0);
-    if (dense) k_target_prep<DIM><<<grid_for(a.nt, 256), 256, 0, st>>>(a.nt, c->y.p, c->nu.p, c->psi.p, a, c->tpack.p);
+    DenseShape ds{};
+    if (dense && c->distance == 0) {
+        ds = dense_shape_of(c, a.eps, prec == SDOT_PREC_FP64);
+        cudaError_t e = c->vpart.alloc(ds.vpart_need(a.nq, a.nt, c->ntblk));
+        if (e == cudaSuccess) e = c->gpart.alloc(ds.gpart_need(a.nt));
+        if (e == cudaSuccess) e = c->blkpart.alloc((size_t)4 * ds.nval);
+        if (e != cudaSuccess) return cuda_error(c, e, "dense sweep partials");
+    }
+    if (ds.lat.cap > 0) launch_lat_prep<DIM>(c, ds, c->psi.p, a, c->tpack.p, c->vpart.p, st);
+    else if (dense)
+        k_target_prep<DIM><<<grid_for(a.nt, 256), 256, 0, st>>>(a.nt, c->y.p, c->nu.p, c->psi.p, a, c->tpack.p);
     mark(1);
     int64_t nval = 0;
     int nks = 1;
@@ -1024,17 +1233,14 @@ static sdot_status run_eval(sdot_ctx *c, const EvalArgs &a, bool dense, const do
         c->klaunch[2] += 1;
         c->klaunch[3] += 1;
     } else if (dense) {
-        const DenseShape ds = dense_shape(a.nq, a.nt, dense_tensor_m(c, a.s), c->ncells);
         nval = ds.nval;
-        if (ds.tm > 0) {
-            const cudaError_t e = c->vpart.alloc((size_t)2 * ds.nvs * a.nq);
-            if (e != cudaSuccess) return cuda_error(c, e, "dense value slices");
+        if (ds.lat.cap > 0) {
+            launch_lat_value<DIM>(c, ds, c->tpack.p, a, c->vpart.p, c->Lq.p, c->blkpart.p, st);
+        } else if (ds.tm > 0) {
             launch_value_dense_tensor<DIM>(c, ds, c->tpack.p, a, c->vpart.p, st);
             k_value_dense_merge<DIM><<<(unsigned)nval, MERGE_THREADS, 0, st>>>(c->x.p, c->rho.p, c->jxw.p, c->vpart.p,
                                                                                ds.nvs, a, c->Lq.p, c->blkpart.p);
         } else if (ds.nvs > 1) {
-            const cudaError_t e = c->vpart.alloc((size_t)2 * ds.nvs * a.nq);
-            if (e != cudaSuccess) return cuda_error(c, e, "dense value slices");
             k_value_dense_slice<DIM><<<dim3((unsigned)nval, (unsigned)ds.nvs), DENSE_A_THREADS, 0, st>>>(
                 c->x.p, c->tpack.p, a, ds.tslice, c->vpart.p);
             k_value_dense_merge<DIM><<<(unsigned)nval, MERGE_THREADS, 0, st>>>(c->x.p, c->rho.p, c->jxw.p, c->vpart.p,
@@ -1046,7 +1252,8 @@ static sdot_status run_eval(sdot_ctx *c, const EvalArgs &a, bool dense, const do
         mark(2);
         // gradient: target blocks x point (or cell) slices
         nks = ds.nks;
-        launch_grad_dense<DIM>(c, ds, prec != SDOT_PREC_FP64, c->Lq.p, c->tpack.p, c->psi.p, a, c->gpart.p, st);
+        if (ds.lat_grad) launch_lat_grad<DIM>(c, ds, c->tpack.p, a, c->vpart.p, c->gpart.p, st);
+        else launch_grad_dense<DIM>(c, ds, prec != SDOT_PREC_FP64, c->Lq.p, c->tpack.p, c->psi.p, a, c->gpart.p, st);
     } else {
         nval = c->nsblk;
         k_target_prep_kd<DIM><<<grid_for(a.nt, 256), 256, 0, st>>>(a.nt, c->y.p, c->nu.p, c->psi.p, a, c->tpack.p);
@@ -1219,7 +1426,7 @@ sdot_status evaluate_enqueue(sdot_ctx *c, const double *p_dir, double comp_tol, 
         k.misc[0] = c->dim;
         k.misc[1] = c->precision;
         k.misc[2] = partial ? 1 : 0;
-        k.misc[3] = (int64_t)c->vpart.n;
+        k.misc[3] = c->geometry_id;
         s = run_graphed(c, k, body);
     } else {
         s = body();
@@ -1315,13 +1522,11 @@ struct NoallocLayout {
     DenseShape ds;
 };
 
-static NoallocLayout noalloc_layout(const sdot_ctx *c)
+static NoallocLayout noalloc_layout(const sdot_ctx *c, const DenseShape &ds)
 {
     const int64_t nq = c->nq, nt = c->nt;
     auto up = [](int64_t n) { return (n + 31) / 32 * 32; };
     NoallocLayout L{};
-    // the launch shape of the allocating dense path
-    const DenseShape ds = dense_shape(nq, nt, dense_tensor_m(c, KAPPA / c->prm.epsilon), c->ncells);
     L.ds = ds;
     L.nval = ds.nval;
     L.nks = ds.nks;
@@ -1336,7 +1541,7 @@ static NoallocLayout noalloc_layout(const sdot_ctx *c)
     L.blkpart = o; o += up(4 * L.nval);
     L.redpart = o; o += up((int64_t)FIN_BLOCKS * NRED);
     L.scal = o;    o += up(SC_COUNT);
-    L.vpart = o;   o += (L.nvs > 1 || ds.tm > 0) ? up((int64_t)2 * L.nvs * nq) : 0;
+    L.vpart = o;   o += up((int64_t)ds.vpart_need(nq, nt, c->ntblk));
     L.total = o;
     return L;
 }
@@ -1362,8 +1567,11 @@ static void noalloc_launch(sdot_ctx *c, const EvalArgs &a, double *S, const Noal
     cudaStream_t st = c->stream;
     double *psi = S + L.psi, *grad = S + L.grad, *tpack = S + L.tpack, *Lq = S + L.Lq, *gpart = S + L.gpart;
     double *blkpart = S + L.blkpart, *redpart = S + L.redpart, *scal = S + L.scal;
-    k_target_prep<DIM><<<grid_for(a.nt, 256), 256, 0, st>>>(a.nt, c->y.p, c->nu.p, psi, a, tpack);
-    if (L.ds.tm > 0) {
+    if (L.ds.lat.cap > 0) launch_lat_prep<DIM>(c, L.ds, psi, a, tpack, S + L.vpart, st);
+    else k_target_prep<DIM><<<grid_for(a.nt, 256), 256, 0, st>>>(a.nt, c->y.p, c->nu.p, psi, a, tpack);
+    if (L.ds.lat.cap > 0) {
+        launch_lat_value<DIM>(c, L.ds, tpack, a, S + L.vpart, Lq, blkpart, st);
+    } else if (L.ds.tm > 0) {
         double *vpart = S + L.vpart;
         launch_value_dense_tensor<DIM>(c, L.ds, tpack, a, vpart, st);
         k_value_dense_merge<DIM><<<(unsigned)L.nval, MERGE_THREADS, 0, st>>>(c->x.p, c->rho.p, c->jxw.p, vpart, L.nvs,
@@ -1378,7 +1586,8 @@ static void noalloc_launch(sdot_ctx *c, const EvalArgs &a, double *S, const Noal
         k_value_dense<DIM><<<(unsigned)L.nval, DENSE_A_THREADS, 0, st>>>(c->x.p, c->rho.p, c->jxw.p, tpack, a, Lq,
                                                                           blkpart);
     }
-    launch_grad_dense<DIM>(c, L.ds, c->precision != SDOT_PREC_FP64, Lq, tpack, psi, a, gpart, st);
+    if (L.ds.lat_grad) launch_lat_grad<DIM>(c, L.ds, tpack, a, S + L.vpart, gpart, st);
+    else launch_grad_dense<DIM>(c, L.ds, c->precision != SDOT_PREC_FP64, Lq, tpack, psi, a, gpart, st);
     const int fb = launch_finalize_grad(a.nt, L.nks, gpart, c->nu.p, psi, nullptr, c->prm.tolerance, 1, grad, redpart,
                                         st);
     launch_finalize_scalars(st, fb, redpart, L.nval, blkpart, scal);
@@ -1398,7 +1607,11 @@ extern "C" sdot_status sdot_evaluate_device_noalloc(sdot_ctx *c, const double *p
         return set_error(c, SDOT_EINVAL,
                          "no-alloc evaluation covers untruncated problems only (pointwise threshold, tau <= 0)");
     if (c->distance != 0) return set_error(c, SDOT_EINVAL, "no-alloc evaluation covers the euclidean distance only");
-    const NoallocLayout L = noalloc_layout(c);
+    // the launch shape of the allocating path; where the lattice sweeps' partials
+    // do not fit the static scratch, the cell or point sweeps'
+    NoallocLayout L = noalloc_layout(c, dense_shape_of(c, p.epsilon, c->precision == SDOT_PREC_FP64));
+    if ((size_t)L.total * sizeof(double) > NOALLOC_BYTES && L.ds.lat.cap > 0)
+        L = noalloc_layout(c, dense_shape(c->nq, c->nt, dense_tensor_m(c, KAPPA / p.epsilon), c->ncells));
     const size_t need = (size_t)L.total * sizeof(double);
     if (need > NOALLOC_BYTES)
         return set_error(c, SDOT_EINVAL,

@@ -173,6 +173,14 @@ struct sdot_ctx {
     double tensor_amax = 0.0;          // largest per-dimension offset of that grid
     bool tensor_uniform = false;       // the same offset per dimension in every cell (within 1e-13)
     double tensor_a[3] = {0, 0, 0};    // that offset
+    bool lat_ok = false;               // the points are a tensor lattice (sdot_lattice.cuh)
+    int lat_n[3] = {1, 1, 1}, lat_xo[3] = {0, 0, 0};
+    int lat_period[3] = {0, 0, 0};     // period and step of its coordinates (sdot_lattice_host.h)
+    double lat_step[3] = {0, 0, 0};
+    std::vector<double> lat_X;         // its coordinates, dimension after dimension
+    sdot::DevBuf<double> lat_x;        // the same on the device
+    sdot::DevBuf<int> lat_q;           // lattice index -> point (internal order)
+    int64_t geometry_id = 0;           // counts the measures set: part of the evaluation graph's key
 
     // ---- truncated path: block-pair lists and gradient partials ----
     sdot::DevBuf<int64_t> fwd_cnt, fwd_off, inv_cnt, inv_off, fwd2inv;
@@ -300,6 +308,8 @@ int64_t hessian_tc_tiles(int64_t n);
 sdot_status hessian_device(sdot_ctx *c, const double *psi_dev, void *H_dev, int method, int out_f32,
                            sdot_hessian_info *info);
 sdot_status ensure_eval_buffers(sdot_ctx *c);
+// Gradient partials (doubles) of an untruncated evaluation at the current parameters (0 where it truncates).
+size_t dense_gpart_need(const sdot_ctx *c);
 // VerboseSolverControl::check on the last evaluation's scalars: 1 converged,
 // 0 iterate, -1 failure (max_iterations reached or NaN).
 int solver_control_check(sdot_ctx *c, unsigned step, double *value);

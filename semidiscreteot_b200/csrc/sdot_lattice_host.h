@@ -1,0 +1,206 @@
+// sdot_lattice_host.h -- host side of the lattice sweeps (sdot_lattice.cuh):
+// detection of a tensor lattice in a point set, and the tile and slice counts.
+#pragma once
+
+#include <math.h>
+#include <stdint.h>
+#include <string.h>
+
+#include <algorithm>
+#include <vector>
+
+namespace sdot {
+
+// A point set that is a tensor lattice: dimension d has n[d] coordinates
+// X[xo[d]..], ascending, and q[i0 + n0 (i1 + n1 i2)] is the point at them.
+struct Lattice {
+    bool ok = false;
+    int n[3] = {1, 1, 1}, xo[3] = {0, 0, 0};
+    // period[d] > 0: X[i + period] = X[i] + step in dimension d (uniform cells of `period` Gauss points)
+    int period[3] = {0, 0, 0};
+    double step[3] = {0.0, 0.0, 0.0};
+    std::vector<double> X;
+    std::vector<int> q;
+};
+constexpr int LAT_MAXP = 4;   // largest period looked for
+
+// Finds the lattice, or leaves ok = false.  Coordinates are told apart by
+// their bits; where that leaves more coordinates than the lattice can have,
+// those within 4 ulp of the largest coordinate are taken as one (meshes that
+// map each cell by itself round a shared coordinate in the last bits): the
+// exponent's own rounding is larger.  Linear in the points; gives up as soon
+// as a dimension has more coordinates than MAXN.
+inline void find_lattice(const double *x, int64_t n, int dim, Lattice &L)
+{
+    constexpr int MAXN = 8192, CAP = 4 * MAXN;
+    L = Lattice();
+    if (n < 4 || n > INT32_MAX) return;
+    struct Slot {
+        uint64_t key;
+        int id;
+    };
+    std::vector<Slot> table[3];
+    std::vector<double> val[3];
+    auto bits = [](double v) {
+        v = v == 0.0 ? 0.0 : v;
+        uint64_t k;
+        memcpy(&k, &v, 8);
+        return k;
+    };
+    auto at = [&](int d, uint64_t k) {
+        uint64_t h = (k * 0x9e3779b97f4a7c15ull) >> 49;  // 15 bits = CAP slots
+        while (table[d][h].id >= 0 && table[d][h].key != k) h = (h + 1) & (CAP - 1);
+        return (int)h;
+    };
+    for (int d = 0; d < dim; ++d) {
+        table[d].assign(CAP, Slot{0, -1});
+        uint64_t last = 0;
+        bool have = false;
+        for (int64_t i = 0; i < n; ++i) {
+            const uint64_t k = bits(x[i * dim + d]);
+            if (have && k == last) continue;
+            last = k;
+            have = true;
+            const int h = at(d, k);
+            if (table[d][h].id >= 0) continue;
+            if ((int)val[d].size() >= MAXN) return;
+            table[d][h] = Slot{k, (int)val[d].size()};
+            val[d].push_back(x[i * dim + d]);
+        }
+    }
+    std::vector<int> rank[3];
+    std::vector<double> coord[3];
+    for (int merge = 0; merge < 2; ++merge) {
+        int64_t total = 1;
+        for (int d = 0; d < dim; ++d) {
+            const int m = (int)val[d].size();
+            std::vector<int> ord(m);
+            for (int i = 0; i < m; ++i) ord[i] = i;
+            std::sort(ord.begin(), ord.end(), [&](int a, int b) { return val[d][a] < val[d][b]; });
+            const double scale = std::max(fabs(val[d][ord[0]]), fabs(val[d][ord[m - 1]]));
+            const double tol = merge ? 4.0 * 2.220446049250313e-16 * scale : -1.0;
+            rank[d].assign(m, 0);
+            coord[d].clear();
+            for (int i = 0; i < m; ++i) {
+                const double v = val[d][ord[i]];
+                if (coord[d].empty() || v - coord[d].back() > tol) coord[d].push_back(v);
+                rank[d][ord[i]] = (int)coord[d].size() - 1;
+            }
+            total *= (int64_t)coord[d].size();
+        }
+        if (total == n) break;
+        if (merge || total < n) return;
+    }
+    std::vector<int> q((size_t)n, -1);
+    int64_t stride[3] = {1, 1, 1};
+    for (int d = 1; d < dim; ++d) stride[d] = stride[d - 1] * (int64_t)coord[d - 1].size();
+    uint64_t last[3] = {0, 0, 0};
+    int lr[3] = {-1, -1, -1};
+    for (int64_t i = 0; i < n; ++i) {
+        int64_t li = 0;
+        for (int d = 0; d < dim; ++d) {
+            const uint64_t k = bits(x[i * dim + d]);
+            if (lr[d] < 0 || k != last[d]) {
+                last[d] = k;
+                lr[d] = rank[d][table[d][at(d, k)].id];
+            }
+            li += stride[d] * lr[d];
+        }
+        if (q[li] >= 0) return;  // two points at one place: no lattice
+        q[li] = (int)i;
+    }
+    int o = 0;
+    for (int d = 0; d < dim; ++d) {
+        L.n[d] = (int)coord[d].size();
+        L.xo[d] = o;
+        o += L.n[d];
+        L.X.insert(L.X.end(), coord[d].begin(), coord[d].end());
+        const std::vector<double> &c = coord[d];
+        const double tol = 4.0 * 2.220446049250313e-16 * std::max(fabs(c.front()), fabs(c.back()));
+        for (int p = 1; p <= LAT_MAXP && L.period[d] == 0 && 2 * p <= L.n[d]; ++p) {
+            const int cells = (L.n[d] - 1) / p;
+            const double h = (c[cells * p] - c[0]) / cells;
+            bool same = true;
+            for (int i = 0; i + p < L.n[d] && same; ++i) same = fabs(c[i + p] - c[i] - h) <= tol;
+            if (same) {
+                L.period[d] = p;
+                L.step[d] = h;
+            }
+        }
+    }
+    L.q.swap(q);
+    L.ok = true;
+}
+
+// Tiles of one evaluation: points per dimension of a tile (0: the lattice
+// sweeps do not apply) and tile counts.
+struct LatTiling {
+    int cap = 0, nt[3] = {1, 1, 1}, ntiles = 0;
+};
+
+// Tile size for scaled exponents s = kappa / eps and targets within reach[d]
+// of the origin: the largest of 64 and 32 points per dimension (2D) or 16
+// (3D) whose factors span at most 2^(+-bits).  A tile's work goes by its
+// padded size (64 or 32 points per dimension, 16 in 3D); where the padding
+// would make that more than LAT_PAD times the points, the cell sweeps (about
+// four multiply-adds per pair against one here, plus a third for the
+// factors) are the faster ones.
+constexpr double LAT_PAD = 2.5;
+inline LatTiling lat_tiling(const int *n, const int *xo, const double *X, int dim, double s, const double *reach,
+                            double bits)
+{
+    LatTiling best;
+    const int caps2[2] = {64, 32}, caps3[1] = {16};
+    const int *caps = dim == 2 ? caps2 : caps3;
+    const int ncaps = dim == 2 ? 2 : 1;
+    int64_t nq = 1;
+    for (int d = 0; d < dim; ++d) nq *= n[d];
+    for (int k = 0; k < ncaps; ++k) {
+        const int cap = caps[k];
+        double span = 0.0, padded = 1.0;
+        LatTiling t;
+        t.cap = cap;
+        int64_t tiles = 1;
+        for (int d = 0; d < dim; ++d) {
+            t.nt[d] = (n[d] + cap - 1) / cap;
+            tiles *= t.nt[d];
+            double h = 0.0;
+            for (int i = 0; i < t.nt[d]; ++i) {
+                const int a = i * cap, b = std::min(n[d], a + cap) - 1;
+                h = std::max(h, 0.5 * (X[xo[d] + b] - X[xo[d] + a]));
+            }
+            span += s * reach[d] * h / 16.0;
+            const int rest = n[d] - (t.nt[d] - 1) * cap;
+            padded *= (t.nt[d] - 1) * (double)cap + (dim == 2 && rest <= 32 ? 32 : cap);
+        }
+        if (!(span <= bits) || padded > LAT_PAD * (double)nq || tiles > (1 << 20)) continue;
+        t.ntiles = (int)tiles;
+        return t;
+    }
+    return best;
+}
+
+// Slices of n items (targets, tiles) over `units` independent work items so
+// that units x slices CTAs fill whole waves of `slots` resident CTAs: the
+// fewest slices that leave less than a tenth of the last wave idle, at most
+// maxs.
+inline int lat_slices(int64_t units, int64_t maxs, int slots)
+{
+    if (units <= 0 || maxs <= 1) return 1;
+    int best = 1;
+    double beff = 0.0;
+    for (int64_t w = 1; w <= 8; ++w) {
+        const int64_t s = std::min<int64_t>(maxs, w * slots / units);
+        if (s < 1) continue;
+        const int64_t waves = (units * s + slots - 1) / slots;
+        const double eff = (double)(units * s) / (double)(waves * slots);
+        if (eff > beff + 1e-9) {
+            beff = eff;
+            best = (int)s;
+        }
+        if (beff >= 0.9 || s == maxs) break;
+    }
+    return best;
+}
+
+}  // namespace sdot
