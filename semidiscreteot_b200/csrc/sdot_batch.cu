@@ -6,13 +6,13 @@
 // holds many untruncated problems of uneven size packed contiguously in HBM
 // and advances all of them together:
 //
-//  * one batched evaluation = four launches over every active problem:
-//    target packing, a persistent value sweep and a persistent gradient
-//    sweep that pull (problem, block) work units from a queue ordered by cost
-//    (largest first, atomic counter), and a finalize with one CTA per
-//    problem.  The per-unit arithmetic is the single-problem dense sweep's
-//    (sdot_dense.cuh), so a problem's gradient is bitwise the one sdot_evaluate
-//    gives for it alone;
+//  * one batched evaluation covers every active problem with a few launches:
+//    target packing, persistent value and gradient sweeps that pull work
+//    units from a queue ordered by cost (largest first, atomic counter), and
+//    a finalize.  Problems whose points are a tensor lattice (found at the
+//    first evaluation; the points come without cells) run the lattice sweeps
+//    of sdot_lattice.cuh, the others, and every FP32 gradient sweep, the
+//    single-problem point sweeps of sdot_dense.cuh;
 //  * L-BFGS per problem with deal.II's SolverBFGS / LineMinimization logic
 //    (the same rules as sdot_solve) run as a resumable state machine on the
 //    host: every problem's next trial step is evaluated in the same batched
@@ -29,17 +29,22 @@
 #include <stdio.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <map>
 #include <mutex>
 #include <numeric>
 #include <tuple>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "sdot_dense.cuh"
 #include "sdot_device.cuh"
 #include "sdot_internal.h"
+#include "sdot_kd_host.h"
+#include "sdot_lattice.cuh"
+#include "sdot_lattice_host.h"
 
 namespace sdot {
 namespace {
@@ -56,7 +61,21 @@ struct BInst {
     int nks, ntb, nvb;  // gradient slices, target blocks, value blocks
     int fp32;           // gradient sweep with FP32 exponentials
     double tol;         // comp tolerance (componentwise control)
+    // lattice sweeps (lat: the points are a lattice and the tiling applies at this eps)
+    int lat;
+    LatArgs L;
+    LatBlocks K;
+    double *ms, *shift, *step;  // slice sums, tile shifts and the targets' step factors
+    int nvs;            // target slices of the value sweep
+    int64_t tslice;
+    int gts, ngs;       // tiles per unit and tile groups of the FP64 gradient sweep
+    __host__ __device__ bool lat_grad() const { return lat && !fp32; }
+    __host__ __device__ int value_parts() const { return lat ? L.ntiles * (LAT_TILE / LAT_THREADS) : nvb; }
+    __host__ __device__ int grad_parts() const { return lat_grad() ? ngs : nks; }
 };
+
+constexpr int BLAT_PREP = 512;      // threads of k_batch_lat_prep
+constexpr int BLAT_PREP_CTAS = 16;  // CTAs per problem over its target blocks
 
 // ---------------------------------------------------------------------------
 // kernels
@@ -132,34 +151,186 @@ k_batch_grad(const BInst *__restrict__ inst, const int4 *__restrict__ units, int
     }
 }
 
-// One CTA per problem: g = sum of slices - nu, the functional and the norms
-// the control and the line search read (same slots as an evaluation's).
-__global__ void __launch_bounds__(BFIN_THREADS)
-k_batch_final(const BInst *__restrict__ inst, const int *__restrict__ act, const double *__restrict__ gpart,
-              const double *__restrict__ part, const double *__restrict__ nu, const double *__restrict__ psi,
-              const double *__restrict__ pdir, double *__restrict__ grad, double *__restrict__ scal)
+// Lattice problems: the target blocks' largest s psi and the targets' step
+// factors (the first BLAT_PREP_CTAS CTAs of a problem, warp <-> block), and
+// the tiles' shifts (one CTA each).
+template <int DIM>
+__global__ void __launch_bounds__(BLAT_PREP)
+k_batch_lat_prep(const BInst *__restrict__ inst, const int *__restrict__ act, const double *__restrict__ y,
+                 const double *__restrict__ psi)
 {
-    const int pi = act[blockIdx.x];
-    const BInst &I = inst[pi];
-    const int64_t nt = I.a.nt;
+    const BInst &I = inst[act[blockIdx.y]];
+    if (!I.lat) return;
+    const EvalArgs &a = I.a;
+    if ((int)blockIdx.x >= BLAT_PREP_CTAS) {
+        const int t = blockIdx.x - BLAT_PREP_CTAS;
+        if (t < I.L.ntiles) lat_shift_block<DIM, BLAT_PREP>(I.L, a, t, y + I.t0 * DIM, psi + I.t0, I.shift);
+        return;
+    }
+    constexpr int NW = BLAT_PREP / 32;
+    const int lane = threadIdx.x & 31;
+    for (int b = blockIdx.x * NW + (threadIdx.x >> 5); b < I.K.n; b += BLAT_PREP_CTAS * NW) {
+        const int64_t k = I.K.off[b] + lane;
+        double v = -CUDART_INF;
+        if (k < I.K.off[b + 1]) {
+            const int64_t j = I.K.mem[k];
+            v = a.s * psi[I.t0 + j];
+            if (I.L.runs > 0) {
+#pragma unroll
+                for (int d = 0; d < DIM; ++d)
+                    I.step[j * DIM + d] = exp2(a.s * (y[(I.t0 + j) * DIM + d] - a.o[d]) * I.L.step16[d]);
+            }
+        }
+        v = warp_max(v);
+        if (lane == 0) const_cast<double *>(I.K.top)[b] = v;
+    }
+}
+
+// Persistent lattice value sweep: units (problem, tile, target slice).
+template <int DIM>
+__global__ void __launch_bounds__(LAT_THREADS, 2)
+k_batch_lat_value(const BInst *__restrict__ inst, const int4 *__restrict__ units, int nunits,
+                  int *__restrict__ counter, const double *__restrict__ tpack)
+{
+    extern __shared__ __align__(16) unsigned char blat_smem[];
+    __shared__ int su;
+    for (;;) {
+        __syncthreads();
+        if (threadIdx.x == 0) su = atomicAdd(counter, 1);
+        __syncthreads();
+        const int u = su;
+        if (u >= nunits) break;
+        const int4 w = units[u];
+        const BInst &I = inst[w.x];
+        const int64_t t0 = w.z * I.tslice;
+        lat_value_block<DIM>(blat_smem, I.L, I.a, tpack + I.t0 * TPACK, I.shift, I.step, w.y, t0,
+                             min(I.a.nt, t0 + I.tslice), I.ms + ((int64_t)w.z * I.L.ntiles + w.y) * LAT_TILE);
+    }
+}
+
+// Lattice merge: CTA <-> (problem, box of a tile).
+template <int DIM>
+__global__ void __launch_bounds__(LAT_THREADS)
+k_batch_lat_merge(const BInst *__restrict__ inst, const int2 *__restrict__ units, const double *__restrict__ tpack,
+                  const double *__restrict__ rho, const double *__restrict__ jxw, double *__restrict__ Lq,
+                  double *__restrict__ part)
+{
+    constexpr int PER = LAT_TILE / LAT_THREADS;
+    const int2 w = units[blockIdx.x];
+    const BInst &I = inst[w.x];
+    lat_merge_block<DIM>(I.L, I.a, I.K, w.y / PER, w.y % PER, I.nvs, I.lat_grad(), I.ms, I.shift,
+                         tpack + I.t0 * TPACK, rho + I.q0, jxw + I.q0, Lq + I.q0, part + (I.part0 + w.y) * 4);
+}
+
+// Persistent FP64 lattice gradient sweep: units (problem, target block, tile group).
+template <int DIM>
+__global__ void __launch_bounds__(LAT_THREADS, 2)
+k_batch_lat_grad(const BInst *__restrict__ inst, const int4 *__restrict__ units, int nunits,
+                 int *__restrict__ counter, const double *__restrict__ tpack, double *__restrict__ gpart)
+{
+    extern __shared__ __align__(16) unsigned char blat_smem[];
+    __shared__ int su;
+    for (;;) {
+        __syncthreads();
+        if (threadIdx.x == 0) su = atomicAdd(counter, 1);
+        __syncthreads();
+        const int u = su;
+        if (u >= nunits) break;
+        const int4 w = units[u];
+        const BInst &I = inst[w.x];
+        lat_grad_block<DIM>(blat_smem, I.L, I.a, tpack + I.t0 * TPACK, I.shift, I.step, I.ms, w.y * (int64_t)LAT_GT,
+                            w.z * I.gts, min(I.L.ntiles, (w.z + 1) * I.gts), gpart + I.gp0 + w.z * I.a.nt);
+    }
+}
+
+// g = sum of slices - nu and the norms the control and the line search read,
+// in two steps: CTA <-> (problem, BFIN_THREADS targets), thread <-> target,
+// the CTA's sums to red; then CTA <-> problem over them and the value
+// partials.  (One CTA per problem for all its targets took 0.48 ms of a
+// 7.9 ms batch of 16 problems: its slice loads are a serial chain.)
+constexpr int BRED = 8;
+__global__ void __launch_bounds__(BFIN_THREADS)
+k_batch_final_grad(const BInst *__restrict__ inst, const int2 *__restrict__ units, const double *__restrict__ gpart,
+                   const double *__restrict__ nu, const double *__restrict__ psi, const double *__restrict__ pdir,
+                   double *__restrict__ grad, double *__restrict__ red)
+{
+    const int2 w = units[blockIdx.x];
+    const BInst &I = inst[w.x];
+    const int64_t nt = I.a.nt, j = w.y * (int64_t)BFIN_THREADS + threadIdx.x;
     double psinu = 0.0, l1 = 0.0, linf = 0.0, comp = -CUDART_INF, l2 = 0.0, gp = 0.0, bad = 0.0;
-    for (int64_t j = threadIdx.x; j < nt; j += BFIN_THREADS) {
+    if (j < nt) {
+        const double *p = gpart + I.gp0 + j;
+        const int nk = I.grad_parts();
         double s = 0.0;
-        for (int k = 0; k < I.nks; ++k) s += gpart[I.gp0 + (int64_t)k * nt + j];
+        int k = 0;
+        for (; k + 8 <= nk; k += 8) {
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = p[(int64_t)(k + u) * nt];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) s += v[u];
+        }
+        for (; k < nk; ++k) s += p[(int64_t)k * nt];
         const int64_t gj = I.t0 + j;
         const double g = s - nu[gj];
         grad[gj] = g;
-        psinu += psi[gj] * nu[gj];
+        psinu = psi[gj] * nu[gj];
         const double ag = fabs(g);
-        l1 += ag;
+        l1 = ag;
         linf = fmax(linf, ag);
         comp = fmax(comp, ag - nu[gj] * I.tol);
-        l2 += g * g;
-        gp += g * pdir[gj];
+        l2 = g * g;
+        gp = g * pdir[gj];
         if (!isfinite(g) || !isfinite(psi[gj])) bad = 1.0;
     }
+    __shared__ double sh[7][BFIN_THREADS / 32];
+    psinu = warp_sum(psinu);
+    l1 = warp_sum(l1);
+    linf = warp_max(linf);
+    comp = warp_max(comp);
+    l2 = warp_sum(l2);
+    gp = warp_sum(gp);
+    bad = warp_max(bad);
+    const int wi = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) {
+        sh[0][wi] = psinu; sh[1][wi] = l1; sh[2][wi] = linf; sh[3][wi] = comp; sh[4][wi] = l2;
+        sh[5][wi] = gp; sh[6][wi] = bad;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double r[7] = {0, 0, 0, -CUDART_INF, 0, 0, 0};
+        for (int i = 0; i < BFIN_THREADS / 32; ++i) {
+            r[0] += sh[0][i]; r[1] += sh[1][i]; r[2] = fmax(r[2], sh[2][i]); r[3] = fmax(r[3], sh[3][i]);
+            r[4] += sh[4][i]; r[5] += sh[5][i]; r[6] = fmax(r[6], sh[6][i]);
+        }
+        double *o = red + (I.t0 / BFIN_THREADS + w.x + w.y) * BRED;
+        for (int k = 0; k < 7; ++k) o[k] = r[k];
+    }
+}
+
+__global__ void __launch_bounds__(BFIN_THREADS)
+k_batch_final(const BInst *__restrict__ inst, const int *__restrict__ act, const double *__restrict__ red,
+              const double *__restrict__ part, double *__restrict__ scal)
+{
+    const int pi = act[blockIdx.x];
+    const BInst &I = inst[pi];
+    const int nred = (int)((I.a.nt + BFIN_THREADS - 1) / BFIN_THREADS);
+    const double *rp = red + (I.t0 / BFIN_THREADS + pi) * BRED;
+    double psinu = 0.0, l1 = 0.0, linf = 0.0, comp = -CUDART_INF, l2 = 0.0, gp = 0.0, bad = 0.0;
+    for (int b = threadIdx.x; b < nred; b += BFIN_THREADS) {
+        const double *o = rp + b * BRED;
+        psinu += o[0];
+        l1 += o[1];
+        linf = fmax(linf, o[2]);
+        comp = fmax(comp, o[3]);
+        l2 += o[4];
+        gp += o[5];
+        bad = fmax(bad, o[6]);
+    }
     double v = 0.0, c = 0.0, sk = 0.0;
-    for (int64_t b = threadIdx.x; b < I.nvb; b += BFIN_THREADS) {
+    const int nv = I.value_parts();
+#pragma unroll 4
+    for (int64_t b = threadIdx.x; b < nv; b += BFIN_THREADS) {
         v += part[(I.part0 + b) * 4 + 0];
         c += part[(I.part0 + b) * 4 + 1];
         sk += part[(I.part0 + b) * 4 + 2];
@@ -200,7 +371,7 @@ k_batch_final(const BInst *__restrict__ inst, const int *__restrict__ act, const
         o[SC_L2SQ] = r[4];
         o[SC_DOT_GP] = r[5];
         o[SC_NONFINITE] = (r[6] != 0.0 || !isfinite(o[SC_VALUE])) ? 1.0 : 0.0;
-        o[SC_PAIRS] = (double)I.a.nq * (double)nt;
+        o[SC_PAIRS] = (double)I.a.nq * (double)I.a.nt;
     }
 }
 
@@ -453,14 +624,24 @@ struct sdot_batch {
     std::vector<double> hx, hrho, hjxw, hy, hnu;  // staged on the host until the first solve
     bool uploaded = false;
     std::vector<BInst> inst;
+    std::vector<Lattice> lat;          // per problem: the points' lattice (coordinates and counts; host)
+    std::vector<double> reach;         // per problem and dimension: the targets' distance from the origin
+    int64_t lat_tslice = 0;            // targets per unit of the lattice value sweep
     int64_t total_q = 0, total_t = 0, total_part = 0, total_gp = 0;
 
     DevBuf<double> x, rho, jxw, w, y, nu, psi, grad, tpack, Lq, part, gpart, x0, g0, pdir, S, Y, rho_h, scal, alpha,
         outv;
     DevBuf<BInst> dinst;
     DevBuf<int> act, counter, spare;
-    DevBuf<int2> vunits;
-    DevBuf<int4> gunits;
+    DevBuf<int2> vunits, munits, funits;
+    DevBuf<int4> gunits, lvunits, lgunits;
+    DevBuf<double> lat_x, lat_sph, lat_top, lat_step, lat_ms, red;
+    DevBuf<int> lat_q, lat_mem;
+    DevBuf<int64_t> lat_off;
+    // unit counts of the lists on the device, and what they were made for
+    int nv = 0, ng = 0, nlv = 0, nlg = 0, nm = 0, nf = 0, lat_tiles = 0;
+    bool units_ok = false;
+    std::vector<int> units_act;
     DevBuf<BHist> dhist;
     std::vector<double> scal_host;
 
@@ -504,6 +685,28 @@ struct DevGuard {
     }
 };
 
+// The most tiles (over the tile sizes), and the most tile groups of the
+// gradient sweep, that problem i may use.
+struct LatMost {
+    int64_t tiles = 0;
+    int groups = 0;
+};
+LatMost lat_most(const sdot_batch *b, int i)
+{
+    LatMost m;
+    const Lattice &G = b->lat[i];
+    if (!G.ok) return m;
+    for (int k = 0; k < (b->dim == 2 ? 2 : 1); ++k) {
+        const int cap = b->dim == 2 ? LAT_CAPS2[k] : LAT_CAPS3[k];
+        int64_t t = 1;
+        for (int d = 0; d < b->dim; ++d) t *= (G.n[d] + cap - 1) / cap;
+        m.tiles = std::max(m.tiles, t);
+    }
+    const int gts = b->inst[i].gts;
+    m.groups = (int)((m.tiles + gts - 1) / gts);
+    return m;
+}
+
 // Gradient slices of every problem for the slice target b->shape[2] (at 8:
 // the single-problem dense path's count): target blocks of DENSE_B_THREADS *
 // TT, slices of at least 256 points, at most 64.  Sets nks, ntb, qslice and
@@ -523,10 +726,28 @@ int64_t plan_slices(sdot_batch *b)
         I.ntb = (int)tb;
         I.qslice = (P.nq + nks - 1) / nks;
         I.gp0 = gp0;
-        gp0 += (int64_t)nks * P.nt;
+        gp0 += (int64_t)std::max(nks, lat_most(b, (int)i).groups) * P.nt;
     }
     b->total_gp = gp0;
+    b->units_ok = false;
     return gp0;
+}
+
+// Lattice tiling of problem i at its current eps (BInst::a.s).
+void plan_lattice(sdot_batch *b, int i)
+{
+    BInst &I = b->inst[i];
+    const Lattice &G = b->lat[i];
+    I.lat = 0;
+    b->units_ok = false;
+    if (!G.ok) return;
+    const LatTiling t = lat_tiling(G.n, G.xo, G.X.data(), b->dim, I.a.s, &b->reach[3 * i], LAT_BITS);
+    if (t.cap == 0) return;
+    for (int d = 0; d < 3; ++d) I.L.nt[d] = t.nt[d];
+    I.L.cap = t.cap;
+    I.L.ntiles = t.ntiles;
+    I.ngs = (t.ntiles + I.gts - 1) / I.gts;
+    I.lat = 1;
 }
 
 // Layout of every problem in the packed arrays and its launch shapes (the
@@ -571,8 +792,133 @@ sdot_status upload(sdot_batch *b)
     }
     b->total_q = q0;
     b->total_t = t0;
+    // lattices: found per problem (threads over the problems), with k-d blocks of their targets
+    struct Blocks {
+        std::vector<int64_t> off;
+        std::vector<int> mem;
+        std::vector<double> sph;
+    };
+    std::vector<Blocks> blk(np);
+    b->lat.assign(np, Lattice());
+    b->reach.assign(3 * np, 0.0);
+    {
+        std::atomic<size_t> next{0};
+        auto one = [&](size_t i) {
+            const auto &P = b->probs[i];
+            find_lattice(b->hx.data() + b->inst[i].q0 * D, P.nq, D, b->lat[i]);
+            if (!b->lat[i].ok) return;
+            const double *y = b->hy.data() + b->inst[i].t0 * D;
+            const std::vector<double> pts(y, y + P.nt * D);
+            const std::vector<int64_t> ord = kd_order(pts, D, P.nt, TBLK_KD, blk[i].off);
+            blk[i].mem.assign(ord.begin(), ord.end());
+            for (size_t k = 0; k + 1 < blk[i].off.size(); ++k) {
+                const std::vector<int64_t> idx(ord.begin() + blk[i].off[k], ord.begin() + blk[i].off[k + 1]);
+                double sp[4];
+                sphere_of(pts.data(), idx, D, sp);
+                blk[i].sph.insert(blk[i].sph.end(), sp, sp + 4);
+            }
+            for (int64_t j = 0; j < P.nt; ++j)
+                for (int d = 0; d < D; ++d)
+                    b->reach[3 * i + d] = std::max(b->reach[3 * i + d], std::fabs(y[j * D + d] - P.origin[d]));
+        };
+        auto work = [&]() {
+            for (size_t i; (i = next.fetch_add(1)) < np;) {
+                try {
+                    one(i);
+                } catch (...) {  // out of host memory: this problem runs the point sweeps
+                    b->lat[i].ok = false;
+                }
+            }
+        };
+        std::vector<std::thread> pool;
+        const size_t nth = std::min<size_t>(np, std::max(1u, std::min(16u, std::thread::hardware_concurrency())));
+        try {
+            for (size_t k = 1; k < nth; ++k) pool.emplace_back(work);
+        } catch (...) {  // fewer threads
+        }
+        work();
+        for (auto &t : pool) t.join();
+    }
+    // units of the lattice sweeps: about eight per resident CTA over the whole batch, of 4,096 points x tslice
+    // targets (value) and 64 targets x tslice / 64 tiles (gradient)
+    double lpairs = 0.0;
+    for (size_t i = 0; i < np; ++i)
+        if (b->lat[i].ok) lpairs += (double)b->probs[i].nq * (double)b->probs[i].nt;
+    b->lat_tslice = std::min<int64_t>(
+        4096, std::max<int64_t>(128, (int64_t)(lpairs / ((double)LAT_TILE * b->sms * 2 * 8)) / 64 * 64));
+    std::vector<double> lx, lsph;
+    std::vector<int> lq, lmem;
+    std::vector<int64_t> loff;
+    int64_t ms = 0, sh = 0, sp = 0;
+    std::vector<int64_t> ms0(np), sh0(np), sp0(np), x0(np), lq0(np), mem0(np), off0(np), sph0(np);
+    part0 = 0;
+    for (size_t i = 0; i < np; ++i) {
+        BInst &I = b->inst[i];
+        const auto &P = b->probs[i];
+        const Lattice &G = b->lat[i];
+        I.tslice = b->lat_tslice;
+        I.nvs = (int)((P.nt + I.tslice - 1) / I.tslice);
+        I.gts = (int)std::max<int64_t>(1, b->lat_tslice / LAT_GT);
+        const LatMost m = lat_most(b, (int)i);
+        I.part0 = part0;
+        part0 += std::max<int64_t>(I.nvb, m.tiles * (LAT_TILE / LAT_THREADS));
+        if (!G.ok) continue;
+        ms0[i] = ms;
+        ms += m.tiles * I.nvs * LAT_TILE;
+        sh0[i] = sh;
+        sh += 2 * m.tiles;
+        sp0[i] = sp;
+        sp += P.nt * D;
+        x0[i] = (int64_t)lx.size();
+        lx.insert(lx.end(), G.X.begin(), G.X.end());
+        lq0[i] = (int64_t)lq.size();
+        lq.insert(lq.end(), G.q.begin(), G.q.end());
+        mem0[i] = (int64_t)lmem.size();
+        lmem.insert(lmem.end(), blk[i].mem.begin(), blk[i].mem.end());
+        off0[i] = (int64_t)loff.size();
+        loff.insert(loff.end(), blk[i].off.begin(), blk[i].off.end());
+        sph0[i] = (int64_t)lsph.size();
+        lsph.insert(lsph.end(), blk[i].sph.begin(), blk[i].sph.end());
+    }
     b->total_part = part0;
     const int64_t gp0 = plan_slices(b);
+    if (!lq.empty()) {
+        BCK(b->lat_x.alloc(lx.size()), "batch lattice");
+        BCK(b->lat_q.alloc(lq.size()), "batch lattice");
+        BCK(b->lat_mem.alloc(lmem.size()), "batch lattice");
+        BCK(b->lat_off.alloc(loff.size()), "batch lattice");
+        BCK(b->lat_sph.alloc(lsph.size()), "batch lattice");
+        BCK(b->lat_top.alloc(lsph.size() / 4), "batch lattice");
+        BCK(b->lat_step.alloc(sp), "batch lattice");
+        BCK(b->lat_ms.alloc(ms + sh), "batch lattice");
+        BCK(cudaMemcpy(b->lat_x.p, lx.data(), lx.size() * 8, cudaMemcpyHostToDevice), "batch lattice");
+        BCK(cudaMemcpy(b->lat_q.p, lq.data(), lq.size() * sizeof(int), cudaMemcpyHostToDevice), "batch lattice");
+        BCK(cudaMemcpy(b->lat_mem.p, lmem.data(), lmem.size() * sizeof(int), cudaMemcpyHostToDevice), "batch lattice");
+        BCK(cudaMemcpy(b->lat_off.p, loff.data(), loff.size() * 8, cudaMemcpyHostToDevice), "batch lattice");
+        BCK(cudaMemcpy(b->lat_sph.p, lsph.data(), lsph.size() * 8, cudaMemcpyHostToDevice), "batch lattice");
+        for (size_t i = 0; i < np; ++i) {
+            BInst &I = b->inst[i];
+            Lattice &G = b->lat[i];
+            if (!G.ok) continue;
+            I.L.X = b->lat_x.p + x0[i];
+            I.L.q = b->lat_q.p + lq0[i];
+            for (int d = 0; d < 3; ++d) {
+                I.L.n[d] = G.n[d];
+                I.L.xo[d] = G.xo[d];
+            }
+            lat_runs(G.period, G.step, D, I.L);
+            I.K.off = b->lat_off.p + off0[i];
+            I.K.mem = b->lat_mem.p + mem0[i];
+            I.K.sph = b->lat_sph.p + sph0[i];
+            I.K.top = b->lat_top.p + sph0[i] / 4;
+            I.K.n = (int)blk[i].off.size() - 1;
+            I.ms = b->lat_ms.p + ms0[i];
+            I.shift = b->lat_ms.p + ms + sh0[i];
+            I.step = b->lat_step.p + sp0[i];
+            std::vector<int>().swap(G.q);  // on the device from here on
+            plan_lattice(b, (int)i);
+        }
+    }
     BCK(b->x.alloc(q0 * D), "batch alloc");
     BCK(b->rho.alloc(q0), "batch alloc");
     BCK(b->jxw.alloc(q0), "batch alloc");
@@ -598,7 +944,8 @@ sdot_status upload(sdot_batch *b)
     BCK(b->act.alloc(np), "batch alloc");
     BCK(b->spare.alloc(np), "batch alloc");
     BCK(b->dhist.alloc(np), "batch alloc");
-    BCK(b->counter.alloc(2), "batch alloc");
+    BCK(b->counter.alloc(4), "batch alloc");
+    BCK(b->red.alloc((size_t)(t0 / BFIN_THREADS + 2 * np + 1) * BRED), "batch alloc");
     std::vector<double> w(q0);
     for (int64_t q = 0; q < q0; ++q) w[q] = b->hrho[q] * b->hjxw[q];
     BCK(cudaMemcpy(b->x.p, b->hx.data(), q0 * D * 8, cudaMemcpyHostToDevice), "batch upload");
@@ -613,6 +960,38 @@ sdot_status upload(sdot_batch *b)
     return SDOT_OK;
 }
 
+// Packing, value and gradient sweeps of the listed units.
+template <int DIM>
+void batch_sweeps(sdot_batch *b, int nact, int64_t maxnt)
+{
+    cudaStream_t st = b->stream;
+    const dim3 pg((unsigned)std::min<int64_t>((maxnt + 255) / 256, 64), (unsigned)nact);
+    const int lgrid = b->sms * 2;
+    k_batch_prep<DIM><<<pg, 256, 0, st>>>(b->dinst.p, b->act.p, b->y.p, b->nu.p, b->psi.p, b->tpack.p);
+    if (b->nlv > 0) {
+        const size_t vs = sizeof(LatValueSmem<DIM>);
+        cudaFuncSetAttribute(k_batch_lat_value<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vs);
+        k_batch_lat_prep<DIM><<<dim3((unsigned)(BLAT_PREP_CTAS + b->lat_tiles), (unsigned)nact), BLAT_PREP, 0, st>>>(
+            b->dinst.p, b->act.p, b->y.p, b->psi.p);
+        k_batch_lat_value<DIM><<<std::min(b->nlv, lgrid), LAT_THREADS, vs, st>>>(b->dinst.p, b->lvunits.p, b->nlv,
+                                                                                 b->counter.p + 2, b->tpack.p);
+        k_batch_lat_merge<DIM><<<(unsigned)b->nm, LAT_THREADS, 0, st>>>(b->dinst.p, b->munits.p, b->tpack.p, b->rho.p,
+                                                                        b->jxw.p, b->Lq.p, b->part.p);
+    }
+    if (b->nv > 0)
+        k_batch_value<DIM><<<std::min(b->nv, b->sms * b->shape[0]), DENSE_A_THREADS, 0, st>>>(
+            b->dinst.p, b->vunits.p, b->nv, b->counter.p, b->x.p, b->rho.p, b->jxw.p, b->tpack.p, b->Lq.p, b->part.p);
+    if (b->nlg > 0) {
+        const size_t gs = sizeof(LatGradSmem<DIM>);
+        cudaFuncSetAttribute(k_batch_lat_grad<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gs);
+        k_batch_lat_grad<DIM><<<std::min(b->nlg, lgrid), LAT_THREADS, gs, st>>>(b->dinst.p, b->lgunits.p, b->nlg,
+                                                                                b->counter.p + 3, b->tpack.p, b->gpart.p);
+    }
+    if (b->ng > 0)
+        k_batch_grad<DIM><<<std::min(b->ng, b->sms * b->shape[1]), DENSE_B_THREADS, 0, st>>>(
+            b->dinst.p, b->gunits.p, b->ng, b->counter.p + 1, b->x.p, b->w.p, b->Lq.p, b->tpack.p, b->psi.p, b->gpart.p);
+}
+
 // One batched evaluation of the listed problems at b->psi (inst[].fp32 and
 // inst[].a.eps as set on the device); fills scal_host for them.
 sdot_status batch_eval(sdot_batch *b, const std::vector<int> &act, double *ms)
@@ -621,44 +1000,67 @@ sdot_status batch_eval(sdot_batch *b, const std::vector<int> &act, double *ms)
     const int D = b->dim;
     cudaStream_t st = b->stream;
     BCK(cudaMemcpyAsync(b->act.p, act.data(), act.size() * sizeof(int), cudaMemcpyHostToDevice, st), "batch act");
-    // work units, largest first
-    std::vector<int2> vu;
-    std::vector<int4> gu;
-    std::vector<std::pair<double, int>> order;
-    for (int p : act) order.push_back({-(double)b->probs[p].nq * (double)b->probs[p].nt, p});
-    std::sort(order.begin(), order.end());
-    for (auto &o : order) {
-        const BInst &I = b->inst[o.second];
-        for (int k = 0; k < I.nvb; ++k) vu.push_back(make_int2(o.second, k));
-        for (int k = 0; k < I.nks; ++k)
-            for (int t = 0; t < I.ntb; ++t) gu.push_back(make_int4(o.second, t, k, 0));
-    }
-    BCK(b->vunits.alloc(vu.size()), "batch units");
-    BCK(b->gunits.alloc(gu.size()), "batch units");
-    BCK(cudaMemcpyAsync(b->vunits.p, vu.data(), vu.size() * sizeof(int2), cudaMemcpyHostToDevice, st), "batch units");
-    BCK(cudaMemcpyAsync(b->gunits.p, gu.data(), gu.size() * sizeof(int4), cudaMemcpyHostToDevice, st), "batch units");
-    BCK(cudaMemsetAsync(b->counter.p, 0, 2 * sizeof(int), st), "batch counter");
+    // work units, largest first (kept on the device while the listed problems and their plans stay the same)
     int64_t maxnt = 0;
     for (int p : act) maxnt = std::max(maxnt, b->probs[p].nt);
-    cudaEventRecord(b->ev0, st);
-    dim3 pg((unsigned)std::min<int64_t>((maxnt + 255) / 256, 64), (unsigned)act.size());
-    const int vgrid = std::min<int>((int)vu.size(), b->sms * b->shape[0]);
-    const int ggrid = std::min<int>((int)gu.size(), b->sms * b->shape[1]);
-    if (D == 2) {
-        k_batch_prep<2><<<pg, 256, 0, st>>>(b->dinst.p, b->act.p, b->y.p, b->nu.p, b->psi.p, b->tpack.p);
-        k_batch_value<2><<<vgrid, DENSE_A_THREADS, 0, st>>>(b->dinst.p, b->vunits.p, (int)vu.size(), b->counter.p,
-                                                            b->x.p, b->rho.p, b->jxw.p, b->tpack.p, b->Lq.p, b->part.p);
-        k_batch_grad<2><<<ggrid, DENSE_B_THREADS, 0, st>>>(b->dinst.p, b->gunits.p, (int)gu.size(), b->counter.p + 1,
-                                                           b->x.p, b->w.p, b->Lq.p, b->tpack.p, b->psi.p, b->gpart.p);
-    } else {
-        k_batch_prep<3><<<pg, 256, 0, st>>>(b->dinst.p, b->act.p, b->y.p, b->nu.p, b->psi.p, b->tpack.p);
-        k_batch_value<3><<<vgrid, DENSE_A_THREADS, 0, st>>>(b->dinst.p, b->vunits.p, (int)vu.size(), b->counter.p,
-                                                            b->x.p, b->rho.p, b->jxw.p, b->tpack.p, b->Lq.p, b->part.p);
-        k_batch_grad<3><<<ggrid, DENSE_B_THREADS, 0, st>>>(b->dinst.p, b->gunits.p, (int)gu.size(), b->counter.p + 1,
-                                                           b->x.p, b->w.p, b->Lq.p, b->tpack.p, b->psi.p, b->gpart.p);
+    if (!b->units_ok || b->units_act != act) {
+        std::vector<int2> vu, mu, fu;
+        std::vector<int4> gu, lv, lg;
+        std::vector<std::pair<double, int>> order;
+        for (int p : act) order.push_back({-(double)b->probs[p].nq * (double)b->probs[p].nt, p});
+        std::sort(order.begin(), order.end());
+        int tiles = 0;
+        for (auto &o : order) {
+            const int p = o.second;
+            const BInst &I = b->inst[p];
+            if (I.lat) {
+                tiles = std::max(tiles, I.L.ntiles);
+                for (int k = 0; k < I.nvs; ++k)
+                    for (int t = 0; t < I.L.ntiles; ++t) lv.push_back(make_int4(p, t, k, 0));
+                for (int k = 0; k < I.value_parts(); ++k) mu.push_back(make_int2(p, k));
+            } else {
+                for (int k = 0; k < I.nvb; ++k) vu.push_back(make_int2(p, k));
+            }
+            if (I.lat_grad()) {
+                const int nb = (int)((I.a.nt + LAT_GT - 1) / LAT_GT);
+                for (int k = 0; k < I.ngs; ++k)
+                    for (int t = 0; t < nb; ++t) lg.push_back(make_int4(p, t, k, 0));
+            } else {
+                for (int k = 0; k < I.nks; ++k)
+                    for (int t = 0; t < I.ntb; ++t) gu.push_back(make_int4(p, t, k, 0));
+            }
+            for (int k = 0; k * (int64_t)BFIN_THREADS < I.a.nt; ++k) fu.push_back(make_int2(p, k));
+        }
+        b->units_ok = false;
+        auto put = [&](auto &buf, const auto &v) {
+            cudaError_t e = buf.alloc(std::max<size_t>(v.size(), 1));
+            if (e == cudaSuccess && !v.empty())
+                e = cudaMemcpyAsync(buf.p, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, st);
+            return e;
+        };
+        BCK(put(b->vunits, vu), "batch units");
+        BCK(put(b->gunits, gu), "batch units");
+        BCK(put(b->lvunits, lv), "batch units");
+        BCK(put(b->lgunits, lg), "batch units");
+        BCK(put(b->munits, mu), "batch units");
+        BCK(put(b->funits, fu), "batch units");
+        b->nv = (int)vu.size();
+        b->ng = (int)gu.size();
+        b->nlv = (int)lv.size();
+        b->nlg = (int)lg.size();
+        b->nm = (int)mu.size();
+        b->nf = (int)fu.size();
+        b->lat_tiles = tiles;
+        b->units_act = act;
+        b->units_ok = true;
     }
-    k_batch_final<<<(unsigned)act.size(), BFIN_THREADS, 0, st>>>(b->dinst.p, b->act.p, b->gpart.p, b->part.p,
-                                                                  b->nu.p, b->psi.p, b->pdir.p, b->grad.p, b->scal.p);
+    BCK(cudaMemsetAsync(b->counter.p, 0, 4 * sizeof(int), st), "batch counter");
+    cudaEventRecord(b->ev0, st);
+    if (D == 2) batch_sweeps<2>(b, (int)act.size(), maxnt);
+    else batch_sweeps<3>(b, (int)act.size(), maxnt);
+    k_batch_final_grad<<<(unsigned)b->nf, BFIN_THREADS, 0, st>>>(b->dinst.p, b->funits.p, b->gpart.p, b->nu.p, b->psi.p,
+                                                                 b->pdir.p, b->grad.p, b->red.p);
+    k_batch_final<<<(unsigned)act.size(), BFIN_THREADS, 0, st>>>(b->dinst.p, b->act.p, b->red.p, b->part.p, b->scal.p);
     cudaEventRecord(b->ev1, st);
     BCK(cudaGetLastError(), "batch evaluate");
     BCK(cudaMemcpyAsync(b->scal_host.data(), b->scal.p, b->scal_host.size() * 8, cudaMemcpyDeviceToHost, st),
@@ -799,6 +1201,7 @@ sdot_status sdot_batch_evaluate(sdot_batch *b, const double *psi, double *grad, 
         if (s != SDOT_OK) return s;
     }
     for (auto &I : b->inst) {
+        if (I.fp32 != (fp32 ? 1 : 0)) b->units_ok = false;
         I.fp32 = fp32 ? 1 : 0;
     }
     BCK(cudaMemcpyAsync(b->dinst.p, b->inst.data(), b->inst.size() * sizeof(BInst), cudaMemcpyHostToDevice, b->stream),
@@ -870,6 +1273,7 @@ sdot_status sdot_batch_solve(sdot_batch *b, double *psi_io, const sdot_batch_opt
         I.a.c32 = LOG2E / (2.0 * eps);
         I.a.l2e_eps = LOG2E / eps;
         I.fp32 = S[p].fp32;
+        plan_lattice(b, p);
     };
     auto reset_lbfgs = [&](int p) {
         St &s = S[p];
@@ -1165,6 +1569,7 @@ sdot_status sdot_batch_autotune(sdot_batch *b, const double *psi, int fp32, int 
         }
     }
     for (auto &I : b->inst) I.fp32 = fp32 ? 1 : 0;
+    b->units_ok = false;
     BCK(cudaMemcpyAsync(b->dinst.p, b->inst.data(), b->inst.size() * sizeof(BInst), cudaMemcpyHostToDevice, b->stream),
         "batch inst");
     BCK(cudaMemcpyAsync(b->psi.p, psi, b->total_t * 8, cudaMemcpyHostToDevice, b->stream), "batch psi");

@@ -182,14 +182,14 @@ k_lat_value(LatArgs L, EvalArgs a, const double *__restrict__ tpack, const doubl
                          ms + ((int64_t)blockIdx.y * L.ntiles + blockIdx.x) * LAT_TILE);
 }
 
-template <int DIM, bool WT>
+template <int DIM>
 __global__ void __launch_bounds__(LAT_THREADS)
-k_lat_merge(LatArgs L, EvalArgs a, LatBlocks K, int nslice, double *__restrict__ ms, const double *__restrict__ shift,
+k_lat_merge(LatArgs L, EvalArgs a, LatBlocks K, int nslice, bool wt, double *__restrict__ ms, const double *__restrict__ shift,
             const double *__restrict__ tpack, const double *__restrict__ rho, const double *__restrict__ jxw, double *__restrict__ Lq,
             double *__restrict__ part)
 {
     constexpr int PER = LAT_TILE / LAT_THREADS;
-    lat_merge_block<DIM, WT>(L, a, K, blockIdx.x / PER, blockIdx.x % PER, nslice, ms, shift, tpack, rho, jxw, Lq,
+    lat_merge_block<DIM>(L, a, K, blockIdx.x / PER, blockIdx.x % PER, nslice, wt, ms, shift, tpack, rho, jxw, Lq,
                              part + (int64_t)blockIdx.x * 4);
 }
 
@@ -1112,17 +1112,13 @@ static void launch_lat_value(const sdot_ctx *c, const DenseShape &ds, const doub
 {
     const LatArgs L = lat_args(c, ds.lat);
     const LatScratch S(ds, vpart, a.nt, DIM);
-    const LatBlocks K{c->tblk_off.p, c->tblk_sph.p, S.top, (int)c->ntblk};
+    const LatBlocks K{c->tblk_off.p, nullptr, c->tblk_sph.p, S.top, (int)c->ntblk};
     const size_t smem = sizeof(LatValueSmem<DIM>);
     lat_smem_limit(k_lat_value<DIM>, smem);
     k_lat_value<DIM><<<dim3((unsigned)L.ntiles, (unsigned)ds.nvs), LAT_THREADS, smem, st>>>(
         L, a, tpack, S.shift, S.step, ds.tslice, vpart);
-    auto merge = [&](auto kern) {
-        kern<<<(unsigned)ds.nval, LAT_THREADS, 0, st>>>(L, a, K, ds.nvs, vpart, S.shift, tpack, c->rho.p, c->jxw.p,
-                                                        Lq, blkpart);
-    };
-    if (ds.lat_grad) merge(k_lat_merge<DIM, true>);
-    else merge(k_lat_merge<DIM, false>);
+    k_lat_merge<DIM><<<(unsigned)ds.nval, LAT_THREADS, 0, st>>>(L, a, K, ds.nvs, ds.lat_grad, vpart, S.shift, tpack,
+                                                                c->rho.p, c->jxw.p, Lq, blkpart);
 }
 
 template <int DIM>

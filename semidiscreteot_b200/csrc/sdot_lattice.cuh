@@ -22,7 +22,7 @@
 // every slice of the targets, so the slices' sums add without rescaling.
 // The caller admits a tile size only when the factors of a tile span at most
 // 2^(+-LAT_BITS): every point's sum is then at least nu 2^-LAT_BITS relative
-// to M, the exponents that exp2_16 clamps are below 2^-1000 times a factor
+// to M, the exponents that exp2_16_full clamps are below 2^-1000 times a factor
 // <= 2^LAT_BITS, and nothing leaves the FP64 range.
 #pragma once
 
@@ -55,10 +55,12 @@ struct LatArgs {
     double step16[3];        // step / 16
 };
 
-// Blocks of at most 32 consecutive targets (k-d tree leaves): bounding
-// sphere (4 doubles) and largest s psi_j.
+// Blocks of at most 32 targets (k-d tree leaves): the targets mem[off[b]..]
+// (consecutive ones, off[b].., without mem), bounding sphere (4 doubles) and
+// largest s psi_j.
 struct LatBlocks {
     const int64_t *off;
+    const int *mem;
     const double *sph;
     const double *top;
     int n;
@@ -305,7 +307,7 @@ __device__ __forceinline__ void lat_value_block(unsigned char *smem, const LatAr
                 if (j < cn) {
                     const double *tp = sm.td[k % 3][j];
                     const double dlt = sm.delta[d * T + i0];
-                    double f = exp2_16(d == 0 ? fma(tp[1], dlt, tp[0]) : tp[1 + d] * dlt, sm.tab);
+                    double f = exp2_16_full(d == 0 ? fma(tp[1], dlt, tp[0]) : tp[1 + d] * dlt, sm.tab);
                     if (d == 0) f *= tp[1 + DIM];
                     lat_run(f, tp[2 + DIM + d], tp[2 + 2 * DIM + d], tp[2 + 3 * DIM + d], o);
                 }
@@ -320,11 +322,11 @@ __device__ __forceinline__ void lat_value_block(unsigned char *smem, const LatAr
 #pragma unroll 4
                 for (; j < cn; j += GS) {
                     const double *tp = sm.td[k % 3][j];
-                    F[j * FS] = tp[1 + DIM] * exp2_16(fma(tp[1], gdelta, tp[0]), sm.tab);
+                    F[j * FS] = tp[1 + DIM] * exp2_16_full(fma(tp[1], gdelta, tp[0]), sm.tab);
                 }
             } else {
 #pragma unroll 4
-                for (; j < cn; j += GS) F[j * FS] = exp2_16_nc(sm.td[k % 3][j][1 + gd] * gdelta, sm.tab);
+                for (; j < cn; j += GS) F[j * FS] = exp2_16_full(sm.td[k % 3][j][1 + gd] * gdelta, sm.tab);
             }
             for (; j < cz; j += GS) F[j * FS] = 0.0;
         }
@@ -413,12 +415,12 @@ __device__ __forceinline__ void lat_value_block(unsigned char *smem, const LatAr
 //    sums; a scan of all targets per box took 0.22 ms at 147,456 points x
 //    16,384 targets.
 //  * The slices' sums added in order of the slices, L_q and the box's
-//    (value, C, skipped, 0) partials.  With WT, the gradient sweep's weights
+//    (value, C, skipped, 0) partials.  With wt, the gradient sweep's weights
 //    w_q / S_q (relative to M; 0 for skipped points and past the tile's
 //    extent) replace slice 0's sums.
-template <int DIM, bool WT>
+template <int DIM>
 __device__ __forceinline__ void lat_merge_block(const LatArgs &L, const EvalArgs &a, const LatBlocks &K, int tile,
-                                                int sub, int nslice, double *__restrict__ ms,
+                                                int sub, int nslice, bool wt, double *__restrict__ ms,
                                                 const double *__restrict__ shift, const double *__restrict__ tpack,
                                                 const double *__restrict__ rho, const double *__restrict__ jxw,
                                                 double *__restrict__ Lq, double *__restrict__ out4)
@@ -640,7 +642,7 @@ __device__ __forceinline__ void lat_merge_block(const LatArgs &L, const EvalArgs
                     }
                 const int64_t j = K.off[bi] + lane;
                 double lb = -CUDART_INF, ub;
-                if (j < K.off[bi + 1]) lb = target_lb(tpack + j * TPACK, ub);
+                if (j < K.off[bi + 1]) lb = target_lb(tpack + (K.mem ? K.mem[j] : j) * TPACK, ub);
                 lb = warp_max(lb);
                 if (lane == 0) slb = lb - slack;
             }
@@ -657,7 +659,7 @@ __device__ __forceinline__ void lat_merge_block(const LatArgs &L, const EvalArgs
                         if (k < nb) {
                             const int64_t j = K.off[blist[k]] + lane;
                             if (j < K.off[blist[k] + 1]) {
-                                const double *tp = tpack + j * TPACK;
+                                const double *tp = tpack + (K.mem ? K.mem[j] : j) * TPACK;
                                 double ub;
                                 target_lb(tp, ub);
                                 if (ub + slack >= lb) push(tp);
@@ -685,7 +687,7 @@ __device__ __forceinline__ void lat_merge_block(const LatArgs &L, const EvalArgs
                 const double xt = L.X[L.xo[d] + B.s[d] + i[d]] - a.o[d];
                 xsq += xt * xt;
             }
-            const double Sref = mx == -CUDART_INF ? 0.0 : S * exp2_16(shift[2 * tile] - mx, tab);
+            const double Sref = mx == -CUDART_INF ? 0.0 : S * exp2_16_full(shift[2 * tile] - mx, tab);
             const double r = rho[q], jw = jxw[q];
             double Lv;
             int sk;
@@ -695,7 +697,7 @@ __device__ __forceinline__ void lat_merge_block(const LatArgs &L, const EvalArgs
             W = sk ? 0.0 : r * jw / S;
         }
     }
-    if (WT) *p = W;
+    if (wt) *p = W;
     block_partials_at(tv, tc, ts, 0.0, out4);
 }
 
@@ -769,7 +771,7 @@ __device__ __forceinline__ void lat_grad_block(unsigned char *smem, const LatArg
                     for (int v = 0; v < LAT_RUN; ++v) o[v] = 0.0;
                     if (i0 < B.e[d]) {
                         const double dlt = lat_delta<DIM>(L, a, B, d, i0);
-                        const double f = d == 0 ? exp2_16(fma(Bj[d], dlt, bb), sm.tab) : exp2_16_nc(Bj[d] * dlt, sm.tab);
+                        const double f = d == 0 ? exp2_16_full(fma(Bj[d], dlt, bb), sm.tab) : exp2_16_full(Bj[d] * dlt, sm.tab);
                         const double r2 = r1[d] * r1[d];
                         lat_run(f, r1[d], r2, r2 * r2, o);
                     }
@@ -789,7 +791,7 @@ __device__ __forceinline__ void lat_grad_block(unsigned char *smem, const LatArg
                 double f = 0.0;
                 if (i < B.e[d]) {
                     const double dlt = lat_delta<DIM>(L, a, B, d, i);
-                    f = d == 0 ? exp2_16(fma(Bd, dlt, bb), sm.tab) : exp2_16_nc(Bd * dlt, sm.tab);
+                    f = d == 0 ? exp2_16_full(fma(Bd, dlt, bb), sm.tab) : exp2_16_full(Bd * dlt, sm.tab);
                 }
                 sm.F[d * T + i][gj] = f;
             }

@@ -138,6 +138,8 @@ struct LatTiling {
     int cap = 0, nt[3] = {1, 1, 1}, ntiles = 0;
 };
 
+constexpr int LAT_CAPS2[2] = {64, 32}, LAT_CAPS3[1] = {16};   // tile sizes (2D, 3D), the largest first
+
 // Tile size for scaled exponents s = kappa / eps and targets within reach[d]
 // of the origin: the largest of 64 and 32 points per dimension (2D) or 16
 // (3D) whose factors span at most 2^(+-bits).  A tile's work goes by its
@@ -150,8 +152,7 @@ inline LatTiling lat_tiling(const int *n, const int *xo, const double *X, int di
                             double bits)
 {
     LatTiling best;
-    const int caps2[2] = {64, 32}, caps3[1] = {16};
-    const int *caps = dim == 2 ? caps2 : caps3;
+    const int *caps = dim == 2 ? LAT_CAPS2 : LAT_CAPS3;
     const int ncaps = dim == 2 ? 2 : 1;
     int64_t nq = 1;
     for (int d = 0; d < dim; ++d) nq *= n[d];
