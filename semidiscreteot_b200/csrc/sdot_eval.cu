@@ -1064,8 +1064,8 @@ size_t dense_gpart_need(const sdot_ctx *c)
 static LatArgs lat_args(const sdot_ctx *c, const LatTiling &t)
 {
     LatArgs L{};
-    L.X = c->lat_x.p;
-    L.q = c->lat_q.p;
+    L.X = c->lat_buf.p;
+    L.q = reinterpret_cast<const int *>(c->lat_buf.p + c->lat_X.size());
     for (int d = 0; d < 3; ++d) {
         L.n[d] = c->lat_n[d];
         L.nt[d] = t.nt[d];

@@ -178,8 +178,7 @@ struct sdot_ctx {
     int lat_period[3] = {0, 0, 0};     // period and step of its coordinates (sdot_lattice_host.h)
     double lat_step[3] = {0, 0, 0};
     std::vector<double> lat_X;         // its coordinates, dimension after dimension
-    sdot::DevBuf<double> lat_x;        // the same on the device
-    sdot::DevBuf<int> lat_q;           // lattice index -> point (internal order)
+    sdot::DevBuf<double> lat_buf;      // the same on the device, then (int) lattice index -> point (internal order)
     int64_t geometry_id = 0;           // counts the measures set: part of the evaluation graph's key
 
     // ---- truncated path: block-pair lists and gradient partials ----

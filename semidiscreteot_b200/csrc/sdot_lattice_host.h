@@ -32,40 +32,57 @@ constexpr int LAT_MAXP = 4;   // largest period looked for
 // as a dimension has more coordinates than MAXN.
 inline void find_lattice(const double *x, int64_t n, int dim, Lattice &L)
 {
-    constexpr int MAXN = 8192, CAP = 4 * MAXN;
+    constexpr int MAXN = 4096, BITS = 13, CAP = 1 << BITS;
     L = Lattice();
     if (n < 4 || n > INT32_MAX) return;
-    struct Slot {
-        uint64_t key;
-        int id;
+    struct Table {
+        uint64_t key[CAP];
+        short id[CAP];
     };
-    std::vector<Slot> table[3];
-    std::vector<double> val[3];
     auto bits = [](double v) {
         v = v == 0.0 ? 0.0 : v;
         uint64_t k;
         memcpy(&k, &v, 8);
         return k;
     };
-    auto at = [&](int d, uint64_t k) {
-        uint64_t h = (k * 0x9e3779b97f4a7c15ull) >> 49;  // 15 bits = CAP slots
-        while (table[d][h].id >= 0 && table[d][h].key != k) h = (h + 1) & (CAP - 1);
-        return (int)h;
-    };
-    for (int d = 0; d < dim; ++d) {
-        table[d].assign(CAP, Slot{0, -1});
-        uint64_t last = 0;
-        bool have = false;
-        for (int64_t i = 0; i < n; ++i) {
-            const uint64_t k = bits(x[i * dim + d]);
-            if (have && k == last) continue;
-            last = k;
-            have = true;
-            const int h = at(d, k);
-            if (table[d][h].id >= 0) continue;
-            if ((int)val[d].size() >= MAXN) return;
-            table[d][h] = Slot{k, (int)val[d].size()};
-            val[d].push_back(x[i * dim + d]);
+    // coordinate of every point per dimension, numbered in order of appearance (stripes of points that share
+    // the previous three points' coordinates, as within a cell, need no search)
+    std::vector<double> val[3];
+    std::vector<short> num((size_t)n * dim);
+    {
+        std::vector<Table> table(1);
+        Table &t = table[0];
+        for (int d = 0; d < dim; ++d) {
+            memset(t.id, 0xff, sizeof t.id);
+            uint64_t lk[4] = {0, 0, 0, 0};
+            short li[4] = {-1, -1, -1, -1};
+            int w = 0;
+            for (int64_t i = 0; i < n; ++i) {
+                const uint64_t k = bits(x[i * dim + d]);
+                short id = -1;
+                for (int m = 0; m < 4; ++m)
+                    if (li[m] >= 0 && lk[m] == k) id = li[m];
+                if (id < 0) {
+                    uint64_t h = (k * 0x9e3779b97f4a7c15ull) >> (64 - BITS);
+                    while (t.id[h] >= 0 && t.key[h] != k) h = (h + 1) & (CAP - 1);
+                    id = t.id[h];
+                    if (id < 0) {
+                        if ((int)val[d].size() >= MAXN) return;
+                        id = (short)val[d].size();
+                        t.key[h] = k;
+                        t.id[h] = id;
+                        val[d].push_back(x[i * dim + d]);
+                    }
+                    lk[w] = k;
+                    li[w] = id;
+                    w = (w + 1) & 3;
+                }
+                num[(size_t)i * dim + d] = id;
+            }
+            // no lattice of n points has this many coordinates in the dimensions seen so far
+            double most = 1.0;
+            for (int e = 0; e <= d; ++e) most *= (double)val[e].size() / 4.0;
+            if (most > (double)n) return;
         }
     }
     std::vector<int> rank[3];
@@ -92,20 +109,14 @@ inline void find_lattice(const double *x, int64_t n, int dim, Lattice &L)
         if (merge || total < n) return;
     }
     std::vector<int> q((size_t)n, -1);
-    int64_t stride[3] = {1, 1, 1};
-    for (int d = 1; d < dim; ++d) stride[d] = stride[d - 1] * (int64_t)coord[d - 1].size();
-    uint64_t last[3] = {0, 0, 0};
-    int lr[3] = {-1, -1, -1};
+    int64_t stride = 1;
+    for (int d = 0; d < dim; ++d) {  // ranks to lattice strides
+        for (int &r : rank[d]) r = (int)(r * stride);
+        stride *= (int64_t)coord[d].size();
+    }
     for (int64_t i = 0; i < n; ++i) {
         int64_t li = 0;
-        for (int d = 0; d < dim; ++d) {
-            const uint64_t k = bits(x[i * dim + d]);
-            if (lr[d] < 0 || k != last[d]) {
-                last[d] = k;
-                lr[d] = rank[d][table[d][at(d, k)].id];
-            }
-            li += stride[d] * lr[d];
-        }
+        for (int d = 0; d < dim; ++d) li += rank[d][num[(size_t)i * dim + d]];
         if (q[li] >= 0) return;  // two points at one place: no lattice
         q[li] = (int)i;
     }
