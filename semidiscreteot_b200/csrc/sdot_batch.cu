@@ -164,7 +164,8 @@ k_batch_lat_prep(const BInst *__restrict__ inst, const int *__restrict__ act, co
     const EvalArgs &a = I.a;
     if ((int)blockIdx.x >= BLAT_PREP_CTAS) {
         const int t = blockIdx.x - BLAT_PREP_CTAS;
-        if (t < I.L.ntiles) lat_shift_block<DIM, BLAT_PREP>(I.L, a, t, y + I.t0 * DIM, psi + I.t0, I.shift);
+        if (t < I.L.ntiles) lat_shift_block<DIM, BLAT_PREP>(
+                I.L, a, t, y + I.t0 * DIM, [&](int64_t j) { return psi[I.t0 + j]; }, I.shift);
         return;
     }
     constexpr int NW = BLAT_PREP / 32;

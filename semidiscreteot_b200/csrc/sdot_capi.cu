@@ -156,13 +156,21 @@ size_t device_bytes(const sdot_ctx *c)
 
 namespace sdot {
 
+sdot_status ensure_tickets(sdot_ctx *c)
+{
+    if (c->ticket.p) return SDOT_OK;
+    CK(c->ticket.alloc(3), "alloc counters");
+    CK(cudaMemsetAsync(c->ticket.p, 0, 3 * sizeof(unsigned), c->stream), "clear counters");
+    return SDOT_OK;
+}
+
 sdot_status ensure_eval_buffers(sdot_ctx *c)
 {
     const int64_t nt = c->nt, nq = c->nq;
     const int64_t dense_blocks = (nq + DENSE_A_THREADS * DENSE_A_QT - 1) / (DENSE_A_THREADS * DENSE_A_QT);
     const int64_t nval = std::max<int64_t>(dense_blocks, c->nsblk);
     const size_t need =
-        (size_t)(nt * (2 + TPACK + dense_grad_slices(INT64_MAX / 2, nt) + 2) + nq + 4 * nval + 148 * 8 + 64) *
+        (size_t)(nt * (2 + TPACK + dense_grad_slices(INT64_MAX / 2, nt) + 2) + nq + 4 * nval + 148 * 12 + 64) *
         sizeof(double);
     if (c->budget && device_bytes(c) + need > c->budget && c->tpack.n < (size_t)(nt * TPACK))
         return set_error(c, SDOT_EBUDGET, "evaluation buffers exceed the context memory budget");
@@ -172,8 +180,15 @@ sdot_status ensure_eval_buffers(sdot_ctx *c)
     CK(c->Lq.alloc(nq), "alloc Lq");
     CK(c->gpart.alloc(std::max<size_t>(nt * dense_grad_slices(INT64_MAX / 2, nt), dense_gpart_need(c))), "alloc gpart");
     CK(c->blkpart.alloc(4 * nval), "alloc blkpart");
-    CK(c->redpart.alloc(148 * 8), "alloc redpart");
+    CK(c->redpart.alloc(148 * 12), "alloc redpart");
     CK(c->scal.alloc(SC_COUNT), "alloc scal");
+    if (!c->io_ptrs.p) {
+        CK(c->io_ptrs.alloc(1), "alloc io");
+        CK(cudaMemsetAsync(c->io_ptrs.p, 0, sizeof(IoPtrs), c->stream), "clear io");
+        c->io_set = IoPtrs();
+    }
+    const sdot_status st = ensure_tickets(c);
+    if (st != SDOT_OK) return st;
     CK(c->io_a.alloc(nt), "alloc io");
     CK(c->io_b.alloc(nt), "alloc io");
     return SDOT_OK;
@@ -186,33 +201,58 @@ sdot_status ensure_eval_buffers(sdot_ctx *c)
 // (SotSolver.cc:431-473; the R-tree nearest query returns the same distance)
 // ---------------------------------------------------------------------------
 
-template <int DIM>
-__global__ void k_covering(const double *__restrict__ cell_ctr, int64_t ncells, const double *__restrict__ y,
-                           int64_t nt, double *__restrict__ blockmax)
+// LANES consecutive threads share a cell and take every LANES-th target (few
+// cells would leave most of the GPU idle with a thread each: 15.6 us against
+// the 4 CTAs of 1,024 cells x 500 targets); the minimum, and the maximum over
+// the cells, do not depend on the order.  The last CTA writes the result to
+// the host.
+constexpr int COVER_THREADS = 256;
+constexpr int COVER_BLOCKS = 148 * 8;
+constexpr int COVER_STAGE = 512;
+
+template <int DIM, int LANES>
+__global__ void __launch_bounds__(COVER_THREADS)
+k_covering(const double *__restrict__ cell_ctr, int64_t ncells, const double *__restrict__ y, int64_t nt,
+           double *__restrict__ blockmax, unsigned *__restrict__ ticket, double *__restrict__ out_host)
 {
-    __shared__ double sy[1024 * DIM];
-    __shared__ double red[32];
-    const int64_t cidx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    double cc[3] = {0, 0, 0};
-    if (cidx < ncells)
-        for (int d = 0; d < DIM; ++d) cc[d] = cell_ctr[cidx * DIM + d];
-    double best = DBL_MAX;
-    for (int64_t t0 = 0; t0 < nt; t0 += 1024) {
-        const int tn = (int)min((int64_t)1024, nt - t0);
-        __syncthreads();
-        for (int i = threadIdx.x; i < tn * DIM; i += blockDim.x) sy[i] = y[t0 * DIM + i];
-        __syncthreads();
-        for (int t = 0; t < tn; ++t) best = fmin(best, dist2_exact<DIM>(sy + t * DIM, cc));
+    constexpr int PER = COVER_THREADS / LANES;
+    constexpr int NW = COVER_THREADS / 32;
+    __shared__ double sy[COVER_STAGE * DIM];
+    __shared__ double red[NW];
+    const int sub = threadIdx.x % LANES;
+    double v = 0.0;
+    for (int64_t c0 = blockIdx.x * (int64_t)PER; c0 < ncells; c0 += (int64_t)gridDim.x * PER) {
+        const int64_t cidx = c0 + threadIdx.x / LANES;
+        double cc[3] = {0, 0, 0};
+        if (cidx < ncells)
+            for (int d = 0; d < DIM; ++d) cc[d] = cell_ctr[cidx * DIM + d];
+        double best = DBL_MAX;
+        for (int64_t t0 = 0; t0 < nt; t0 += COVER_STAGE) {
+            const int tn = (int)min((int64_t)COVER_STAGE, nt - t0);
+            __syncthreads();
+            for (int i = threadIdx.x; i < tn * DIM; i += COVER_THREADS) sy[i] = y[t0 * DIM + i];
+            __syncthreads();
+#pragma unroll 4
+            for (int t = sub; t < tn; t += LANES) best = fmin(best, dist2_exact<DIM>(sy + t * DIM, cc));
+        }
+#pragma unroll
+        for (int o = 1; o < LANES; o <<= 1) best = fmin(best, __shfl_xor_sync(0xffffffffu, best, o));
+        if (cidx < ncells) v = fmax(v, __dsqrt_rn(best));
     }
-    double v = cidx < ncells ? __dsqrt_rn(best) : 0.0;
-    v = warp_max(v);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double m = 0.0;
-        for (int i = 0; i < (int)(blockDim.x >> 5); ++i) m = fmax(m, red[i]);
-        blockmax[blockIdx.x] = m;
-    }
+    auto reduce = [&]() {
+        v = warp_max(v);
+        __syncthreads();
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+        __syncthreads();
+        for (int i = 0; i < NW; ++i) v = fmax(v, red[i]);
+    };
+    reduce();
+    if (threadIdx.x == 0) blockmax[blockIdx.x] = v;
+    if (!last_block(ticket)) return;
+    v = 0.0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += COVER_THREADS) v = fmax(v, __ldcg(blockmax + i));
+    reduce();
+    if (threadIdx.x == 0) *out_host = v;
 }
 
 // ---------------------------------------------------------------------------
@@ -227,78 +267,89 @@ struct Hist {
     int slot[6];
 };
 
-// Two-loop recursion (deal.II SolverBFGS::solve, wasserstein_solver_bfgs.h
-// :420-441), H0 = I; one CTA, order-fixed reductions.  Also writes g.p.
+// One L-BFGS step between two line searches, by one CTA (order-fixed
+// reductions, every thread adds the warps' sums over the same tree):
+//  * with spare >= 0, s = x - x_old and y = g - g_old of the accepted step go
+//    to history slot spare, with rho = 1 / (s.y); the history is `with` when
+//    s.y > 0 and `without` otherwise;
+//  * x_old = x, g_old = g;
+//  * the direction p by the two-loop recursion (deal.II SolverBFGS::solve,
+//    wasserstein_solver_bfgs.h:420-441), H0 = I;
+//  * g.p and s.y to the host.
+// One launch and one wait; as separate kernels and copies with a wait each
+// (s.y, rho, g.p) a step took 40 us beside its evaluations at 500 targets.
 __global__ void __launch_bounds__(1024)
-k_two_loop(int64_t n, Hist h, const double *__restrict__ S, const double *__restrict__ Y,
-           const double *__restrict__ rho, const double *__restrict__ g, double *__restrict__ p,
-           double *__restrict__ gp_out)
+k_lbfgs_step(int64_t n, Hist with, Hist without, int spare, double *__restrict__ S, double *__restrict__ Y,
+             double *__restrict__ rho, const double *__restrict__ x, double *__restrict__ x_old,
+             const double *__restrict__ g, double *__restrict__ g_old, double *__restrict__ p,
+             double *__restrict__ out_host)
 {
-    __shared__ double red[32];
-    __shared__ double bc;
+    __shared__ double red[2][32];
     __shared__ double c1[8];
-    const int tid = threadIdx.x;
-    auto block_dot = [&](const double *a, const double *b) -> double {
-        double s = 0.0;
-        for (int64_t i = tid; i < n; i += blockDim.x) s += a[i] * b[i];
+    const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5, nw = blockDim.x >> 5;
+    int par = 0;
+    auto block_sum = [&](double s) -> double {  // one barrier: the two rows alternate
         s = warp_sum(s);
+        if (lane == 0) red[par][wp] = s;
         __syncthreads();
-        if ((tid & 31) == 0) red[tid >> 5] = s;
-        __syncthreads();
-        if (tid == 0) {
-            double t = 0.0;
-            for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += red[i];
-            bc = t;
-        }
-        __syncthreads();
-        return bc;
+        s = warp_sum(lane < nw ? red[par][lane] : 0.0);
+        par ^= 1;
+        return s;
     };
-    for (int64_t i = tid; i < n; i += blockDim.x) p[i] = g[i];
-    __syncthreads();
+    Hist h = without;
+    double sy = 0.0;
+    if (spare >= 0) {
+        double *s = S + (int64_t)spare * n, *yv = Y + (int64_t)spare * n;
+        double acc = 0.0;
+        for (int64_t i = tid; i < n; i += blockDim.x) {
+            const double a = x[i] - x_old[i];
+            const double b = g[i] - g_old[i];
+            s[i] = a;
+            yv[i] = b;
+            acc += a * b;
+        }
+        sy = block_sum(acc);
+        if (sy > 0.0) {
+            h = with;
+            if (tid == 0) rho[spare] = 1. / sy;
+        }
+    }
+    for (int64_t i = tid; i < n; i += blockDim.x) {
+        const double gi = g[i];
+        p[i] = gi;
+        g_old[i] = gi;
+        x_old[i] = x[i];
+    }
+    __syncthreads();  // rho
+    // each thread reads and writes its own entries of p, S and Y only
     for (int i = 0; i < h.m; ++i) {
         const int slot = h.slot[i];
-        const double ci = rho[slot] * block_dot(S + (int64_t)slot * n, p);
+        const double *sv = S + (int64_t)slot * n, *yv = Y + (int64_t)slot * n;
+        double acc = 0.0;
+        for (int64_t t = tid; t < n; t += blockDim.x) acc += sv[t] * p[t];
+        const double ci = rho[slot] * block_sum(acc);
         if (tid == 0) c1[i] = ci;
-        const double a = -ci;
-        const double *yv = Y + (int64_t)slot * n;
-        for (int64_t t = tid; t < n; t += blockDim.x) p[t] += a * yv[t];
-        __syncthreads();
+        for (int64_t t = tid; t < n; t += blockDim.x) p[t] += -ci * yv[t];
     }
     for (int i = h.m - 1; i >= 0; --i) {
         const int slot = h.slot[i];
-        const double c2 = rho[slot] * block_dot(Y + (int64_t)slot * n, p);
+        const double *sv = S + (int64_t)slot * n, *yv = Y + (int64_t)slot * n;
+        double acc = 0.0;
+        for (int64_t t = tid; t < n; t += blockDim.x) acc += yv[t] * p[t];
+        const double c2 = rho[slot] * block_sum(acc);
         const double a = c1[i] - c2;
-        const double *sv = S + (int64_t)slot * n;
         for (int64_t t = tid; t < n; t += blockDim.x) p[t] += a * sv[t];
-        __syncthreads();
     }
-    for (int64_t i = tid; i < n; i += blockDim.x) p[i] *= -1.;
-    __syncthreads();
-    const double gp = block_dot(g, p);
-    if (tid == 0) gp_out[0] = gp;
-}
-
-// s_k = x - x_old, y_k = g - g_old into a history slot; out = s_k . y_k
-__global__ void __launch_bounds__(1024)
-k_sy(int64_t n, const double *__restrict__ x, const double *__restrict__ xold, const double *__restrict__ g,
-     const double *__restrict__ gold, double *__restrict__ s, double *__restrict__ yv, double *__restrict__ out)
-{
-    __shared__ double red[32];
     double acc = 0.0;
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const double a = x[i] - xold[i];
-        const double b = g[i] - gold[i];
-        s[i] = a;
-        yv[i] = b;
-        acc += a * b;
+    for (int64_t i = tid; i < n; i += blockDim.x) {
+        const double v = -p[i];
+        p[i] = v;
+        acc += g[i] * v;
     }
-    acc = warp_sum(acc);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += red[i];
-        out[0] = t;
+    const double gp = block_sum(acc);
+    if (tid == 0) {
+        out_host[0] = gp;
+        out_host[1] = sy;
     }
 }
 
@@ -387,6 +438,7 @@ void sdot_destroy(sdot_ctx *c)
         c->y.release(); c->nu.release();
         c->perm.release(); c->tblk_sph.release(); c->psi.release(); c->grad.release(); c->tpack.release();
         c->Lq.release(); c->gpart.release(); c->blkpart.release(); c->scal.release(); c->redpart.release();
+        c->io_ptrs.release(); c->ticket.release(); c->cover.release();
         c->vpart.release(); c->lat_buf.release();
         c->io_a.release(); c->io_b.release(); c->x0.release(); c->pdir.release(); c->sk.release(); c->yk.release();
         c->hist_s.release(); c->hist_y.release(); c->gtmp.release();
@@ -722,14 +774,16 @@ sdot_status sdot_evaluate(sdot_ctx *c, const double *psi, double *grad, double *
     sdot_status s = prepare_eval(c);
     if (s != SDOT_OK) return s;
     CK(cudaMemcpyAsync(c->io_a.p, psi, c->nt * 8, cudaMemcpyHostToDevice, c->stream), "copy psi");
-    if ((s = launch_gather(c, c->psi.p, c->io_a.p, c->nt)) != SDOT_OK) return s;
     double ms = 0;
-    // one wait for the stream: the gradient's scatter and copy are queued behind the evaluation
+    // one wait for the stream: the gradient's copy is queued behind the evaluation
     EvalPending pend;
-    s = evaluate_enqueue(c, nullptr, c->prm.tolerance, false, pend);
+    IoPtrs io;
+    io.psi = c->io_a.p;
+    io.grad = c->io_b.p;
+    s = evaluate_enqueue(c, nullptr, c->prm.tolerance, false, pend, &io);
     if (s != SDOT_OK && s != SDOT_ENONFINITE) return s;
     const bool queued = s == SDOT_OK;   // ENONFINITE here: non-finite psi, nothing was queued
-    sdot_status s2 = launch_scatter(c, c->io_b.p, c->grad.p, c->nt);
+    sdot_status s2 = queued ? SDOT_OK : launch_scatter(c, c->io_b.p, c->grad.p, c->nt);
     if (s2 != SDOT_OK) return s2;
     CK(cudaMemcpyAsync(grad, c->io_b.p, c->nt * 8, cudaMemcpyDeviceToHost, c->stream), "copy grad");
     CK(cudaStreamSynchronize(c->stream), "evaluate sync");
@@ -747,13 +801,15 @@ sdot_status sdot_evaluate_device(sdot_ctx *c, const double *psi_dev, double *gra
     DeviceGuard g(c->device);
     sdot_status s = prepare_eval(c);
     if (s != SDOT_OK) return s;
-    if ((s = launch_gather(c, c->psi.p, psi_dev, c->nt)) != SDOT_OK) return s;
     double ms = 0;
     EvalPending pend;
-    s = evaluate_enqueue(c, nullptr, c->prm.tolerance, false, pend);
+    IoPtrs io;
+    io.psi = psi_dev;
+    io.grad = grad_dev;
+    s = evaluate_enqueue(c, nullptr, c->prm.tolerance, false, pend, &io);
     if (s != SDOT_OK && s != SDOT_ENONFINITE) return s;
     const bool queued = s == SDOT_OK;
-    sdot_status s2 = launch_scatter(c, grad_dev, c->grad.p, c->nt);
+    sdot_status s2 = queued ? SDOT_OK : launch_scatter(c, grad_dev, c->grad.p, c->nt);
     if (s2 != SDOT_OK) return s2;
     CK(cudaStreamSynchronize(c->stream), "evaluate sync");
     if (queued) s = evaluate_complete(c, pend, &ms);
@@ -768,21 +824,23 @@ sdot_status sdot_compute_covering_radius(sdot_ctx *c, double *radius)
     if (!c || !radius) return SDOT_EINVAL;
     if (c->nq == 0 || c->nt == 0) return set_error(c, SDOT_ESTATE, "Invalid measures configuration for computing covering radius");
     DeviceGuard g(c->device);
-    const int threads = 256;
-    const int64_t nb = (c->ncells + threads - 1) / threads;
-    sdot::DevBuf<double> bm;
-    CK(bm.alloc(nb), "alloc covering");
-    if (c->dim == 2)
-        k_covering<2><<<(unsigned)nb, threads, 0, c->stream>>>(c->cell_ctr.p, c->ncells, c->y.p, c->nt, bm.p);
-    else
-        k_covering<3><<<(unsigned)nb, threads, 0, c->stream>>>(c->cell_ctr.p, c->ncells, c->y.p, c->nt, bm.p);
+    sdot_status s = ensure_tickets(c);
+    if (s != SDOT_OK) return s;
+    CK(c->cover.alloc(COVER_BLOCKS), "alloc covering");
+    // threads per cell: as many as it takes to fill the GPU
+    const int lanes = c->ncells >= (int64_t)COVER_BLOCKS * COVER_THREADS / 4 ? 1
+                      : (c->ncells >= (int64_t)COVER_BLOCKS * COVER_THREADS / 32 ? 8 : 32);
+    const int64_t per = COVER_THREADS / lanes;
+    const unsigned nb = (unsigned)std::min<int64_t>(COVER_BLOCKS, (c->ncells + per - 1) / per);
+    auto go = [&](auto kern) {
+        kern<<<nb, COVER_THREADS, 0, c->stream>>>(c->cell_ctr.p, c->ncells, c->y.p, c->nt, c->cover.p, c->ticket.p + 2,
+                                                  c->scal_host + SC_COVER);
+    };
+    if (c->dim == 2) lanes == 1 ? go(k_covering<2, 1>) : (lanes == 8 ? go(k_covering<2, 8>) : go(k_covering<2, 32>));
+    else lanes == 1 ? go(k_covering<3, 1>) : (lanes == 8 ? go(k_covering<3, 8>) : go(k_covering<3, 32>));
     CK(cudaGetLastError(), "covering launch");
-    std::vector<double> h(nb);
-    CK(cudaMemcpyAsync(h.data(), bm.p, nb * 8, cudaMemcpyDeviceToHost, c->stream), "covering copy");
     CK(cudaStreamSynchronize(c->stream), "covering sync");
-    double m = 0.0;
-    for (double v : h) m = std::max(m, v);
-    *radius = m;
+    *radius = c->scal_host[SC_COVER];
     return SDOT_OK;
 }
 
@@ -994,29 +1052,40 @@ sdot_status sdot_solve(sdot_ctx *c, double *psi, const sdot_solver_params *param
     unsigned k = 0;
     int first_step = 1;
     double f_prev = 0.;
-    Hist hist{};
-    hist.m = 0;
     std::vector<int> order;  // physical slots, newest first
     int spare = 0;
+    bool stepped = false;    // a line search has been accepted: its (s, y) go to the spare slot
     std::vector<int> free_slots = {1, 2, 3, 4, 5};
     double *rho_dev = c->sk.p;
-    double *scratch = c->sk.p + 6;
+    const unsigned step_threads = (unsigned)std::min<int64_t>(1024, (n + 31) / 32 * 32);
     sdot_status result = SDOT_OK;
     int conv;
     if ((s = S.eval_at(&f, &gp)) != SDOT_OK) return s;
     conv = control_check(c, k, &check_value);
-    double host2[2];
     while (conv == 0) {
-        hist.m = (int)order.size();
-        for (int i = 0; i < hist.m; ++i) hist.slot[i] = order[i];
-        k_two_loop<<<1, 1024, 0, c->stream>>>(n, hist, c->hist_s.p, c->hist_y.p, rho_dev, c->grad.p, c->pdir.p,
-                                               scratch);
-        CK(cudaGetLastError(), "two-loop");
-        CK(cudaMemcpyAsync(c->x0.p, c->psi.p, n * 8, cudaMemcpyDeviceToDevice, c->stream), "copy x0");
-        CK(cudaMemcpyAsync(c->gtmp.p, c->grad.p, n * 8, cudaMemcpyDeviceToDevice, c->stream), "copy g");
-        CK(cudaMemcpyAsync(host2, scratch, 8, cudaMemcpyDeviceToHost, c->stream), "g0 copy");
-        CK(cudaStreamSynchronize(c->stream), "g0 sync");
-        const double g0 = host2[0];
+        // s_k, y_k into the spare slot, kept iff their curvature s.y > 0 (the device picks the history), and the
+        // next direction
+        Hist with{}, without{};
+        for (int i = 0; i < (int)order.size(); ++i) without.slot[without.m++] = order[i];
+        if (stepped) with.slot[with.m++] = spare;
+        for (int i = 0; i < (int)order.size() && with.m < M; ++i) with.slot[with.m++] = order[i];
+        k_lbfgs_step<<<1, step_threads, 0, c->stream>>>(n, with, without, stepped ? spare : -1, c->hist_s.p, c->hist_y.p,
+                                                        rho_dev, c->psi.p, c->x0.p, c->grad.p, c->gtmp.p, c->pdir.p,
+                                                        c->scal_host + SC_STEP_GP);
+        CK(cudaGetLastError(), "direction");
+        CK(cudaStreamSynchronize(c->stream), "direction sync");
+        static_assert(SC_STEP_SY == SC_STEP_GP + 1, "step slots");
+        const double g0 = c->scal_host[SC_STEP_GP];
+        if (stepped && c->scal_host[SC_STEP_SY] > 0.) {
+            order.insert(order.begin(), spare);
+            if ((int)order.size() > M) {
+                spare = order.back();
+                order.pop_back();
+            } else {
+                spare = free_slots.back();
+                free_slots.pop_back();
+            }
+        }
         // default line search lambda (wasserstein_solver_bfgs.h:316-389)
         const double f0 = f;
         double df = f_prev - f;
@@ -1052,26 +1121,7 @@ sdot_status sdot_solve(sdot_ctx *c, double *psi, const sdot_solver_params *param
         ++k;
         conv = control_check(c, k, &check_value);
         if (conv != 0) break;
-        // s_k = x - x0, y_k = g - g0 into the spare slot; keep it iff curvature > 0
-        k_sy<<<1, 1024, 0, c->stream>>>(n, c->psi.p, c->x0.p, c->grad.p, c->gtmp.p, c->hist_s.p + (int64_t)spare * n,
-                                        c->hist_y.p + (int64_t)spare * n, scratch);
-        CK(cudaGetLastError(), "sy");
-        CK(cudaMemcpyAsync(host2, scratch, 8, cudaMemcpyDeviceToHost, c->stream), "curv copy");
-        CK(cudaStreamSynchronize(c->stream), "curv sync");
-        const double curvature = host2[0];
-        if (curvature > 0.) {
-            const double r = 1. / curvature;
-            CK(cudaMemcpyAsync(rho_dev + spare, &r, 8, cudaMemcpyHostToDevice, c->stream), "rho");
-            CK(cudaStreamSynchronize(c->stream), "rho sync");
-            order.insert(order.begin(), spare);
-            if ((int)order.size() > M) {
-                spare = order.back();
-                order.pop_back();
-            } else {
-                spare = free_slots.back();
-                free_slots.pop_back();
-            }
-        }
+        stepped = true;
     }
     c->last_iterations = k;
     c->last_converged = (conv == 1);
@@ -1108,13 +1158,15 @@ sdot_status sdot_evaluate_partial_device(sdot_ctx *c, const double *psi_dev, dou
     DeviceGuard g(c->device);
     sdot_status s = prepare_eval(c);
     if (s != SDOT_OK) return s;
-    if ((s = launch_gather(c, c->psi.p, psi_dev, c->nt)) != SDOT_OK) return s;
     double ms = 0;
     EvalPending pend;
-    s = evaluate_enqueue(c, nullptr, c->prm.tolerance, true, pend);
+    IoPtrs io;
+    io.psi = psi_dev;
+    io.grad = out_dev;
+    s = evaluate_enqueue(c, nullptr, c->prm.tolerance, true, pend, &io);
     if (s != SDOT_OK && s != SDOT_ENONFINITE) return s;
     const bool queued = s == SDOT_OK;
-    sdot_status s2 = launch_scatter(c, out_dev, c->grad.p, c->nt);
+    sdot_status s2 = queued ? SDOT_OK : launch_scatter(c, out_dev, c->grad.p, c->nt);
     if (s2 != SDOT_OK) return s2;
     k_partial_tail<<<1, 1, 0, c->stream>>>(c->scal.p, out_dev + c->nt);
     CK(cudaGetLastError(), "partial tail");

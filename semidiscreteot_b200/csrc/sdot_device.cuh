@@ -199,6 +199,20 @@ __device__ __forceinline__ void lse_update(double b, double nu, double &M, doubl
     S = fma(nu, exp2_16(u, tab), S);
 }
 
+// Whether this CTA is the last of the grid to arrive (all threads get the
+// answer; what the others wrote before is visible then).  The counter wraps
+// back to zero.
+__device__ __forceinline__ bool last_block(unsigned *ticket)
+{
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
 // Block-level ordered sum of (value, C, skipped, pairs) -> out4[0..3].
 __device__ __forceinline__ void block_partials_at(double v, double c, double sk, double np, double *out4)
 {

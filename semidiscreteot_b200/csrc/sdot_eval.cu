@@ -59,60 +59,80 @@ __global__ void k_axpy(double *x, const double *x0, double a, const double *p, i
         x[i] = x0[i] + a * p[i];
 }
 
-// max/min/non-finite flag of a vector: out[0]=max, out[1]=min, out[2]=1 if non-finite.
-__global__ void k_minmax(const double *v, int64_t n, double *out)
+// Range of the potential, gathered on the way (dst[i] = src[perm[i]]; without
+// perm dst is read): max, min and 1 if an entry is not finite, to out and
+// out_host.  Four entries per thread and pass, so that their loads overlap;
+// the last CTA reduces the CTAs' results.
+constexpr int RANGE_THREADS = 256;
+constexpr int RANGE_BLOCKS = 148;
+__global__ void __launch_bounds__(RANGE_THREADS)
+k_psi_range(int64_t n, const double *__restrict__ src, const int64_t *__restrict__ perm, double *__restrict__ dst,
+            double *__restrict__ part, unsigned *__restrict__ ticket, double *__restrict__ out,
+            double *__restrict__ out_host)
 {
-    __shared__ double smx[32], smn[32];
-    __shared__ int sbad[32];
-    double mx = -DBL_MAX, mn = DBL_MAX;
-    int bad = 0;
-    // sixteen independent loads in flight per thread (max, min and the flag do
-    // not depend on the order): the single CTA is bound by load latency
-    constexpr int U = 16;
-    const int64_t step = blockDim.x;
-    int64_t i = threadIdx.x;
-    for (; i + (U - 1) * step < n; i += U * step) {
+    constexpr int U = 4, NW = RANGE_THREADS / 32;
+    __shared__ double sh[3][NW];
+    double mx = -DBL_MAX, mn = DBL_MAX, bad = 0.0;
+    for (int64_t base = blockIdx.x * (int64_t)(RANGE_THREADS * U); base < n;
+         base += (int64_t)gridDim.x * (RANGE_THREADS * U)) {
         double a[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) a[u] = v[i + u * step];
+        for (int u = 0; u < U; ++u) {
+            const int64_t i = base + u * RANGE_THREADS + threadIdx.x;
+            a[u] = i < n ? (perm ? src[perm[i]] : dst[i]) : 0.0;
+        }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            if (!isfinite(a[u])) bad = 1;
+            const int64_t i = base + u * RANGE_THREADS + threadIdx.x;
+            if (i >= n) continue;
+            if (perm) dst[i] = a[u];
+            if (!isfinite(a[u])) bad = 1.0;
             mx = a[u] > mx ? a[u] : mx;
             mn = a[u] < mn ? a[u] : mn;
         }
     }
-    for (; i < n; i += step) {
-        const double a = v[i];
-        if (!isfinite(a)) bad = 1;
-        mx = a > mx ? a : mx;
-        mn = a < mn ? a : mn;
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-        bad |= __shfl_xor_sync(0xffffffffu, bad, o);
-    }
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0) { smx[w] = mx; smn[w] = mn; sbad[w] = bad; }
-    __syncthreads();
+    auto reduce = [&]() {  // over the CTA, to thread 0
+        mx = warp_max(mx);
+        mn = -warp_max(-mn);
+        bad = warp_max(bad);
+        const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+        __syncthreads();
+        if (l == 0) { sh[0][w] = mx; sh[1][w] = mn; sh[2][w] = bad; }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int i = 1; i < NW; ++i) {
+                mx = fmax(mx, sh[0][i]);
+                mn = fmin(mn, sh[1][i]);
+                bad = fmax(bad, sh[2][i]);
+            }
+    };
+    reduce();
     if (threadIdx.x == 0) {
-        for (int i = 1; i < (int)(blockDim.x >> 5); ++i) {
-            mx = fmax(mx, smx[i]);
-            mn = fmin(mn, smn[i]);
-            bad |= sbad[i];
-        }
-        out[0] = mx;
-        out[1] = mn;
-        out[2] = bad;
+        part[blockIdx.x * 3 + 0] = mx;
+        part[blockIdx.x * 3 + 1] = mn;
+        part[blockIdx.x * 3 + 2] = bad;
+    }
+    if (!last_block(ticket)) return;
+    mx = -DBL_MAX;
+    mn = DBL_MAX;
+    bad = 0.0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += RANGE_THREADS) {
+        mx = fmax(mx, __ldcg(part + i * 3));
+        mn = fmin(mn, __ldcg(part + i * 3 + 1));
+        bad = fmax(bad, __ldcg(part + i * 3 + 2));
+    }
+    reduce();
+    if (threadIdx.x == 0) {
+        out[0] = out_host[0] = mx;
+        out[1] = out_host[1] = mn;
+        out[2] = out_host[2] = bad;
     }
 }
 
 // tpack[j] = {A_j, B_j(DIM), nu_j, y_j(DIM)}: scaled exponent coefficients.
 template <int DIM>
 __device__ __forceinline__ void target_prep_one(int64_t j, const double *__restrict__ y, const double *__restrict__ nu,
-                                                const double *__restrict__ psi, const EvalArgs &a,
-                                                double *__restrict__ tpack)
+                                                double psi, const EvalArgs &a, double *__restrict__ tpack)
 {
     double yt[3], ysq = 0.0;
 #pragma unroll
@@ -121,7 +141,7 @@ __device__ __forceinline__ void target_prep_one(int64_t j, const double *__restr
         ysq += yt[d] * yt[d];
     }
     double *t = tpack + j * TPACK;
-    t[0] = a.s * psi[j] - a.halfs * ysq;
+    t[0] = a.s * psi - a.halfs * ysq;
 #pragma unroll
     for (int d = 0; d < DIM; ++d) t[1 + d] = a.s * yt[d];
     t[1 + DIM] = nu[j];
@@ -129,12 +149,17 @@ __device__ __forceinline__ void target_prep_one(int64_t j, const double *__restr
     for (int d = 0; d < DIM; ++d) t[2 + DIM + d] = y[j * DIM + d];
 }
 
+// With io, psi is gathered from the caller's array (io->psi) on the way.
 template <int DIM>
 __global__ void k_target_prep(int64_t nt, const double *__restrict__ y, const double *__restrict__ nu,
-                              const double *__restrict__ psi, EvalArgs a, double *__restrict__ tpack)
+                              double *__restrict__ psi, const IoPtrs *__restrict__ io,
+                              const int64_t *__restrict__ perm, EvalArgs a, double *__restrict__ tpack)
 {
-    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < nt; j += (int64_t)gridDim.x * blockDim.x)
-        target_prep_one<DIM>(j, y, nu, psi, a, tpack);
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < nt; j += (int64_t)gridDim.x * blockDim.x) {
+        const double p = io ? io->psi[perm[j]] : psi[j];
+        if (io) psi[j] = p;
+        target_prep_one<DIM>(j, y, nu, p, a, tpack);
+    }
 }
 
 // Target packing (with the target blocks' largest s psi and the targets' step
@@ -144,12 +169,15 @@ __global__ void k_target_prep(int64_t nt, const double *__restrict__ y, const do
 constexpr int LAT_PREP_THREADS = 512;
 template <int DIM>
 __global__ void __launch_bounds__(LAT_PREP_THREADS)
-k_lat_prep(const double *__restrict__ y, const double *__restrict__ nu, const double *__restrict__ psi, EvalArgs a,
-           LatArgs L, const int64_t *__restrict__ tblk_off, int ntb, int npb, double *__restrict__ tpack,
+k_lat_prep(const double *__restrict__ y, const double *__restrict__ nu, double *__restrict__ psi,
+           const IoPtrs *__restrict__ io, const int64_t *__restrict__ perm, EvalArgs a, LatArgs L,
+           const int64_t *__restrict__ tblk_off, int ntb, int npb, double *__restrict__ tpack,
            double *__restrict__ top, double *__restrict__ shift, double *__restrict__ step)
 {
+    const double *src = io ? io->psi : nullptr;
     if ((int)blockIdx.x >= npb) {
-        lat_shift_block<DIM, LAT_PREP_THREADS>(L, a, blockIdx.x - npb, y, psi, shift);
+        lat_shift_block<DIM, LAT_PREP_THREADS>(
+            L, a, blockIdx.x - npb, y, [&](int64_t j) { return src ? src[perm[j]] : psi[j]; }, shift);
         return;
     }
     constexpr int NW = LAT_PREP_THREADS / 32;
@@ -158,8 +186,10 @@ k_lat_prep(const double *__restrict__ y, const double *__restrict__ nu, const do
         const int64_t j = tblk_off[b] + lane;
         double v = -CUDART_INF;
         if (j < tblk_off[b + 1]) {
-            target_prep_one<DIM>(j, y, nu, psi, a, tpack);
-            v = a.s * psi[j];
+            const double p = src ? src[perm[j]] : psi[j];
+            if (src) psi[j] = p;
+            target_prep_one<DIM>(j, y, nu, p, a, tpack);
+            v = a.s * p;
             if (L.runs > 0) {
 #pragma unroll
                 for (int d = 0; d < DIM; ++d) step[j * DIM + d] = exp2(tpack[j * TPACK + 1 + d] * L.step16[d]);
@@ -670,17 +700,17 @@ k_grad_dense(const double *__restrict__ x, const double *__restrict__ w, const d
 // ---------------------------------------------------------------------------
 
 constexpr int FIN_THREADS = 256;
-constexpr int FIN_BLOCKS = 148;  // largest grid of k_finalize_grad
-constexpr int NRED = 8;  // psinu, l1, linf, comp, l2sq, gp, nonfinite, unused
+constexpr int FIN_BLOCKS = 148;  // largest grid of k_finalize
+constexpr int NRED = 12;  // psinu, l1, linf, comp, l2sq, gp, nonfinite; value, C, skipped, pairs; unused
 
-// Lanes per target of k_finalize_grad for nks slice partials: the smallest
+// Lanes per target of k_finalize for nks slice partials: the smallest
 // power of two >= nks, at most 8.
 static int fin_parts(int nks)
 {
     return nks <= 1 ? 1 : (nks <= 2 ? 2 : (nks <= 4 ? 4 : 8));
 }
 
-// Grid of k_finalize_grad for nt targets (FIN_THREADS / parts targets per CTA and pass).
+// Grid of k_finalize for nt targets (FIN_THREADS / parts targets per CTA and pass).
 static int fin_blocks(int64_t nt, int parts)
 {
     const int64_t per = FIN_THREADS / parts;
@@ -694,180 +724,156 @@ static int fin_blocks(int64_t nt, int parts)
 // s3), ...  PARTS = 8, or any power of two PARTS >= nks, gives the sums of
 // eight interleaved sums k mod 8 added in the tree ((s0 + s1) + (s2 + s3)) +
 // ((s4 + s5) + (s6 + s7)) (the lanes past nks hold zeros).
+//
+// Each CTA also sums its share of the nval value partials; the last CTA to
+// arrive adds the CTAs' results (in order of the CTAs over a fixed tree) and
+// writes the evaluation's scalars to scal and to the host.  With io, the
+// gradient also goes to the caller's array.  One launch and no copy at the
+// end of an evaluation: two kernels, a scatter and a copy engine's transfer
+// took 20 us of a 71 us evaluation of 2,304 points x 256 targets.
+struct FinArgs {
+    int64_t nt;
+    int nks;
+    const double *gpart, *nu, *psi, *pdir;
+    double tol;
+    int sub_nu;
+    double *grad;
+    const IoPtrs *io;
+    const int64_t *perm;
+    int64_t nval;
+    const double *valpart;
+    double *redpart;
+    unsigned *ticket;
+    double *scal, *scal_host;
+};
+
 template <int PARTS>
 __global__ void __launch_bounds__(FIN_THREADS)
-k_finalize_grad(int64_t nt, int nks, const double *__restrict__ gpart, const double *__restrict__ nu,
-                const double *__restrict__ psi, const double *__restrict__ pdir, double tol, int sub_nu,
-                double *__restrict__ grad, double *__restrict__ redpart)
+k_finalize(FinArgs f)
 {
-    constexpr int FIN_PARTS = PARTS;
-    constexpr int TPB = FIN_THREADS / FIN_PARTS;  // targets per CTA and pass
-    const int u = threadIdx.x % FIN_PARTS;
-    double psinu = 0.0, l1 = 0.0, linf = 0.0, comp = -CUDART_INF, l2 = 0.0, gp = 0.0, bad = 0.0;
+    constexpr int TPB = FIN_THREADS / PARTS;  // targets per CTA and pass
+    constexpr int NW = FIN_THREADS / 32;
+    constexpr int NR = 11;
+    const int u = threadIdx.x % PARTS;
+    const int64_t nt = f.nt;
+    const int nks = f.nks;
+    const double *gpart = f.gpart;
+    // sums: 0 psinu, 1 l1, 4 l2sq, 5 dot_gp, 7 value, 8 C, 9 skipped, 10 pairs; maxima: 2 linf, 3 comp, 6 bad
+    double r[NR] = {0, 0, 0, -CUDART_INF, 0, 0, 0, 0, 0, 0, 0};
+    double *gout = f.io ? f.io->grad : nullptr;
     for (int64_t base = blockIdx.x * (int64_t)TPB; base < nt; base += (int64_t)gridDim.x * TPB) {
-        const int64_t j = base + threadIdx.x / FIN_PARTS;
+        const int64_t j = base + threadIdx.x / PARTS;
         const bool ok = j < nt;
         double acc = 0.0;
         if (ok) {
             int k = u;
-            for (; k + 3 * FIN_PARTS < nks; k += 4 * FIN_PARTS) {
+            for (; k + 3 * PARTS < nks; k += 4 * PARTS) {
                 const double v0 = gpart[(int64_t)k * nt + j];
-                const double v1 = gpart[(int64_t)(k + FIN_PARTS) * nt + j];
-                const double v2 = gpart[(int64_t)(k + 2 * FIN_PARTS) * nt + j];
-                const double v3 = gpart[(int64_t)(k + 3 * FIN_PARTS) * nt + j];
+                const double v1 = gpart[(int64_t)(k + PARTS) * nt + j];
+                const double v2 = gpart[(int64_t)(k + 2 * PARTS) * nt + j];
+                const double v3 = gpart[(int64_t)(k + 3 * PARTS) * nt + j];
                 acc += v0;
                 acc += v1;
                 acc += v2;
                 acc += v3;
             }
-            for (; k < nks; k += FIN_PARTS) acc += gpart[(int64_t)k * nt + j];
+            for (; k < nks; k += PARTS) acc += gpart[(int64_t)k * nt + j];
         }
 #pragma unroll
-        for (int o = 1; o < FIN_PARTS; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        for (int o = 1; o < PARTS; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
         if (ok && u == 0) {
-            const double s = acc;
-            const double g = s - nu[j];
-            grad[j] = sub_nu ? g : s;
-            psinu += psi[j] * nu[j];
+            const double s = acc, nuj = f.nu[j], ps = f.psi[j];
+            const double g = s - nuj, w = f.sub_nu ? g : s;
+            f.grad[j] = w;
+            if (gout) gout[f.perm[j]] = w;
+            r[0] += ps * nuj;
             const double ag = fabs(g);
-            l1 += ag;
-            linf = fmax(linf, ag);
-            comp = fmax(comp, ag - nu[j] * tol);
-            l2 += g * g;
-            if (pdir) gp += g * pdir[j];
-            if (!isfinite(g) || !isfinite(psi[j])) bad = 1.0;
+            r[1] += ag;
+            r[2] = fmax(r[2], ag);
+            r[3] = fmax(r[3], ag - nuj * f.tol);
+            r[4] += g * g;
+            if (f.pdir) r[5] += g * f.pdir[j];
+            if (!isfinite(g) || !isfinite(ps)) r[6] = 1.0;
         }
     }
-    __shared__ double sh[NRED][FIN_THREADS / 32];
-    psinu = warp_sum(psinu);
-    l1 = warp_sum(l1);
-    linf = warp_max(linf);
-    comp = warp_max(comp);
-    l2 = warp_sum(l2);
-    gp = warp_sum(gp);
-    bad = warp_max(bad);
-    const int wi = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) {
-        sh[0][wi] = psinu; sh[1][wi] = l1; sh[2][wi] = linf; sh[3][wi] = comp;
-        sh[4][wi] = l2; sh[5][wi] = gp; sh[6][wi] = bad;
+    const double4 *vp = reinterpret_cast<const double4 *>(f.valpart);
+    const int64_t per = (f.nval + gridDim.x - 1) / gridDim.x;
+    const int64_t v1 = min(f.nval, (blockIdx.x + 1) * per);
+#pragma unroll 4
+    for (int64_t b = blockIdx.x * per + threadIdx.x; b < v1; b += FIN_THREADS) {
+        const double4 t = vp[b];
+        r[7] += t.x;
+        r[8] += t.y;
+        r[9] += t.z;
+        r[10] += t.w;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double r[7] = {0, 0, 0, -CUDART_INF, 0, 0, 0};
-        for (int i = 0; i < FIN_THREADS / 32; ++i) {
-            r[0] += sh[0][i]; r[1] += sh[1][i]; r[2] = fmax(r[2], sh[2][i]); r[3] = fmax(r[3], sh[3][i]);
-            r[4] += sh[4][i]; r[5] += sh[5][i]; r[6] = fmax(r[6], sh[6][i]);
-        }
-        for (int k = 0; k < 7; ++k) redpart[blockIdx.x * NRED + k] = r[k];
-    }
-}
-
-// k_finalize_grad with fin_parts(nks) lanes per target; returns its grid size.
-static int launch_finalize_grad(int64_t nt, int nks, const double *gpart, const double *nu, const double *psi,
-                                const double *pdir, double tol, int sub_nu, double *grad, double *redpart,
-                                cudaStream_t st)
-{
-    const int parts = fin_parts(nks);
-    const int fb = fin_blocks(nt, parts);
-    auto go = [&](auto kern) {
-        kern<<<fb, FIN_THREADS, 0, st>>>(nt, nks, gpart, nu, psi, pdir, tol, sub_nu, grad, redpart);
-    };
-    if (parts == 1) go(k_finalize_grad<1>);
-    else if (parts == 2) go(k_finalize_grad<2>);
-    else if (parts == 4) go(k_finalize_grad<4>);
-    else go(k_finalize_grad<8>);
-    return fb;
-}
-
-// One CTA of T threads: thread i sums value partials i, i + T, i + 2T, ...
-// into four accumulators (partial i + kT into accumulator k mod 4, eight
-// loads in flight), added in a fixed order, and the gradient blocks'
-// reductions i, i + T, ...; then warp reductions, and warp 0 reduces the
-// warps' results (a fixed tree throughout).  T = 256 for up to 2,048 value
-// partials (the dense path), 1,024 above (one per source block).
-template <int T>
-__global__ void __launch_bounds__(T)
-k_finalize_scalars(int nred, const double *__restrict__ redpart, int64_t nval, const double *__restrict__ valpart,
-                   double *__restrict__ scal)
-{
-    constexpr int NW = T / 32;
-    __shared__ double sh[11][NW];
-    double va[4] = {0, 0, 0, 0}, ca[4] = {0, 0, 0, 0}, ska[4] = {0, 0, 0, 0}, npa[4] = {0, 0, 0, 0};
-    const double4 *vp = reinterpret_cast<const double4 *>(valpart);
-    int64_t b0 = threadIdx.x;
-    for (; b0 + 7 * T < nval; b0 += 8 * T) {
-        double4 t[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) t[u] = vp[b0 + u * T];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            va[u & 3] += t[u].x;
-            ca[u & 3] += t[u].y;
-            ska[u & 3] += t[u].z;
-            npa[u & 3] += t[u].w;
-        }
-    }
-#pragma unroll
-    for (int u = 0; u < 7; ++u) {
-        if (b0 + u * T < nval) {
-            const double4 t = vp[b0 + u * T];
-            va[u & 3] += t.x;
-            ca[u & 3] += t.y;
-            ska[u & 3] += t.z;
-            npa[u & 3] += t.w;
-        }
-    }
-    double v = (va[0] + va[1]) + (va[2] + va[3]), c = (ca[0] + ca[1]) + (ca[2] + ca[3]);
-    double sk = (ska[0] + ska[1]) + (ska[2] + ska[3]), np = (npa[0] + npa[1]) + (npa[2] + npa[3]);
-    double r[7] = {0, 0, 0, -CUDART_INF, 0, 0, 0};
-    for (int b = threadIdx.x; b < nred; b += T) {
-        const double *p = redpart + (int64_t)b * NRED;
-        r[0] += p[0]; r[1] += p[1]; r[2] = fmax(r[2], p[2]); r[3] = fmax(r[3], p[3]);
-        r[4] += p[4]; r[5] += p[5]; r[6] = fmax(r[6], p[6]);
-    }
-    v = warp_sum(v); c = warp_sum(c); sk = warp_sum(sk); np = warp_sum(np);
-    r[0] = warp_sum(r[0]); r[1] = warp_sum(r[1]); r[2] = warp_max(r[2]); r[3] = warp_max(r[3]);
-    r[4] = warp_sum(r[4]); r[5] = warp_sum(r[5]); r[6] = warp_max(r[6]);
+    __shared__ double sh[NR][NW];
     const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) {
-        sh[0][wi] = v; sh[1][wi] = c; sh[2][wi] = sk; sh[10][wi] = np;
+    auto is_max = [](int k) { return k == 2 || k == 3 || k == 6; };
+    auto reduce = [&]() {  // over the CTA, to warp 0's lane 0
 #pragma unroll
-        for (int k = 0; k < 7; ++k) sh[3 + k][wi] = r[k];
-    }
-    __syncthreads();
-    if (wi == 0) {
-        double t[11];
-        // sums: 0 value, 1 C, 2 skipped, 3 psinu, 4 l1, 7 l2sq, 8 dot_gp, 10 pairs; maxima: 5 linf, 6 comp, 9 bad
-#pragma unroll
-        for (int k = 0; k < 11; ++k)
-            t[k] = lane < NW ? sh[k][lane] : ((k == 5 || k == 6 || k == 9) ? -CUDART_INF : 0.0);
-#pragma unroll
-        for (int k = 0; k < 11; ++k) t[k] = (k == 5 || k == 6 || k == 9) ? warp_max(t[k]) : warp_sum(t[k]);
+        for (int k = 0; k < NR; ++k) r[k] = is_max(k) ? warp_max(r[k]) : warp_sum(r[k]);
         if (lane == 0) {
-            const double psinu = t[3];
-            const double value = t[0] - psinu;
-            scal[SC_VALUE] = value;
-            scal[SC_VALSRC] = t[0];
-            scal[SC_C] = t[1];
-            scal[SC_SKIPPED] = t[2];
-            scal[SC_PSINU] = psinu;
-            scal[SC_L1] = t[4];
-            scal[SC_LINF] = t[5];
-            scal[SC_COMP] = t[6];
-            scal[SC_L2SQ] = t[7];
-            scal[SC_DOT_GP] = t[8];
-            scal[SC_NONFINITE] = (t[9] != 0.0 || !isfinite(value)) ? 1.0 : 0.0;
-            scal[SC_PAIRS] = t[10];
+#pragma unroll
+            for (int k = 0; k < NR; ++k) sh[k][wi] = r[k];
+        }
+        __syncthreads();
+        if (wi == 0) {
+#pragma unroll
+            for (int k = 0; k < NR; ++k) {
+                const double t = lane < NW ? sh[k][lane] : (is_max(k) ? -CUDART_INF : 0.0);
+                r[k] = is_max(k) ? warp_max(t) : warp_sum(t);
+            }
+        }
+    };
+    reduce();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < NR; ++k) f.redpart[blockIdx.x * NRED + k] = r[k];
+    }
+    if (!last_block(f.ticket)) return;
+#pragma unroll
+    for (int k = 0; k < NR; ++k) {
+        r[k] = is_max(k) ? -CUDART_INF : 0.0;
+        if (threadIdx.x < gridDim.x) r[k] = __ldcg(f.redpart + threadIdx.x * NRED + k);
+    }
+    static_assert(FIN_BLOCKS <= FIN_THREADS, "one CTA's result per thread");
+    reduce();
+    if (threadIdx.x == 0) {
+        const double value = r[7] - r[0];
+        double o[SC_COUNT];
+        o[SC_VALUE] = value;
+        o[SC_C] = r[8];
+        o[SC_DOT_GP] = r[5];
+        o[SC_L1] = r[1];
+        o[SC_LINF] = fmax(r[2], 0.0);
+        o[SC_COMP] = r[3];
+        o[SC_L2SQ] = r[4];
+        o[SC_PSINU] = r[0];
+        o[SC_SKIPPED] = r[9];
+        o[SC_NONFINITE] = (r[6] > 0.0 || !isfinite(value)) ? 1.0 : 0.0;
+        o[SC_PAIRS] = r[10];
+        o[SC_VALSRC] = r[7];
+        constexpr int slot[] = {SC_VALUE, SC_C, SC_DOT_GP, SC_L1, SC_LINF, SC_COMP, SC_L2SQ,
+                                SC_PSINU, SC_SKIPPED, SC_NONFINITE, SC_PAIRS, SC_VALSRC};
+#pragma unroll
+        for (int k = 0; k < (int)(sizeof(slot) / sizeof(int)); ++k) {
+            f.scal[slot[k]] = o[slot[k]];
+            f.scal_host[slot[k]] = o[slot[k]];
         }
     }
 }
 
-// k_finalize_scalars with its CTA size for nval value partials.
-static void launch_finalize_scalars(cudaStream_t st, int nred, const double *redpart, int64_t nval,
-                                    const double *valpart, double *scal)
+// k_finalize with fin_parts(nks) lanes per target.
+static void launch_finalize(const FinArgs &f, cudaStream_t st)
 {
-    if (nval <= 2048) k_finalize_scalars<256><<<1, 256, 0, st>>>(nred, redpart, nval, valpart, scal);
-    else k_finalize_scalars<1024><<<1, 1024, 0, st>>>(nred, redpart, nval, valpart, scal);
+    const int parts = fin_parts(f.nks);
+    const int fb = fin_blocks(f.nt, parts);
+    auto go = [&](auto kern) { kern<<<fb, FIN_THREADS, 0, st>>>(f); };
+    if (parts == 1) go(k_finalize<1>);
+    else if (parts == 2) go(k_finalize<2>);
+    else if (parts == 4) go(k_finalize<4>);
+    else go(k_finalize<8>);
 }
 
 // ---------------------------------------------------------------------------
@@ -882,12 +888,16 @@ static int grid_for(int64_t n, int threads, int cap = 148 * 8)
     return (int)g;
 }
 
+template <int DIM>
+static void launch_target_prep(const sdot_ctx *c, const EvalArgs &a, double *psi, const IoPtrs *io, double *tpack)
+{
+    k_target_prep<DIM><<<grid_for(a.nt, 256), 256, 0, c->stream>>>(a.nt, c->y.p, c->nu.p, psi, io, c->perm.p, a, tpack);
+}
+
 void launch_target_prep_dense(sdot_ctx *c, const EvalArgs &a)
 {
-    if (c->dim == 2)
-        k_target_prep<2><<<grid_for(a.nt, 256), 256, 0, c->stream>>>(a.nt, c->y.p, c->nu.p, c->psi.p, a, c->tpack.p);
-    else
-        k_target_prep<3><<<grid_for(a.nt, 256), 256, 0, c->stream>>>(a.nt, c->y.p, c->nu.p, c->psi.p, a, c->tpack.p);
+    if (c->dim == 2) launch_target_prep<2>(c, a, c->psi.p, nullptr, c->tpack.p);
+    else launch_target_prep<3>(c, a, c->psi.p, nullptr, c->tpack.p);
 }
 
 void k_axpy_launch(cudaStream_t s, double *x, const double *x0, double a, const double *p, int64_t n)
@@ -1095,14 +1105,14 @@ struct LatScratch {
 };
 
 template <int DIM>
-static void launch_lat_prep(const sdot_ctx *c, const DenseShape &ds, const double *psi, const EvalArgs &a,
+static void launch_lat_prep(const sdot_ctx *c, const DenseShape &ds, double *psi, const IoPtrs *io, const EvalArgs &a,
                             double *tpack, double *vpart, cudaStream_t st)
 {
     constexpr int NW = LAT_PREP_THREADS / 32;
     const int npb = (int)std::min<int64_t>((c->ntblk + NW - 1) / NW, 148);
     const LatScratch S(ds, vpart, a.nt, DIM);
     k_lat_prep<DIM><<<(unsigned)(npb + ds.lat.ntiles), LAT_PREP_THREADS, 0, st>>>(
-        c->y.p, c->nu.p, psi, a, lat_args(c, ds.lat), c->tblk_off.p, (int)c->ntblk, npb, tpack, S.top, S.shift,
+        c->y.p, c->nu.p, psi, io, c->perm.p, a, lat_args(c, ds.lat), c->tblk_off.p, (int)c->ntblk, npb, tpack, S.top, S.shift,
         S.step);
 }
 
@@ -1197,7 +1207,8 @@ static void launch_grad_dense(const sdot_ctx *c, const DenseShape &ds, bool fp32
 }
 
 template <int DIM>
-static sdot_status run_eval(sdot_ctx *c, const EvalArgs &a, bool dense, const double *pdir, double tol, bool partial)
+static sdot_status run_eval(sdot_ctx *c, const EvalArgs &a, bool dense, const double *pdir, double tol, bool partial,
+                            const IoPtrs *gather, const IoPtrs *scatter)
 {
     cudaStream_t st = c->stream;
     const int prec = c->precision;
@@ -1213,9 +1224,8 @@ static sdot_status run_eval(sdot_ctx *c, const EvalArgs &a, bool dense, const do
         if (e == cudaSuccess) e = c->blkpart.alloc((size_t)4 * ds.nval);
         if (e != cudaSuccess) return cuda_error(c, e, "dense sweep partials");
     }
-    if (ds.lat.cap > 0) launch_lat_prep<DIM>(c, ds, c->psi.p, a, c->tpack.p, c->vpart.p, st);
-    else if (dense)
-        k_target_prep<DIM><<<grid_for(a.nt, 256), 256, 0, st>>>(a.nt, c->y.p, c->nu.p, c->psi.p, a, c->tpack.p);
+    if (ds.lat.cap > 0) launch_lat_prep<DIM>(c, ds, c->psi.p, gather, a, c->tpack.p, c->vpart.p, st);
+    else if (dense) launch_target_prep<DIM>(c, a, c->psi.p, gather, c->tpack.p);
     mark(1);
     int64_t nval = 0;
     int nks = 1;
@@ -1257,16 +1267,32 @@ static sdot_status run_eval(sdot_ctx *c, const EvalArgs &a, bool dense, const do
         if (s != SDOT_OK) return s;
     }
     if (dense) mark(3);
-    const int fb = launch_finalize_grad(a.nt, nks, c->gpart.p, c->nu.p, c->psi.p, pdir, tol, partial ? 0 : 1, c->grad.p,
-                                        c->redpart.p, st);
-    launch_finalize_scalars(st, fb, c->redpart.p, nval, c->blkpart.p, c->scal.p);
+    FinArgs f{};
+    f.nt = a.nt;
+    f.nks = nks;
+    f.gpart = c->gpart.p;
+    f.nu = c->nu.p;
+    f.psi = c->psi.p;
+    f.pdir = pdir;
+    f.tol = tol;
+    f.sub_nu = partial ? 0 : 1;
+    f.grad = c->grad.p;
+    f.io = scatter;
+    f.perm = c->perm.p;
+    f.nval = nval;
+    f.valpart = c->blkpart.p;
+    f.redpart = c->redpart.p;
+    f.ticket = c->ticket.p;
+    f.scal = c->scal.p;
+    f.scal_host = c->scal_host;
+    launch_finalize(f, st);
     mark(4);
     c->klaunch[1] += 1;
     if (dense && c->distance == 0) {
         c->klaunch[2] += 1;
         c->klaunch[3] += 1;
     }
-    c->klaunch[4] += 2;
+    c->klaunch[4] += 1;
     return cuda_error(c, cudaGetLastError(), "evaluate launch");
 }
 
@@ -1339,7 +1365,8 @@ sdot_status evaluate_internal(sdot_ctx *c, const double *p_dir, double comp_tol,
     return evaluate_complete(c, pend, ms_out);
 }
 
-sdot_status evaluate_enqueue(sdot_ctx *c, const double *p_dir, double comp_tol, bool partial, EvalPending &pend)
+sdot_status evaluate_enqueue(sdot_ctx *c, const double *p_dir, double comp_tol, bool partial, EvalPending &pend,
+                             const IoPtrs *io)
 {
     if (c->dim == 0 || c->nq == 0) return set_error(c, SDOT_ESTATE, "source measure not set");
     if (c->nt == 0) return set_error(c, SDOT_ESTATE, "target measure not set");
@@ -1351,23 +1378,31 @@ sdot_status evaluate_enqueue(sdot_ctx *c, const double *p_dir, double comp_tol, 
     const bool may_truncate = (p.threshold_type != SDOT_THRESH_POINTWISE) ||
                               (p.tau > 0 && (c->min_target_density > 0.0 ? c->min_target_density
                                                                           : c->nu_min) > 0);
+    if (io && !(*io == c->io_set)) {
+        const cudaError_t e = cudaMemcpyAsync(c->io_ptrs.p, io, sizeof *io, cudaMemcpyHostToDevice, c->stream);
+        if (e != cudaSuccess) return cuda_error(c, e, "caller arrays");
+        c->io_set = *io;
+    }
     cudaEventRecord(c->ev0, c->stream);
-    double mm[3] = {0, 0, 0};
-    auto launch_minmax = [&] {
+    const IoPtrs *gather = io ? c->io_ptrs.p : nullptr, *scatter = gather;  // of the evaluation's first and last kernel
+    if (may_truncate) {
         if (c->profiling) cudaEventRecord(c->pev[5], c->stream);
-        k_minmax<<<1, 1024, 0, c->stream>>>(c->psi.p, c->nt, c->scal.p + SC_MAXPSI);
+        const int64_t blocks = (c->nt + RANGE_THREADS * 4 - 1) / (RANGE_THREADS * 4);
+        k_psi_range<<<(unsigned)std::min<int64_t>(RANGE_BLOCKS, blocks), RANGE_THREADS, 0, c->stream>>>(
+            c->nt, io ? io->psi : nullptr, io ? c->perm.p : nullptr, c->psi.p, c->redpart.p, c->ticket.p + 1,
+            c->scal.p + SC_MAXPSI, c->scal_host + SC_MAXPSI);
+        static_assert(SC_MINPSI == SC_MAXPSI + 1 && SC_PSIBAD == SC_MAXPSI + 2, "range slots");
+        gather = nullptr;
         if (c->profiling) cudaEventRecord(c->pev[6], c->stream);
         c->klaunch[0] += 1;
-    };
-    if (may_truncate) {
-        launch_minmax();
-        cudaError_t e = cudaMemcpyAsync(mm, c->scal.p + SC_MAXPSI, 3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+        const cudaError_t e = cudaStreamSynchronize(c->stream);
         if (e != cudaSuccess) return cuda_error(c, e, "threshold readback");
-        if (mm[2] != 0.0) return set_error(c, SDOT_ENONFINITE, "non-finite potential");
-        c->scal_host[SC_MAXPSI] = mm[0];
-        c->scal_host[SC_MINPSI] = mm[1];
-        r = host_threshold(c, mm[0], mm[1]);
+        if (c->scal_host[SC_PSIBAD] != 0.0) return set_error(c, SDOT_ENONFINITE, "non-finite potential");
+        r = host_threshold(c, c->scal_host[SC_MAXPSI], c->scal_host[SC_MINPSI]);
+    } else if (io && c->distance != 0) {
+        const sdot_status s = launch_gather(c, c->psi.p, io->psi, c->nt);
+        if (s != SDOT_OK) return s;
+        gather = nullptr;
     }
     c->current_distance_threshold = r;
     const double sstar = sstar_of(r);
@@ -1396,15 +1431,10 @@ sdot_status evaluate_enqueue(sdot_ctx *c, const double *p_dir, double comp_tol, 
         // NaN threshold: the reference's predicate d <= NaN rejects everything
         a.sstar = NAN;
     }
-    // everything after the threshold, up to the copy of the scalars to the host
-    // (an untruncated evaluation needs no ψ range: k_minmax runs only for the threshold)
+    // everything after the threshold (an untruncated evaluation needs no ψ range)
     auto body = [&]() -> sdot_status {
-        const sdot_status s = (c->dim == 2) ? run_eval<2>(c, a, dense_ok, p_dir, comp_tol, partial)
-                                            : run_eval<3>(c, a, dense_ok, p_dir, comp_tol, partial);
-        if (s != SDOT_OK) return s;
-        const cudaError_t e = cudaMemcpyAsync(c->scal_host, c->scal.p, SC_COUNT * sizeof(double),
-                                              cudaMemcpyDeviceToHost, c->stream);
-        return e == cudaSuccess ? SDOT_OK : cuda_error(c, e, "evaluate");
+        return (c->dim == 2) ? run_eval<2>(c, a, dense_ok, p_dir, comp_tol, partial, gather, scatter)
+                             : run_eval<3>(c, a, dense_ok, p_dir, comp_tol, partial, gather, scatter);
     };
     // An untruncated euclidean evaluation has no host step between its
     // launches, so it runs as one CUDA graph once its launch key repeats.
@@ -1415,13 +1445,13 @@ sdot_status evaluate_enqueue(sdot_ctx *c, const double *p_dir, double comp_tol, 
         k.a = a;
         const void *ptrs[] = {c->psi.p, c->y.p, c->nu.p, c->x.p, c->rho.p, c->jxw.p, c->w.p, c->tpack.p,
                               c->vpart.p, c->Lq.p, c->blkpart.p, c->gpart.p, c->grad.p, c->redpart.p,
-                              c->scal.p, c->scal_host, p_dir};
+                              c->scal.p, c->scal_host, p_dir, c->io_ptrs.p, c->ticket.p};
         static_assert(sizeof(ptrs) <= sizeof(k.p), "key pointer slots");
         memcpy(k.p, ptrs, sizeof(ptrs));
         k.tol = comp_tol;
         k.misc[0] = c->dim;
         k.misc[1] = c->precision;
-        k.misc[2] = partial ? 1 : 0;
+        k.misc[2] = (partial ? 1 : 0) + (io ? 2 : 0);
         k.misc[3] = c->geometry_id;
         s = run_graphed(c, k, body);
     } else {
@@ -1503,7 +1533,8 @@ namespace sdot {
 constexpr size_t NOALLOC_BYTES = size_t(8) << 20;  // == SDOT_NOALLOC_SCRATCH_BYTES
 constexpr int NOALLOC_MAX_DEVICES = 64;
 
-static __device__ __align__(256) double g_noalloc_scratch[NOALLOC_BYTES / sizeof(double)];
+// (its last words are the finalize kernel's arrival counter: zero at load and between evaluations)
+static __device__ __align__(256) double g_noalloc_scratch[NOALLOC_BYTES / sizeof(double) + 32];
 
 static double *g_noalloc_ptr[NOALLOC_MAX_DEVICES] = {};
 static std::mutex g_noalloc_mu;
@@ -1558,13 +1589,13 @@ static sdot_status noalloc_scratch(sdot_ctx *c, double **out)
 }
 
 template <int DIM>
-static void noalloc_launch(sdot_ctx *c, const EvalArgs &a, double *S, const NoallocLayout &L)
+static void noalloc_launch(sdot_ctx *c, const EvalArgs &a, double *S, unsigned *ticket, const NoallocLayout &L)
 {
     cudaStream_t st = c->stream;
     double *psi = S + L.psi, *grad = S + L.grad, *tpack = S + L.tpack, *Lq = S + L.Lq, *gpart = S + L.gpart;
     double *blkpart = S + L.blkpart, *redpart = S + L.redpart, *scal = S + L.scal;
-    if (L.ds.lat.cap > 0) launch_lat_prep<DIM>(c, L.ds, psi, a, tpack, S + L.vpart, st);
-    else k_target_prep<DIM><<<grid_for(a.nt, 256), 256, 0, st>>>(a.nt, c->y.p, c->nu.p, psi, a, tpack);
+    if (L.ds.lat.cap > 0) launch_lat_prep<DIM>(c, L.ds, psi, nullptr, a, tpack, S + L.vpart, st);
+    else launch_target_prep<DIM>(c, a, psi, nullptr, tpack);
     if (L.ds.lat.cap > 0) {
         launch_lat_value<DIM>(c, L.ds, tpack, a, S + L.vpart, Lq, blkpart, st);
     } else if (L.ds.tm > 0) {
@@ -1584,9 +1615,23 @@ static void noalloc_launch(sdot_ctx *c, const EvalArgs &a, double *S, const Noal
     }
     if (L.ds.lat_grad) launch_lat_grad<DIM>(c, L.ds, tpack, a, S + L.vpart, gpart, st);
     else launch_grad_dense<DIM>(c, L.ds, c->precision != SDOT_PREC_FP64, Lq, tpack, psi, a, gpart, st);
-    const int fb = launch_finalize_grad(a.nt, L.nks, gpart, c->nu.p, psi, nullptr, c->prm.tolerance, 1, grad, redpart,
-                                        st);
-    launch_finalize_scalars(st, fb, redpart, L.nval, blkpart, scal);
+    FinArgs f{};
+    f.nt = a.nt;
+    f.nks = L.nks;
+    f.gpart = gpart;
+    f.nu = c->nu.p;
+    f.psi = psi;
+    f.tol = c->prm.tolerance;
+    f.sub_nu = 1;
+    f.grad = grad;
+    f.perm = c->perm.p;
+    f.nval = L.nval;
+    f.valpart = blkpart;
+    f.redpart = redpart;
+    f.ticket = ticket;
+    f.scal = scal;
+    f.scal_host = c->scal_host;
+    launch_finalize(f, st);
 }
 
 }  // namespace sdot
@@ -1648,18 +1693,16 @@ extern "C" sdot_status sdot_evaluate_device_noalloc(sdot_ctx *c, const double *p
     a.l2e_eps = LOG2E / p.epsilon;
 
     if ((s = launch_gather(c, S + L.psi, psi_dev, c->nt)) != SDOT_OK) return s;
-    if (c->dim == 2) noalloc_launch<2>(c, a, S, L);
-    else noalloc_launch<3>(c, a, S, L);
+    unsigned *ticket = reinterpret_cast<unsigned *>(S + NOALLOC_BYTES / sizeof(double));
+    if (c->dim == 2) noalloc_launch<2>(c, a, S, ticket, L);
+    else noalloc_launch<3>(c, a, S, ticket, L);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_error(c, e, "no-alloc evaluation launch");
     if ((s = launch_scatter(c, grad_dev, S + L.grad, c->nt)) != SDOT_OK) return s;
-    // k_finalize_scalars writes slots SC_VALUE .. SC_VALSRC except the psi range,
-    // the psi check and the threshold slots (the untruncated path needs none of
-    // them); those are set on the host below, so nothing an earlier call left in
-    // the shared array reaches the context.
-    e = cudaMemcpyAsync(c->scal_host, S + L.scal, (SC_VALSRC + 1) * sizeof(double), cudaMemcpyDeviceToHost,
-                        c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    // k_finalize writes slots SC_VALUE .. SC_VALSRC of the host's array except the
+    // psi range, the psi check and the threshold slots (the untruncated path needs
+    // none of them), which are set below.
+    e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_error(c, e, "no-alloc evaluation");
     c->scal_host[SC_MAXPSI] = NAN;
     c->scal_host[SC_MINPSI] = NAN;
@@ -1669,7 +1712,7 @@ extern "C" sdot_status sdot_evaluate_device_noalloc(sdot_ctx *c, const double *p
     c->klaunch[1] += 1;
     c->klaunch[2] += 1;
     c->klaunch[3] += 1;
-    c->klaunch[4] += 2;
+    c->klaunch[4] += 1;
     c->current_distance_threshold = DBL_MAX;
     c->scal_host[SC_R] = DBL_MAX;
     c->global_functional = c->scal_host[SC_VALUE];

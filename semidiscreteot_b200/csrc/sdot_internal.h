@@ -78,6 +78,9 @@ enum ScalarSlot {
     SC_NONFINITE = 14, // 1 if value or gradient not finite
     SC_PAIRS = 15,     // candidate pairs of the evaluation
     SC_VALSRC = 16,    // source part of J (before the linear term)
+    SC_STEP_GP = 17,   // g . p of an L-BFGS direction (host array only)
+    SC_STEP_SY = 18,   // s . y of the step before it (host array only)
+    SC_COVER = 19,     // covering radius (host array only)
     SC_COUNT = 20
 };
 
@@ -117,6 +120,15 @@ struct DevBuf {
         return e;
     }
     size_t bytes() const { return n * sizeof(T); }
+};
+
+// The caller's device arrays (caller order) of an evaluation: read and
+// written by its first and last kernel through device memory, so that a
+// captured evaluation serves any arrays.
+struct IoPtrs {
+    const double *psi = nullptr;
+    double *grad = nullptr;
+    bool operator==(const IoPtrs &o) const { return psi == o.psi && grad == o.grad; }
 };
 
 struct EvalPlan {
@@ -195,7 +207,11 @@ struct sdot_ctx {
     sdot::DevBuf<double> psi, grad, tpack, Lq, gpart, blkpart, scal, redpart;
     sdot::DevBuf<double> vpart;        // dense value sweep: per (target slice, point) largest exponent and sum
     sdot::DevBuf<double> io_a, io_b;   // caller-order staging
-    double *scal_host = nullptr;       // pinned, SC_COUNT doubles
+    double *scal_host = nullptr;       // pinned, SC_COUNT doubles, written by the kernels that compute them
+    sdot::DevBuf<sdot::IoPtrs> io_ptrs;  // the caller's arrays of the evaluation under way, as the kernels read them
+    sdot::IoPtrs io_set;               // what io_ptrs holds
+    sdot::DevBuf<double> cover;        // covering radius: the CTAs' maxima
+    sdot::DevBuf<unsigned> ticket;     // arrival counters of the kernels whose last CTA finishes (zero between launches)
 
     // ---- parameters and reference-like persistent state ----
     sdot_solver_params prm{};
@@ -264,15 +280,18 @@ sdot_status evaluate_internal(sdot_ctx *c, const double *p_dir, double comp_tol,
                               double *ms_out, bool partial = false);
 // The same in two halves, so that a caller can queue more work (the
 // gradient's scatter, its copy to the host) before the one wait for the
-// stream: evaluate_enqueue queues the evaluation and the copy of its scalars
-// to c->scal_host; after the caller has synchronised c->stream,
+// stream: evaluate_enqueue queues the evaluation, whose last kernel writes
+// its scalars to c->scal_host; after the caller has synchronised c->stream,
 // evaluate_complete reads them (and the timing events) and updates the state.
+// With io, the potential is taken from io->psi and the gradient also written
+// to io->grad (device, caller order); without, from and to c->psi and c->grad.
 struct EvalPending {
     double r = 0.0;
     bool dense = false;
     bool ranged = false;   // the ψ range was computed (for the threshold)
 };
-sdot_status evaluate_enqueue(sdot_ctx *c, const double *p_dir, double comp_tol, bool partial, EvalPending &pend);
+sdot_status evaluate_enqueue(sdot_ctx *c, const double *p_dir, double comp_tol, bool partial, EvalPending &pend,
+                             const IoPtrs *io = nullptr);
 sdot_status evaluate_complete(sdot_ctx *c, const EvalPending &pend, double *ms_out);
 
 // Threshold for the current psi (host computation mirroring
@@ -284,7 +303,6 @@ double sstar_of(double r);
 
 sdot_status launch_gather(sdot_ctx *c, double *dst, const double *src, int64_t n);
 sdot_status launch_scatter(sdot_ctx *c, double *dst, const double *src, int64_t n);
-sdot_status launch_minmax(sdot_ctx *c, const double *v, int64_t n, double *mx, double *mn);
 
 struct EvalArgs;
 // truncated evaluation (block-pair lists, fused sweeps, partial reduction)
@@ -307,6 +325,7 @@ int64_t hessian_tc_tiles(int64_t n);
 sdot_status hessian_device(sdot_ctx *c, const double *psi_dev, void *H_dev, int method, int out_f32,
                            sdot_hessian_info *info);
 sdot_status ensure_eval_buffers(sdot_ctx *c);
+sdot_status ensure_tickets(sdot_ctx *c);  // c->ticket
 // Gradient partials (doubles) of an untruncated evaluation at the current parameters (0 where it truncates).
 size_t dense_gpart_need(const sdot_ctx *c);
 // VerboseSolverControl::check on the last evaluation's scalars: 1 converged,

@@ -160,10 +160,9 @@ __device__ __forceinline__ void lat_run(double f, double r, double r2, double r4
 // Shift of tile t over all targets by one CTA: shift[2 t] = M = max_j B0_j,
 // shift[2 t + 1] the largest magnitude of a term of an exponent, for the
 // rounding of the bounds in lat_merge_block.
-template <int DIM, int NTH>
+template <int DIM, int NTH, class Psi>
 __device__ __forceinline__ void lat_shift_block(const LatArgs &L, const EvalArgs &a, int t,
-                                                const double *__restrict__ y, const double *__restrict__ psi,
-                                                double *__restrict__ shift)
+                                                const double *__restrict__ y, Psi &&psi, double *__restrict__ shift)
 {
     __shared__ double red[2][NTH / 32];
     LatBox<DIM> B;
@@ -171,7 +170,7 @@ __device__ __forceinline__ void lat_shift_block(const LatArgs &L, const EvalArgs
     double M = -CUDART_INF, mag = 0.0;
 #pragma unroll 4
     for (int64_t j = threadIdx.x; j < a.nt; j += NTH) {
-        const double sp = a.s * psi[j];
+        const double sp = a.s * psi(j);
         double ysq = 0.0, b0 = sp, am = fabs(sp);
 #pragma unroll
         for (int d = 0; d < DIM; ++d) {
