@@ -140,8 +140,8 @@ size_t device_bytes(const sdot_ctx *c)
     return c->x.bytes() + c->rho.bytes() + c->jxw.bytes() + c->w.bytes() + c->cell_ctr.bytes() +
            c->sblk_sph.bytes() + c->sblk_sph32.bytes() + c->sblk_cell.bytes() + c->tblk_off.bytes() +
            c->lat_buf.bytes() +
-           c->tblk_sph32.bytes() + c->part.bytes() + c->fwd_t.bytes() + c->pmask.bytes() + c->pmpre.bytes() +
-           c->inv_b.bytes() + c->fwd2inv.bytes() + c->inv_tmpb.bytes() + c->inv_tmpk.bytes() + c->inv_off.bytes() +
+           c->tblk_sph32.bytes() + c->part.bytes() + c->fwd_t.bytes() + c->pmask.bytes() +
+           c->inv_b.bytes() + c->inv_k.bytes() + c->inv_tmpb.bytes() + c->inv_tmpk.bytes() + c->inv_off.bytes() +
            c->y.bytes() + c->nu.bytes() + c->perm.bytes() +
            c->tblk_sph.bytes() + c->psi.bytes() + c->grad.bytes() + c->tpack.bytes() + c->Lq.bytes() +
            c->gpart.bytes() + c->blkpart.bytes() + c->scal.bytes() + c->redpart.bytes() + c->vpart.bytes() +
@@ -404,7 +404,13 @@ sdot_status sdot_create(sdot_ctx **out, const sdot_options *opts)
         return e != cudaSuccess ? SDOT_ECUDA : SDOT_EINVAL;
     }
     DeviceGuard g(c->device);
+    int least = 0, greatest = 0;
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
+        // the highest priority: its small kernels take the slots that the sweeps' CTAs free
+        cudaDeviceGetStreamPriorityRange(&least, &greatest) != cudaSuccess ||
+        cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, greatest) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->join, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
         cudaMallocHost(&c->scal_host, SC_COUNT * sizeof(double)) != cudaSuccess) {
         sdot_destroy(c);
@@ -428,13 +434,14 @@ void sdot_destroy(sdot_ctx *c)
     {
         DeviceGuard g(c->device);
         if (c->stream) cudaStreamSynchronize(c->stream);
+        if (c->side) cudaStreamSynchronize(c->side);
         c->x.release(); c->rho.release(); c->jxw.release(); c->w.release();
         c->cell_ctr.release(); c->sblk_sph.release(); c->sblk_sph32.release(); c->sblk_cell.release();
         c->tblk_off.release(); c->tblk_sph32.release(); c->part.release(); c->fwd_t.release();
-        c->fwd_cnt.release(); c->fwd_off.release(); c->shit.release(); c->spidx.release(); c->scount.release();
-        c->inv_cnt.release(); c->inv_off.release(); c->inv_b.release(); c->fwd2inv.release();
+        c->fwd_cnt.release(); c->fwd_off.release(); c->shit.release(); c->scount.release();
+        c->inv_cnt.release(); c->inv_off.release(); c->inv_b.release(); c->inv_k.release();
         c->inv_tmpb.release(); c->inv_tmpk.release();
-        c->pmask.release(); c->pmpre.release(); c->superpair.release(); c->ssup_sph32.release(); c->tsup_sph32.release();
+        c->pmask.release(); c->superpair.release(); c->ssup_sph32.release(); c->tsup_sph32.release();
         c->y.release(); c->nu.release();
         c->perm.release(); c->tblk_sph.release(); c->psi.release(); c->grad.release(); c->tpack.release();
         c->Lq.release(); c->gpart.release(); c->blkpart.release(); c->scal.release(); c->redpart.release();
@@ -446,6 +453,9 @@ void sdot_destroy(sdot_ctx *c)
         if (c->dg_exec) cudaGraphExecDestroy(c->dg_exec);
         for (int i = 0; i < 8; ++i)
             if (c->pev[i]) cudaEventDestroy(c->pev[i]);
+        if (c->side) cudaStreamDestroy(c->side);
+        if (c->fork) cudaEventDestroy(c->fork);
+        if (c->join) cudaEventDestroy(c->join);
         if (c->ev0) cudaEventDestroy(c->ev0);
         if (c->ev1) cudaEventDestroy(c->ev1);
         if (c->stream) cudaStreamDestroy(c->stream);

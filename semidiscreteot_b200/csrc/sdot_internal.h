@@ -80,7 +80,7 @@ enum ScalarSlot {
     SC_VALSRC = 16,    // source part of J (before the linear term)
     SC_STEP_GP = 17,   // g . p of an L-BFGS direction (host array only)
     SC_STEP_SY = 18,   // s . y of the step before it (host array only)
-    SC_COVER = 19,     // covering radius (host array only)
+    SC_COVER = 19,     // covering radius; block pairs of a truncated evaluation (host array only)
     SC_COUNT = 20
 };
 
@@ -142,6 +142,8 @@ struct EvalPlan {
 struct sdot_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
+    cudaStream_t side = nullptr;       // beside stream within a truncated evaluation (inverse pair lists)
+    cudaEvent_t fork = nullptr, join = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int precision = SDOT_PREC_HYBRID;
     size_t budget = 0;
@@ -194,8 +196,8 @@ struct sdot_ctx {
     int64_t geometry_id = 0;           // counts the measures set: part of the evaluation graph's key
 
     // ---- truncated path: block-pair lists and gradient partials ----
-    sdot::DevBuf<int64_t> fwd_cnt, fwd_off, inv_cnt, inv_off, fwd2inv;
-    sdot::DevBuf<int> fwd_t, inv_b, shit, spidx, scount, pmpre, inv_tmpb;
+    sdot::DevBuf<int64_t> fwd_cnt, fwd_off, inv_cnt, inv_off, inv_k;
+    sdot::DevBuf<int> fwd_t, inv_b, shit, scount, inv_tmpb;
     sdot::DevBuf<int64_t> inv_tmpk;    // inverse-list scatter (forward position per entry)
     sdot::DevBuf<unsigned> pmask;
     sdot::DevBuf<unsigned char> superpair;

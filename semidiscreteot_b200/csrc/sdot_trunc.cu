@@ -13,9 +13,9 @@
 // Per evaluation:
 //   1. block-pair lists.  (b, t) is a pair iff dist(c_b, c_t) <= r + R_b + R_t
 //      (FP32, conservatively enlarged).  The forward list (per b, t ascending)
-//      and the inverse list (per t, b ascending) are built by count / scan /
-//      fill kernels that evaluate the identical expression, so they hold the
-//      same pairs.
+//      is filled from masks; the inverse list (per t, b ascending, with the
+//      pairs' forward positions) is its transpose, built on a second stream
+//      beside step 2, which does not need it.
 //   2. k_fused (CTA <-> source block, warp <-> unit):
 //      staging: the targets of the block's pairs, culled per target against
 //        the block sphere (|y - c_b| <= r + R_b), compacted in order;
@@ -33,8 +33,8 @@
 //        small, into the warp's partial row (FP32 rows in the hybrid mode,
 //        FP64 rows in the FP64 mode); the rows are added in warp order in
 //        FP64.  The block's partial for each target of each pair is written
-//        to a slot of the pair in the inverse list order.
-//   3. k_grad_reduce (warp <-> target block): sum of the partials over the
+//        to the pair's forward position.
+//   3. k_grad_reduce (CTA <-> target block): sum of the partials over the
 //      pairs in ascending source-block order, lane <-> target.  No atomics;
 //      the summation order is fixed, results are bitwise reproducible.
 #include <float.h>
@@ -73,15 +73,13 @@ struct FusedArgs {
     const int64_t *tblk_off;     // target block -> first target (ntblk + 1)
     const int64_t *fwd_off;
     const int *fwd_t;
-    const int64_t *fwd2inv;      // inverse position of each forward pair
-    double *part;                // partials, 32 per pair, at inverse positions minus part_base (FP64 sweeps)
+    double *part;                // partials, 32 per pair, at forward positions minus part_base (FP64 sweeps)
     float *part32;               // the same in FP32 (hybrid sweeps: their rows are FP32 already)
     double *Lq;                  // per q (written by the value sweep)
     double *valpart;             // per source block: value, C, skipped, pairs
-    int do_a, do_b;
     int w_nonneg;                // all w_q >= 0: log2 w_q folded into the FP32 exponent
-    int tlo, thi;                // gradient partials only for target blocks [tlo, thi)
-    int64_t part_base;           // inverse position of the first pair of tlo
+    int b0;                      // first source block of the launch
+    int64_t part_base;           // forward position of its first pair
     double cullt;                // per-target cull radius addend (r, enlarged)
 };
 
@@ -100,15 +98,12 @@ struct FTSmem {
     float pvw[FT_WARPS][CAP];     // gradient partial of each unit (warp) per staged target (FP32 mode)
     unsigned short cand[FT_WARPS][CAP];
     short smap[FT_MAXT][TBLK_KD]; // (chunk target block, slot) -> staged position or -1
-    int ctb[FT_MAXT];             // target blocks of the chunk
-    int64_t cpos[FT_MAXT];        // their partial base index
     int ecnt[32];                 // survivors per examined forward entry (-1: none)
     int epre[32];                 // staged position of the first survivor of each accepted entry
     int eacc, etot;
     int wcount[FT_WARPS];
     int nstg;
-    int ent_t[FT_PREF];            // forward entries of the block: target block,
-    int ent_j0[FT_PREF];           // its first target
+    int ent_j0[FT_PREF];           // forward entries of the block: the target block's first target
     unsigned char ent_sz[FT_PREF]; // and its size (prefetched once per block)
 };
 
@@ -155,11 +150,10 @@ k_super_pairs(const float4 *__restrict__ ssph, int nss, const float4 *__restrict
 }
 
 // Warp <-> source super-block: its paired target super-blocks in ascending
-// order (shit[si * nts + h]), their count, and the inverse map
-// spidx[si * nts + ti] = h (or -1).
+// order (shit[si * nts + h]) and their count.
 __global__ void __launch_bounds__(256)
 k_super_compact(const unsigned char *__restrict__ sp, int nss, int nts, int *__restrict__ shit,
-                int *__restrict__ scount, int *__restrict__ spidx)
+                int *__restrict__ scount)
 {
     const int si = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
@@ -170,7 +164,6 @@ k_super_compact(const unsigned char *__restrict__ sp, int nss, int nts, int *__r
         const bool on = ti < nts && sp[(int64_t)si * nts + ti];
         const unsigned bal = __ballot_sync(0xffffffffu, on);
         const int pos = h + __popc(bal & ((1u << lane) - 1u));
-        if (ti < nts) spidx[(int64_t)si * nts + ti] = on ? pos : -1;
         if (on) shit[(int64_t)si * nts + pos] = ti;
         h += __popc(bal);
     }
@@ -178,13 +171,11 @@ k_super_compact(const unsigned char *__restrict__ sp, int nss, int nts, int *__r
 }
 
 // Warp <-> source block b: for each paired target super-block h, the 32-bit
-// mask of its target blocks t with pair_test(b, t), and the number of b's
-// pairs before it; cnt[b] = total.  Pairs are ordered by t, so the forward
-// position of (b, t) is fwd_off[b] + mpre[b, h] + popc(mask[b, h] below t).
+// mask of its target blocks t with pair_test(b, t); cnt[b] = total.
 __global__ void __launch_bounds__(256)
 k_fwd_masks(const float4 *__restrict__ sph, int nsb, const float4 *__restrict__ tph, int ntb, int nts, int hmax,
             float cr, const int *__restrict__ shit, const int *__restrict__ scount, unsigned *__restrict__ mask,
-            int *__restrict__ mpre, int64_t *__restrict__ cnt)
+            int64_t *__restrict__ cnt)
 {
     const int b = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
@@ -197,16 +188,15 @@ k_fwd_masks(const float4 *__restrict__ sph, int nsb, const float4 *__restrict__ 
         const int t = shit[(int64_t)si * nts + h] * SUPER + lane;
         const bool hit = t < ntb && pair_test(me, tph[t], cr);
         const unsigned bal = __ballot_sync(0xffffffffu, hit);
-        if (lane == 0) {
-            mask[(int64_t)b * hmax + h] = bal;
-            mpre[(int64_t)b * hmax + h] = k;
-        }
+        if (lane == 0) mask[(int64_t)b * hmax + h] = bal;
         k += __popc(bal);
     }
     if (lane == 0) cnt[b] = k;
 }
 
 // Forward lists from the masks: fwd_t[fwd_off[b] ..] = paired t, ascending.
+// Inverse lists are the forward lists transposed (the same pair set by
+// construction).
 __global__ void __launch_bounds__(256)
 k_fwd_fill(int nsb, int nts, int hmax, const int *__restrict__ shit, const int *__restrict__ scount,
            const unsigned *__restrict__ mask, const int64_t *__restrict__ fwd_off, int *__restrict__ fwd_t)
@@ -224,9 +214,8 @@ k_fwd_fill(int nsb, int nts, int hmax, const int *__restrict__ shit, const int *
     }
 }
 
-// Inverse lists by transposing the forward lists (the same pair set by
-// construction).  Warp <-> source block b, lanes over its forward entries:
-// count the pairs of each target block (integer atomics, exact totals).
+// Warp <-> source block b, lanes over its forward entries: count the pairs of
+// each target block (integer atomics, exact totals).
 __global__ void __launch_bounds__(256)
 k_inv_count(int nsb, const int64_t *__restrict__ fwd_off, const int *__restrict__ fwd_t,
             unsigned long long *__restrict__ cnt)
@@ -264,12 +253,12 @@ k_inv_scatter(int nsb, const int64_t *__restrict__ fwd_off, const int *__restric
 // segments: the rank of each entry = the number of entries with a smaller b,
 // counted against INV_TILE-entry tiles.  Every way, inv_b[off + rank] = b
 // (ascending b, the order the gradient reduction sums in) and
-// fwd2inv[k] = off + rank.
+// inv_k[off + rank] = the pair's forward position.
 constexpr int INV_TILE = 2048;
 constexpr int INV_PER = INV_TILE / 256;
 __global__ void __launch_bounds__(256)
 k_inv_order(int nsb, const int64_t *__restrict__ inv_off, const int *__restrict__ tmp_b,
-            const int64_t *__restrict__ tmp_k, int *__restrict__ inv_b, int64_t *__restrict__ fwd2inv)
+            const int64_t *__restrict__ tmp_k, int *__restrict__ inv_b, int64_t *__restrict__ inv_k)
 {
     __shared__ int sb[INV_TILE];
     __shared__ short si[INV_TILE];
@@ -315,7 +304,7 @@ k_inv_order(int nsb, const int64_t *__restrict__ inv_off, const int *__restrict_
             const int b = tmp_b[off + i];
             const int r = pre[b >> 5] + __popc(bm[b >> 5] & ((1u << (b & 31)) - 1u));
             inv_b[off + r] = b;
-            fwd2inv[tmp_k[off + i]] = off + r;
+            inv_k[off + r] = tmp_k[off + i];
         }
         return;
     }
@@ -347,7 +336,7 @@ k_inv_order(int nsb, const int64_t *__restrict__ inv_off, const int *__restrict_
         }
         for (int i = tid; i < L; i += 256) {
             inv_b[off + i] = sb[i];
-            fwd2inv[tmp_k[off + si[i]]] = off + i;
+            inv_k[off + i] = tmp_k[off + si[i]];
         }
         return;
     }
@@ -375,14 +364,16 @@ k_inv_order(int nsb, const int64_t *__restrict__ inv_off, const int *__restrict_
             const int64_t i = i0 + tid + 256 * u;
             if (i < L) {
                 inv_b[off + rank[u]] = mine[u];
-                fwd2inv[tmp_k[off + i]] = off + rank[u];
+                inv_k[off + rank[u]] = tmp_k[off + i];
             }
         }
     }
 }
 
 // exclusive scan of n counts into off[0..n] (single CTA, order-fixed)
-__global__ void __launch_bounds__(1024) k_scan(const int64_t *__restrict__ cnt, int64_t n, int64_t *__restrict__ off)
+// total_host (may be null): the total, for the host
+__global__ void __launch_bounds__(1024)
+k_scan(const int64_t *__restrict__ cnt, int64_t n, int64_t *__restrict__ off, double *__restrict__ total_host)
 {
     // passes of 1,024 x SP counts: each thread loads SP consecutive counts at
     // once (the CTA is bound by load latency), the thread sums are scanned by
@@ -426,7 +417,10 @@ __global__ void __launch_bounds__(1024) k_scan(const int64_t *__restrict__ cnt, 
         carry += wsum[31];
         __syncthreads();  // wsum is rewritten by the next pass
     }
-    if (tid == 0) off[n] = (int64_t)carry;
+    if (tid == 0) {
+        off[n] = (int64_t)carry;
+        if (total_host) *total_host = (double)carry;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -440,7 +434,7 @@ __global__ void __launch_bounds__(1024) k_scan(const int64_t *__restrict__ cnt, 
 // number of forward entries consumed; staged order = (target block, slot).
 template <int DIM, class SM>
 __device__ int stage_chunk(SM &sm, const FusedArgs &f, int64_t kb, int64_t k0, int64_t k1, const double *bc,
-                           double rcull2, bool for_b)
+                           double rcull2)
 {
     constexpr int SUB = 4;                       // target blocks per warp per iteration
     constexpr int PER = FT_WARPS * SUB;          // entries examined per iteration
@@ -449,29 +443,25 @@ __device__ int stage_chunk(SM &sm, const FusedArgs &f, int64_t kb, int64_t k0, i
     int64_t k = k0;
     while (k < k1 && nb < FT_MAXT) {
         unsigned bal[SUB];
-        int tt[SUB];
         int64_t jj[SUB];
 #pragma unroll
         for (int s = 0; s < SUB; ++s) {
             const int idx = s * FT_WARPS + wp;
             const int64_t e = k + idx;
             bal[s] = 0u;
-            tt[s] = -1;
             jj[s] = 0;
             int cntv = -1;
             if (e < k1 && nb + idx < FT_MAXT) {
-                int t, sz;
+                int sz;
                 int64_t j0;
                 if (e - kb < FT_PREF) {
-                    t = sm.ent_t[e - kb];
                     j0 = sm.ent_j0[e - kb];
                     sz = sm.ent_sz[e - kb];
                 } else {
-                    t = f.fwd_t[e];
+                    const int t = f.fwd_t[e];
                     j0 = f.tblk_off[t];
                     sz = (int)(f.tblk_off[t + 1] - j0);
                 }
-                tt[s] = t;
                 jj[s] = j0;
                 bool keep = false;
                 if (lane < sz) {
@@ -528,13 +518,6 @@ __device__ int stage_chunk(SM &sm, const FusedArgs &f, int64_t kb, int64_t k0, i
                     for (int d = 0; d < FT_TS; ++d) sm.stg[d][pos] = tp[d];
                 }
                 sm.smap[slot][lane] = pos;
-                if (lane == 0) {
-                    const int tb = tt[s];
-                    sm.ctb[slot] = tb;
-                    const int64_t ip = f.fwd2inv[k + idx];
-                    sm.cpos[slot] = (for_b && ip >= 0 && tb >= f.tlo && tb < f.thi) ? (ip - f.part_base) * TBLK_KD
-                                                                                    : (int64_t)-1;
-                }
             }
         }
         total = run;
@@ -895,16 +878,16 @@ __device__ __forceinline__ void grad_pairs_tensor(SM &sm, int wp, int lane, int 
 }
 
 // CTA sum of the warp partial rows (warp order) and the write of every slot
-// of every pair of the chunk (zeros where a target was not staged).
+// of every pair of the chunk, forward positions k.. (zeros where a target was
+// not staged).
 template <bool FP32B, class SM>
-__device__ __forceinline__ void write_partials(SM &sm, const FusedArgs &f, int nt, int nunit)
+__device__ __forceinline__ void write_partials(SM &sm, const FusedArgs &f, int64_t k, int nt, int nunit)
 {
     const typename PRow<FP32B>::T *rows = partial_rows<FP32B>(sm);
     const int tid = threadIdx.x;
     for (int i = tid; i < nt * TBLK_KD; i += blockDim.x) {
         const int ti = i / TBLK_KD, sl = i - ti * TBLK_KD;
-        const int64_t base = sm.cpos[ti];
-        if (base < 0) continue;
+        const int64_t base = (k + ti - f.part_base) * TBLK_KD;
         const short p = sm.smap[ti][sl];
         double v = 0.0;
         if (p >= 0)
@@ -922,7 +905,7 @@ k_fused(FusedArgs f, EvalArgs a)
     using SMem = FTSmem<fused_cap(DIM, TQ, FP32B)>;
     SMem &sm = *reinterpret_cast<SMem *>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
-    const int b = blockIdx.x;
+    const int b = f.b0 + blockIdx.x;
     if (tid < 16) sm.tab[tid] = c_exp2_tab[tid];
     const int64_t cb0 = f.sblk_cell[b], cb1 = f.sblk_cell[b + 1];
     const int ncell = (int)(cb1 - cb0);
@@ -946,7 +929,6 @@ k_fused(FusedArgs f, EvalArgs a)
     for (int i = tid; i < (int)min((int64_t)FT_PREF, k1 - k0); i += blockDim.x) {
         const int t = f.fwd_t[k0 + i];
         const int64_t j0 = f.tblk_off[t];
-        sm.ent_t[i] = t;
         sm.ent_j0[i] = (int)j0;
         sm.ent_sz[i] = (unsigned char)(f.tblk_off[t + 1] - j0);
     }
@@ -970,7 +952,7 @@ k_fused(FusedArgs f, EvalArgs a)
     int ncand_single = 0;
 
     // ---------------- value sweep ----------------
-    if (f.do_a) {
+    {
         // Shift of the online sums.  MODE 0/1: Munit = max_j B0_Kj + s r
         // max_q |delta_q| bounds every exponent of the unit from above
         // (|G_Kj| <= s r for a candidate), so no per-pair rescale is needed;
@@ -988,7 +970,7 @@ k_fused(FusedArgs f, EvalArgs a)
         double bmax_run = -CUDART_INF;  // largest B0 of the candidates so far
         const double sr = a.s * a.cull;
         for (int64_t k = k0; k < k1;) {
-            const int nt = stage_chunk<DIM>(sm, f, k0, k, k1, bc, rcull2, f.do_b != 0);
+            const int nt = stage_chunk<DIM>(sm, f, k0, k, k1, bc, rcull2);
             const int nstg = sm.nstg;
             if (valid) {
                 double bmax;
@@ -1093,12 +1075,8 @@ k_fused(FusedArgs f, EvalArgs a)
             tcv = cv;
             tsk = sk;
         }
-        block_partials(tv, tcv, tsk, lane == 0 ? npairs : 0.0, f.valpart);  // contains __syncthreads
-    } else {
-        for (int i = tid; i < nqb; i += blockDim.x) sm.qL[i] = f.Lq[qblk0 + i];
-        __syncthreads();
+        block_partials_at(tv, tcv, tsk, lane == 0 ? npairs : 0.0, f.valpart + (int64_t)b * 4);  // contains __syncthreads
     }
-    if (!f.do_b) return;
 
     // ---------------- gradient sweep ----------------
     // per-unit reference L_Kref = min L over the unit's q; per-q FP32 data
@@ -1138,19 +1116,14 @@ k_fused(FusedArgs f, EvalArgs a)
                 else grad_pairs<DIM, FP32B>(sm, f, wp, lane, ncand_single, qoff, nql, cc, Lref, qblk0, a);
             }
         }
-        if (tid < nt) {
-            const int tb = sm.ctb[tid];
-            const int64_t ip = f.fwd2inv[k0 + tail_off + tid];
-            sm.cpos[tid] = (ip >= 0 && tb >= f.tlo && tb < f.thi) ? (ip - f.part_base) * TBLK_KD : (int64_t)-1;
-        }
         __syncthreads();
-        write_partials<FP32B>(sm, f, nt, nunit);
+        write_partials<FP32B>(sm, f, k0 + tail_off, nt, nunit);
         if (tail_off == 0) return;
         kend = k0 + tail_off;
         __syncthreads();  // the earlier chunks overwrite the staged targets
     }
     for (int64_t k = k0; k < kend;) {
-        const int nt = stage_chunk<DIM>(sm, f, k0, k, kend, bc, rcull2, true);
+        const int nt = stage_chunk<DIM>(sm, f, k0, k, kend, bc, rcull2);
         const int nstg = sm.nstg;
         if (valid) {
             double bmax;
@@ -1163,7 +1136,7 @@ k_fused(FusedArgs f, EvalArgs a)
             }
         }
         __syncthreads();
-        write_partials<FP32B>(sm, f, nt, nunit);
+        write_partials<FP32B>(sm, f, k, nt, nunit);
         k += nt;
         __syncthreads();
     }
@@ -1171,18 +1144,51 @@ k_fused(FusedArgs f, EvalArgs a)
 
 // gradient of target block t = sum of its pair partials in inverse order
 // (ascending source block), lane <-> target.  CTA <-> target block: warp w
-// sums rows w, w+8, ...; the 8 warp sums are added in warp order.
+// sums entries w, w + 8, ... (the positions of 32 of them fetched at once,
+// eight partials in flight: with a position fetched per partial it took 316 us
+// for 2.8 million pairs); the 8 warp sums are added in warp order.  Of the pairs at forward positions [k0, k1) only (one
+// launch's source blocks; a target's positions ascend), added to gacc after
+// the first launch.
 template <typename PT>
 __global__ void __launch_bounds__(256)
-k_grad_reduce(const int64_t *__restrict__ tblk_off, const int64_t *__restrict__ inv_off, int tlo, int thi,
-              int64_t part_base, const PT *__restrict__ part, double *__restrict__ gacc)
+k_grad_reduce(const int64_t *__restrict__ tblk_off, const int64_t *__restrict__ inv_off,
+              const int64_t *__restrict__ inv_k, int64_t k0, int64_t k1, int add, const PT *__restrict__ part,
+              double *__restrict__ gacc)
 {
     __shared__ double ws[8][32];
-    const int t = tlo + blockIdx.x;
+    const int t = blockIdx.x;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int64_t p0 = inv_off[t], p1 = inv_off[t + 1];
+    int64_t p0 = inv_off[t], p1 = inv_off[t + 1];
+    if (add || (p1 > p0 && inv_k[p1 - 1] >= k1)) {  // a part of the list: binary searches for its ends
+        auto first = [&](int64_t k) {
+            int64_t lo = p0, hi = p1;
+            while (lo < hi) {
+                const int64_t m = (lo + hi) >> 1;
+                if (inv_k[m] < k) lo = m + 1;
+                else hi = m;
+            }
+            return lo;
+        };
+        const int64_t a = first(k0), b = first(k1);
+        p0 = a;
+        p1 = b;
+    }
     double acc = 0.0;
-    for (int64_t p = p0 + w; p < p1; p += 8) acc += (double)part[(p - part_base) * TBLK_KD + lane];
+    for (int64_t p = p0 + w; p < p1; p += 256) {
+        const int64_t mine = p + 8 * lane < p1 ? inv_k[p + 8 * lane] - k0 : 0;
+        const int n = (int)min((int64_t)32, (p1 - p + 7) / 8);
+        for (int u0 = 0; u0 < n; u0 += 8) {
+            PT v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int64_t k = __shfl_sync(0xffffffffu, mine, u0 + u);
+                v[u] = u0 + u < n ? part[k * TBLK_KD + lane] : PT(0);
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (u0 + u < n) acc += (double)v[u];
+        }
+    }
     ws[w][lane] = acc;
     __syncthreads();
     if (w == 0) {
@@ -1190,7 +1196,7 @@ k_grad_reduce(const int64_t *__restrict__ tblk_off, const int64_t *__restrict__ 
 #pragma unroll
         for (int i = 0; i < 8; ++i) s += ws[i][lane];
         const int64_t j = tblk_off[t] + lane;
-        if (j < tblk_off[t + 1]) gacc[j] = s;
+        if (j < tblk_off[t + 1]) gacc[j] = add ? gacc[j] + s : s;
     }
 }
 
@@ -1288,19 +1294,18 @@ sdot_status run_trunc(sdot_ctx *c, const EvalArgs &a, double r)
     if (e == cudaSuccess) e = c->fwd_off.alloc(nsb + 1);
     if (e == cudaSuccess) e = c->superpair.alloc((size_t)nss * nts);
     if (e == cudaSuccess) e = c->shit.alloc((size_t)nss * nts);
-    if (e == cudaSuccess) e = c->spidx.alloc((size_t)nss * nts);
     if (e == cudaSuccess) e = c->scount.alloc(nss + 1);
     if (e != cudaSuccess) return cuda_error(c, e, "pair list alloc");
     k_super_pairs<<<(unsigned)(((int64_t)nss * nts + 255) / 256), 256, 0, st>>>(c->ssup_sph32.p, nss, c->tsup_sph32.p,
                                                                              nts, cr, c->superpair.p);
     k_super_compact<<<(unsigned)(((int64_t)nss * 32 + 255) / 256), 256, 0, st>>>(c->superpair.p, nss, nts, c->shit.p,
-                                                                              c->scount.p, c->spidx.p);
+                                                                              c->scount.p);
     // Row length of the per-block pair masks: the most target super-blocks any
     // source super-block pairs with.  Every count is at most nts, so when the
-    // nts-wide rows are small (<= 128 MiB for both arrays) they are used as
+    // nts-wide rows are small (<= 64 MiB) they are used as
     // they are and the counts are not read back (one host round trip fewer).
     int hmax = std::max(1, nts);
-    if ((size_t)nsb * (size_t)nts * 2 * sizeof(int) > ((size_t)128 << 20)) {
+    if ((size_t)nsb * (size_t)nts * sizeof(int) > ((size_t)64 << 20)) {
         std::vector<int> sc((size_t)nss);
         e = cudaMemcpyAsync(sc.data(), c->scount.p, nss * sizeof(int), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -1309,67 +1314,73 @@ sdot_status run_trunc(sdot_ctx *c, const EvalArgs &a, double r)
         for (int v : sc) hmax = std::max(hmax, v);
     }
     e = c->pmask.alloc((size_t)nsb * hmax);
-    if (e == cudaSuccess) e = c->pmpre.alloc((size_t)nsb * hmax);
     if (e != cudaSuccess) return cuda_error(c, e, "pair mask alloc");
     const unsigned gw = (unsigned)(((int64_t)nsb * 32 + 255) / 256);
     k_fwd_masks<<<gw, 256, 0, st>>>(c->sblk_sph32.p, nsb, c->tblk_sph32.p, ntb, nts, hmax, cr, c->shit.p, c->scount.p,
-                                    c->pmask.p, c->pmpre.p, c->fwd_cnt.p);
-    k_scan<<<1, 1024, 0, st>>>(c->fwd_cnt.p, nsb, c->fwd_off.p);
-    int64_t npairs = 0;
-    e = cudaMemcpyAsync(&npairs, c->fwd_off.p + nsb, 8, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+                                    c->pmask.p, c->fwd_cnt.p);
+    k_scan<<<1, 1024, 0, st>>>(c->fwd_cnt.p, nsb, c->fwd_off.p, c->scal_host + SC_COVER);
+    e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_error(c, e, "pair list count");
+    const int64_t npairs = (int64_t)c->scal_host[SC_COVER];  // (a whole number below 2^53)
     e = c->fwd_t.alloc(npairs + 1);
     if (e == cudaSuccess) e = c->inv_b.alloc(npairs + 1);
-    if (e == cudaSuccess) e = c->fwd2inv.alloc(npairs + 1);
+    if (e == cudaSuccess) e = c->inv_k.alloc(npairs + 1);
     if (e == cudaSuccess) e = c->inv_tmpb.alloc(npairs + 1);
     if (e == cudaSuccess) e = c->inv_tmpk.alloc(npairs + 1);
-    if (e == cudaSuccess) e = c->inv_cnt.alloc(ntb + 1);
+    if (e == cudaSuccess) e = c->inv_cnt.alloc(2 * (size_t)(ntb + 1));
     if (e == cudaSuccess) e = c->inv_off.alloc(ntb + 1);
     if (e != cudaSuccess) return cuda_error(c, e, "pair list alloc");
     k_fwd_fill<<<gw, 256, 0, st>>>(nsb, nts, hmax, c->shit.p, c->scount.p, c->pmask.p, c->fwd_off.p, c->fwd_t.p);
-    unsigned long long *icnt = reinterpret_cast<unsigned long long *>(c->inv_cnt.p);
-    e = cudaMemsetAsync(c->inv_cnt.p, 0, (ntb + 1) * sizeof(int64_t), st);
-    if (e != cudaSuccess) return cuda_error(c, e, "pair list clear");
-    k_inv_count<<<gw, 256, 0, st>>>(nsb, c->fwd_off.p, c->fwd_t.p, icnt);
-    k_scan<<<1, 1024, 0, st>>>(c->inv_cnt.p, ntb, c->inv_off.p);
-    e = cudaMemsetAsync(c->inv_cnt.p, 0, (ntb + 1) * sizeof(int64_t), st);
-    if (e != cudaSuccess) return cuda_error(c, e, "pair list clear");
-    k_inv_scatter<<<gw, 256, 0, st>>>(nsb, c->fwd_off.p, c->fwd_t.p, c->inv_off.p, icnt, c->inv_tmpb.p, c->inv_tmpk.p);
-    k_inv_order<<<(unsigned)ntb, 256, 0, st>>>(nsb, c->inv_off.p, c->inv_tmpb.p, c->inv_tmpk.p, c->inv_b.p, c->fwd2inv.p);
     c->klaunch[6] += 9;
     if (c->profiling) cudaEventRecord(c->pev[7], st);
-    // 2. partial buffer (inverse order): all pairs at once under the cap, else target-block groups
-    // partials are FP32 in the hybrid mode (the sweeps' rows are FP32), FP64 otherwise
+    // 2. partial buffer (forward order): all pairs at once under the cap, else groups of source blocks.
+    // Partials are FP32 in the hybrid mode (the sweeps' rows are FP32), FP64 otherwise.
     const bool fp32b = c->precision != SDOT_PREC_FP64;
     const size_t pel = fp32b ? sizeof(float) : sizeof(double);
     const int64_t cap_pairs = std::max<int64_t>(1, (int64_t)(c->part_cap_bytes / (TBLK_KD * pel)));
-    std::vector<std::pair<int, int>> groups;
-    std::vector<int64_t> inv_host;
+    struct Group {
+        int b0, b1;
+        int64_t k0, k1;
+    };
+    std::vector<Group> groups;
     int64_t part_pairs = npairs;
     if (npairs <= cap_pairs) {
-        groups.push_back({0, ntb});
+        groups.push_back({0, nsb, 0, npairs});
     } else {
-        inv_host.resize((size_t)ntb + 1);
-        e = cudaMemcpyAsync(inv_host.data(), c->inv_off.p, (ntb + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, st);
+        std::vector<int64_t> off((size_t)nsb + 1);
+        e = cudaMemcpyAsync(off.data(), c->fwd_off.p, (nsb + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) return cuda_error(c, e, "pair list copy");
         part_pairs = 0;
-        int t0 = 0;
-        while (t0 < ntb) {
-            int t1 = t0 + 1;
-            while (t1 < ntb && inv_host[t1 + 1] - inv_host[t0] <= cap_pairs) ++t1;
-            groups.push_back({t0, t1});
-            part_pairs = std::max(part_pairs, inv_host[t1] - inv_host[t0]);
-            t0 = t1;
+        int b0 = 0;
+        while (b0 < nsb) {
+            int b1 = b0 + 1;
+            while (b1 < nsb && off[b1 + 1] - off[b0] <= cap_pairs) ++b1;
+            groups.push_back({b0, b1, off[b0], off[b1]});
+            part_pairs = std::max(part_pairs, off[b1] - off[b0]);
+            b0 = b1;
         }
     }
     e = c->part.alloc(((size_t)std::max<int64_t>(1, part_pairs) * TBLK_KD * pel + sizeof(double) - 1) / sizeof(double));
     if (e != cudaSuccess) return cuda_error(c, e, "partial buffer alloc");
+    // the inverse lists, on the second stream: k_fused needs the forward lists only
+    e = cudaEventRecord(c->fork, st);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(c->side, c->fork, 0);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->inv_cnt.p, 0, 2 * (ntb + 1) * sizeof(int64_t), c->side);
+    if (e != cudaSuccess) return cuda_error(c, e, "pair list fork");
+    unsigned long long *icnt = reinterpret_cast<unsigned long long *>(c->inv_cnt.p), *ifill = icnt + ntb + 1;
+    k_inv_count<<<gw, 256, 0, c->side>>>(nsb, c->fwd_off.p, c->fwd_t.p, icnt);
+    k_scan<<<1, 1024, 0, c->side>>>(c->inv_cnt.p, ntb, c->inv_off.p, nullptr);
+    k_inv_scatter<<<gw, 256, 0, c->side>>>(nsb, c->fwd_off.p, c->fwd_t.p, c->inv_off.p, ifill, c->inv_tmpb.p,
+                                           c->inv_tmpk.p);
+    k_inv_order<<<(unsigned)ntb, 256, 0, c->side>>>(nsb, c->inv_off.p, c->inv_tmpb.p, c->inv_tmpk.p, c->inv_b.p,
+                                                    c->inv_k.p);
+    e = cudaEventRecord(c->join, c->side);
+    if (e != cudaSuccess) return cuda_error(c, e, "pair list join");
     FusedArgs f{};
     f.x = c->x.p; f.rho = c->rho.p; f.jxw = c->jxw.p; f.w = c->w.p; f.cell_ctr = c->cell_ctr.p;
     f.tpk = c->tpack.p; f.sblk_cell = c->sblk_cell.p; f.sblk_sph = c->sblk_sph.p; f.tblk_off = c->tblk_off.p;
-    f.fwd_off = c->fwd_off.p; f.fwd_t = c->fwd_t.p; f.fwd2inv = c->fwd2inv.p;
+    f.fwd_off = c->fwd_off.p; f.fwd_t = c->fwd_t.p;
     f.part = c->part.p; f.part32 = reinterpret_cast<float *>(c->part.p); f.Lq = c->Lq.p; f.valpart = c->blkpart.p;
     f.cullt = std::isnan(r) ? 0.0 : std::min(r, 1e300);
     f.w_nonneg = c->w_nonneg ? 1 : 0;
@@ -1377,21 +1388,22 @@ sdot_status run_trunc(sdot_ctx *c, const EvalArgs &a, double r)
     const double prange = std::isfinite(prange0) ? prange0 : 1e300;
     const int tmode = fused_tensor_mode(c, a, prange);
     for (size_t gi = 0; gi < groups.size(); ++gi) {
-        f.do_a = gi == 0;
-        f.do_b = 1;
-        f.tlo = groups[gi].first;
-        f.thi = groups[gi].second;
-        f.part_base = groups.size() == 1 ? 0 : inv_host[f.tlo];
-        if (c->dim == 2) dispatch_fused<2>(c, f, a, fp32b, nsb, prange, tmode);
-        else dispatch_fused<3>(c, f, a, fp32b, nsb, prange, tmode);
+        const Group &g = groups[gi];
+        f.b0 = g.b0;
+        f.part_base = g.k0;
+        if (c->dim == 2) dispatch_fused<2>(c, f, a, fp32b, g.b1 - g.b0, prange, tmode);
+        else dispatch_fused<3>(c, f, a, fp32b, g.b1 - g.b0, prange, tmode);
         if (c->profiling && gi + 1 == groups.size()) cudaEventRecord(c->pev[2], st);
-        const int nw = f.thi - f.tlo;
+        if (gi == 0) {
+            e = cudaStreamWaitEvent(st, c->join, 0);
+            if (e != cudaSuccess) return cuda_error(c, e, "pair list join");
+        }
         if (fp32b)
-            k_grad_reduce<float><<<(unsigned)nw, 256, 0, st>>>(c->tblk_off.p, c->inv_off.p, f.tlo, f.thi, f.part_base,
-                                                               f.part32, c->gpart.p);
+            k_grad_reduce<float><<<(unsigned)ntb, 256, 0, st>>>(c->tblk_off.p, c->inv_off.p, c->inv_k.p, g.k0, g.k1,
+                                                                gi > 0, f.part32, c->gpart.p);
         else
-            k_grad_reduce<double><<<(unsigned)nw, 256, 0, st>>>(c->tblk_off.p, c->inv_off.p, f.tlo, f.thi,
-                                                                f.part_base, c->part.p, c->gpart.p);
+            k_grad_reduce<double><<<(unsigned)ntb, 256, 0, st>>>(c->tblk_off.p, c->inv_off.p, c->inv_k.p, g.k0, g.k1,
+                                                                 gi > 0, c->part.p, c->gpart.p);
         c->klaunch[2] += 1;
         c->klaunch[3] += 1;
     }
