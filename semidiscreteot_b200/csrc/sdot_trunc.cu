@@ -56,8 +56,12 @@ constexpr int FT_MAXS = 1024;               // staged targets per chunk
 // 16; registers capped at 80): measured 3.99 ms per trunc_3d evaluation against
 // 4.19 ms with 1,024 targets and 2 CTAs, although more blocks need several chunks.
 constexpr int FT_MAXS_TENSOR = 624;
-__host__ __device__ constexpr bool fused_small(int dim, int tq, bool fp32b) { return dim == 3 && tq > 0 && fp32b; }
-__host__ __device__ constexpr int fused_cap(int dim, int tq, bool fp32b) { return fused_small(dim, tq, fp32b) ? FT_MAXS_TENSOR : FT_MAXS; }
+constexpr int FT_MAXS_TENSOR64 = 448;
+__host__ __device__ constexpr bool fused_small(int dim, int tq, bool fp32b) { return tq > 0; }
+__host__ __device__ constexpr int fused_cap(int dim, int tq, bool fp32b)
+{
+    return !fused_small(dim, tq, fp32b) ? FT_MAXS : (fp32b ? FT_MAXS_TENSOR : FT_MAXS_TENSOR64);
+}
 __host__ __device__ constexpr int fused_min_blocks(int dim, int tq, bool fp32b) { return fused_small(dim, tq, fp32b) ? 3 : 2; }
 constexpr int FT_TS = 6;                    // doubles per staged target: y(3), nu, log2 nu, s*psi
 constexpr int FT_MAXT = 96;                 // target blocks per chunk
@@ -83,44 +87,43 @@ struct FusedArgs {
     double cullt;                // per-target cull radius addend (r, enlarged)
 };
 
-template <int CAP>
+constexpr int FT_NEAR = 64;                 // candidates per warp and chunk that may hold a point's maximum
+
+// Row: the type of the gradient sweep's partial rows, FP32 in the hybrid mode
+// and FP64 in the FP64 mode (which keeps its precision through the sum of the
+// warps' rows).
+template <int CAP, class Row>
 struct FTSmem {
     static constexpr int MAXS = CAP;
     double tab[16];
     double stg[FT_TS][CAP];    // staged targets, structure of arrays (conflict-free lane access)
     double qd[FT_MAXQ][4];        // delta_q (FP64) and C'_q
-    double qn[FT_MAXQ];           // |delta_q|
     double qL[FT_MAXQ];           // L_q of the block
+    double uL[FT_WARPS];          // smallest L_q of each unit
     __align__(16) float qb[FT_MAXQ][4];  // pass B: delta (3) as float, D_q (+ log2 w_q)
-    float qw[FT_MAXQ];            // pass B: w_q
-    float qtw[FT_MAXQ];           // pass B, tensor path: w_q 2^(D_q)
+    Row qw[FT_MAXQ];              // pass B: w_q
+    Row qtw[FT_MAXQ];             // pass B, tensor path: w_q 2^(D_q)
     double cellc[FT_WARPS][3];    // centre of each cell of the block
-    float pvw[FT_WARPS][CAP];     // gradient partial of each unit (warp) per staged target (FP32 mode)
+    // gradient partial of each unit (warp) per staged target; before that, in the value sweep:
+    union {
+        Row rows[FT_WARPS][CAP];
+        struct {
+            double S[FT_MAXQ], mx[FT_MAXQ], U[FT_MAXQ];   // per point: sum relative to U, largest exponent
+            unsigned short near_list[FT_WARPS][FT_NEAR];  // candidates that may hold a point's maximum
+            int nnear[FT_WARPS];
+        } v;
+    };
     unsigned short cand[FT_WARPS][CAP];
     short smap[FT_MAXT][TBLK_KD]; // (chunk target block, slot) -> staged position or -1
     int ecnt[32];                 // survivors per examined forward entry (-1: none)
     int epre[32];                 // staged position of the first survivor of each accepted entry
     int eacc, etot;
-    int wcount[FT_WARPS];
     int nstg;
     int ent_j0[FT_PREF];           // forward entries of the block: the target block's first target
     unsigned char ent_sz[FT_PREF]; // and its size (prefetched once per block)
 };
-
-// Partial rows of the gradient sweep: FP32 in the hybrid mode (inside
-// FTSmem), FP64 in the FP64 mode (appended after FTSmem in dynamic shared
-// memory, so that the FP64 gradient keeps its precision through the sum of
-// the warps' rows).
 template <bool FP32B> struct PRow { using T = double; };
 template <> struct PRow<true> { using T = float; };
-__host__ __device__ constexpr size_t ft_rows64_bytes(int cap) { return sizeof(double) * FT_WARPS * cap; }
-
-template <bool FP32B, class SM>
-__device__ __forceinline__ typename PRow<FP32B>::T *partial_rows(SM &sm)
-{
-    if constexpr (FP32B) return &sm.pvw[0][0];
-    else return reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(&sm) + sizeof(SM));
-}
 
 // ---------------------------------------------------------------------------
 // block-pair lists
@@ -531,14 +534,6 @@ __device__ int stage_chunk(SM &sm, const FusedArgs &f, int64_t kb, int64_t k0, i
     return nb;
 }
 
-// Exact squared distance from a staged target (SoA) to a cell centre.
-template <int DIM, class SM>
-__device__ __forceinline__ double stg_dist2(const SM &sm, int t, const double *c)
-{
-    const double y[3] = {sm.stg[0][t], sm.stg[1][t], DIM == 3 ? sm.stg[2][t] : 0.0};
-    return dist2_exact<DIM>(y, c);
-}
-
 // Value-sweep pair loop of one unit over its compacted candidates.
 // MODE 0: shift M = per-unit upper bound, exponents provably >= -16000 (no
 //         clamp); MODE 1: same with the clamp; MODE 2: per-pair lazy rescale
@@ -608,14 +603,17 @@ __device__ __noinline__ void value_pairs_partial(const SM &sm, int wp, int lane,
 
 // Exact candidate test of the staged targets for the warp's cell, in-order
 // compaction into sm.cand[wp]; returns the count and (through bmax) the
-// largest B0_Kj = kappa (psi_j - d2/2)/eps over the candidates.
-template <int DIM, class SM>
+// largest B0_Kj = kappa (psi_j - d2/2)/eps over the candidates.  With TQ > 0
+// also (through lb) the largest lower bound B0_Kj - sum_d |G_Kj,d| a_d of a
+// candidate's exponents at the cell's points (a: their offsets; gh = s a).
+template <int DIM, int TQ, class SM>
 __device__ __forceinline__ int compact_candidates(SM &sm, int wp, int lane, int nstg, const double *cc,
-                                                  const EvalArgs &a, double &bmax)
+                                                  const EvalArgs &a, const double *gh, double &bmax, double &lb)
 {
     constexpr int U = 4;  // staged targets per lane in flight (independent distance chains)
     int ncand = 0;
     bmax = -CUDART_INF;
+    lb = -CUDART_INF;
     for (int b0 = 0; b0 < nstg; b0 += 32 * U) {
         bool in[U];
 #pragma unroll
@@ -623,9 +621,19 @@ __device__ __forceinline__ int compact_candidates(SM &sm, int wp, int lane, int 
             const int t = b0 + 32 * u + lane;
             in[u] = false;
             if (t < nstg) {
-                const double d2 = stg_dist2<DIM>(sm, t, cc);
+                const double y[3] = {sm.stg[0][t], sm.stg[1][t], DIM == 3 ? sm.stg[2][t] : 0.0};
+                const double d2 = dist2_exact<DIM>(y, cc);
                 in[u] = d2 <= a.sstar;
-                if (in[u]) bmax = fmax(bmax, fma(-a.halfs, d2, sm.stg[5][t]));
+                if (in[u]) {
+                    const double B0 = fma(-a.halfs, d2, sm.stg[5][t]);
+                    bmax = fmax(bmax, B0);
+                    if (TQ > 0) {
+                        double l = B0;
+#pragma unroll
+                        for (int d = 0; d < DIM; ++d) l = fma(-fabs(y[d] - cc[d]), gh[d], l);
+                        lb = fmax(lb, l);
+                    }
+                }
             }
         }
 #pragma unroll
@@ -636,6 +644,7 @@ __device__ __forceinline__ int compact_candidates(SM &sm, int wp, int lane, int 
         }
     }
     bmax = warp_max(bmax);
+    if (TQ > 0) lb = warp_max(lb);
     __syncwarp();
     return ncand;
 }
@@ -702,11 +711,11 @@ __device__ __forceinline__ void grad_pairs(SM &sm, const FusedArgs &f, int wp, i
                 double u = fma(G0, dq[0], U0 + dq[3] - KAPPA * (L - Lref));
                 u = fma(G1, dq[1], u);
                 if (DIM == 3) u = fma(G2, dq[2], u);
-                acc = fma(f.w[qblk0 + qoff + q], exp2_16(u, sm.tab), acc);
+                acc = fma(sm.qw[qoff + q], exp2_16(u, sm.tab), acc);
             }
             val = acc;
         }
-        partial_rows<FP32B>(sm)[wp * SM::MAXS + ti] = (typename PRow<FP32B>::T)val;
+        sm.rows[wp][ti] = (typename PRow<FP32B>::T)val;
     }
 }
 
@@ -722,20 +731,17 @@ __device__ __forceinline__ constexpr int tstride()
 }
 
 // The per-q maximum exponent (the reference's m of the log-sum-exp, which
-// C_global depends on) is taken exactly, as in value_pairs, but only over the
-// candidates that can attain it: b_qj lies within s r |delta|max of B0_Kj, so
-// a candidate with B0 below (running max B0) - 2 s r |delta|max is never a
-// maximum; thr is that bound relative to Munit.
+// C_global depends on) is taken exactly, but only over the candidates that
+// can attain it: those whose upper bound B0 + sum_d |G_d| a_d reaches the
+// largest lower bound lb of any candidate (relative to Munit here).  They are
+// listed (one in 20 to 100 of a cell's candidates) and their exponents taken
+// afterwards by near_maxima, lane <-> point, so that the loop keeps no maxima
+// in registers.
 template <int DIM, int TM, int TS, class SM>
-__device__ __forceinline__ void value_pairs_tensor(const SM &sm, int wp, int lane, int ncand, int qoff,
-                                                   const double *cc, const EvalArgs &a, double Munit, double thr,
-                                                   double *S, double *mx)
+__device__ __forceinline__ void value_pairs_tensor(SM &sm, int wp, int lane, int ncand, const double *ah,
+                                                   const double *cc, const EvalArgs &a, double Munit, double lb,
+                                                   double *S)
 {
-    constexpr int NQ = DIM == 3 ? TM * TM * TM : TM * TM;
-    double ah[3];
-    ah[0] = sm.qd[qoff + (TM - 1) * tstride<TM, 0>()][0];
-    ah[1] = sm.qd[qoff + (TM - 1) * tstride<TM, 1>()][1];
-    ah[2] = DIM == 3 ? sm.qd[qoff + (TM - 1) * tstride<TM, 2>()][2] : 0.0;
     for (int p = lane; p < ncand; p += 32) {
         const int ti = sm.cand[wp][p];
         const double g0 = sm.stg[0][ti] - cc[0], g1 = sm.stg[1][ti] - cc[1];
@@ -743,27 +749,25 @@ __device__ __forceinline__ void value_pairs_tensor(const SM &sm, int wp, int lan
         const double d2 = DIM == 3 ? g0 * g0 + g1 * g1 + g2 * g2 : g0 * g0 + g1 * g1;
         const double B0 = fma(-a.halfs, d2, sm.stg[5][ti]) - Munit;
         const double G[3] = {a.s * g0, a.s * g1, a.s * g2};
-        if (B0 >= thr) {
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) {
-                const double *dq = sm.qd[qoff + q];
-                double bb = fma(G[0], dq[0], B0);
-                bb = fma(G[1], dq[1], bb);
-                if (DIM == 3) bb = fma(G[2], dq[2], bb);
-                mx[q] = fmax(mx[q], bb);
-            }
-        }
         // per-dimension factors 2^(G_d delta_d): with TS, relative to the lowest
         // point (1, r, r^2 with the shift folded into P); otherwise 2^(-G a), (1), 2^(G a)
-        double F[3][TM];
+        double F[3][TM], ga[3], ub = B0;
         double P;
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+            ga[d] = G[d] * ah[d];
+            ub += fabs(ga[d]);
+        }
+        if (ub >= lb) {
+            const int at = atomicAdd(&sm.v.nnear[wp], 1);
+            if (at < FT_NEAR) sm.v.near_list[wp][at] = (unsigned short)ti;
+        }
         if constexpr (TS >= 1) {
             double sga = 0.0;
 #pragma unroll
             for (int d = 0; d < DIM; ++d) {
-                const double ga = G[d] * ah[d];
-                sga += ga;
-                const double r = exp2_16(TM == 2 ? 2.0 * ga : ga, sm.tab);
+                sga += ga[d];
+                const double r = exp2_16(TM == 2 ? 2.0 * ga[d] : ga[d], sm.tab);
                 F[d][0] = 1.0;
                 F[d][1] = r;
                 if (TM == 3) F[d][2] = r * r;
@@ -772,7 +776,7 @@ __device__ __forceinline__ void value_pairs_tensor(const SM &sm, int wp, int lan
         } else {
 #pragma unroll
             for (int d = 0; d < DIM; ++d) {
-                const double xp = exp2_16(G[d] * ah[d], sm.tab);
+                const double xp = exp2_16(ga[d], sm.tab);
                 F[d][0] = __drcp_rn(xp);
                 F[d][TM - 1] = xp;
                 if (TM == 3) F[d][1] = 1.0;
@@ -798,6 +802,65 @@ __device__ __forceinline__ void value_pairs_tensor(const SM &sm, int wp, int lan
             }
         }
     }
+}
+
+// Largest exponents (absolute) of the unit's points over the listed
+// candidates (all of them where the list overflowed): lanes <-> (point q =
+// lane mod NQ, every EP-th candidate), one running maximum per lane.
+template <int DIM, int NQ, class SM>
+__device__ __forceinline__ void near_maxima(const SM &sm, int wp, int lane, int ncand, int qoff, const double *cc,
+                                            const EvalArgs &a, double &mx)
+{
+    constexpr int EP = 32 / NQ;
+    const int q = lane % NQ, sub = lane / NQ;
+    const int n = sm.v.nnear[wp];
+    const bool all = n > FT_NEAR;
+    const int cnt = all ? ncand : n;
+    if (sub >= EP) return;
+    const double *dq = sm.qd[qoff + q];
+    for (int p = sub; p < cnt; p += EP) {
+        const int ti = all ? sm.cand[wp][p] : sm.v.near_list[wp][p];
+        const double g0 = sm.stg[0][ti] - cc[0], g1 = sm.stg[1][ti] - cc[1];
+        const double g2 = DIM == 3 ? sm.stg[2][ti] - cc[2] : 0.0;
+        const double d2 = DIM == 3 ? g0 * g0 + g1 * g1 + g2 * g2 : g0 * g0 + g1 * g1;
+        double bb = fma(a.s * g0, dq[0], fma(-a.halfs, d2, sm.stg[5][ti]));
+        bb = fma(a.s * g1, dq[1], bb);
+        if (DIM == 3) bb = fma(a.s * g2, dq[2], bb);
+        mx = fmax(mx, bb);
+    }
+}
+
+// Sums over the lanes of the unit's NQ per-lane sums; q's total ends in lane
+// q * (32 / 2^ceil(log2 NQ)) for q < 8 (transposed butterflies: each exchange
+// halves the sums a lane keeps, NQ + log2 exchanges instead of 5 NQ) and, for
+// NQ = 9, the ninth in every lane (last).
+template <int NQ>
+__device__ __forceinline__ double lane_totals(const double *S, int lane, double &last)
+{
+    constexpr int H = NQ == 4 ? 2 : 4;   // sums kept after the first exchange
+    constexpr int FIRST = 16;
+    double s[H];
+    const bool b4 = lane & FIRST;
+#pragma unroll
+    for (int k = 0; k < H; ++k) {
+        const double keep = b4 ? S[H + k] : S[k], give = b4 ? S[k] : S[H + k];
+        s[k] = keep + __shfl_xor_sync(0xffffffffu, give, FIRST);
+    }
+    int o = 8;
+#pragma unroll
+    for (int h = H / 2; h > 0; h >>= 1, o >>= 1) {
+        const bool b = lane & o;
+#pragma unroll
+        for (int k = 0; k < H / 2; ++k) {
+            if (k >= h) continue;
+            const double keep = b ? s[h + k] : s[k], give = b ? s[k] : s[h + k];
+            s[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+#pragma unroll
+    for (int e = NQ == 4 ? 4 : 2; e > 0; e >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], e);
+    last = NQ == 9 ? warp_sum(S[NQ - 1]) : 0.0;
+    return s[0];
 }
 
 __device__ __forceinline__ float rcp_approx(float x)
@@ -873,7 +936,53 @@ __device__ __forceinline__ void grad_pairs_tensor(SM &sm, int wp, int lane, int 
                 w = fmaf(u, F[0][i0], w);
             }
         }
-        partial_rows<true>(sm)[wp * SM::MAXS + ti] = ex2_approx(e0) * w;
+        sm.rows[wp][ti] = ex2_approx(e0) * w;
+    }
+}
+
+// FP64 gradient sweep on tensor-product points: the same sums with FP64
+// factors relative to the lowest point (1 + DIM exponentials per candidate
+// instead of one per point).
+template <int DIM, int TM, class SM>
+__device__ __forceinline__ void grad_pairs_tensor64(SM &sm, int wp, int lane, int ncand, int qoff, const double *ah,
+                                                    const double *cc, double Lref, const EvalArgs &a)
+{
+    constexpr int NQ = DIM == 3 ? TM * TM * TM : TM * TM;
+    double W[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) W[q] = sm.qtw[qoff + q];
+    for (int p = lane; p < ncand; p += 32) {
+        const int ti = sm.cand[wp][p];
+        const double g[3] = {sm.stg[0][ti] - cc[0], sm.stg[1][ti] - cc[1], DIM == 3 ? sm.stg[2][ti] - cc[2] : 0.0};
+        const double d2 = DIM == 3 ? g[0] * g[0] + g[1] * g[1] + g[2] * g[2] : g[0] * g[0] + g[1] * g[1];
+        double U = 16.0 * sm.stg[4][ti] + fma(-a.halfs, d2, sm.stg[5][ti]) - KAPPA * Lref;
+        double r[3];
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+            const double ga = a.s * g[d] * ah[d];
+            U -= ga;
+            r[d] = exp2_16(TM == 2 ? 2.0 * ga : ga, sm.tab);
+        }
+        double w = 0.0;
+#pragma unroll
+        for (int i0 = TM - 1; i0 >= 0; --i0) {
+            double u = 0.0;
+#pragma unroll
+            for (int i1 = TM - 1; i1 >= 0; --i1) {
+                double v = 0.0;
+                if (DIM == 2) {
+                    v = W[i0 + TM * i1];
+                } else {
+#pragma unroll
+                    for (int i2 = TM - 1; i2 >= 0; --i2)
+                        v = i2 == TM - 1 ? W[i0 + TM * i1 + TM * TM * i2]
+                                         : fma(v, r[2], W[i0 + TM * i1 + TM * TM * i2]);
+                }
+                u = i1 == TM - 1 ? v : fma(u, r[1], v);
+            }
+            w = i0 == TM - 1 ? u : fma(w, r[0], u);
+        }
+        sm.rows[wp][ti] = exp2_16(U, sm.tab) * w;
     }
 }
 
@@ -883,7 +992,6 @@ __device__ __forceinline__ void grad_pairs_tensor(SM &sm, int wp, int lane, int 
 template <bool FP32B, class SM>
 __device__ __forceinline__ void write_partials(SM &sm, const FusedArgs &f, int64_t k, int nt, int nunit)
 {
-    const typename PRow<FP32B>::T *rows = partial_rows<FP32B>(sm);
     const int tid = threadIdx.x;
     for (int i = tid; i < nt * TBLK_KD; i += blockDim.x) {
         const int ti = i / TBLK_KD, sl = i - ti * TBLK_KD;
@@ -891,7 +999,7 @@ __device__ __forceinline__ void write_partials(SM &sm, const FusedArgs &f, int64
         const short p = sm.smap[ti][sl];
         double v = 0.0;
         if (p >= 0)
-            for (int w = 0; w < nunit; ++w) v += (double)rows[w * SM::MAXS + p];
+            for (int w = 0; w < nunit; ++w) v += (double)sm.rows[w][p];
         if constexpr (FP32B) f.part32[base + sl] = (float)v;
         else f.part[base + sl] = v;
     }
@@ -902,7 +1010,7 @@ __global__ void __launch_bounds__(FT_WARPS * 32, fused_min_blocks(DIM, TQ, FP32B
 k_fused(FusedArgs f, EvalArgs a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    using SMem = FTSmem<fused_cap(DIM, TQ, FP32B)>;
+    using SMem = FTSmem<fused_cap(DIM, TQ, FP32B), typename PRow<FP32B>::T>;
     SMem &sm = *reinterpret_cast<SMem *>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
     const int b = f.b0 + blockIdx.x;
@@ -943,10 +1051,18 @@ k_fused(FusedArgs f, EvalArgs a)
             dsq += dl * dl;
         }
         sm.qd[i][3] = -a.halfs * dsq;
-        sm.qn[i] = sqrt(dsq);
     }
     __syncthreads();
     const double cc[3] = {sm.cellc[cl][0], sm.cellc[cl][1], sm.cellc[cl][2]};
+    // tensor points: the largest offset per dimension, and s times it
+    double ah[3] = {0.0, 0.0, 0.0}, gh[3] = {0.0, 0.0, 0.0};
+    if constexpr (TQ > 0) {
+        ah[0] = sm.qd[qoff + (TQ - 1) * tstride<TQ, 0>()][0];
+        ah[1] = sm.qd[qoff + (TQ - 1) * tstride<TQ, 1>()][1];
+        if (DIM == 3) ah[2] = sm.qd[qoff + (TQ - 1) * tstride<TQ, 2>()][2];
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) gh[d] = a.s * ah[d];
+    }
     int tail_off = -1;  // first entry (minus k0) of the value sweep's last chunk, still staged for the gradient sweep
     int tail_nt = 0;
     int ncand_single = 0;
@@ -956,25 +1072,33 @@ k_fused(FusedArgs f, EvalArgs a)
         // Shift of the online sums.  MODE 0/1: Munit = max_j B0_Kj + s r
         // max_q |delta_q| bounds every exponent of the unit from above
         // (|G_Kj| <= s r for a candidate), so no per-pair rescale is needed;
-        // exponents are kept relative to Munit (mx too) and a chunk that raises
-        // the bound rescales S once.  MODE 2 keeps a per-q lazy shift M[q].
-        double M[MODE == 2 ? QL : 1], S[QL], mx[QL];
+        // exponents are kept relative to Munit (mx too, on the per-point
+        // sweeps) and a chunk that raises the bound rescales S once.  MODE 2
+        // keeps a per-q lazy shift M[q].
+        constexpr bool TENS = TQ > 0;
+        double M[MODE == 2 ? QL : 1], S[QL], mx[TENS ? 1 : QL];
 #pragma unroll
-        for (int k = 0; k < QL; ++k) { S[k] = 0.0; mx[k] = -CUDART_INF; }
+        for (int k = 0; k < QL; ++k) S[k] = 0.0;
+#pragma unroll
+        for (int k = 0; k < (TENS ? 1 : QL); ++k) mx[k] = -CUDART_INF;
 #pragma unroll
         for (int k = 0; k < (MODE == 2 ? QL : 1); ++k) M[k] = -CUDART_INF;
         double Munit = -CUDART_INF;
         double dqmax = 0.0;
-        for (int q = 0; q < nql; ++q) dqmax = fmax(dqmax, sm.qn[qoff + q]);
+        for (int q = 0; q < nql; ++q) {
+            const double *dq = sm.qd[qoff + q];
+            dqmax = fmax(dqmax, dq[0] * dq[0] + dq[1] * dq[1] + dq[2] * dq[2]);
+        }
+        dqmax = sqrt(dqmax);
         double npairs = 0.0;
-        double bmax_run = -CUDART_INF;  // largest B0 of the candidates so far
+        double lb_run = -CUDART_INF;  // largest lower bound of the candidates so far
         const double sr = a.s * a.cull;
         for (int64_t k = k0; k < k1;) {
             const int nt = stage_chunk<DIM>(sm, f, k0, k, k1, bc, rcull2);
             const int nstg = sm.nstg;
             if (valid) {
-                double bmax;
-                const int ncand = compact_candidates<DIM>(sm, wp, lane, nstg, cc, a, bmax);
+                double bmax, lb;
+                const int ncand = compact_candidates<DIM, TQ>(sm, wp, lane, nstg, cc, a, gh, bmax, lb);
                 ncand_single = ncand;
                 npairs += (double)ncand * nql;
                 if (MODE != 2 && bmax > -CUDART_INF) {
@@ -985,17 +1109,23 @@ k_fused(FusedArgs f, EvalArgs a)
 #pragma unroll
                             for (int q = 0; q < QL; ++q) {
                                 S[q] *= sc;
-                                mx[q] += Munit - mnew;
+                                if (!TENS) mx[TENS ? 0 : q] += Munit - mnew;
                             }
                         }
                         Munit = mnew;
                     }
                 }
-                if (bmax > bmax_run) bmax_run = bmax;
-                if constexpr (TQ > 0)
-                    value_pairs_tensor<DIM, TQ, TS>(sm, wp, lane, ncand, qoff, cc, a, Munit,
-                                                    bmax_run - 2.0 * sr * dqmax - Munit, S, mx);
-                else if (nql == QL)
+                if constexpr (TENS) {
+                    if (lb > lb_run) lb_run = lb;
+                    if (lane == 0) sm.v.nnear[wp] = 0;
+                    __syncwarp();
+                    // the bounds' rounding: a few ulp of the exponents, far below 1e-12 of their range
+                    const double lbr = lb_run - Munit;
+                    value_pairs_tensor<DIM, TQ, TS>(sm, wp, lane, ncand, ah, cc, a, Munit,
+                                                    lbr - 1e-12 * (fabs(lb_run) + fabs(Munit)), S);
+                    __syncwarp();
+                    near_maxima<DIM, QL>(sm, wp, lane, ncand, qoff, cc, a, mx[0]);
+                } else if (nql == QL)
                     value_pairs<DIM, QL, QL, MODE>(sm, wp, lane, ncand, qoff, cc[0], cc[1], cc[2], a, Munit, M, S, mx);
                 else
                     value_pairs_partial<DIM, QL, MODE>(sm, wp, lane, ncand, qoff, nql, cc[0], cc[1], cc[2], a, Munit,
@@ -1009,96 +1139,83 @@ k_fused(FusedArgs f, EvalArgs a)
                 __syncthreads();  // the next chunk overwrites the staged targets
             }
         }
-        // merge the lanes of each q (max, sum); the lane that ends with q's
-        // totals runs q's epilogue, so the QL epilogues proceed in parallel
-        double my_mx = -CUDART_INF, my_S = 0.0;
-        int my_q = lane;   // the q whose totals this lane holds
-        bool epi = lane < nql;
-        if constexpr (MODE != 2 && QL == 8) {
-            // Transposed butterflies: the xor-16, -8 and -4 exchanges each
-            // halve the q's a lane keeps (q = lane >> 2 after them), the xor-2
-            // and -1 exchanges finish: 9 exchanges per reduction instead of 40.
-            // Every lane's sums are relative to Munit, so they add directly and
-            // one exponential per q rescales the total to its maximum.
-            const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
-            double m4[4], s4[4], m2[2], s2[2];
+        // the lanes' sums and maxima of each q, to shared memory
+        if (valid) {
+            if constexpr (TENS) {
+                double last;
+                const double tot = lane_totals<QL>(S, lane, last);
+                constexpr int EP = 32 / QL;
+                double m = mx[0];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const double mk = b4 ? mx[4 + k] : mx[k], ms = b4 ? mx[k] : mx[4 + k];
-                const double sk = b4 ? S[4 + k] : S[k], ss = b4 ? S[k] : S[4 + k];
-                m4[k] = fmax(mk, __shfl_xor_sync(0xffffffffu, ms, 16));
-                s4[k] = sk + __shfl_xor_sync(0xffffffffu, ss, 16);
-            }
+                for (int e = 1; e < EP; ++e) m = fmax(m, __shfl_down_sync(0xffffffffu, mx[0], e * QL));
+                constexpr int LPQ = QL == 4 ? 8 : 4;   // lanes that hold a total
+                if (lane % LPQ == 0) sm.v.S[qoff + lane / LPQ] = tot;
+                if (QL == 9 && lane == 0) sm.v.S[qoff + QL - 1] = last;
+                if (lane < QL) {
+                    sm.v.mx[qoff + lane] = m;
+                    sm.v.U[qoff + lane] = Munit;
+                }
+            } else {
 #pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                const double mk = b3 ? m4[2 + k] : m4[k], ms = b3 ? m4[k] : m4[2 + k];
-                const double sk = b3 ? s4[2 + k] : s4[k], ss = b3 ? s4[k] : s4[2 + k];
-                m2[k] = fmax(mk, __shfl_xor_sync(0xffffffffu, ms, 8));
-                s2[k] = sk + __shfl_xor_sync(0xffffffffu, ss, 8);
-            }
-            double m1 = fmax(b2 ? m2[1] : m2[0], __shfl_xor_sync(0xffffffffu, b2 ? m2[0] : m2[1], 4));
-            double s1 = (b2 ? s2[1] : s2[0]) + __shfl_xor_sync(0xffffffffu, b2 ? s2[0] : s2[1], 4);
-#pragma unroll
-            for (int o = 2; o > 0; o >>= 1) {
-                m1 = fmax(m1, __shfl_xor_sync(0xffffffffu, m1, o));
-                s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-            }
-            my_q = lane >> 2;
-            epi = (lane & 3) == 0 && my_q < nql;
-            my_mx = m1;
-            my_S = (Munit == -CUDART_INF || m1 == -CUDART_INF) ? 0.0 : s1 * exp2_16(-m1, sm.tab);
-        } else {
-#pragma unroll
-            for (int q = 0; q < QL; ++q) {
-                const double mxw = warp_max(mx[q]);
-                // shift of this lane's sum: Munit (exponents relative to it: 0) or the lazy M[q]
-                const double Ml = MODE == 2 ? M[MODE == 2 ? q : 0] : (Munit > -CUDART_INF ? 0.0 : -CUDART_INF);
-                const double sl = (Ml == -CUDART_INF || mxw == -CUDART_INF) ? 0.0 : S[q] * exp2_16(Ml - mxw, sm.tab);
-                const double Sw = warp_sum(sl);
-                if (lane == q) {
-                    my_mx = mxw;
-                    my_S = Sw;
+                for (int q = 0; q < QL; ++q) {
+                    const double mxw = warp_max(mx[TENS ? 0 : q]);
+                    // shift of this lane's sum: Munit (exponents relative to it: 0) or the lazy M[q]
+                    const double Ml = MODE == 2 ? M[MODE == 2 ? q : 0] : (Munit > -CUDART_INF ? 0.0 : -CUDART_INF);
+                    const double sl =
+                        (Ml == -CUDART_INF || mxw == -CUDART_INF) ? 0.0 : S[q] * exp2_16(Ml - mxw, sm.tab);
+                    const double Sw = warp_sum(sl);
+                    if (lane == 0 && q < nql) {
+                        const double m = MODE == 2 ? mxw : mxw + Munit;
+                        sm.v.S[qoff + q] = Sw;
+                        sm.v.mx[qoff + q] = m;
+                        sm.v.U[qoff + q] = m;   // the sum is relative to the maximum
+                    }
                 }
             }
         }
+        __syncthreads();
+        // the points' epilogues, thread <-> point of the block: one or three warps run the logarithms instead of
+        // every warp for the eight or nine lanes of its unit
         double tv = 0.0, tcv = 0.0, tsk = 0.0;
-        if (valid && epi) {
-            const int qi = qoff + my_q;
-            const int64_t qg = qblk0 + qi;
-            double v, cv, L;
+        if (tid < nqb) {
+            const int64_t qg = qblk0 + tid;
+            const double m = sm.v.mx[tid], U = sm.v.U[tid];
+            const double Sr =
+                (m == -CUDART_INF || U == -CUDART_INF) ? 0.0 : sm.v.S[tid] * (TENS ? exp2_16(U - m, sm.tab) : 1.0);
+            double L;
             int sk;
-            value_epilogue(a, MODE == 2 ? my_mx : my_mx + Munit, my_S, sm.qd[qi][3], f.rho[qg], f.jxw[qg], v, cv, L,
-                           sk);
+            value_epilogue(a, m, Sr, sm.qd[tid][3], f.rho[qg], f.jxw[qg], tv, tcv, L, sk);
             f.Lq[qg] = L;
-            sm.qL[qi] = L;
-            tv = v;
-            tcv = cv;
+            sm.qL[tid] = L;
             tsk = sk;
         }
         block_partials_at(tv, tcv, tsk, lane == 0 ? npairs : 0.0, f.valpart + (int64_t)b * 4);  // contains __syncthreads
     }
 
     // ---------------- gradient sweep ----------------
-    // per-unit reference L_Kref = min L over the unit's q; per-q FP32 data
-    double Lref = CUDART_INF;
-    if (valid) {
-        double lv = lane < nql ? sm.qL[qoff + lane] : CUDART_INF;
-        Lref = -warp_max(-lv);
-        if (lane < nql) {
-            const int i = qoff + lane;
-            const double L = sm.qL[i];
-            const double D = (!isfinite(Lref) || !isfinite(L)) ? -CUDART_INF
-                                                                : (sm.qd[i][3] - KAPPA * (L - Lref)) * (1.0 / 16.0);
-            const double wq = f.w[qblk0 + i];
+    // per-unit reference L_Kref = min L over the unit's q; per-q data
+    if (tid < nqb) {
+        const int i = tid, c = i / a.qpc, gr = (i - c * a.qpc) / a.ql;
+        const int u0 = c * a.qpc + gr * a.ql, un = min(a.ql, a.qpc - gr * a.ql);
+        double Lr = CUDART_INF;
+        for (int q = 0; q < un; ++q) Lr = fmin(Lr, sm.qL[u0 + q]);
+        if (i == u0) sm.uL[c * a.ngroups + gr] = Lr;
+        const double L = sm.qL[i];
+        const double D = (!isfinite(Lr) || !isfinite(L)) ? -CUDART_INF
+                                                         : (sm.qd[i][3] - KAPPA * (L - Lr)) * (1.0 / 16.0);
+        const double wq = f.w[qblk0 + i];
+        using Row = typename PRow<FP32B>::T;
+        if (FP32B && TQ == 0) {
             sm.qb[i][0] = (float)sm.qd[i][0];
             sm.qb[i][1] = (float)sm.qd[i][1];
             sm.qb[i][2] = (float)sm.qd[i][2];
             sm.qb[i][3] = (float)(f.w_nonneg ? D + log2(wq) : D);  // w_q folded in: p = 2^e directly
-            sm.qw[i] = (float)wq;
-            if (TQ > 0) sm.qtw[i] = (float)(wq * exp2(D));
         }
-        __syncwarp();
+        sm.qw[i] = (Row)wq;
+        if (TQ > 0) sm.qtw[i] = (Row)(wq * exp2(D));
     }
+    __syncthreads();
+    const double Lref = valid ? sm.uL[wp] : CUDART_INF;
     // The value sweep's last chunk (the only one when everything fit) is still
     // staged with each warp's candidates: its gradient comes first, then the
     // earlier chunks are staged again (the same chunks: the greedy rule over
@@ -1109,10 +1226,11 @@ k_fused(FusedArgs f, EvalArgs a)
         const int nt = tail_nt;
         const int nstg = sm.nstg;
         if (valid) {
-            for (int t = lane; t < nstg; t += 32) partial_rows<FP32B>(sm)[wp * SMem::MAXS + t] = 0;
+            for (int t = lane; t < nstg; t += 32) sm.rows[wp][t] = 0;
             __syncwarp();
             if (isfinite(Lref)) {
                 if constexpr (TQ > 0 && FP32B) grad_pairs_tensor<DIM, TQ, TS>(sm, wp, lane, ncand_single, qoff, cc, Lref, a);
+                else if constexpr (TQ > 0) grad_pairs_tensor64<DIM, TQ>(sm, wp, lane, ncand_single, qoff, ah, cc, Lref, a);
                 else grad_pairs<DIM, FP32B>(sm, f, wp, lane, ncand_single, qoff, nql, cc, Lref, qblk0, a);
             }
         }
@@ -1126,12 +1244,13 @@ k_fused(FusedArgs f, EvalArgs a)
         const int nt = stage_chunk<DIM>(sm, f, k0, k, kend, bc, rcull2);
         const int nstg = sm.nstg;
         if (valid) {
-            double bmax;
-            const int ncand = compact_candidates<DIM>(sm, wp, lane, nstg, cc, a, bmax);
-            for (int t = lane; t < nstg; t += 32) partial_rows<FP32B>(sm)[wp * SMem::MAXS + t] = 0;
+            double bmax, lb;
+            const int ncand = compact_candidates<DIM, 0>(sm, wp, lane, nstg, cc, a, gh, bmax, lb);
+            for (int t = lane; t < nstg; t += 32) sm.rows[wp][t] = 0;
             __syncwarp();
             if (isfinite(Lref)) {
                 if constexpr (TQ > 0 && FP32B) grad_pairs_tensor<DIM, TQ, TS>(sm, wp, lane, ncand, qoff, cc, Lref, a);
+                else if constexpr (TQ > 0) grad_pairs_tensor64<DIM, TQ>(sm, wp, lane, ncand, qoff, ah, cc, Lref, a);
                 else grad_pairs<DIM, FP32B>(sm, f, wp, lane, ncand, qoff, nql, cc, Lref, qblk0, a);
             }
         }
@@ -1212,10 +1331,8 @@ static void launch_fused(sdot_ctx *c, const FusedArgs &f, const EvalArgs &a, siz
 template <int DIM, int QL, int MODE, int TQ = 0, int TS = 0>
 static void dispatch_fused_b(sdot_ctx *c, const FusedArgs &f, const EvalArgs &a, bool fp32b, int nb)
 {
-    if (fp32b) launch_fused<DIM, QL, true, MODE, TQ, TS>(c, f, a, sizeof(FTSmem<fused_cap(DIM, TQ, true)>), nb);
-    else
-        launch_fused<DIM, QL, false, MODE, TQ, TS>(c, f, a, sizeof(FTSmem<fused_cap(DIM, TQ, false)>) + ft_rows64_bytes(fused_cap(DIM, TQ, false)),
-                                               nb);
+    if (fp32b) launch_fused<DIM, QL, true, MODE, TQ, TS>(c, f, a, sizeof(FTSmem<fused_cap(DIM, TQ, true), float>), nb);
+    else launch_fused<DIM, QL, false, MODE, TQ, TS>(c, f, a, sizeof(FTSmem<fused_cap(DIM, TQ, false), double>), nb);
 }
 
 template <int DIM, int MODE>
