@@ -51,18 +51,12 @@ namespace sdot {
 
 constexpr int FT_WARPS = 8;
 constexpr int FT_MAXS = 1024;               // staged targets per chunk
-// The 3D tensor-factored hybrid sweeps stage at most 624 targets per chunk so that
-// their shared memory (75,312 B) lets 3 CTAs share an SM (24 warps instead of
-// 16; registers capped at 80): measured 3.99 ms per trunc_3d evaluation against
-// 4.19 ms with 1,024 targets and 2 CTAs, although more blocks need several chunks.
-constexpr int FT_MAXS_TENSOR = 624;
-constexpr int FT_MAXS_TENSOR64 = 448;
-__host__ __device__ constexpr bool fused_small(int dim, int tq, bool fp32b) { return tq > 0; }
-__host__ __device__ constexpr int fused_cap(int dim, int tq, bool fp32b)
-{
-    return !fused_small(dim, tq, fp32b) ? FT_MAXS : (fp32b ? FT_MAXS_TENSOR : FT_MAXS_TENSOR64);
-}
-__host__ __device__ constexpr int fused_min_blocks(int dim, int tq, bool fp32b) { return fused_small(dim, tq, fp32b) ? 3 : 2; }
+// The tensor-factored sweeps stage at most 936 targets per chunk, so that three
+// CTAs share an SM (24 warps; 80 registers): fewer chunks per block, which
+// are staged twice but for the last, against occupancy.
+constexpr int FT_MAXS_TENSOR = 936;
+__host__ __device__ constexpr int fused_cap(int tq) { return tq > 0 ? FT_MAXS_TENSOR : FT_MAXS; }
+__host__ __device__ constexpr int fused_min_blocks(int tq) { return tq > 0 ? 3 : 2; }
 constexpr int FT_TS = 6;                    // doubles per staged target: y(3), nu, log2 nu, s*psi
 constexpr int FT_MAXT = 96;                 // target blocks per chunk
 constexpr int FT_MAXQ = 80;                 // quadrature points of one source block
@@ -89,9 +83,8 @@ struct FusedArgs {
 
 constexpr int FT_NEAR = 64;                 // candidates per warp and chunk that may hold a point's maximum
 
-// Row: the type of the gradient sweep's partial rows, FP32 in the hybrid mode
-// and FP64 in the FP64 mode (which keeps its precision through the sum of the
-// warps' rows).
+// Row: the type of a unit's gradient terms and weights, FP32 in the hybrid
+// mode and FP64 in the FP64 mode.
 template <int CAP, class Row>
 struct FTSmem {
     static constexpr int MAXS = CAP;
@@ -99,22 +92,18 @@ struct FTSmem {
     double stg[FT_TS][CAP];    // staged targets, structure of arrays (conflict-free lane access)
     double qd[FT_MAXQ][4];        // delta_q (FP64) and C'_q
     double qL[FT_MAXQ];           // L_q of the block
+    double qS[FT_MAXQ], qm[FT_MAXQ], qU[FT_MAXQ];  // value sweep, per point: sum relative to U, largest exponent, U
     double uL[FT_WARPS];          // smallest L_q of each unit
-    __align__(16) float qb[FT_MAXQ][4];  // pass B: delta (3) as float, D_q (+ log2 w_q)
-    Row qw[FT_MAXQ];              // pass B: w_q
-    Row qtw[FT_MAXQ];             // pass B, tensor path: w_q 2^(D_q)
-    double cellc[FT_WARPS][3];    // centre of each cell of the block
-    // gradient partial of each unit (warp) per staged target; before that, in the value sweep:
-    union {
-        Row rows[FT_WARPS][CAP];
-        struct {
-            double S[FT_MAXQ], mx[FT_MAXQ], U[FT_MAXQ];   // per point: sum relative to U, largest exponent
-            unsigned short near_list[FT_WARPS][FT_NEAR];  // candidates that may hold a point's maximum
-            int nnear[FT_WARPS];
-        } v;
-    };
+    double cellc[FT_WARPS][3];    // centre of each unit's cell
+    double uah[FT_WARPS][3];      // tensor path: largest offsets of its points
+    __align__(16) float qb[FT_MAXQ][4];  // gradient sweep: delta (3) as float, D_q (+ log2 w_q)
+    __align__(16) Row qw[FT_MAXQ];       // gradient sweep: w_q
+    __align__(16) Row qtw[FT_MAXQ];      // gradient sweep, tensor path: w_q 2^(D_q)
     unsigned short cand[FT_WARPS][CAP];
-    short smap[FT_MAXT][TBLK_KD]; // (chunk target block, slot) -> staged position or -1
+    unsigned short dst[CAP];      // (chunk target block, slot) of each staged target
+    unsigned keep[FT_MAXT];       // staged slots of each target block of the chunk
+    unsigned short near_list[FT_WARPS][FT_NEAR];  // candidates that may hold a point's maximum
+    int nnear[FT_WARPS];
     int ecnt[32];                 // survivors per examined forward entry (-1: none)
     int epre[32];                 // staged position of the first survivor of each accepted entry
     int eacc, etot;
@@ -513,14 +502,14 @@ __device__ int stage_chunk(SM &sm, const FusedArgs &f, int64_t kb, int64_t k0, i
                 const int slot = nb + idx;
                 const int64_t j0 = jj[s];
                 const bool keep = (bal[s] >> lane) & 1u;
-                short pos = -1;
                 if (keep) {
-                    pos = (short)(sm.epre[idx] + __popc(bal[s] & ((1u << lane) - 1u)));
+                    const int pos = sm.epre[idx] + __popc(bal[s] & ((1u << lane) - 1u));
+                    sm.dst[pos] = (unsigned short)(slot * TBLK_KD + lane);
                     const double *tp = f.tpk + (j0 + lane) * TPACK;
 #pragma unroll
                     for (int d = 0; d < FT_TS; ++d) sm.stg[d][pos] = tp[d];
                 }
-                sm.smap[slot][lane] = pos;
+                if (lane == 0) sm.keep[slot] = bal[s];
             }
         }
         total = run;
@@ -649,73 +638,68 @@ __device__ __forceinline__ int compact_candidates(SM &sm, int wp, int lane, int 
     return ncand;
 }
 
-// Gradient sweep of one unit over its compacted candidates: for each
-// candidate target j (lane-strided) the unit's part of sum_q w_q nu_j
-// e^{t_qj - L_q}, written to the warp's partial row (FP32).  E0 and G' are
-// formed in FP64 per (cell, target) so that every FP32 operand is small.
+// A unit's part of the gradient of one target, sum over the unit's q of
+// w_q nu_j e^{t_qj - L_q} at g = y_j - c_K: E0 and G' are formed in FP64 per
+// (cell, target) so that every FP32 operand of the hybrid form is small.
+// lognu = log2 nu_j, sp = kappa psi_j / eps.
 template <int DIM, bool FP32B, class SM>
-__device__ __forceinline__ void grad_pairs(SM &sm, const FusedArgs &f, int wp, int lane, int ncand, int qoff,
-                                           int nql, const double *cc, double Lref, int64_t qblk0, const EvalArgs &a)
+__device__ __forceinline__ typename PRow<FP32B>::T grad_term(const SM &sm, int w_nonneg, int qoff, int nql,
+                                                             const double *g, double lognu, double sp, double Lref,
+                                                             const EvalArgs &a)
 {
-    const float sf = (float)(a.s * (1.0 / 16.0));
-    for (int p = lane; p < ncand; p += 32) {
-        const int ti = sm.cand[wp][p];
-        const double g0 = sm.stg[0][ti] - cc[0], g1 = sm.stg[1][ti] - cc[1];
-        const double g2 = DIM == 3 ? sm.stg[2][ti] - cc[2] : 0.0;
-        const double d2 = DIM == 3 ? g0 * g0 + g1 * g1 + g2 * g2 : g0 * g0 + g1 * g1;
-        double val;
-        if (FP32B) {
-            const float e0 = (float)(sm.stg[4][ti] + (fma(-a.halfs, d2, sm.stg[5][ti]) - KAPPA * Lref) * (1.0 / 16.0));
-            const float G0 = sf * (float)g0, G1 = sf * (float)g1, G2 = sf * (float)g2;
-            float acc0 = 0.f, acc1 = 0.f;
-            if (f.w_nonneg) {
-                int q = 0;
-                for (; q + 1 < nql; q += 2) {
-                    const float4 v0 = *reinterpret_cast<const float4 *>(sm.qb[qoff + q]);
-                    const float4 v1 = *reinterpret_cast<const float4 *>(sm.qb[qoff + q + 1]);
-                    float ea = fmaf(G0, v0.x, e0 + v0.w), eb = fmaf(G0, v1.x, e0 + v1.w);
-                    ea = fmaf(G1, v0.y, ea);
-                    eb = fmaf(G1, v1.y, eb);
-                    if (DIM == 3) {
-                        ea = fmaf(G2, v0.z, ea);
-                        eb = fmaf(G2, v1.z, eb);
-                    }
-                    acc0 += ex2_approx(ea);
-                    acc1 += ex2_approx(eb);
+    const double g0 = g[0], g1 = g[1], g2 = DIM == 3 ? g[2] : 0.0;
+    const double d2 = DIM == 3 ? g0 * g0 + g1 * g1 + g2 * g2 : g0 * g0 + g1 * g1;
+    if constexpr (FP32B) {
+        const float sf = (float)(a.s * (1.0 / 16.0));
+        const float e0 = (float)(lognu + (fma(-a.halfs, d2, sp) - KAPPA * Lref) * (1.0 / 16.0));
+        const float G0 = sf * (float)g0, G1 = sf * (float)g1, G2 = sf * (float)g2;
+        float acc0 = 0.f, acc1 = 0.f;
+        if (w_nonneg) {
+            int q = 0;
+            for (; q + 1 < nql; q += 2) {
+                const float4 v0 = *reinterpret_cast<const float4 *>(sm.qb[qoff + q]);
+                const float4 v1 = *reinterpret_cast<const float4 *>(sm.qb[qoff + q + 1]);
+                float ea = fmaf(G0, v0.x, e0 + v0.w), eb = fmaf(G0, v1.x, e0 + v1.w);
+                ea = fmaf(G1, v0.y, ea);
+                eb = fmaf(G1, v1.y, eb);
+                if (DIM == 3) {
+                    ea = fmaf(G2, v0.z, ea);
+                    eb = fmaf(G2, v1.z, eb);
                 }
-                if (q < nql) {
-                    const float4 v0 = *reinterpret_cast<const float4 *>(sm.qb[qoff + q]);
-                    float ea = fmaf(G0, v0.x, e0 + v0.w);
-                    ea = fmaf(G1, v0.y, ea);
-                    if (DIM == 3) ea = fmaf(G2, v0.z, ea);
-                    acc0 += ex2_approx(ea);
-                }
-            } else {
-                for (int q = 0; q < nql; ++q) {
-                    const float *qb = sm.qb[qoff + q];
-                    float e = fmaf(G0, qb[0], e0 + qb[3]);
-                    e = fmaf(G1, qb[1], e);
-                    if (DIM == 3) e = fmaf(G2, qb[2], e);
-                    acc0 = fmaf(sm.qw[qoff + q], ex2_approx(e), acc0);
-                }
+                acc0 += ex2_approx(ea);
+                acc1 += ex2_approx(eb);
             }
-            val = (double)(acc0 + acc1);
+            if (q < nql) {
+                const float4 v0 = *reinterpret_cast<const float4 *>(sm.qb[qoff + q]);
+                float ea = fmaf(G0, v0.x, e0 + v0.w);
+                ea = fmaf(G1, v0.y, ea);
+                if (DIM == 3) ea = fmaf(G2, v0.z, ea);
+                acc0 += ex2_approx(ea);
+            }
         } else {
-            const double U0 = 16.0 * sm.stg[4][ti] + fma(-a.halfs, d2, sm.stg[5][ti]) - KAPPA * Lref;
-            const double G0 = a.s * g0, G1 = a.s * g1, G2 = a.s * g2;
-            double acc = 0.0;
             for (int q = 0; q < nql; ++q) {
-                const double *dq = sm.qd[qoff + q];
-                const double L = sm.qL[qoff + q];
-                if (!isfinite(L)) continue;
-                double u = fma(G0, dq[0], U0 + dq[3] - KAPPA * (L - Lref));
-                u = fma(G1, dq[1], u);
-                if (DIM == 3) u = fma(G2, dq[2], u);
-                acc = fma(sm.qw[qoff + q], exp2_16(u, sm.tab), acc);
+                const float *qb = sm.qb[qoff + q];
+                float e = fmaf(G0, qb[0], e0 + qb[3]);
+                e = fmaf(G1, qb[1], e);
+                if (DIM == 3) e = fmaf(G2, qb[2], e);
+                acc0 = fmaf(sm.qw[qoff + q], ex2_approx(e), acc0);
             }
-            val = acc;
         }
-        sm.rows[wp][ti] = (typename PRow<FP32B>::T)val;
+        return acc0 + acc1;
+    } else {
+        const double U0 = 16.0 * lognu + fma(-a.halfs, d2, sp) - KAPPA * Lref;
+        const double G0 = a.s * g0, G1 = a.s * g1, G2 = a.s * g2;
+        double acc = 0.0;
+        for (int q = 0; q < nql; ++q) {
+            const double *dq = sm.qd[qoff + q];
+            const double L = sm.qL[qoff + q];
+            if (!isfinite(L)) continue;
+            double u = fma(G0, dq[0], U0 + dq[3] - KAPPA * (L - Lref));
+            u = fma(G1, dq[1], u);
+            if (DIM == 3) u = fma(G2, dq[2], u);
+            acc = fma(sm.qw[qoff + q], exp2_16(u, sm.tab), acc);
+        }
+        return acc;
     }
 }
 
@@ -759,8 +743,8 @@ __device__ __forceinline__ void value_pairs_tensor(SM &sm, int wp, int lane, int
             ub += fabs(ga[d]);
         }
         if (ub >= lb) {
-            const int at = atomicAdd(&sm.v.nnear[wp], 1);
-            if (at < FT_NEAR) sm.v.near_list[wp][at] = (unsigned short)ti;
+            const int at = atomicAdd(&sm.nnear[wp], 1);
+            if (at < FT_NEAR) sm.near_list[wp][at] = (unsigned short)ti;
         }
         if constexpr (TS >= 1) {
             double sga = 0.0;
@@ -813,13 +797,13 @@ __device__ __forceinline__ void near_maxima(const SM &sm, int wp, int lane, int 
 {
     constexpr int EP = 32 / NQ;
     const int q = lane % NQ, sub = lane / NQ;
-    const int n = sm.v.nnear[wp];
+    const int n = sm.nnear[wp];
     const bool all = n > FT_NEAR;
     const int cnt = all ? ncand : n;
     if (sub >= EP) return;
     const double *dq = sm.qd[qoff + q];
     for (int p = sub; p < cnt; p += EP) {
-        const int ti = all ? sm.cand[wp][p] : sm.v.near_list[wp][p];
+        const int ti = all ? sm.cand[wp][p] : sm.near_list[wp][p];
         const double g0 = sm.stg[0][ti] - cc[0], g1 = sm.stg[1][ti] - cc[1];
         const double g2 = DIM == 3 ? sm.stg[2][ti] - cc[2] : 0.0;
         const double d2 = DIM == 3 ? g0 * g0 + g1 * g1 + g2 * g2 : g0 * g0 + g1 * g1;
@@ -870,34 +854,28 @@ __device__ __forceinline__ float rcp_approx(float x)
     return y;
 }
 
-// FP32 gradient sweep on tensor-product points: per candidate
-// 2^(e0) sum_q W_q prod_d F_d[i_d], W_q = w_q 2^(D_q), summed dimension by
-// dimension (Horner order), into the warp's partial row.
-template <int DIM, int TM, int TS, class SM>
-__device__ __forceinline__ void grad_pairs_tensor(SM &sm, int wp, int lane, int ncand, int qoff,
-                                                  const double *cc, double Lref, const EvalArgs &a)
+// grad_term on tensor-product points: 2^(e0) sum_q W_q prod_d F_d[i_d],
+// W_q = w_q 2^(D_q), summed dimension by dimension (Horner order).  The FP64
+// form takes the factors relative to the lowest point.
+template <int DIM, int TM, int TS, bool FP32B, class SM>
+__device__ __forceinline__ typename PRow<FP32B>::T grad_term_tensor(const SM &sm, int qoff, const double *ahd,
+                                                                    const double *g, double lognu, double sp,
+                                                                    double Lref, const EvalArgs &a)
 {
     constexpr int NQ = DIM == 3 ? TM * TM * TM : TM * TM;
-    const float sf = (float)(a.s * (1.0 / 16.0));
-    float ah[3];
-    ah[0] = (float)sm.qd[qoff + (TM - 1) * tstride<TM, 0>()][0];
-    ah[1] = (float)sm.qd[qoff + (TM - 1) * tstride<TM, 1>()][1];
-    ah[2] = DIM == 3 ? (float)sm.qd[qoff + (TM - 1) * tstride<TM, 2>()][2] : 0.f;
-    float W[NQ];
+    using Row = typename PRow<FP32B>::T;
+    Row W[NQ];
 #pragma unroll
     for (int q = 0; q < NQ; ++q) W[q] = sm.qtw[qoff + q];
-    for (int p = lane; p < ncand; p += 32) {
-        const int ti = sm.cand[wp][p];
-        const double g0 = sm.stg[0][ti] - cc[0], g1 = sm.stg[1][ti] - cc[1];
-        const double g2 = DIM == 3 ? sm.stg[2][ti] - cc[2] : 0.0;
-        const double d2 = DIM == 3 ? g0 * g0 + g1 * g1 + g2 * g2 : g0 * g0 + g1 * g1;
-        float e0 = (float)(sm.stg[4][ti] + (fma(-a.halfs, d2, sm.stg[5][ti]) - KAPPA * Lref) * (1.0 / 16.0));
-        const float gd[3] = {(float)g0, (float)g1, (float)g2};
+    const double d2 = DIM == 3 ? g[0] * g[0] + g[1] * g[1] + g[2] * g[2] : g[0] * g[0] + g[1] * g[1];
+    if constexpr (FP32B) {
+        const float sf = (float)(a.s * (1.0 / 16.0));
+        float e0 = (float)(lognu + (fma(-a.halfs, d2, sp) - KAPPA * Lref) * (1.0 / 16.0));
         float F[3][TM];
         if constexpr (TS >= 1) {
 #pragma unroll
             for (int d = 0; d < DIM; ++d) {
-                const float ga = sf * gd[d] * ah[d];
+                const float ga = sf * (float)g[d] * (float)ahd[d];
                 e0 -= ga;
                 const float r = ex2_approx(TM == 2 ? 2.f * ga : ga);
                 F[d][0] = 1.f;
@@ -907,7 +885,7 @@ __device__ __forceinline__ void grad_pairs_tensor(SM &sm, int wp, int lane, int 
         } else {
 #pragma unroll
             for (int d = 0; d < DIM; ++d) {
-                const float xp = ex2_approx(sf * gd[d] * ah[d]);
+                const float xp = ex2_approx(sf * (float)g[d] * (float)ahd[d]);
                 F[d][0] = rcp_approx(xp);
                 F[d][TM - 1] = xp;
                 if (TM == 3) F[d][1] = 1.f;
@@ -936,30 +914,13 @@ __device__ __forceinline__ void grad_pairs_tensor(SM &sm, int wp, int lane, int 
                 w = fmaf(u, F[0][i0], w);
             }
         }
-        sm.rows[wp][ti] = ex2_approx(e0) * w;
-    }
-}
-
-// FP64 gradient sweep on tensor-product points: the same sums with FP64
-// factors relative to the lowest point (1 + DIM exponentials per candidate
-// instead of one per point).
-template <int DIM, int TM, class SM>
-__device__ __forceinline__ void grad_pairs_tensor64(SM &sm, int wp, int lane, int ncand, int qoff, const double *ah,
-                                                    const double *cc, double Lref, const EvalArgs &a)
-{
-    constexpr int NQ = DIM == 3 ? TM * TM * TM : TM * TM;
-    double W[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) W[q] = sm.qtw[qoff + q];
-    for (int p = lane; p < ncand; p += 32) {
-        const int ti = sm.cand[wp][p];
-        const double g[3] = {sm.stg[0][ti] - cc[0], sm.stg[1][ti] - cc[1], DIM == 3 ? sm.stg[2][ti] - cc[2] : 0.0};
-        const double d2 = DIM == 3 ? g[0] * g[0] + g[1] * g[1] + g[2] * g[2] : g[0] * g[0] + g[1] * g[1];
-        double U = 16.0 * sm.stg[4][ti] + fma(-a.halfs, d2, sm.stg[5][ti]) - KAPPA * Lref;
+        return ex2_approx(e0) * w;
+    } else {
+        double U = 16.0 * lognu + fma(-a.halfs, d2, sp) - KAPPA * Lref;
         double r[3];
 #pragma unroll
         for (int d = 0; d < DIM; ++d) {
-            const double ga = a.s * g[d] * ah[d];
+            const double ga = a.s * g[d] * ahd[d];
             U -= ga;
             r[d] = exp2_16(TM == 2 ? 2.0 * ga : ga, sm.tab);
         }
@@ -982,35 +943,59 @@ __device__ __forceinline__ void grad_pairs_tensor64(SM &sm, int wp, int lane, in
             }
             w = i0 == TM - 1 ? u : fma(w, r[0], u);
         }
-        sm.rows[wp][ti] = exp2_16(U, sm.tab) * w;
+        return exp2_16(U, sm.tab) * w;
     }
 }
 
-// CTA sum of the warp partial rows (warp order) and the write of every slot
-// of every pair of the chunk, forward positions k.. (zeros where a target was
-// not staged).
-template <bool FP32B, class SM>
-__device__ __forceinline__ void write_partials(SM &sm, const FusedArgs &f, int64_t k, int nt, int nunit)
+// Gradient sweep of the staged chunk (forward positions k..): thread <->
+// staged target, over the block's units in order (the unit terms, FP32 in the
+// hybrid mode, added in FP64), and the write of every slot of every pair
+// (zeros where a target was not staged).  The exact candidate test is taken
+// again per (cell, target) instead of a compacted list per cell: a target's
+// data stay in registers over the units and no partial rows go through
+// shared memory (rows, their zeroing and their sums, with the lists, were
+// two thirds of a re-staged chunk's instructions).
+template <int DIM, bool FP32B, int TQ, int TS, class SM>
+__device__ __forceinline__ void grad_chunk(SM &sm, const FusedArgs &f, int64_t k, int nt, int nunit,
+                                           const EvalArgs &a)
 {
     const int tid = threadIdx.x;
-    for (int i = tid; i < nt * TBLK_KD; i += blockDim.x) {
-        const int ti = i / TBLK_KD, sl = i - ti * TBLK_KD;
-        const int64_t base = (k + ti - f.part_base) * TBLK_KD;
-        const short p = sm.smap[ti][sl];
+    using Row = typename PRow<FP32B>::T;
+    const int64_t base = (k - f.part_base) * TBLK_KD;
+    Row *out = (FP32B ? reinterpret_cast<Row *>(f.part32) : reinterpret_cast<Row *>(f.part)) + base;
+    const int nstg = sm.nstg;
+    for (int p = tid; p < nstg; p += FT_WARPS * 32) {
+        const double y[3] = {sm.stg[0][p], sm.stg[1][p], DIM == 3 ? sm.stg[2][p] : 0.0};
+        const double lognu = sm.stg[4][p], sp = sm.stg[5][p];
         double v = 0.0;
-        if (p >= 0)
-            for (int w = 0; w < nunit; ++w) v += (double)sm.rows[w][p];
-        if constexpr (FP32B) f.part32[base + sl] = (float)v;
-        else f.part[base + sl] = v;
+#pragma unroll 2
+        for (int u = 0; u < nunit; ++u) {
+            const double *cc = sm.cellc[u];
+            const double Lref = sm.uL[u];
+            const double g[3] = {y[0] - cc[0], y[1] - cc[1], DIM == 3 ? y[2] - cc[2] : 0.0};
+            if (dist2_exact<DIM>(y, cc) <= a.sstar && isfinite(Lref)) {
+                const int cl = TQ > 0 ? u : u / a.ngroups, qoff = cl * a.qpc + (TQ > 0 ? 0 : (u - cl * a.ngroups) * a.ql);
+                Row t;
+                if constexpr (TQ > 0)
+                    t = grad_term_tensor<DIM, TQ, TS, FP32B>(sm, qoff, sm.uah[u], g, lognu, sp, Lref, a);
+                else
+                    t = grad_term<DIM, FP32B>(sm, f.w_nonneg, qoff, min(a.ql, (cl + 1) * a.qpc - qoff), g, lognu, sp,
+                                              Lref, a);
+                v += (double)t;
+            }
+        }
+        out[sm.dst[p]] = (Row)v;
     }
+    for (int i = tid; i < nt * TBLK_KD; i += FT_WARPS * 32)
+        if (!((sm.keep[i / TBLK_KD] >> (i % TBLK_KD)) & 1u)) out[i] = Row(0);
 }
 
 template <int DIM, int QL, bool FP32B, int MODE, int TQ, int TS>
-__global__ void __launch_bounds__(FT_WARPS * 32, fused_min_blocks(DIM, TQ, FP32B))
+__global__ void __launch_bounds__(FT_WARPS * 32, fused_min_blocks(TQ))
 k_fused(FusedArgs f, EvalArgs a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    using SMem = FTSmem<fused_cap(DIM, TQ, FP32B), typename PRow<FP32B>::T>;
+    using SMem = FTSmem<fused_cap(TQ), typename PRow<FP32B>::T>;
     SMem &sm = *reinterpret_cast<SMem *>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
     const int b = f.b0 + blockIdx.x;
@@ -1030,9 +1015,9 @@ k_fused(FusedArgs f, EvalArgs a)
     const double rc = (f.cullt + bs[3]) * (1.0 + 1e-12) + 1e-300;
     const double rcull2 = rc * rc;
     const int64_t k0 = f.fwd_off[b], k1 = f.fwd_off[b + 1];
-    for (int i = tid; i < ncell * 3; i += blockDim.x) {
-        const int c = i / 3, d = i - c * 3;
-        sm.cellc[c][d] = d < DIM ? f.cell_ctr[(cb0 + c) * DIM + d] : 0.0;
+    for (int i = tid; i < nunit * 3; i += blockDim.x) {
+        const int u = i / 3, d = i - u * 3;
+        sm.cellc[u][d] = d < DIM ? f.cell_ctr[(cb0 + u / a.ngroups) * DIM + d] : 0.0;
     }
     for (int i = tid; i < (int)min((int64_t)FT_PREF, k1 - k0); i += blockDim.x) {
         const int t = f.fwd_t[k0 + i];
@@ -1046,14 +1031,15 @@ k_fused(FusedArgs f, EvalArgs a)
         double dsq = 0.0;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            const double dl = d < DIM ? f.x[(qblk0 + i) * DIM + d] - sm.cellc[c][d] : 0.0;
+            const double dl = d < DIM ? f.x[(qblk0 + i) * DIM + d] - sm.cellc[c * a.ngroups][d] : 0.0;
             sm.qd[i][d] = dl;
             dsq += dl * dl;
         }
         sm.qd[i][3] = -a.halfs * dsq;
     }
     __syncthreads();
-    const double cc[3] = {sm.cellc[cl][0], sm.cellc[cl][1], sm.cellc[cl][2]};
+    const int wu = valid ? wp : 0;
+    const double cc[3] = {sm.cellc[wu][0], sm.cellc[wu][1], sm.cellc[wu][2]};
     // tensor points: the largest offset per dimension, and s times it
     double ah[3] = {0.0, 0.0, 0.0}, gh[3] = {0.0, 0.0, 0.0};
     if constexpr (TQ > 0) {
@@ -1062,10 +1048,10 @@ k_fused(FusedArgs f, EvalArgs a)
         if (DIM == 3) ah[2] = sm.qd[qoff + (TQ - 1) * tstride<TQ, 2>()][2];
 #pragma unroll
         for (int d = 0; d < DIM; ++d) gh[d] = a.s * ah[d];
+        if (valid && lane < 3) sm.uah[wp][lane] = lane == 0 ? ah[0] : (lane == 1 ? ah[1] : ah[2]);
     }
     int tail_off = -1;  // first entry (minus k0) of the value sweep's last chunk, still staged for the gradient sweep
     int tail_nt = 0;
-    int ncand_single = 0;
 
     // ---------------- value sweep ----------------
     {
@@ -1099,7 +1085,6 @@ k_fused(FusedArgs f, EvalArgs a)
             if (valid) {
                 double bmax, lb;
                 const int ncand = compact_candidates<DIM, TQ>(sm, wp, lane, nstg, cc, a, gh, bmax, lb);
-                ncand_single = ncand;
                 npairs += (double)ncand * nql;
                 if (MODE != 2 && bmax > -CUDART_INF) {
                     const double mnew = bmax + sr * dqmax;
@@ -1117,7 +1102,7 @@ k_fused(FusedArgs f, EvalArgs a)
                 }
                 if constexpr (TENS) {
                     if (lb > lb_run) lb_run = lb;
-                    if (lane == 0) sm.v.nnear[wp] = 0;
+                    if (lane == 0) sm.nnear[wp] = 0;
                     __syncwarp();
                     // the bounds' rounding: a few ulp of the exponents, far below 1e-12 of their range
                     const double lbr = lb_run - Munit;
@@ -1133,7 +1118,7 @@ k_fused(FusedArgs f, EvalArgs a)
             }
             k += nt;
             if (k >= k1) {
-                tail_off = (int)(k - nt - k0);  // kept staged (with each warp's candidates) for the gradient sweep
+                tail_off = (int)(k - nt - k0);  // kept staged for the gradient sweep
                 tail_nt = nt;
             } else {
                 __syncthreads();  // the next chunk overwrites the staged targets
@@ -1149,11 +1134,11 @@ k_fused(FusedArgs f, EvalArgs a)
 #pragma unroll
                 for (int e = 1; e < EP; ++e) m = fmax(m, __shfl_down_sync(0xffffffffu, mx[0], e * QL));
                 constexpr int LPQ = QL == 4 ? 8 : 4;   // lanes that hold a total
-                if (lane % LPQ == 0) sm.v.S[qoff + lane / LPQ] = tot;
-                if (QL == 9 && lane == 0) sm.v.S[qoff + QL - 1] = last;
+                if (lane % LPQ == 0) sm.qS[qoff + lane / LPQ] = tot;
+                if (QL == 9 && lane == 0) sm.qS[qoff + QL - 1] = last;
                 if (lane < QL) {
-                    sm.v.mx[qoff + lane] = m;
-                    sm.v.U[qoff + lane] = Munit;
+                    sm.qm[qoff + lane] = m;
+                    sm.qU[qoff + lane] = Munit;
                 }
             } else {
 #pragma unroll
@@ -1166,9 +1151,9 @@ k_fused(FusedArgs f, EvalArgs a)
                     const double Sw = warp_sum(sl);
                     if (lane == 0 && q < nql) {
                         const double m = MODE == 2 ? mxw : mxw + Munit;
-                        sm.v.S[qoff + q] = Sw;
-                        sm.v.mx[qoff + q] = m;
-                        sm.v.U[qoff + q] = m;   // the sum is relative to the maximum
+                        sm.qS[qoff + q] = Sw;
+                        sm.qm[qoff + q] = m;
+                        sm.qU[qoff + q] = m;   // the sum is relative to the maximum
                     }
                 }
             }
@@ -1179,9 +1164,9 @@ k_fused(FusedArgs f, EvalArgs a)
         double tv = 0.0, tcv = 0.0, tsk = 0.0;
         if (tid < nqb) {
             const int64_t qg = qblk0 + tid;
-            const double m = sm.v.mx[tid], U = sm.v.U[tid];
+            const double m = sm.qm[tid], U = sm.qU[tid];
             const double Sr =
-                (m == -CUDART_INF || U == -CUDART_INF) ? 0.0 : sm.v.S[tid] * (TENS ? exp2_16(U - m, sm.tab) : 1.0);
+                (m == -CUDART_INF || U == -CUDART_INF) ? 0.0 : sm.qS[tid] * (TENS ? exp2_16(U - m, sm.tab) : 1.0);
             double L;
             int sk;
             value_epilogue(a, m, Sr, sm.qd[tid][3], f.rho[qg], f.jxw[qg], tv, tcv, L, sk);
@@ -1215,49 +1200,21 @@ k_fused(FusedArgs f, EvalArgs a)
         if (TQ > 0) sm.qtw[i] = (Row)(wq * exp2(D));
     }
     __syncthreads();
-    const double Lref = valid ? sm.uL[wp] : CUDART_INF;
     // The value sweep's last chunk (the only one when everything fit) is still
-    // staged with each warp's candidates: its gradient comes first, then the
-    // earlier chunks are staged again (the same chunks: the greedy rule over
-    // [k0, k0 + tail_off) ends where the value sweep's did).  Every pair's partial
-    // is written once, so the order of the chunks does not change any sum.
+    // staged: its gradient comes first, then the earlier chunks are staged again
+    // (the same chunks: the greedy rule over [k0, k0 + tail_off) ends where the
+    // value sweep's did).  Every pair's partial is written once, so the order of
+    // the chunks does not change any sum.
     int64_t kend = k1;
     if (tail_off >= 0) {
-        const int nt = tail_nt;
-        const int nstg = sm.nstg;
-        if (valid) {
-            for (int t = lane; t < nstg; t += 32) sm.rows[wp][t] = 0;
-            __syncwarp();
-            if (isfinite(Lref)) {
-                if constexpr (TQ > 0 && FP32B) grad_pairs_tensor<DIM, TQ, TS>(sm, wp, lane, ncand_single, qoff, cc, Lref, a);
-                else if constexpr (TQ > 0) grad_pairs_tensor64<DIM, TQ>(sm, wp, lane, ncand_single, qoff, ah, cc, Lref, a);
-                else grad_pairs<DIM, FP32B>(sm, f, wp, lane, ncand_single, qoff, nql, cc, Lref, qblk0, a);
-            }
-        }
-        __syncthreads();
-        write_partials<FP32B>(sm, f, k0 + tail_off, nt, nunit);
-        if (tail_off == 0) return;
+        grad_chunk<DIM, FP32B, TQ, TS>(sm, f, k0 + tail_off, tail_nt, nunit, a);
         kend = k0 + tail_off;
-        __syncthreads();  // the earlier chunks overwrite the staged targets
     }
     for (int64_t k = k0; k < kend;) {
+        __syncthreads();  // the staged targets are consumed
         const int nt = stage_chunk<DIM>(sm, f, k0, k, kend, bc, rcull2);
-        const int nstg = sm.nstg;
-        if (valid) {
-            double bmax, lb;
-            const int ncand = compact_candidates<DIM, 0>(sm, wp, lane, nstg, cc, a, gh, bmax, lb);
-            for (int t = lane; t < nstg; t += 32) sm.rows[wp][t] = 0;
-            __syncwarp();
-            if (isfinite(Lref)) {
-                if constexpr (TQ > 0 && FP32B) grad_pairs_tensor<DIM, TQ, TS>(sm, wp, lane, ncand, qoff, cc, Lref, a);
-                else if constexpr (TQ > 0) grad_pairs_tensor64<DIM, TQ>(sm, wp, lane, ncand, qoff, ah, cc, Lref, a);
-                else grad_pairs<DIM, FP32B>(sm, f, wp, lane, ncand, qoff, nql, cc, Lref, qblk0, a);
-            }
-        }
-        __syncthreads();
-        write_partials<FP32B>(sm, f, k, nt, nunit);
+        grad_chunk<DIM, FP32B, TQ, TS>(sm, f, k, nt, nunit, a);
         k += nt;
-        __syncthreads();
     }
 }
 
@@ -1331,8 +1288,8 @@ static void launch_fused(sdot_ctx *c, const FusedArgs &f, const EvalArgs &a, siz
 template <int DIM, int QL, int MODE, int TQ = 0, int TS = 0>
 static void dispatch_fused_b(sdot_ctx *c, const FusedArgs &f, const EvalArgs &a, bool fp32b, int nb)
 {
-    if (fp32b) launch_fused<DIM, QL, true, MODE, TQ, TS>(c, f, a, sizeof(FTSmem<fused_cap(DIM, TQ, true), float>), nb);
-    else launch_fused<DIM, QL, false, MODE, TQ, TS>(c, f, a, sizeof(FTSmem<fused_cap(DIM, TQ, false), double>), nb);
+    if (fp32b) launch_fused<DIM, QL, true, MODE, TQ, TS>(c, f, a, sizeof(FTSmem<fused_cap(TQ), float>), nb);
+    else launch_fused<DIM, QL, false, MODE, TQ, TS>(c, f, a, sizeof(FTSmem<fused_cap(TQ), double>), nb);
 }
 
 template <int DIM, int MODE>
