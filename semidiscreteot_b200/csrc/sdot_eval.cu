@@ -234,18 +234,17 @@ k_lat_grad(LatArgs L, EvalArgs a, const double *__restrict__ tpack, const double
                         gpart + blockIdx.y * a.nt);
 }
 
-// truncated-path layout: {y(3), nu, log2 nu, kappa psi / eps}
+// truncated-path layout: component after component (y(3), nu, log2 nu, kappa psi / eps), nt doubles each
 template <int DIM>
 __global__ void k_target_prep_kd(int64_t nt, const double *__restrict__ y, const double *__restrict__ nu,
                                  const double *__restrict__ psi, EvalArgs a, double *__restrict__ tpack)
 {
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < nt; j += (int64_t)gridDim.x * blockDim.x) {
-        double *t = tpack + j * TPACK;
 #pragma unroll
-        for (int d = 0; d < 3; ++d) t[d] = d < DIM ? y[j * DIM + d] : 0.0;
-        t[3] = nu[j];
-        t[4] = log2(nu[j]);
-        t[5] = a.s * psi[j];
+        for (int d = 0; d < 3; ++d) tpack[d * nt + j] = d < DIM ? y[j * DIM + d] : 0.0;
+        tpack[3 * nt + j] = nu[j];
+        tpack[4 * nt + j] = log2(nu[j]);
+        tpack[5 * nt + j] = a.s * psi[j];
     }
 }
 

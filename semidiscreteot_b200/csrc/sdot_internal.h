@@ -10,7 +10,7 @@
 //   tpack[j], 8 doubles: dense path {A_j, B_j(dim), nu_j, y_j(dim)} where the
 //     scaled exponent is b_qj = A_j + B_j.xt_q + C_q = kappa*(psi_j-|x_q-y_j|^2/2)/eps,
 //     kappa = 16/ln 2 (units of 2^(1/16)), xt = x - origin; truncated path
-//     {y_j(3), nu_j, log2 nu_j, kappa psi_j / eps};
+//     y_j(3), nu_j, log2 nu_j, kappa psi_j / eps, component after component;
 //   Lq[q] = log of the reference's total_sum_exp at q (natural units, +inf if
 //     the point is skipped), written by the value sweep and read by the
 //     gradient sweep.

@@ -65,7 +65,8 @@ constexpr int FT_PREF = 192;                // forward entries of a block prefet
 
 struct FusedArgs {
     const double *x, *rho, *jxw, *w, *cell_ctr;
-    const double *tpk;           // per target: y(3), nu, log2 nu, s*psi, -, -
+    const double *tpk;           // y(3), nu, log2 nu, s*psi of all targets, component after component
+    int64_t nt;                  // targets
     const int64_t *sblk_cell;    // source block -> first cell (nsblk + 1)
     const double *sblk_sph;      // FP64 centre(3), radius
     const int64_t *tblk_off;     // target block -> first target (ntblk + 1)
@@ -457,11 +458,11 @@ __device__ int stage_chunk(SM &sm, const FusedArgs &f, int64_t kb, int64_t k0, i
                 jj[s] = j0;
                 bool keep = false;
                 if (lane < sz) {
-                    const double *tp = f.tpk + (j0 + lane) * TPACK;
+                    const double *tp = f.tpk + j0 + lane;
                     double d2 = 0.0;
 #pragma unroll
                     for (int d = 0; d < DIM; ++d) {
-                        const double q = tp[d] - bc[d];
+                        const double q = tp[d * f.nt] - bc[d];
                         d2 += q * q;
                     }
                     keep = d2 <= rcull2;
@@ -505,9 +506,9 @@ __device__ int stage_chunk(SM &sm, const FusedArgs &f, int64_t kb, int64_t k0, i
                 if (keep) {
                     const int pos = sm.epre[idx] + __popc(bal[s] & ((1u << lane) - 1u));
                     sm.dst[pos] = (unsigned short)(slot * TBLK_KD + lane);
-                    const double *tp = f.tpk + (j0 + lane) * TPACK;
+                    const double *tp = f.tpk + j0 + lane;
 #pragma unroll
-                    for (int d = 0; d < FT_TS; ++d) sm.stg[d][pos] = tp[d];
+                    for (int d = 0; d < FT_TS; ++d) sm.stg[d][pos] = tp[d * f.nt];
                 }
                 if (lane == 0) sm.keep[slot] = bal[s];
             }
@@ -1453,7 +1454,7 @@ sdot_status run_trunc(sdot_ctx *c, const EvalArgs &a, double r)
     if (e != cudaSuccess) return cuda_error(c, e, "pair list join");
     FusedArgs f{};
     f.x = c->x.p; f.rho = c->rho.p; f.jxw = c->jxw.p; f.w = c->w.p; f.cell_ctr = c->cell_ctr.p;
-    f.tpk = c->tpack.p; f.sblk_cell = c->sblk_cell.p; f.sblk_sph = c->sblk_sph.p; f.tblk_off = c->tblk_off.p;
+    f.tpk = c->tpack.p; f.nt = c->nt; f.sblk_cell = c->sblk_cell.p; f.sblk_sph = c->sblk_sph.p; f.tblk_off = c->tblk_off.p;
     f.fwd_off = c->fwd_off.p; f.fwd_t = c->fwd_t.p;
     f.part = c->part.p; f.part32 = reinterpret_cast<float *>(c->part.p); f.Lq = c->Lq.p; f.valpart = c->blkpart.p;
     f.cullt = std::isnan(r) ? 0.0 : std::min(r, 1e300);
