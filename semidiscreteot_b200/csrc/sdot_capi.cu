@@ -91,13 +91,22 @@ cudaError_t update_geometry(sdot_ctx *c)
     double sc = 1e-30;
     for (int d = 0; d < c->dim; ++d) sc = std::max(sc, std::max(std::fabs(lo[d]), std::fabs(hi[d])));
     c->coord_scale = sc;
-    // conservative FP32 spheres depend on the common coordinate scale
-    std::vector<float4> s32(c->nsblk), t32(c->ntblk);
-    for (int64_t b = 0; b < c->nsblk; ++b) s32[b] = sphere32(&c->src_sph_host[b * 4], sc);
-    for (int64_t b = 0; b < c->ntblk; ++b) t32[b] = sphere32(&c->tgt_sph_host[b * 4], sc);
-    cudaError_t e = cudaMemcpy(c->sblk_sph32.p, s32.data(), s32.size() * sizeof(float4), cudaMemcpyHostToDevice);
+    // conservative FP32 boxes depend on the common coordinate scale
+    auto boxes = [&](const std::vector<double> &box, int64_t nb, std::vector<float4> &out) {
+        const double m = 1e-6 * sc;
+        out.resize(2 * nb);
+        for (int64_t b = 0; b < nb; ++b) {
+            const double *p = &box[b * 6];
+            out[2 * b] = make_float4((float)(p[0] - m), (float)(p[1] - m), (float)(p[2] - m), 0.f);
+            out[2 * b + 1] = make_float4((float)(p[3] + m), (float)(p[4] + m), (float)(p[5] + m), 0.f);
+        }
+    };
+    std::vector<float4> s32, t32;
+    boxes(c->src_box_host, c->nsblk, s32);
+    boxes(c->tgt_box_host, c->ntblk, t32);
+    cudaError_t e = cudaMemcpy(c->sblk_box32.p, s32.data(), s32.size() * sizeof(float4), cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
-        e = cudaMemcpy(c->tblk_sph32.p, t32.data(), t32.size() * sizeof(float4), cudaMemcpyHostToDevice);
+        e = cudaMemcpy(c->tblk_box32.p, t32.data(), t32.size() * sizeof(float4), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return e;
     // super-blocks of 32 consecutive blocks: sphere containing the member spheres
     auto supers = [&](const std::vector<double> &sph, int64_t nb, std::vector<float4> &out) {
@@ -138,9 +147,9 @@ cudaError_t update_geometry(sdot_ctx *c)
 size_t device_bytes(const sdot_ctx *c)
 {
     return c->x.bytes() + c->rho.bytes() + c->jxw.bytes() + c->w.bytes() + c->cell_ctr.bytes() +
-           c->sblk_sph.bytes() + c->sblk_sph32.bytes() + c->sblk_cell.bytes() + c->tblk_off.bytes() +
+           c->sblk_sph.bytes() + c->sblk_box32.bytes() + c->sblk_cell.bytes() + c->tblk_off.bytes() +
            c->lat_buf.bytes() +
-           c->tblk_sph32.bytes() + c->part.bytes() + c->fwd_t.bytes() + c->pmask.bytes() +
+           c->tblk_box32.bytes() + c->part.bytes() + c->fwd_t.bytes() + c->pmask.bytes() +
            c->inv_b.bytes() + c->inv_k.bytes() + c->inv_tmpb.bytes() + c->inv_tmpk.bytes() + c->inv_off.bytes() +
            c->y.bytes() + c->nu.bytes() + c->perm.bytes() +
            c->tblk_sph.bytes() + c->psi.bytes() + c->grad.bytes() + c->tpack.bytes() + c->Lq.bytes() +
@@ -436,9 +445,9 @@ void sdot_destroy(sdot_ctx *c)
         if (c->stream) cudaStreamSynchronize(c->stream);
         if (c->side) cudaStreamSynchronize(c->side);
         c->x.release(); c->rho.release(); c->jxw.release(); c->w.release();
-        c->cell_ctr.release(); c->sblk_sph.release(); c->sblk_sph32.release(); c->sblk_cell.release();
-        c->tblk_off.release(); c->tblk_sph32.release(); c->part.release(); c->fwd_t.release();
-        c->fwd_cnt.release(); c->fwd_off.release(); c->shit.release(); c->scount.release();
+        c->cell_ctr.release(); c->sblk_sph.release(); c->sblk_box32.release(); c->sblk_cell.release();
+        c->tblk_off.release(); c->tblk_box32.release(); c->part.release(); c->fwd_t.release();
+        c->fwd_cnt.release(); c->fwd_off.release(); c->fwd_hist.release(); c->fwd_order.release(); c->shit.release(); c->scount.release();
         c->inv_cnt.release(); c->inv_off.release(); c->inv_b.release(); c->inv_k.release();
         c->inv_tmpb.release(); c->inv_tmpk.release();
         c->pmask.release(); c->superpair.release(); c->ssup_sph32.release(); c->tsup_sph32.release();
@@ -589,11 +598,11 @@ sdot_status sdot_set_source(sdot_ctx *c, int dim, int64_t n_q, const double *x, 
     c->tensor_uniform = uni;
     for (int d = 0; d < 3; ++d) c->tensor_a[d] = (uni && d < dim) ? ahi[d] : 0.0;
     const int64_t nsblk = (int64_t)bounds.size() - 1;
-    std::vector<double> ssph(nsblk * 4);
+    std::vector<double> ssph(nsblk * 4), sbox(nsblk * 6);
     for (int64_t b = 0; b < nsblk; ++b) {
         std::vector<int64_t> cells;
         for (int64_t k = bounds[b]; k < bounds[b + 1]; ++k) cells.push_back(k);
-        sphere_of(hc.data(), cells, dim, &ssph[b * 4]);
+        sphere_of(hc.data(), cells, dim, &ssph[b * 4], &sbox[b * 6]);
     }
     c->dim = dim;
     c->nq = n_q;
@@ -627,7 +636,7 @@ sdot_status sdot_set_source(sdot_ctx *c, int dim, int64_t n_q, const double *x, 
     CK(c->w.alloc(n_q), "alloc w");
     CK(c->cell_ctr.alloc(n_cells * dim), "alloc cells");
     CK(c->sblk_sph.alloc(nsblk * 4), "alloc spheres");
-    CK(c->sblk_sph32.alloc(nsblk), "alloc spheres");
+    CK(c->sblk_box32.alloc(2 * nsblk), "alloc boxes");
     CK(c->sblk_cell.alloc(nsblk + 1), "alloc blocks");
     CK(cudaMemcpy(c->x.p, hx.data(), hx.size() * 8, cudaMemcpyHostToDevice), "copy x");
     CK(cudaMemcpy(c->rho.p, hr.data(), hr.size() * 8, cudaMemcpyHostToDevice), "copy rho");
@@ -659,6 +668,7 @@ sdot_status sdot_set_source(sdot_ctx *c, int dim, int64_t n_q, const double *x, 
         c->lat_ok = true;
     }
     c->src_sph_host = ssph;
+    c->src_box_host = sbox;
     c->covering_radius = 0.0;  // reference: recomputed by the next solve
     c->nq = n_q;
     c->ncells = n_cells;
@@ -691,18 +701,18 @@ sdot_status sdot_set_target(sdot_ctx *c, int64_t n, const double *y, const doubl
         hn[k] = nu[ord[k]];
     }
     const int64_t ntblk = (int64_t)bounds.size() - 1;
-    std::vector<double> tsph(ntblk * 4);
+    std::vector<double> tsph(ntblk * 4), tbox(ntblk * 6);
     for (int64_t b = 0; b < ntblk; ++b) {
         std::vector<int64_t> idx;
         for (int64_t k = bounds[b]; k < bounds[b + 1]; ++k) idx.push_back(k);
-        sphere_of(hy.data(), idx, dim, &tsph[b * 4]);
+        sphere_of(hy.data(), idx, dim, &tsph[b * 4], &tbox[b * 6]);
     }
     c->nt = 0;  // no usable target until its buffers are in place (see set_source)
     CK(c->y.alloc(n * dim), "alloc y");
     CK(c->nu.alloc(n), "alloc nu");
     CK(c->perm.alloc(n), "alloc perm");
     CK(c->tblk_sph.alloc(ntblk * 4), "alloc spheres");
-    CK(c->tblk_sph32.alloc(ntblk), "alloc spheres");
+    CK(c->tblk_box32.alloc(2 * ntblk), "alloc boxes");
     CK(c->tblk_off.alloc(ntblk + 1), "alloc blocks");
     CK(cudaMemcpy(c->y.p, hy.data(), hy.size() * 8, cudaMemcpyHostToDevice), "copy y");
     CK(cudaMemcpy(c->nu.p, hn.data(), hn.size() * 8, cudaMemcpyHostToDevice), "copy nu");
@@ -710,6 +720,7 @@ sdot_status sdot_set_target(sdot_ctx *c, int64_t n, const double *y, const doubl
     CK(cudaMemcpy(c->tblk_sph.p, tsph.data(), tsph.size() * 8, cudaMemcpyHostToDevice), "copy spheres");
     CK(cudaMemcpy(c->tblk_off.p, bounds.data(), bounds.size() * 8, cudaMemcpyHostToDevice), "copy blocks");
     c->tgt_sph_host = tsph;
+    c->tgt_box_host = tbox;
     c->nt = n;
     c->ntblk = ntblk;
     c->nu_host.assign(nu, nu + n);

@@ -160,10 +160,11 @@ struct sdot_ctx {
     int64_t nsblk = 0;                 // source blocks (k-d leaves)
     sdot::DevBuf<int64_t> sblk_cell;   // first cell of each block (nsblk + 1)
     sdot::DevBuf<double> sblk_sph;     // 4 per block: centre(3), radius (FP64)
-    sdot::DevBuf<float4> sblk_sph32;   // conservative FP32 spheres
+    sdot::DevBuf<float4> sblk_box32;   // conservative FP32 boxes of the cell centres (lo, hi per block)
     int ql = 0, ngroups = 1;           // quadrature points per warp unit, units per cell
     std::vector<double> cell_ctr_host; // internal order, for the covering radius
     std::vector<double> src_sph_host, tgt_sph_host;  // FP64 block spheres (4 per block)
+    std::vector<double> src_box_host, tgt_box_host;  // and boxes (6 per block)
     double src_lo[3] = {0, 0, 0}, src_hi[3] = {0, 0, 0};
 
     // ---- target (internal order) ----
@@ -173,7 +174,7 @@ struct sdot_ctx {
     int64_t ntblk = 0;                 // target blocks (k-d leaves)
     sdot::DevBuf<int64_t> tblk_off;    // first target of each block (ntblk + 1)
     sdot::DevBuf<double> tblk_sph;     // 4 per block
-    sdot::DevBuf<float4> tblk_sph32;
+    sdot::DevBuf<float4> tblk_box32;   // conservative FP32 boxes of the targets (lo, hi per block)
     std::vector<double> nu_host;       // caller order
     double nu_min = 0.0;               // min of nu_host (set with the targets)
     std::vector<double> y_host;        // caller order
@@ -197,7 +198,7 @@ struct sdot_ctx {
 
     // ---- truncated path: block-pair lists and gradient partials ----
     sdot::DevBuf<int64_t> fwd_cnt, fwd_off, inv_cnt, inv_off, inv_k;
-    sdot::DevBuf<int> fwd_t, inv_b, shit, scount, inv_tmpb;
+    sdot::DevBuf<int> fwd_t, fwd_hist, fwd_order, inv_b, shit, scount, inv_tmpb;
     sdot::DevBuf<int64_t> inv_tmpk;    // inverse-list scatter (forward position per entry)
     sdot::DevBuf<unsigned> pmask;
     sdot::DevBuf<unsigned char> superpair;

@@ -72,8 +72,9 @@ inline std::vector<int64_t> kd_order(const std::vector<double> &pts, int dim, in
     return dim == 2 ? kd_order_of<2>(pts, n, leaf, bounds) : kd_order_of<3>(pts, n, leaf, bounds);
 }
 
-// Bounding sphere (bbox centre, max distance, enlarged by 1e-12 relative).
-inline void sphere_of(const double *pts, const std::vector<int64_t> &idx, int dim, double *out)
+// Bounding sphere (bbox centre, max distance, enlarged by 1e-12 relative);
+// box (may be null): the bounding box, lo(3) and hi(3), 0 past dim.
+inline void sphere_of(const double *pts, const std::vector<int64_t> &idx, int dim, double *out, double *box = nullptr)
 {
     double lo[3] = {DBL_MAX, DBL_MAX, DBL_MAX}, hi[3] = {-DBL_MAX, -DBL_MAX, -DBL_MAX};
     for (int64_t i : idx)
@@ -83,6 +84,11 @@ inline void sphere_of(const double *pts, const std::vector<int64_t> &idx, int di
         }
     double c[3] = {0, 0, 0};
     for (int d = 0; d < dim; ++d) c[d] = 0.5 * (lo[d] + hi[d]);
+    if (box)
+        for (int d = 0; d < 3; ++d) {
+            box[d] = d < dim ? lo[d] : 0.0;
+            box[3 + d] = d < dim ? hi[d] : 0.0;
+        }
     double R = 0.0;
     for (int64_t i : idx) {
         double s = 0.0;

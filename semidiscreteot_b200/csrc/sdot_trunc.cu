@@ -11,8 +11,10 @@
 // bounding sphere (FP64 and a conservative FP32 copy).
 //
 // Per evaluation:
-//   1. block-pair lists.  (b, t) is a pair iff dist(c_b, c_t) <= r + R_b + R_t
-//      (FP32, conservatively enlarged).  The forward list (per b, t ascending)
+//   1. block-pair lists.  (b, t) is a pair iff the box of b's cell centres is
+//      within r of the box of t's targets (FP32, conservatively enlarged;
+//      super-blocks by their spheres).  With the blocks' spheres in place of
+//      their boxes a third more pairs were listed, staged and reduced.  The forward list (per b, t ascending)
 //      is filled from masks; the inverse list (per t, b ascending, with the
 //      pairs' forward positions) is its transpose, built on a second stream
 //      beside step 2, which does not need it.
@@ -61,6 +63,7 @@ constexpr int FT_TS = 6;                    // doubles per staged target: y(3), 
 constexpr int FT_MAXT = 96;                 // target blocks per chunk
 constexpr int FT_MAXQ = 80;                 // quadrature points of one source block
 constexpr int SUPER = 32;                   // blocks per super-block of the pair-list hierarchy
+constexpr int ORDER_BUCKETS = 256;          // weight classes of the source blocks (the sweeps' order)
 constexpr int FT_PREF = 192;                // forward entries of a block prefetched into smem
 
 struct FusedArgs {
@@ -77,6 +80,7 @@ struct FusedArgs {
     double *Lq;                  // per q (written by the value sweep)
     double *valpart;             // per source block: value, C, skipped, pairs
     int w_nonneg;                // all w_q >= 0: log2 w_q folded into the FP32 exponent
+    const int *order;            // source block of each CTA (null: b0, b0 + 1, ...)
     int b0;                      // first source block of the launch
     int64_t part_base;           // forward position of its first pair
     double cullt;                // per-target cull radius addend (r, enlarged)
@@ -119,8 +123,6 @@ template <> struct PRow<true> { using T = float; };
 // block-pair lists
 // ---------------------------------------------------------------------------
 
-// Rounded operation by operation (no contraction): the forward and inverse
-// list kernels must reach bitwise identical decisions.
 __device__ __forceinline__ bool pair_test(float4 s, float4 t, float cr)
 {
     const float dx = __fsub_rn(s.x, t.x), dy = __fsub_rn(s.y, t.y), dz = __fsub_rn(s.z, t.z);
@@ -143,11 +145,12 @@ k_super_pairs(const float4 *__restrict__ ssph, int nss, const float4 *__restrict
 }
 
 // Warp <-> source super-block: its paired target super-blocks in ascending
-// order (shit[si * nts + h]) and their count.
+// order (shit[si * nts + h]) and their count; hist is cleared.
 __global__ void __launch_bounds__(256)
 k_super_compact(const unsigned char *__restrict__ sp, int nss, int nts, int *__restrict__ shit,
-                int *__restrict__ scount)
+                int *__restrict__ scount, int *__restrict__ hist)
 {
+    if (blockIdx.x == 0 && threadIdx.x < ORDER_BUCKETS) hist[threadIdx.x] = 0;
     const int si = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if (si >= nss) return;
@@ -163,36 +166,76 @@ k_super_compact(const unsigned char *__restrict__ sp, int nss, int nts, int *__r
     if (lane == 0) scount[si] = h;
 }
 
-// Warp <-> source block b: for each paired target super-block h, the 32-bit
-// mask of its target blocks t with pair_test(b, t); cnt[b] = total.
-__global__ void __launch_bounds__(256)
-k_fwd_masks(const float4 *__restrict__ sph, int nsb, const float4 *__restrict__ tph, int ntb, int nts, int hmax,
-            float cr, const int *__restrict__ shit, const int *__restrict__ scount, unsigned *__restrict__ mask,
-            int64_t *__restrict__ cnt)
+// Whether two boxes are within cr of each other.
+__device__ __forceinline__ bool box_test(float4 slo, float4 shi, float4 tlo, float4 thi, float cr)
 {
-    const int b = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
+    const float dx = fmaxf(0.f, fmaxf(tlo.x - shi.x, slo.x - thi.x));
+    const float dy = fmaxf(0.f, fmaxf(tlo.y - shi.y, slo.y - thi.y));
+    const float dz = fmaxf(0.f, fmaxf(tlo.z - shi.z, slo.z - thi.z));
+    return dx * dx + dy * dy + dz * dz <= cr * cr;
+}
+
+// Bucket of a source block with c of at most ntb pairs in the order of the
+// sweeps, the heaviest blocks first.  Clustered targets make some blocks many
+// times the average; started last, they left a quarter of the SM time of a
+// launch idle (4,096 blocks x 100,000 targets).
+__device__ __forceinline__ int order_bucket(int c, int ntb)
+{
+    return ORDER_BUCKETS - 1 - min(ORDER_BUCKETS - 1, (int)((int64_t)c * ORDER_BUCKETS / (ntb + 1)));
+}
+
+// Warp <-> FM_B consecutive source blocks (of one super-block): for each
+// paired target super-block h, the 32-bit mask of its target blocks t with
+// box_test(b, t); cnt[b] = total, hist[bucket of b] counts the blocks.
+constexpr int FM_B = 4;
+__global__ void __launch_bounds__(256)
+k_fwd_masks(const float4 *__restrict__ sbox, int nsb, const float4 *__restrict__ tbox, int ntb, int nts, int hmax,
+            float cr, const int *__restrict__ shit, const int *__restrict__ scount, unsigned *__restrict__ mask,
+            int64_t *__restrict__ cnt, int *__restrict__ hist)
+{
+    const int b0 = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * FM_B;
     const int lane = threadIdx.x & 31;
-    if (b >= nsb) return;
-    const float4 me = sph[b];
-    const int si = b / SUPER;
+    if (b0 >= nsb) return;
+    static_assert(SUPER % FM_B == 0, "the warp's blocks share a super-block");
+    float4 slo[FM_B], shi[FM_B];
+    int k[FM_B];
+#pragma unroll
+    for (int i = 0; i < FM_B; ++i) {
+        const int b = min(b0 + i, nsb - 1);
+        slo[i] = sbox[2 * b];
+        shi[i] = sbox[2 * b + 1];
+        k[i] = 0;
+    }
+    const int si = b0 / SUPER;
     const int nh = scount[si];
-    int k = 0;
+#pragma unroll 2
     for (int h = 0; h < nh; ++h) {
         const int t = shit[(int64_t)si * nts + h] * SUPER + lane;
-        const bool hit = t < ntb && pair_test(me, tph[t], cr);
-        const unsigned bal = __ballot_sync(0xffffffffu, hit);
-        if (lane == 0) mask[(int64_t)b * hmax + h] = bal;
-        k += __popc(bal);
+        const float4 tlo = tbox[2 * min(t, ntb - 1)], thi = tbox[2 * min(t, ntb - 1) + 1];
+#pragma unroll
+        for (int i = 0; i < FM_B; ++i) {
+            const bool hit = t < ntb && box_test(slo[i], shi[i], tlo, thi, cr);
+            const unsigned bal = __ballot_sync(0xffffffffu, hit);
+            if (lane == i && b0 + i < nsb) mask[(int64_t)(b0 + i) * hmax + h] = bal;
+            k[i] += __popc(bal);
+        }
     }
-    if (lane == 0) cnt[b] = k;
+#pragma unroll
+    for (int i = 0; i < FM_B; ++i)
+        if (lane == i && b0 + i < nsb) {
+            cnt[b0 + i] = k[i];
+            atomicAdd(&hist[order_bucket(k[i], ntb)], 1);
+        }
 }
 
 // Forward lists from the masks: fwd_t[fwd_off[b] ..] = paired t, ascending.
+// order: the blocks by bucket (hist: the buckets' first positions, advanced).
 // Inverse lists are the forward lists transposed (the same pair set by
 // construction).
 __global__ void __launch_bounds__(256)
 k_fwd_fill(int nsb, int nts, int hmax, const int *__restrict__ shit, const int *__restrict__ scount,
-           const unsigned *__restrict__ mask, const int64_t *__restrict__ fwd_off, int *__restrict__ fwd_t)
+           const unsigned *__restrict__ mask, const int64_t *__restrict__ fwd_off, int *__restrict__ fwd_t, int ntb,
+           int *__restrict__ hist, int *__restrict__ order)
 {
     const int b = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
@@ -205,6 +248,8 @@ k_fwd_fill(int nsb, int nts, int hmax, const int *__restrict__ shit, const int *
         if ((bal >> lane) & 1u) fwd_t[k + __popc(bal & ((1u << lane) - 1u))] = shit[(int64_t)si * nts + h] * SUPER + lane;
         k += __popc(bal);
     }
+    // (the blocks of a bucket in any order: no result depends on it)
+    if (lane == 0) order[atomicAdd(&hist[order_bucket((int)(k - fwd_off[b]), ntb)], 1)] = b;
 }
 
 // Warp <-> source block b, lanes over its forward entries: count the pairs of
@@ -364,9 +409,11 @@ k_inv_order(int nsb, const int64_t *__restrict__ inv_off, const int *__restrict_
 }
 
 // exclusive scan of n counts into off[0..n] (single CTA, order-fixed)
-// total_host (may be null): the total, for the host
+// total_host (may be null): the total, for the host; hist (may be null): bucket
+// counts, replaced by the buckets' first positions
 __global__ void __launch_bounds__(1024)
-k_scan(const int64_t *__restrict__ cnt, int64_t n, int64_t *__restrict__ off, double *__restrict__ total_host)
+k_scan(const int64_t *__restrict__ cnt, int64_t n, int64_t *__restrict__ off, double *__restrict__ total_host,
+       int *__restrict__ hist)
 {
     // passes of 1,024 x SP counts: each thread loads SP consecutive counts at
     // once (the CTA is bound by load latency), the thread sums are scanned by
@@ -413,6 +460,27 @@ k_scan(const int64_t *__restrict__ cnt, int64_t n, int64_t *__restrict__ off, do
     if (tid == 0) {
         off[n] = (int64_t)carry;
         if (total_host) *total_host = (double)carry;
+    }
+    if (hist && w == 31) {
+        constexpr int PER = ORDER_BUCKETS / 32;
+        int h[PER], sum = 0;
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            h[k] = hist[lane * PER + k];
+            sum += h[k];
+        }
+        int x = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        x -= sum;
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            hist[lane * PER + k] = x;
+            x += h[k];
+        }
     }
 }
 
@@ -999,7 +1067,7 @@ k_fused(FusedArgs f, EvalArgs a)
     using SMem = FTSmem<fused_cap(TQ), typename PRow<FP32B>::T>;
     SMem &sm = *reinterpret_cast<SMem *>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
-    const int b = f.b0 + blockIdx.x;
+    const int b = f.order ? f.order[blockIdx.x] : f.b0 + (int)blockIdx.x;
     if (tid < 16) sm.tab[tid] = c_exp2_tab[tid];
     const int64_t cb0 = f.sblk_cell[b], cb1 = f.sblk_cell[b + 1];
     const int ncell = (int)(cb1 - cb0);
@@ -1370,11 +1438,13 @@ sdot_status run_trunc(sdot_ctx *c, const EvalArgs &a, double r)
     if (e == cudaSuccess) e = c->superpair.alloc((size_t)nss * nts);
     if (e == cudaSuccess) e = c->shit.alloc((size_t)nss * nts);
     if (e == cudaSuccess) e = c->scount.alloc(nss + 1);
+    if (e == cudaSuccess) e = c->fwd_hist.alloc(ORDER_BUCKETS);
+    if (e == cudaSuccess) e = c->fwd_order.alloc(nsb);
     if (e != cudaSuccess) return cuda_error(c, e, "pair list alloc");
     k_super_pairs<<<(unsigned)(((int64_t)nss * nts + 255) / 256), 256, 0, st>>>(c->ssup_sph32.p, nss, c->tsup_sph32.p,
                                                                              nts, cr, c->superpair.p);
     k_super_compact<<<(unsigned)(((int64_t)nss * 32 + 255) / 256), 256, 0, st>>>(c->superpair.p, nss, nts, c->shit.p,
-                                                                              c->scount.p);
+                                                                              c->scount.p, c->fwd_hist.p);
     // Row length of the per-block pair masks: the most target super-blocks any
     // source super-block pairs with.  Every count is at most nts, so when the
     // nts-wide rows are small (<= 64 MiB) they are used as
@@ -1391,9 +1461,10 @@ sdot_status run_trunc(sdot_ctx *c, const EvalArgs &a, double r)
     e = c->pmask.alloc((size_t)nsb * hmax);
     if (e != cudaSuccess) return cuda_error(c, e, "pair mask alloc");
     const unsigned gw = (unsigned)(((int64_t)nsb * 32 + 255) / 256);
-    k_fwd_masks<<<gw, 256, 0, st>>>(c->sblk_sph32.p, nsb, c->tblk_sph32.p, ntb, nts, hmax, cr, c->shit.p, c->scount.p,
-                                    c->pmask.p, c->fwd_cnt.p);
-    k_scan<<<1, 1024, 0, st>>>(c->fwd_cnt.p, nsb, c->fwd_off.p, c->scal_host + SC_COVER);
+    const unsigned gm = (unsigned)(((int64_t)((nsb + FM_B - 1) / FM_B) * 32 + 255) / 256);
+    k_fwd_masks<<<gm, 256, 0, st>>>(c->sblk_box32.p, nsb, c->tblk_box32.p, ntb, nts, hmax, cr, c->shit.p, c->scount.p,
+                                    c->pmask.p, c->fwd_cnt.p, c->fwd_hist.p);
+    k_scan<<<1, 1024, 0, st>>>(c->fwd_cnt.p, nsb, c->fwd_off.p, c->scal_host + SC_COVER, c->fwd_hist.p);
     e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_error(c, e, "pair list count");
     const int64_t npairs = (int64_t)c->scal_host[SC_COVER];  // (a whole number below 2^53)
@@ -1405,7 +1476,8 @@ sdot_status run_trunc(sdot_ctx *c, const EvalArgs &a, double r)
     if (e == cudaSuccess) e = c->inv_cnt.alloc(2 * (size_t)(ntb + 1));
     if (e == cudaSuccess) e = c->inv_off.alloc(ntb + 1);
     if (e != cudaSuccess) return cuda_error(c, e, "pair list alloc");
-    k_fwd_fill<<<gw, 256, 0, st>>>(nsb, nts, hmax, c->shit.p, c->scount.p, c->pmask.p, c->fwd_off.p, c->fwd_t.p);
+    k_fwd_fill<<<gw, 256, 0, st>>>(nsb, nts, hmax, c->shit.p, c->scount.p, c->pmask.p, c->fwd_off.p, c->fwd_t.p, ntb,
+                                   c->fwd_hist.p, c->fwd_order.p);
     c->klaunch[6] += 9;
     if (c->profiling) cudaEventRecord(c->pev[7], st);
     // 2. partial buffer (forward order): all pairs at once under the cap, else groups of source blocks.
@@ -1445,7 +1517,7 @@ sdot_status run_trunc(sdot_ctx *c, const EvalArgs &a, double r)
     if (e != cudaSuccess) return cuda_error(c, e, "pair list fork");
     unsigned long long *icnt = reinterpret_cast<unsigned long long *>(c->inv_cnt.p), *ifill = icnt + ntb + 1;
     k_inv_count<<<gw, 256, 0, c->side>>>(nsb, c->fwd_off.p, c->fwd_t.p, icnt);
-    k_scan<<<1, 1024, 0, c->side>>>(c->inv_cnt.p, ntb, c->inv_off.p, nullptr);
+    k_scan<<<1, 1024, 0, c->side>>>(c->inv_cnt.p, ntb, c->inv_off.p, nullptr, nullptr);
     k_inv_scatter<<<gw, 256, 0, c->side>>>(nsb, c->fwd_off.p, c->fwd_t.p, c->inv_off.p, ifill, c->inv_tmpb.p,
                                            c->inv_tmpk.p);
     k_inv_order<<<(unsigned)ntb, 256, 0, c->side>>>(nsb, c->inv_off.p, c->inv_tmpb.p, c->inv_tmpk.p, c->inv_b.p,
@@ -1464,6 +1536,7 @@ sdot_status run_trunc(sdot_ctx *c, const EvalArgs &a, double r)
     const int tmode = fused_tensor_mode(c, a, prange);
     for (size_t gi = 0; gi < groups.size(); ++gi) {
         const Group &g = groups[gi];
+        f.order = groups.size() == 1 ? c->fwd_order.p : nullptr;
         f.b0 = g.b0;
         f.part_base = g.k0;
         if (c->dim == 2) dispatch_fused<2>(c, f, a, fp32b, g.b1 - g.b0, prange, tmode);
