@@ -752,7 +752,7 @@ void plan_lattice(sdot_batch *b, int i)
 }
 
 // Layout of every problem in the packed arrays and its launch shapes (the
-// single-problem dense path's: value blocks of DENSE_A_THREADS * QT points,
+// single-problem dense path's: value blocks of DENSE_A_THREADS points,
 // gradient target blocks of DENSE_B_THREADS * TT and the same slice count).
 sdot_status upload(sdot_batch *b)
 {
@@ -782,7 +782,7 @@ sdot_status upload(sdot_batch *b)
         a.l2e_eps = LOG2E / a.eps;
         I.q0 = q0;
         I.t0 = t0;
-        const int64_t per = (int64_t)DENSE_A_THREADS * DENSE_A_QT;
+        const int64_t per = DENSE_A_THREADS;
         I.nvb = (int)((P.nq + per - 1) / per);
         I.part0 = part0;
         I.fp32 = 0;

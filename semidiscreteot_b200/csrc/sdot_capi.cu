@@ -176,7 +176,7 @@ sdot_status ensure_tickets(sdot_ctx *c)
 sdot_status ensure_eval_buffers(sdot_ctx *c)
 {
     const int64_t nt = c->nt, nq = c->nq;
-    const int64_t dense_blocks = (nq + DENSE_A_THREADS * DENSE_A_QT - 1) / (DENSE_A_THREADS * DENSE_A_QT);
+    const int64_t dense_blocks = (nq + DENSE_A_THREADS - 1) / DENSE_A_THREADS;
     const int64_t nval = std::max<int64_t>(dense_blocks, c->nsblk);
     const size_t need =
         (size_t)(nt * (2 + TPACK + dense_grad_slices(INT64_MAX / 2, nt) + 2) + nq + 4 * nval + 148 * 12 + 64) *

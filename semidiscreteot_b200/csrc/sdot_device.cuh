@@ -24,6 +24,7 @@ __device__ __constant__ double c_exp2_tab[16] = {
 // FP64 sum stays far from overflow and the rescale branch is rare.
 constexpr double LSE_THR = 16.0 * 512.0;
 constexpr double EXP2_CLAMP = -16.0 * 1000.0;
+constexpr int LSE_THR_HI = 0x40C00000, CLAMP_HI = (int)0xC0CF4000u;  // their high words
 
 // FP64 2^(u/16) for u <= 16*1022, relative error <= 1.5e-13.
 // Method: u = 16 e + k + f with n = rint(u) (k = n mod 16, e = n div 16,
@@ -129,6 +130,45 @@ __device__ __forceinline__ float ex2_approx(float x)
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+
+// Two FP32 values in one 64-bit register pair: one packed instruction rounds
+// each half as the scalar one does.
+typedef unsigned long long f32x2;
+
+__device__ __forceinline__ f32x2 pack2(float lo, float hi)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float &lo, float &hi)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 ex2_approx2(f32x2 v)
+{
+    float a, b;
+    unpack2(v, a, b);
+    return pack2(ex2_approx(a), ex2_approx(b));
 }
 
 // Exact floor(p / d) for p < 2^16, d <= 64 with m = ceil(2^32 / d).
