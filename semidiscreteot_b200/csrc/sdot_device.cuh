@@ -10,14 +10,23 @@
 
 namespace sdot {
 
-// 2^(k/16), k = 0..15, correctly rounded.  Kept in shared memory by every
-// kernel that calls exp2_16: 16 doubles occupy all 32 banks, so any per-lane
-// index pattern is conflict-free.
+// 2^(k/16), k = 0..15, correctly rounded, with k 2^16 taken off the high word:
+// that word plus n 2^16, n = 16 e + k, is the high word of 2^(n/16) (one
+// integer instruction; masking the fraction of n off first took two more).
+// Kept in shared memory by every kernel that calls exp2_16: 16 doubles occupy
+// all 32 banks, so any per-lane index pattern is conflict-free.
 __device__ __constant__ double c_exp2_tab[16] = {
-    0x1.0000000000000p+0, 0x1.0b5586cf9890fp+0, 0x1.172b83c7d517bp+0, 0x1.2387a6e756238p+0,
-    0x1.306fe0a31b715p+0, 0x1.3dea64c123422p+0, 0x1.4bfdad5362a27p+0, 0x1.5ab07dd485429p+0,
-    0x1.6a09e667f3bcdp+0, 0x1.7a11473eb0187p+0, 0x1.8ace5422aa0dbp+0, 0x1.9c49182a3f090p+0,
-    0x1.ae89f995ad3adp+0, 0x1.c199bdd85529cp+0, 0x1.d5818dcfba487p+0, 0x1.ea4afa2a490dap+0};
+    0x1.0000000000000p+0, 0x1.fb5586cf9890fp-1, 0x1.f72b83c7d517bp-1, 0x1.f387a6e756238p-1,
+    0x1.f06fe0a31b715p-1, 0x1.edea64c123422p-1, 0x1.ebfdad5362a27p-1, 0x1.eab07dd485429p-1,
+    0x1.ea09e667f3bcdp-1, 0x1.ea11473eb0187p-1, 0x1.eace5422aa0dbp-1, 0x1.ec49182a3f090p-1,
+    0x1.ee89f995ad3adp-1, 0x1.f199bdd85529cp-1, 0x1.f5818dcfba487p-1, 0x1.fa4afa2a490dap-1};
+
+// 2^(n/16) from the table above, for |n| < 16 * 1022.
+__device__ __forceinline__ double exp2_int(int n, const double *tab)
+{
+    const double t = tab[n & 15];
+    return __hiloint2double(__double2hiint(t) + (n << 16), __double2loint(t));
+}
 
 // Lazy-rescale threshold of the online log-sum-exp, in units of 2^(1/16):
 // the running shift M is only moved when a term would exceed 2^512, so the
@@ -30,8 +39,7 @@ constexpr int LSE_THR_HI = 0x40C00000, CLAMP_HI = (int)0xC0CF4000u;  // their hi
 // Method: u = 16 e + k + f with n = rint(u) (k = n mod 16, e = n div 16,
 // |f| <= 1/2); 2^(u/16) = 2^e * 2^(k/16) * exp(f ln2/16).  The last factor is
 // the degree-5 Taylor polynomial of exp on |f ln2/16| <= 0.0217 (remainder
-// < 1.5e-13); 2^(k/16) comes from a 16-entry table and 2^e is added to the
-// exponent field.  Arguments below -16000 are clamped (result ~2^-1000, far
+// < 1.5e-13); 2^(n/16) comes from a 16-entry table (exp2_int).  Arguments below -16000 are clamped (result ~2^-1000, far
 // below any sum it is added to).
 __device__ __forceinline__ double exp2_16(double u, const double *tab)
 {
@@ -45,9 +53,7 @@ __device__ __forceinline__ double exp2_16(double u, const double *tab)
     p = fma(f, p, 0x1.ebfbdff82c58fp-11);
     p = fma(f, p, 0x1.62e42fefa39efp-5);
     p = fma(f, p, 1.0);
-    const double r = tab[n & 15] * p;
-    const int hi = __double2hiint(r) + ((n >> 4) << 20);
-    return __hiloint2double(hi, __double2loint(r));
+    return exp2_int(n, tab) * p;
 }
 
 // exp2_16 without the lower clamp, for arguments proven >= -16000 by the caller.
@@ -62,9 +68,7 @@ __device__ __forceinline__ double exp2_16_nc(double u, const double *tab)
     p = fma(f, p, 0x1.ebfbdff82c58fp-11);
     p = fma(f, p, 0x1.62e42fefa39efp-5);
     p = fma(f, p, 1.0);
-    const double r = tab[n & 15] * p;
-    const int hi = __double2hiint(r) + ((n >> 4) << 20);
-    return __hiloint2double(hi, __double2loint(r));
+    return exp2_int(n, tab) * p;
 }
 
 // exp2_16 with one more term of the polynomial (remainder < 5e-16), for
@@ -82,9 +86,7 @@ __device__ __forceinline__ double exp2_16_full(double u, const double *tab)
     p = fma(f, p, 0x1.ebfbdff82c58fp-11);
     p = fma(f, p, 0x1.62e42fefa39efp-5);
     p = fma(f, p, 1.0);
-    const double r = tab[n & 15] * p;
-    const int hi = __double2hiint(r) + ((n >> 4) << 20);
-    return __hiloint2double(hi, __double2loint(r));
+    return exp2_int(n, tab) * p;
 }
 
 // Squared distance rounded exactly like the reference's
