@@ -14,8 +14,8 @@
 //   1. block-pair lists.  (b, t) is a pair iff the box of b's cell centres is
 //      within r of the box of t's targets (FP32, conservatively enlarged;
 //      super-blocks by their spheres).  With the blocks' spheres in place of
-//      their boxes a third more pairs were listed, staged and reduced.  The forward list (per b, t ascending)
-//      is filled from masks; the inverse list (per t, b ascending, with the
+//      their boxes a third more pairs were listed, staged and reduced.  The
+//      forward list (per b, t ascending) is filled from masks; the inverse list (per t, b ascending, with the
 //      pairs' forward positions) is its transpose, built on a second stream
 //      beside step 2, which does not need it.
 //   2. k_fused (CTA <-> source block, warp <-> unit):
@@ -28,14 +28,14 @@
 //        B0_Kj = kappa (psi_j - d2/2)/eps, G_Kj = kappa (y_j - c_K)/eps,
 //        delta_q = x_q - c_K, C'_q = -kappa |delta_q|^2 / (2 eps)
 //        (kappa = 16/ln 2; the same expansion as |x_q - y_j|^2 about c_K);
-//      gradient sweep: each warp over the same compacted candidates, lane <->
-//        candidate, sum over the unit's q of
+//      gradient sweep: sum over a cell's q of
 //        w_q nu_j 2^(E0_Kj + G'_Kj.delta_q + D_q) in FP32 ex2 (or FP64 exp2),
 //        E0 and G' formed in FP64 per (cell, target) so every FP32 operand is
-//        small, into the warp's partial row (FP32 rows in the hybrid mode,
-//        FP64 rows in the FP64 mode); the rows are added in warp order in
-//        FP64.  The block's partial for each target of each pair is written
-//        to the pair's forward position.
+//        small; thread <-> staged target for the chunk that is still staged,
+//        lane <-> target of a forward entry for the others (tensor-product
+//        points; staged again otherwise), over the block's cells in FP64.  The
+//        block's partial for each target of each pair is written to the pair's
+//        forward position.
 //   3. k_grad_reduce (CTA <-> target block): sum of the partials over the
 //      pairs in ascending source-block order, lane <-> target.  No atomics;
 //      the summation order is fixed, results are bitwise reproducible.
@@ -113,6 +113,13 @@ struct FTSmem {
     int epre[32];                 // staged position of the first survivor of each accepted entry
     int eacc, etot;
     int nstg;
+    // tensor path, gradient sweep: centres of the units' cells relative to the block's, and the cells' centre
+    // coordinates where there are at most two per dimension (brick), the unit at (i0, i1, i2) of them, the offsets
+    float uf[FT_WARPS][3];
+    double cs[3][2];
+    float csf[3][2], ahf[3];
+    int cell_at[8];
+    int brick;
     int ent_j0[FT_PREF];           // forward entries of the block: the target block's first target
     unsigned char ent_sz[FT_PREF]; // and its size (prefetched once per block)
 };
@@ -1016,6 +1023,94 @@ __device__ __forceinline__ typename PRow<FP32B>::T grad_term_tensor(const SM &sm
     }
 }
 
+// A target's gradient terms over the block's units, tensor-product points:
+// the exact candidate test (the FP32 squared distance about the block's
+// centre decides outside [lo, hi], the FP64 one, rounded like the
+// reference's, inside) and grad_term_tensor.  FP32 in 3D is bound by the
+// special-function unit (exponentials and conversions between FP32 and
+// FP64); where the block's cells have at most two centre coordinates per
+// dimension (brick), the target's differences, factors and their conversions
+// are taken once per coordinate: 12 per target and 3 per cell instead of 9
+// per cell, the same operations on the same operands.
+template <int DIM, int TM, bool FP32B, int TS, class SM>
+__device__ __forceinline__ double unit_terms(const SM &sm, const double *y, double lognu, double sp, bool on,
+                                             bool brick, int nunit, const double *bc, float lo, float hi,
+                                             const EvalArgs &a)
+{
+    constexpr int NQ = DIM == 3 ? TM * TM * TM : TM * TM;
+    float z[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) z[d] = d < DIM ? (float)(y[d] - bc[d]) : 0.f;
+    double v = 0.0;
+    if (brick) {
+        if constexpr (DIM == 3 && FP32B && TM == 2) {
+            const float sf = (float)(a.s * (1.0 / 16.0));
+            double g[3][2];
+            float zz[3][2], ga[3][2], Fl[3][2], Fh[3][2];
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    g[d][i] = y[d] - sm.cs[d][i];
+                    const float zc = z[d] - sm.csf[d][i];
+                    zz[d][i] = zc * zc;
+                    ga[d][i] = sf * (float)g[d][i] * sm.ahf[d];
+                    if (TS >= 1) {
+                        Fl[d][i] = 1.f;
+                        Fh[d][i] = ex2_approx(2.f * ga[d][i]);
+                    } else {
+                        Fh[d][i] = ex2_approx(ga[d][i]);
+                        Fl[d][i] = rcp_approx(Fh[d][i]);
+                    }
+                }
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const int u = sm.cell_at[c];
+                if (u < 0) continue;
+                const int i0 = c & 1, i1 = (c >> 1) & 1, i2 = c >> 2;
+                const float d2f = zz[2][i2] + (zz[1][i1] + zz[0][i0]);
+                bool in = d2f < lo;
+                if (!in && !(d2f > hi)) in = dist2_exact<3>(y, sm.cellc[u]) <= a.sstar;
+                const double Lref = sm.uL[u];
+                if (!in || !on || !isfinite(Lref)) continue;
+                float W[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) W[q] = sm.qtw[8 * u + q];
+                const double d2 = fma(g[2][i2], g[2][i2], fma(g[1][i1], g[1][i1], g[0][i0] * g[0][i0]));
+                float e0 = (float)(lognu + (fma(-a.halfs, d2, sp) - KAPPA * Lref) * (1.0 / 16.0));
+                if (TS >= 1) e0 = ((e0 - ga[0][i0]) - ga[1][i1]) - ga[2][i2];
+                float w = 0.f;
+#pragma unroll
+                for (int p0 = 0; p0 < 2; ++p0) {
+                    float t1 = 0.f;
+#pragma unroll
+                    for (int p1 = 0; p1 < 2; ++p1) {
+                        const float t2 = fmaf(W[p0 + 2 * p1 + 4], Fh[2][i2], W[p0 + 2 * p1] * Fl[2][i2]);
+                        t1 = p1 ? fmaf(t2, Fh[1][i1], t1) : t2 * Fl[1][i1];
+                    }
+                    w = p0 ? fmaf(t1, Fh[0][i0], w) : t1 * Fl[0][i0];
+                }
+                v += (double)(ex2_approx(e0) * w);
+            }
+        }
+    } else {
+#pragma unroll 1
+        for (int u = 0; u < nunit; ++u) {
+            const float gx = z[0] - sm.uf[u][0], gy = z[1] - sm.uf[u][1], gz = DIM == 3 ? z[2] - sm.uf[u][2] : 0.f;
+            float d2f = fmaf(gy, gy, gx * gx);
+            if (DIM == 3) d2f = fmaf(gz, gz, d2f);
+            bool in = d2f < lo;
+            if (!in && !(d2f > hi)) in = dist2_exact<DIM>(y, sm.cellc[u]) <= a.sstar;
+            const double Lref = sm.uL[u];
+            if (!in || !on || !isfinite(Lref)) continue;
+            const double *cc = sm.cellc[u];
+            const double g[3] = {y[0] - cc[0], y[1] - cc[1], DIM == 3 ? y[2] - cc[2] : 0.0};
+            v += (double)grad_term_tensor<DIM, TM, TS, FP32B>(sm, u * NQ, sm.uah[u], g, lognu, sp, Lref, a);
+        }
+    }
+    return v;
+}
+
 // Gradient sweep of the staged chunk (forward positions k..): thread <->
 // staged target, over the block's units in order (the unit terms, FP32 in the
 // hybrid mode, added in FP64), and the write of every slot of every pair
@@ -1057,6 +1152,77 @@ __device__ __forceinline__ void grad_chunk(SM &sm, const FusedArgs &f, int64_t k
     }
     for (int i = tid; i < nt * TBLK_KD; i += FT_WARPS * 32)
         if (!((sm.keep[i / TBLK_KD] >> (i % TBLK_KD)) & 1u)) out[i] = Row(0);
+}
+
+// Gradient sweep of the block's forward entries [k0, k1) whose targets are no
+// longer staged: warp <-> entry (target block), lane <-> target, straight from
+// the packed targets; every slot of the pair's partial is written.  Staging
+// these chunks again took their culling, compaction and barriers a second
+// time (2,097,152 points x 100,000 targets, both sweeps: 6,020 -> 5,740 us).
+// The last chunk stays with grad_chunk, whose lanes are all within reach of
+// the block (direct for it too: 5,907 us, and 10% slower where every block has
+// one chunk; the FP32 test and bricks in grad_chunk: no gain).
+template <int DIM, int TM, bool FP32B, int TS, class SM>
+__device__ __forceinline__ void grad_direct(SM &sm, const FusedArgs &f, int64_t k0, int64_t k1, int nunit,
+                                            const double *bc, float lo, float hi, const EvalArgs &a)
+{
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    using Row = typename PRow<FP32B>::T;
+    Row *out = (FP32B ? reinterpret_cast<Row *>(f.part32) : reinterpret_cast<Row *>(f.part)) +
+               (k0 - f.part_base) * TBLK_KD + lane;
+    const bool brick = DIM == 3 && FP32B && TM == 2 && sm.brick;
+    for (int e = wp; e < (int)(k1 - k0); e += FT_WARPS) {
+        int64_t j0;
+        int sz;
+        if (e < FT_PREF) {
+            j0 = sm.ent_j0[e];
+            sz = sm.ent_sz[e];
+        } else {
+            const int t = f.fwd_t[k0 + e];
+            j0 = f.tblk_off[t];
+            sz = (int)(f.tblk_off[t + 1] - j0);
+        }
+        const double *tp = f.tpk + j0 + min(lane, sz - 1);
+        double y[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) y[d] = tp[d * f.nt];
+        const double lognu = tp[4 * f.nt], sp = tp[5 * f.nt];
+        out[(int64_t)e * TBLK_KD] = (Row)unit_terms<DIM, TM, FP32B, TS>(sm, y, lognu, sp, lane < sz, brick, nunit, bc,
+                                                                        lo, hi, a);
+    }
+}
+
+// One warp's preparation of grad_direct: the units' centres in FP32 and
+// whether the block is a brick.
+template <int DIM, class SM>
+__device__ __forceinline__ void direct_setup(SM &sm, int lane, int nunit, const double *bc)
+{
+    for (int i = lane; i < nunit * 3; i += 32) sm.uf[i / 3][i % 3] = (float)(sm.cellc[i / 3][i % 3] - bc[i % 3]);
+    if (DIM == 2) return;
+    // at most two centre coordinates per dimension, each cell at its own place, the same offsets in all?
+    const int u = min(lane, nunit - 1);
+    bool ok = true;
+    int at = 0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const double c0 = sm.cellc[0][d], cu = sm.cellc[u][d];
+        const unsigned other = __ballot_sync(0xffffffffu, cu != c0);
+        const double c1 = other ? sm.cellc[__ffs(other) - 1][d] : c0;
+        ok = ok && (cu == c0 || cu == c1) && (float)sm.uah[u][d] == (float)sm.uah[0][d];
+        at |= cu == c0 ? 0 : 1 << d;
+        if (lane < 2) {
+            sm.cs[d][lane] = lane ? c1 : c0;
+            sm.csf[d][lane] = (float)((lane ? c1 : c0) - bc[d]);
+        }
+        if (lane == 2) sm.ahf[d] = (float)sm.uah[0][d];
+    }
+    if (lane < 8) sm.cell_at[lane] = -1;
+    const unsigned same = __match_any_sync(0xffffffffu, lane < nunit ? at : 32 + lane);
+    ok = ok && (same & (same - 1)) == 0;
+    const bool all = __all_sync(0xffffffffu, ok);
+    __syncwarp();
+    if (lane < nunit) sm.cell_at[at] = lane;
+    if (lane == 0) sm.brick = all;
 }
 
 template <int DIM, int QL, bool FP32B, int MODE, int TQ, int TS>
@@ -1270,20 +1436,31 @@ k_fused(FusedArgs f, EvalArgs a)
     }
     __syncthreads();
     // The value sweep's last chunk (the only one when everything fit) is still
-    // staged: its gradient comes first, then the earlier chunks are staged again
-    // (the same chunks: the greedy rule over [k0, k0 + tail_off) ends where the
-    // value sweep's did).  Every pair's partial is written once, so the order of
-    // the chunks does not change any sum.
+    // staged: its gradient comes first, then the earlier entries' (tensor-product
+    // points: unstaged; otherwise the earlier chunks are staged again, the same
+    // ones: the greedy rule over [k0, k0 + tail_off) ends where the value sweep's
+    // did).  Every pair's partial is written once, so the order does not change
+    // any sum.
     int64_t kend = k1;
     if (tail_off >= 0) {
         grad_chunk<DIM, FP32B, TQ, TS>(sm, f, k0 + tail_off, tail_nt, nunit, a);
         kend = k0 + tail_off;
     }
-    for (int64_t k = k0; k < kend;) {
-        __syncthreads();  // the staged targets are consumed
-        const int nt = stage_chunk<DIM>(sm, f, k0, k, kend, bc, rcull2);
-        grad_chunk<DIM, FP32B, TQ, TS>(sm, f, k, nt, nunit, a);
-        k += nt;
+    if constexpr (TQ > 0) {
+        if (kend == k0) return;
+        if (wp == 0) direct_setup<DIM>(sm, lane, nunit, bc);
+        __syncthreads();
+        // The FP32 squared distance about the block centre is off by less than
+        // 1.4e-6 rc^2 (components up to 2 rc, rounded three times).
+        grad_direct<DIM, TQ, FP32B, TS>(sm, f, k0, kend, nunit, bc, (float)(a.sstar - 4e-6 * rc * rc),
+                                        (float)(a.sstar + 4e-6 * rc * rc), a);
+    } else {
+        for (int64_t k = k0; k < kend;) {
+            __syncthreads();  // the staged targets are consumed
+            const int nt = stage_chunk<DIM>(sm, f, k0, k, kend, bc, rcull2);
+            grad_chunk<DIM, FP32B, TQ, TS>(sm, f, k, nt, nunit, a);
+            k += nt;
+        }
     }
 }
 
@@ -1391,7 +1568,7 @@ static int fused_tensor_mode(const sdot_ctx *c, const EvalArgs &a, double psi_ra
     // 2^300 (FP64 value sweep) and 2^40 (FP32 gradient sweep)
     const double fac = a.s * a.cull * c->tensor_amax / 16.0;
     const bool tensor = c->tensor_m > 0 && a.lse && a.ngroups == 1 && fac <= 40.0 && umin > -15000.0 &&
-                        gap < 16.0 * 500.0;
+                        gap < 16.0 * 500.0 && a.cull > 1e-12 && a.cull < 1e12;  // (FP32 squared distances)
     const bool shape = (c->dim == 3 && c->tensor_m == 2 && a.ql == 8) ||
                        (c->dim == 2 && c->tensor_m == 3 && a.ql == 9) || (c->dim == 2 && c->tensor_m == 2 && a.ql == 4);
     if (!tensor || !shape) return -1;

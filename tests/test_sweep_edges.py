@@ -65,10 +65,11 @@ def test_point_sweep_reference_moves(oracle_mod, order):
 
 
 @pytest.mark.parametrize("precision", ["fp64", "hybrid"])
-@pytest.mark.parametrize("dim,n,order", [(2, 24, 2), (2, 24, 3), (3, 8, 2), (2, 12, 4)])
+@pytest.mark.parametrize("dim,n,order", [(2, 24, 2), (2, 24, 3), (3, 8, 2), (3, 7, 2), (2, 12, 4)])
 def test_truncated_lists_and_chunks(oracle_mod, dim, n, order, precision):
     """A tight cluster (several chunks per source block) around 300 targets that nearly coincide (more candidates for
-    a point's largest exponent than its list holds), and a few targets far away."""
+    a point's largest exponent than its list holds), and a few targets far away; in 3D, source blocks of 2 x 2 x 2
+    cells and ragged ones."""
     rng = np.random.default_rng(dim * n + order)
     y = np.concatenate([0.5 + 0.02 * rng.standard_normal((2500, dim)), 0.45 + 1e-7 * rng.standard_normal((300, dim)),
                         rng.random((101, dim))])
