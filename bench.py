@@ -279,14 +279,14 @@ class ClockSampler:
 # DRAM traffic per launch of the dominant kernels (dram__bytes_read.sum +
 # dram__bytes_write.sum), from one ncu capture each:
 #   k_fused, trunc_3d (2,097,152 points x 100,000 targets), HYBRID (FP32
-#   gradient partials): 130,609,408 read + 167,453,952 written, from
+#   gradient partials): 115,030,784 read + 143,745,792 written, from
 #     ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,gpu__time_duration.sum
 #         --clock-control none -k regex:k_fused -s 3 -c 1 --csv
 #         python bench.py --steps 1 --warmup 3 --no-cpu-baseline --no-extra
-#   dense sweeps (k_value_dense_tensor, k_grad_dense_tensor, ...), dense_2d: the inputs (0.9 MB) stay in L2, so
+#   dense sweeps (k_lat_value, k_grad_dense_tensor, ...), dense_2d: the inputs (0.9 MB) stay in L2, so
 #     DRAM traffic is not a meaningful bound there (null).
 TRAFFIC_BYTES = {
-    ("trunc_3d", "hybrid"): 298063360.0,
+    ("trunc_3d", "hybrid"): 258776576.0,
 }
 
 
@@ -461,9 +461,9 @@ def roofline_of(m, wl, peaks, precision):
     if tv >= tg or truncated:
         ach = VALUE_FLOPS_PER_PAIR[dim] * pairs / (tv * 1e-3) / 1e12
         kname = ("k_fused (FP64 exp2 value sweep + FP32 ex2 gradient sweep, one kernel)" if truncated else
-                 "dense FP64 value sweep: k_value_dense_tensor (per tensor-grid cell and target slice; one "
-                 "exponential per cell and target on uniform grids) + k_value_dense_merge, or per point; flops "
-                 "counted for the unfactored form")
+                 "dense FP64 value sweep: k_lat_value (points on a tensor lattice: per-dimension factors as FP64 "
+                 "matrix products) + k_lat_merge, or per tensor-grid cell or point; flops counted for the "
+                 "unfactored form")
         return {"kernel": kname, "bound": "fp64", "achieved": ach, "peak": peaks["fp64_tflops"], "unit": "TFLOP/s",
                 "frac": ach / peaks["fp64_tflops"], "traffic": TRAFFIC_BYTES.get((wl["name"], precision)),
                 "flops_per_pair": VALUE_FLOPS_PER_PAIR[dim], "ms_per_launch": tv,

@@ -310,7 +310,7 @@ struct EvalArgs;
 // truncated evaluation (block-pair lists, fused sweeps, partial reduction)
 sdot_status run_trunc(sdot_ctx *c, const EvalArgs &a, double r);
 // value and gradient sweeps with the spherical distance (sdot_spherical.cu);
-// *nval: the value blocks whose partials k_finalize_scalars sums
+// *nval: the value blocks whose partials k_finalize sums
 sdot_status run_spherical(sdot_ctx *c, const EvalArgs &a, double r, int64_t *nval);
 // dense-layout tpack for the current psi (used by the Hessian)
 void launch_target_prep_dense(sdot_ctx *c, const EvalArgs &a);
