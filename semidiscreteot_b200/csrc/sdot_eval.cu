@@ -1081,6 +1081,11 @@ static DenseShape dense_shape_of(const sdot_ctx *c, double eps, bool fp64)
     for (int k = 0; k < 3; ++k)
         reach[k] = std::max(std::fabs(c->tgt_lo[k] - c->origin[k]), std::fabs(c->tgt_hi[k] - c->origin[k]));
     d.lat = lat_tiling(c->lat_n, c->lat_xo, c->lat_X.data(), c->dim, s, reach, LAT_BITS);
+    // The merge takes the points' maxima over the targets in one CTA per
+    // LAT_THREADS points: with fewer of them than SMs and more targets than it
+    // lists at once it is a serial chain (4,096 points x 10,538 targets: value
+    // 298 us against 63 on the cell or point sweeps).
+    if ((int64_t)d.lat.ntiles * (LAT_TILE / LAT_THREADS) < 148 && c->nt > 1024) d.lat = LatTiling{};
     if (d.lat.cap == 0) return d;
     constexpr int SLOTS = 148 * 2;
     d.nvs = lat_slices(d.lat.ntiles, (c->nt + 15) / 16, SLOTS);
