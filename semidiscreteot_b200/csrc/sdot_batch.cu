@@ -742,11 +742,12 @@ void plan_lattice(sdot_batch *b, int i)
     I.lat = 0;
     b->units_ok = false;
     if (!G.ok) return;
-    const LatTiling t = lat_tiling(G.n, G.xo, G.X.data(), b->dim, I.a.s, &b->reach[3 * i], LAT_BITS);
+    const LatTiling t = lat_tiling(G.n, G.xo, G.X.data(), b->dim, I.a.s, &b->reach[3 * i]);
     if (t.cap == 0) return;
     for (int d = 0; d < 3; ++d) I.L.nt[d] = t.nt[d];
     I.L.cap = t.cap;
     I.L.ntiles = t.ntiles;
+    lat_runs(G.period, G.step, b->dim, t.span, I.L);
     I.ngs = (t.ntiles + I.gts - 1) / I.gts;
     I.lat = 1;
 }
@@ -907,7 +908,6 @@ sdot_status upload(sdot_batch *b)
                 I.L.n[d] = G.n[d];
                 I.L.xo[d] = G.xo[d];
             }
-            lat_runs(G.period, G.step, D, I.L);
             I.K.off = b->lat_off.p + off0[i];
             I.K.mem = b->lat_mem.p + mem0[i];
             I.K.sph = b->lat_sph.p + sph0[i];

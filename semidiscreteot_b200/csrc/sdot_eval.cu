@@ -1080,7 +1080,7 @@ static DenseShape dense_shape_of(const sdot_ctx *c, double eps, bool fp64)
     double reach[3];
     for (int k = 0; k < 3; ++k)
         reach[k] = std::max(std::fabs(c->tgt_lo[k] - c->origin[k]), std::fabs(c->tgt_hi[k] - c->origin[k]));
-    d.lat = lat_tiling(c->lat_n, c->lat_xo, c->lat_X.data(), c->dim, s, reach, LAT_BITS);
+    d.lat = lat_tiling(c->lat_n, c->lat_xo, c->lat_X.data(), c->dim, s, reach);
     // The merge takes the points' maxima over the targets in one CTA per
     // LAT_THREADS points: with fewer of them than SMs and more targets than it
     // lists at once it is a serial chain (4,096 points x 10,538 targets: value
@@ -1119,7 +1119,7 @@ static LatArgs lat_args(const sdot_ctx *c, const LatTiling &t)
     }
     L.cap = t.cap;
     L.ntiles = t.ntiles;
-    lat_runs(c->lat_period, c->lat_step, c->dim, L);
+    lat_runs(c->lat_period, c->lat_step, c->dim, t.span, L);
     return L;
 }
 

@@ -22,11 +22,18 @@
 // every slice of the targets, so the slices' sums add without rescaling.
 // The caller admits a tile size only when the factors of a tile span at most
 // 2^(+-LAT_BITS): every point's sum is then at least nu 2^-LAT_BITS relative
-// to M, the exponents that exp2_16_full clamps are below 2^-1000 times a factor
-// <= 2^LAT_BITS, and nothing leaves the FP64 range.
+// to M, and nothing leaves the FP64 range.  exp2_16_full clamps at 2^-1000.
+// With an exponential for each factor a clamped one is multiplied by the other
+// dimensions' only, at most 2^LAT_BITS: what it adds is 300 bits below the
+// least sum.  A run multiplies its clamped first factor by up to seven steps
+// too, as much as from one end of the tile to the other: with factors of
+// 2^(+-b) a clamped 2^-1000 grows to 2^(2 b - 1000) against a sum of 2^-b, so
+// runs are taken up to b = LAT_RUN_BITS only (310 bits apart), and factor by
+// factor beyond.
 #pragma once
 
 #include "sdot_device.cuh"
+#include "sdot_lattice_host.h"
 
 namespace sdot {
 
@@ -34,7 +41,6 @@ constexpr int LAT_THREADS = 256;
 constexpr int LAT_TILE = 4096;    // points of a tile: 64 x 64 or 16 x 16 x 16
 constexpr int LAT_CK = 32;        // targets of a chunk of the value sweep
 constexpr int LAT_GT = 64;        // targets of a CTA of the gradient sweep
-constexpr double LAT_BITS = 350.0;
 constexpr int LAT_RUN = 8;        // points of a factor run
 constexpr int LAT_MAXRUNS = 32;   // 2D: 2 x period x ceil(64 / (8 period)) <= 24 for periods up to 4
 constexpr int LAT_LIST = 1024;    // candidates of a pass over the points' maxima (32 target blocks)
@@ -83,11 +89,13 @@ struct LatDims {
     static constexpr int FS = FD + LAT_PAD_F;      // row of one target's factors in shared memory
 };
 
-// Run counts of a launch from the lattice's periods (host).
-inline void lat_runs(const int *period, const double *step, int dim, LatArgs &L)
+// Run counts of a launch from the lattice's periods; span: the bits that the
+// factors of a tile span (host).
+inline void lat_runs(const int *period, const double *step, int dim, double span, LatArgs &L)
 {
     const int T = dim == 2 ? 64 : 16;
     L.runs = 0;
+    if (!(span <= LAT_RUN_BITS)) return;
     for (int d = 0; d < dim; ++d) {
         const int p = period[d];
         if (p <= 0) {

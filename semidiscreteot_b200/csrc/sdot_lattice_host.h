@@ -147,20 +147,24 @@ inline void find_lattice(const double *x, int64_t n, int dim, Lattice &L)
 // sweeps do not apply) and tile counts.
 struct LatTiling {
     int cap = 0, nt[3] = {1, 1, 1}, ntiles = 0;
+    double span = 0.0;   // the factors of a tile lie within 2^(+-span)
 };
+
+// The largest span that the sweeps admit, and with factor runs (sdot_lattice.cuh says why).
+constexpr double LAT_BITS = 350.0;
+constexpr double LAT_RUN_BITS = 230.0;
 
 constexpr int LAT_CAPS2[2] = {64, 32}, LAT_CAPS3[1] = {16};   // tile sizes (2D, 3D), the largest first
 
 // Tile size for scaled exponents s = kappa / eps and targets within reach[d]
 // of the origin: the largest of 64 and 32 points per dimension (2D) or 16
-// (3D) whose factors span at most 2^(+-bits).  A tile's work goes by its
+// (3D) whose factors span at most 2^(+-LAT_BITS).  A tile's work goes by its
 // padded size (64 or 32 points per dimension, 16 in 3D); where the padding
 // would make that more than LAT_PAD times the points, the cell sweeps (about
 // four multiply-adds per pair against one here, plus a third for the
 // factors) are the faster ones.
 constexpr double LAT_PAD = 2.5;
-inline LatTiling lat_tiling(const int *n, const int *xo, const double *X, int dim, double s, const double *reach,
-                            double bits)
+inline LatTiling lat_tiling(const int *n, const int *xo, const double *X, int dim, double s, const double *reach)
 {
     LatTiling best;
     const int *caps = dim == 2 ? LAT_CAPS2 : LAT_CAPS3;
@@ -185,8 +189,9 @@ inline LatTiling lat_tiling(const int *n, const int *xo, const double *X, int di
             const int rest = n[d] - (t.nt[d] - 1) * cap;
             padded *= (t.nt[d] - 1) * (double)cap + (dim == 2 && rest <= 32 ? 32 : cap);
         }
-        if (!(span <= bits) || padded > LAT_PAD * (double)nq || tiles > (1 << 20)) continue;
+        if (!(span <= LAT_BITS) || padded > LAT_PAD * (double)nq || tiles > (1 << 20)) continue;
         t.ntiles = (int)tiles;
+        t.span = span;
         return t;
     }
     return best;
