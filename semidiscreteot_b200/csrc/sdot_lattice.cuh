@@ -41,7 +41,6 @@ constexpr int LAT_THREADS = 256;
 constexpr int LAT_TILE = 4096;    // points of a tile: 64 x 64 or 16 x 16 x 16
 constexpr int LAT_CK = 32;        // targets of a chunk of the value sweep
 constexpr int LAT_GT = 64;        // targets of a CTA of the gradient sweep
-constexpr int LAT_RUN = 8;        // points of a factor run
 constexpr int LAT_MAXRUNS = 32;   // 2D: 2 x period x ceil(64 / (8 period)) <= 24 for periods up to 4
 constexpr int LAT_LIST = 1024;    // candidates of a pass over the points' maxima (32 target blocks)
 constexpr int LAT_PAD_F = 4;      // row padding of the operands in shared memory: the four rows a fragment

@@ -23,13 +23,20 @@ struct Lattice {
     std::vector<int> q;
 };
 constexpr int LAT_MAXP = 4;   // largest period looked for
+constexpr int LAT_RUN = 8;    // points of a factor run
+
+constexpr double LAT_ULPS = 4.0 * 2.220446049250313e-16;
 
 // Finds the lattice, or leaves ok = false.  Coordinates are told apart by
 // their bits; where that leaves more coordinates than the lattice can have,
-// those within 4 ulp of the largest coordinate are taken as one (meshes that
-// map each cell by itself round a shared coordinate in the last bits): the
-// exponent's own rounding is larger.  Linear in the points; gives up as soon
-// as a dimension has more coordinates than MAXN.
+// those within LAT_ULPS of the points' extent are taken as one (meshes that
+// map each cell by itself round a shared coordinate in the last bits).  The
+// sweeps form the exponents about the source's centre, so their own rounding
+// goes by the extent, and so has what merged coordinates and a run's equal
+// steps (below) add.  Far from the origin, where coordinates are rounded more
+// coarsely than that, a source is a lattice only if its coordinates agree in
+// their bits.  Linear in the points; gives up as soon as a dimension has more
+// coordinates than MAXN.
 inline void find_lattice(const double *x, int64_t n, int dim, Lattice &L)
 {
     constexpr int MAXN = 4096, BITS = 13, CAP = 1 << BITS;
@@ -94,8 +101,7 @@ inline void find_lattice(const double *x, int64_t n, int dim, Lattice &L)
             std::vector<int> ord(m);
             for (int i = 0; i < m; ++i) ord[i] = i;
             std::sort(ord.begin(), ord.end(), [&](int a, int b) { return val[d][a] < val[d][b]; });
-            const double scale = std::max(fabs(val[d][ord[0]]), fabs(val[d][ord[m - 1]]));
-            const double tol = merge ? 4.0 * 2.220446049250313e-16 * scale : -1.0;
+            const double tol = merge ? LAT_ULPS * (val[d][ord[m - 1]] - val[d][ord[0]]) : -1.0;
             rank[d].assign(m, 0);
             coord[d].clear();
             for (int i = 0; i < m; ++i) {
@@ -127,12 +133,15 @@ inline void find_lattice(const double *x, int64_t n, int dim, Lattice &L)
         o += L.n[d];
         L.X.insert(L.X.end(), coord[d].begin(), coord[d].end());
         const std::vector<double> &c = coord[d];
-        const double tol = 4.0 * 2.220446049250313e-16 * std::max(fabs(c.front()), fabs(c.back()));
+        const double tol = LAT_ULPS * (c.back() - c.front());
         for (int p = 1; p <= LAT_MAXP && L.period[d] == 0 && 2 * p <= L.n[d]; ++p) {
             const int cells = (L.n[d] - 1) / p;
             const double h = (c[cells * p] - c[0]) / cells;
+            // every point of every run of LAT_RUN from its first one: the steps' differences add up along a run
             bool same = true;
-            for (int i = 0; i + p < L.n[d] && same; ++i) same = fabs(c[i + p] - c[i] - h) <= tol;
+            for (int i = 0; i + p < L.n[d] && same; ++i)
+                for (int k = 1; k < LAT_RUN && i + k * p < L.n[d] && same; ++k)
+                    same = fabs(c[i + k * p] - c[i] - k * h) <= tol;
             if (same) {
                 L.period[d] = p;
                 L.step[d] = h;

@@ -1,5 +1,6 @@
 """The ends of the range of the lattice sweeps (csrc/sdot_lattice.cuh) against the FP64 oracle: elongated sources,
-whose factors span the whole admitted range along one axis.
+whose factors span the whole admitted range along one axis, and sources away from the origin, whose coordinates are
+rounded.
 
 Tolerances as in test_gpu_parity.py: value and C 1e-10 relative, gradient 1e-12 absolute in FP64. Where it runs in
 FP32, the exponent's terms of up to D^2 / (2 eps) (D: the largest distance) are rounded four times: a relative
@@ -96,3 +97,34 @@ def test_beams_in_a_batch(oracle_mod, fp32):
         assert abs(J - J0) <= 1e-10 * max(abs(J0), 1e-6), (eps, J, J0)
         assert np.max(np.abs(g - g0)) <= tolerance(src, y, nu, eps, want, fp32), (eps, np.max(np.abs(g - g0)))
     b.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "hybrid"])
+@pytest.mark.parametrize("offset", [-300.0, 1e3, 1e5])
+@pytest.mark.parametrize("dim,n,order,N,eps", [(2, 64, 2, 400, 1.7e-3), (2, 43, 3, 400, 1.7e-3), (3, 8, 2, 64, 5e-3)])
+def test_source_away_from_the_origin(oracle_mod, dim, n, order, N, eps, offset, precision):
+    """The unit cube moved by `offset`: its coordinates are rounded to ulps of the offset, which neither equal
+    steps nor merged coordinates may add to the exponents (those are formed about the source's centre)."""
+    rng = np.random.default_rng(n)
+    src = structured_source(dim, n, order, lo=offset, hi=offset + 1.0,
+                            nodal_density=lambda p: 1.0 + 0.5 * np.sin(3.0 * p[:, 0]))
+    y, nu = offset + rng.random((N, dim)), rng.dirichlet(np.ones(N) * 5)
+    psi = 0.5 * eps * rng.standard_normal(N)
+    s = solver_of(src, y, nu, eps, precision)
+    want = oracle_of(oracle_mod, src, y, nu, eps, psi)
+    check(s, want, psi, tolerance(src, y, nu, eps, want, precision != "fp64"))
+    s.close()
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-3, 1e4])
+def test_coordinates_rounded_cell_by_cell(oracle_mod, scale):
+    """Points whose shared coordinates differ in the last bits (each cell mapped by itself)."""
+    rng = np.random.default_rng(2)
+    src = dict(structured_source(2, 64, 2))
+    src["x"] = src["x"] + 2.0 ** -53 * rng.integers(-1, 2, src["x"].shape)
+    src["x"], src["cell_centers"] = scale * src["x"], scale * src["cell_centers"]
+    N, eps = 400, 1.7e-3 * scale ** 2
+    y, nu, psi = scale * rng.random((N, 2)), rng.dirichlet(np.ones(N) * 5), 0.5 * eps * rng.standard_normal(N)
+    s = solver_of(src, y, nu, eps, "fp64")
+    check(s, oracle_of(oracle_mod, src, y, nu, eps, psi), psi, 1e-12)
+    s.close()
