@@ -1558,10 +1558,10 @@ sdot_status evaluate_complete(sdot_ctx *c, const EvalPending &pend, double *ms_o
 // life of the process; a cudaDeviceReset by the host application frees the
 // module instance the cached address points into, so no-alloc calls must not
 // follow one.  Every scratch word the evaluation reads is written earlier by
-// the same evaluation on the same stream: nothing has to start at zero, and
-// only the scalar slots the evaluation writes are copied back to the context.
-// The array is shared by every context of the process on a device, so calls
-// whose executions overlap corrupt each other.
+// the same evaluation on the same stream (the finalize kernel's arrival
+// counter is cleared first): nothing has to start at zero.  The array is
+// shared by every context of the process on a device, so calls whose
+// executions overlap corrupt each other, but no call after them.
 // ---------------------------------------------------------------------------
 
 namespace sdot {
@@ -1569,7 +1569,7 @@ namespace sdot {
 constexpr size_t NOALLOC_BYTES = size_t(8) << 20;  // == SDOT_NOALLOC_SCRATCH_BYTES
 constexpr int NOALLOC_MAX_DEVICES = 64;
 
-// (its last words are the finalize kernel's arrival counter: zero at load and between evaluations)
+// (its last words hold the finalize kernel's arrival counter)
 static __device__ __align__(256) double g_noalloc_scratch[NOALLOC_BYTES / sizeof(double) + 32];
 
 static double *g_noalloc_ptr[NOALLOC_MAX_DEVICES] = {};
@@ -1730,9 +1730,12 @@ extern "C" sdot_status sdot_evaluate_device_noalloc(sdot_ctx *c, const double *p
 
     if ((s = launch_gather(c, S + L.psi, psi_dev, c->nt)) != SDOT_OK) return s;
     unsigned *ticket = reinterpret_cast<unsigned *>(S + NOALLOC_BYTES / sizeof(double));
+    // not left to the kernel's own wrap to zero: two overlapping calls of different grids can leave it elsewhere
+    cudaError_t e = cudaMemsetAsync(ticket, 0, sizeof *ticket, c->stream);
+    if (e != cudaSuccess) return cuda_error(c, e, "no-alloc evaluation");
     if (c->dim == 2) noalloc_launch<2>(c, a, S, ticket, L);
     else noalloc_launch<3>(c, a, S, ticket, L);
-    cudaError_t e = cudaGetLastError();
+    e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_error(c, e, "no-alloc evaluation launch");
     if ((s = launch_scatter(c, grad_dev, S + L.grad, c->nt)) != SDOT_OK) return s;
     // k_finalize writes slots SC_VALUE .. SC_VALSRC of the host's array except the
