@@ -529,13 +529,20 @@ int64_t sdot_debug_allocation_count(void);
  * latency-bound loop that cannot absorb cudaMalloc / cudaFree and the
  * synchronisation they imply.  The set-up calls (sdot_create,
  * sdot_set_source, sdot_set_target) still allocate, as before.
- *   - Requests whose scratch exceeds the limit (about 8 * n_q * (1 + 2 * vs)
- *     + (10 + slices) * 8 * n_targets bytes, where vs <= 16 is the number of
- *     target slices of the value sweep when n_q < 75,776 and 0 otherwise, and
- *     slices <= 64 that of the gradient sweep) are rejected with SDOT_EINVAL and
+ *   - Requests whose scratch exceeds the limit are rejected with SDOT_EINVAL and
  *     a message giving the need and the limit; truncated problems likewise.
+ *     The scratch is about 8 * n_q * (1 + 2 * vs) + (10 + gs) * 8 * n_targets
+ *     bytes: gs <= 64 slices of the gradient sweep, vs target slices of the
+ *     value sweep (over cells of a tensor grid of points vs <= 64, over single
+ *     points vs <= 16 when n_q < 75,776 and 0 otherwise).  Sources whose
+ *     points form a tensor lattice (untruncated sweeps as matrix products)
+ *     take 32 KiB per lattice tile of 64^2, 32^2 or 16^3 points and target
+ *     slice instead of the 16 * n_q * vs bytes; a request that fits either way
+ *     is accepted, with as many slices at a time as fit.  Only where fewer
+ *     than two do, the cell or point sweeps run in place of the lattice's, and
+ *     the results differ from sdot_evaluate_device's by rounding.
  *   - Nothing in the scratch has to start at zero: every word a call reads is
- *     written earlier by the same call on the context's stream.
+ *     written (or cleared) earlier by the same call on the context's stream.
  *   - The scratch is shared by all contexts of the process on a device: calls
  *     whose executions overlap (other threads, streams or contexts on the same
  *     device) race and corrupt each other's results.  Serialise them.

@@ -203,13 +203,25 @@ k_lat_prep(const double *__restrict__ y, const double *__restrict__ nu, double *
 template <int DIM>
 __global__ void __launch_bounds__(LAT_THREADS, 2)
 k_lat_value(LatArgs L, EvalArgs a, const double *__restrict__ tpack, const double *__restrict__ shift,
-            const double *__restrict__ step, int64_t tslice, double *__restrict__ ms)
+            const double *__restrict__ step, int64_t tslice, int slice0, double *__restrict__ ms)
 {
     extern __shared__ __align__(16) unsigned char lat_smem[];
-    const int64_t t0 = blockIdx.y * tslice;
+    const int64_t t0 = (slice0 + (int)blockIdx.y) * tslice;
     const int64_t t1 = min(a.nt, t0 + tslice);
     lat_value_block<DIM>(lat_smem, L, a, tpack, shift, step, blockIdx.x, t0, t1,
                          ms + ((int64_t)blockIdx.y * L.ntiles + blockIdx.x) * LAT_TILE);
+}
+
+// ms[i] += the n - 1 slices after it, in their order: the sums that
+// lat_merge_block forms over the slices, begun where not all of them fit the
+// scratch at once.
+__global__ void k_lat_fold(int64_t stride, int n, double *__restrict__ ms)
+{
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= stride) return;
+    double s = ms[i];
+    for (int k = 1; k < n; ++k) s += ms[i + k * stride];
+    ms[i] = s;
 }
 
 template <int DIM>
@@ -1025,10 +1037,11 @@ struct DenseShape {
     LatTiling lat;    // cap > 0: the lattice sweeps
     bool lat_grad;    // the gradient sweep too
     int gts;          // tiles per CTA of the lattice gradient sweep (nks groups)
+    int slots;        // slices of the lattice value sweep that the partials hold at a time
     // doubles of the value sweep's partials and of the gradient partials
     size_t vpart_need(int64_t nq, int64_t nt, int64_t ntblk) const
     {
-        if (lat.cap > 0) return (size_t)lat.ntiles * ((size_t)nvs * LAT_TILE + 2) + (size_t)(3 * nt + ntblk);
+        if (lat.cap > 0) return (size_t)lat.ntiles * ((size_t)slots * LAT_TILE + 2) + (size_t)(3 * nt + ntblk);
         return (nvs > 1 || tm > 0) ? (size_t)2 * nvs * nq : 0;
     }
     size_t gpart_need(int64_t nt) const { return (size_t)nks * nt; }
@@ -1091,6 +1104,7 @@ static DenseShape dense_shape_of(const sdot_ctx *c, double eps, bool fp64)
     d.nvs = lat_slices(d.lat.ntiles, (c->nt + 15) / 16, SLOTS);
     d.tslice = (c->nt + d.nvs - 1) / d.nvs;
     d.nvs = (int)((c->nt + d.tslice - 1) / d.tslice);
+    d.slots = d.nvs;
     d.nval = (int64_t)d.lat.ntiles * (LAT_TILE / LAT_THREADS);
     d.lat_grad = fp64;
     if (fp64) {
@@ -1135,7 +1149,7 @@ static void lat_smem_limit(K k, size_t bytes)
 struct LatScratch {
     double *shift, *step, *top;
     LatScratch(const DenseShape &ds, double *vpart, int64_t nt, int dim)
-        : shift(vpart + (size_t)ds.lat.ntiles * ds.nvs * LAT_TILE), step(shift + 2 * ds.lat.ntiles), top(step + nt * dim)
+        : shift(vpart + (size_t)ds.lat.ntiles * ds.slots * LAT_TILE), step(shift + 2 * ds.lat.ntiles), top(step + nt * dim)
     {
     }
 };
@@ -1161,9 +1175,19 @@ static void launch_lat_value(const sdot_ctx *c, const DenseShape &ds, const doub
     const LatBlocks K{c->tblk_off.p, nullptr, c->tblk_sph.p, S.top, (int)c->ntblk};
     const size_t smem = sizeof(LatValueSmem<DIM>);
     lat_smem_limit(k_lat_value<DIM>, smem);
-    k_lat_value<DIM><<<dim3((unsigned)L.ntiles, (unsigned)ds.nvs), LAT_THREADS, smem, st>>>(
-        L, a, tpack, S.shift, S.step, ds.tslice, vpart);
-    k_lat_merge<DIM><<<(unsigned)ds.nval, LAT_THREADS, 0, st>>>(L, a, K, ds.nvs, ds.lat_grad, vpart, S.shift, tpack,
+    // all slices at once where the partials hold them, else a pass at a time into the slots after the sum so far
+    const int64_t stride = (int64_t)L.ntiles * LAT_TILE;
+    int held = 0;
+    for (int s = 0; s < ds.nvs;) {
+        if (held > 1) k_lat_fold<<<(unsigned)(stride / LAT_THREADS), LAT_THREADS, 0, st>>>(stride, held, vpart);
+        held = std::min(held, 1);
+        const int n = std::min(ds.nvs - s, ds.slots - held);
+        k_lat_value<DIM><<<dim3((unsigned)L.ntiles, (unsigned)n), LAT_THREADS, smem, st>>>(
+            L, a, tpack, S.shift, S.step, ds.tslice, s, vpart + held * stride);
+        s += n;
+        held += n;
+    }
+    k_lat_merge<DIM><<<(unsigned)ds.nval, LAT_THREADS, 0, st>>>(L, a, K, held, ds.lat_grad, vpart, S.shift, tpack,
                                                                 c->rho.p, c->jxw.p, Lq, blkpart);
 }
 
@@ -1684,11 +1708,19 @@ extern "C" sdot_status sdot_evaluate_device_noalloc(sdot_ctx *c, const double *p
         return set_error(c, SDOT_EINVAL,
                          "no-alloc evaluation covers untruncated problems only (pointwise threshold, tau <= 0)");
     if (c->distance != 0) return set_error(c, SDOT_EINVAL, "no-alloc evaluation covers the euclidean distance only");
-    // the launch shape of the allocating path; where the lattice sweeps' partials
-    // do not fit the static scratch, the cell or point sweeps'
-    NoallocLayout L = noalloc_layout(c, dense_shape_of(c, p.epsilon, c->precision == SDOT_PREC_FP64));
-    if ((size_t)L.total * sizeof(double) > NOALLOC_BYTES && L.ds.lat.cap > 0)
-        L = noalloc_layout(c, dense_shape(c->nq, c->nt, dense_tensor_m(c, KAPPA / p.epsilon), c->ncells));
+    // The launch shape of the allocating path.  Where the lattice sweeps' partials exceed the scratch but the cell
+    // or point sweeps' would not, as many target slices at a time as fit (the sums keep their order); only where not
+    // even two fit, the cell or point sweeps, which round differently.
+    DenseShape ds = dense_shape_of(c, p.epsilon, c->precision == SDOT_PREC_FP64);
+    NoallocLayout L = noalloc_layout(c, ds);
+    constexpr int64_t CAP = NOALLOC_BYTES / sizeof(double);
+    if (L.total > CAP && ds.lat.cap > 0) {
+        const int64_t per = (int64_t)ds.lat.ntiles * LAT_TILE;
+        ds.slots = (int)(ds.nvs - std::min<int64_t>(ds.nvs, (L.total - CAP + per - 1) / per));
+        const NoallocLayout other =
+            noalloc_layout(c, dense_shape(c->nq, c->nt, dense_tensor_m(c, KAPPA / p.epsilon), c->ncells));
+        L = other.total <= CAP && ds.slots >= 2 ? noalloc_layout(c, ds) : other;
+    }
     const size_t need = (size_t)L.total * sizeof(double);
     if (need > NOALLOC_BYTES)
         return set_error(c, SDOT_EINVAL,
