@@ -362,6 +362,8 @@ sdot_status sdot_batch_problem_info(const sdot_batch *batch, int index, sdot_sol
  * which each target's FP64 partial sums are added. */
 sdot_status sdot_batch_set_shape(sdot_batch *batch, const int *shape);
 sdot_status sdot_batch_get_shape(const sdot_batch *batch, int *shape);
+/* sdot_get_dense_sweeps of one problem, as of the last evaluation. */
+sdot_status sdot_batch_get_sweeps(sdot_batch *batch, int index, int *sweeps);
 /* Device milliseconds (CUDA events) of the batch's last batched evaluation. */
 double sdot_batch_last_eval_ms(const sdot_batch *batch);
 /* The batch's own autotuner: times `reps` batched evaluations at psi (host,
@@ -444,6 +446,15 @@ double sdot_get_last_distance_threshold(const sdot_ctx *ctx);
 double sdot_get_C_global(const sdot_ctx *ctx);
 sdot_status sdot_set_distance_threshold(sdot_ctx *ctx, double threshold);
 
+/* Sweeps of an untruncated evaluation at the context's measures and
+ * parameters (no reference counterpart; for tests and measurements):
+ * [0] points per dimension of a lattice tile (0: the points are no lattice, or
+ * its sweeps do not apply), [1] lattice tiles, [2] 1 if the gradient sweep runs
+ * on the lattice too, [3] 1 if the lattice factors come in runs, [4] points per
+ * dimension of the cells on the cell sweeps (0: lattice or point sweeps),
+ * [5] target slices of the value sweep. */
+#define SDOT_DENSE_SWEEPS 6
+sdot_status sdot_get_dense_sweeps(sdot_ctx *ctx, int *sweeps);
 /* Replaces SotSolver::compute_covering_radius (SotSolver.h:275; SotSolver.cc:431-473). */
 sdot_status sdot_compute_covering_radius(sdot_ctx *ctx, double *radius);
 /* Replaces SotSolver::compute_geometric_radius_bound (SotSolver.h:296-299;

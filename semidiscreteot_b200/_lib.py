@@ -47,7 +47,10 @@ EXPORTED = [
     "sdot_debug_fail_allocation", "sdot_debug_allocation_count", "sdot_weighted_barycenters_spherical",
     "sdot_server_create", "sdot_server_destroy", "sdot_server_last_error", "sdot_server_submit", "sdot_server_poll",
     "sdot_server_wait", "sdot_server_get_stats", "sdot_server_reset_stats",
+    "sdot_get_dense_sweeps", "sdot_batch_get_sweeps",
 ]
+
+DENSE_SWEEPS = ("tile", "tiles", "lattice_gradient", "runs", "cell", "slices")  # sdot_get_dense_sweeps
 
 NOALLOC_SCRATCH_BYTES = 8 << 20  # SDOT_NOALLOC_SCRATCH_BYTES
 
@@ -169,6 +172,10 @@ def load():
     lib.sdot_measure_peaks.argtypes = [ip, vp]
     lib.sdot_evaluate_device_noalloc.argtypes = [vp, vp, vp, C.POINTER(d)]
     lib.sdot_evaluate_device_noalloc.restype = ip
+    lib.sdot_get_dense_sweeps.argtypes = [vp, vp]
+    lib.sdot_get_dense_sweeps.restype = ip
+    lib.sdot_batch_get_sweeps.argtypes = [vp, ip, vp]
+    lib.sdot_batch_get_sweeps.restype = ip
     lib.sdot_hessian_device.argtypes = [vp, vp, vp, ip, ip, C.POINTER(HessianInfo)]
     lib.sdot_hessian_device.restype = ip
     lib.sdot_set_hessian_chunk.argtypes = [vp, ip]

@@ -123,6 +123,12 @@ class BatchSolver:
         arr = np.ascontiguousarray(shape, dtype=np.int32)
         self._check(self._L.sdot_batch_set_shape(self._h, arr.ctypes.data))
 
+    def sweeps(self, index: int) -> dict:
+        """Sweeps of one problem's last evaluation (see SotSolver.dense_sweeps)."""
+        out = np.zeros(len(_lib.DENSE_SWEEPS), dtype=np.int32)
+        self._check(self._L.sdot_batch_get_sweeps(self._h, int(index), out.ctypes.data))
+        return dict(zip(_lib.DENSE_SWEEPS, out.tolist()))
+
     def last_eval_ms(self) -> float:
         """Device milliseconds of the last batched evaluation."""
         return float(self._L.sdot_batch_last_eval_ms(self._h))

@@ -1135,6 +1135,17 @@ void sdot_batch_destroy(sdot_batch *b)
     delete b;
 }
 
+sdot_status sdot_batch_get_sweeps(sdot_batch *b, int index, int *sweeps)
+{
+    if (!b || !sweeps || index < 0 || index >= (int)b->probs.size()) return SDOT_EINVAL;
+    if (!b->uploaded) return berr(b, SDOT_ESTATE, "no evaluation yet");
+    const BInst &I = b->inst[index];
+    const int v[SDOT_DENSE_SWEEPS] = {I.lat ? I.L.cap : 0, I.lat ? I.L.ntiles : 0, I.lat_grad(),
+                                      I.lat && I.L.runs > 0, 0, I.lat ? I.nvs : 1};
+    std::copy(v, v + SDOT_DENSE_SWEEPS, sweeps);
+    return SDOT_OK;
+}
+
 const char *sdot_batch_last_error(const sdot_batch *b) { return b ? b->err.c_str() : "null batch"; }
 
 int sdot_batch_size(const sdot_batch *b) { return b ? (int)b->probs.size() : 0; }

@@ -840,6 +840,16 @@ sdot_status sdot_evaluate_device(sdot_ctx *c, const double *psi_dev, double *gra
     return s;
 }
 
+sdot_status sdot_get_dense_sweeps(sdot_ctx *c, int *sweeps)
+{
+    if (!c || !sweeps) return SDOT_EINVAL;
+    if (c->nq == 0 || c->nt == 0) return set_error(c, SDOT_ESTATE, "measures not set");
+    if (!(c->prm.epsilon > 0) || c->distance != 0)
+        return set_error(c, SDOT_EINVAL, "no dense sweeps for these parameters");
+    dense_sweeps(c, sweeps);
+    return SDOT_OK;
+}
+
 sdot_status sdot_compute_covering_radius(sdot_ctx *c, double *radius)
 {
     if (!c || !radius) return SDOT_EINVAL;

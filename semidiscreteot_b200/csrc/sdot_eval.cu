@@ -1094,11 +1094,17 @@ static DenseShape dense_shape_of(const sdot_ctx *c, double eps, bool fp64)
     for (int k = 0; k < 3; ++k)
         reach[k] = std::max(std::fabs(c->tgt_lo[k] - c->origin[k]), std::fabs(c->tgt_hi[k] - c->origin[k]));
     d.lat = lat_tiling(c->lat_n, c->lat_xo, c->lat_X.data(), c->dim, s, reach);
-    // The merge takes the points' maxima over the targets in one CTA per
-    // LAT_THREADS points: with fewer of them than SMs and more targets than it
-    // lists at once it is a serial chain (4,096 points x 10,538 targets: value
-    // 298 us against 63 on the cell or point sweeps).
-    if ((int64_t)d.lat.ntiles * (LAT_TILE / LAT_THREADS) < 148 && c->nt > 1024) d.lat = LatTiling{};
+    // The merge takes the points' maxima in one CTA per LAT_THREADS points, and with more targets than it lists at
+    // once it goes through their blocks in turn: few points are few CTAs with a long chain each.  Lattice against
+    // cell sweeps, us per FP64 evaluation at eps = 1e-2, 1,025 / 3,001 / 10,538 targets: 2D 64^2 points 60 / 85 / 187
+    // against 52 / 66 / 110, 96^2 58 / 76 / 153 against 60 / 84 / 175 (hybrid 66 / 86 / 168 against 62 / 84 / 164),
+    // 112^2 58 / 75 / 136 against 64 / 97 / 222, 192^2 62 / 83 / 161 against 98 / 181 / 507; 3D 24^3 64 / 98 / 247
+    // against 66 / 97 / 208, 26^3 65 / 101 / 249 against 71 / 111 / 254 (hybrid 78 / 110 / 261 against 76 / 111 /
+    // 239), 28^3 63 / 102 / 234 against 76 / 120 / 287, 32^3 63 / 96 / 205 against 90 / 148 / 390.
+    // (Batches have no such line: their other sweeps go by points without target slices, 1,468 us against 390 for
+    // 16^3 points x 10,538 targets alone, and all problems' merges are one launch.)
+    constexpr int64_t FEW_2D = 12000, FEW_3D = 18000;
+    if (c->nt > LAT_LIST && c->nq < (c->dim == 2 ? FEW_2D : FEW_3D)) d.lat = LatTiling{};
     if (d.lat.cap == 0) return d;
     constexpr int SLOTS = 148 * 2;
     d.nvs = lat_slices(d.lat.ntiles, (c->nt + 15) / 16, SLOTS);
@@ -1113,6 +1119,16 @@ static DenseShape dense_shape_of(const sdot_ctx *c, double eps, bool fp64)
         d.nks = (d.lat.ntiles + d.gts - 1) / d.gts;
     }
     return d;
+}
+
+void dense_sweeps(const sdot_ctx *c, int *sweeps)
+{
+    const DenseShape d = dense_shape_of(c, c->prm.epsilon, c->precision == SDOT_PREC_FP64);
+    const bool lat = d.lat.cap > 0;
+    LatArgs L{};
+    if (lat) lat_runs(c->lat_period, c->lat_step, c->dim, d.lat.span, L);
+    const int v[SDOT_DENSE_SWEEPS] = {d.lat.cap, d.lat.ntiles, lat && d.lat_grad, L.runs > 0, lat ? 0 : d.tm, d.nvs};
+    std::copy(v, v + SDOT_DENSE_SWEEPS, sweeps);
 }
 
 size_t dense_gpart_need(const sdot_ctx *c)

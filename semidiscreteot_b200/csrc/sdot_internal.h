@@ -330,6 +330,7 @@ sdot_status ensure_eval_buffers(sdot_ctx *c);
 sdot_status ensure_tickets(sdot_ctx *c);  // c->ticket
 // Gradient partials (doubles) of an untruncated evaluation at the current parameters (0 where it truncates).
 size_t dense_gpart_need(const sdot_ctx *c);
+void dense_sweeps(const sdot_ctx *c, int *sweeps);  // sdot_get_dense_sweeps
 // VerboseSolverControl::check on the last evaluation's scalars: 1 converged,
 // 0 iterate, -1 failure (max_iterations reached or NaN).
 int solver_control_check(sdot_ctx *c, unsigned step, double *value);

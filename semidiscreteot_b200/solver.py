@@ -158,6 +158,12 @@ class SotSolver:
                                                          C.byref(val)))
         return val.value
 
+    def dense_sweeps(self) -> dict:
+        """Sweeps that an untruncated evaluation runs at the configured parameters (sdot_get_dense_sweeps)."""
+        out = np.zeros(len(_lib.DENSE_SWEEPS), dtype=np.int32)
+        self._check(self._L.sdot_get_dense_sweeps(self._h, out.ctypes.data))
+        return dict(zip(_lib.DENSE_SWEEPS, out.tolist()))
+
     def solve(self, potential: np.ndarray, params: Optional[SolverParameters] = None) -> np.ndarray:
         """SotSolver::solve (SotSolver.cc:105-215): L-BFGS on the device.
         ``potential`` is updated in place when it is a float64 C-contiguous array."""

@@ -53,7 +53,8 @@ def test_calls_of_different_grids_in_turn():
 
 # lattice partials beyond the scratch (63 or 64 slices x 4 tiles, 37 x 8), those of the cell or point sweeps within it
 @pytest.mark.parametrize("precision", ["fp64", "hybrid"])
-@pytest.mark.parametrize("dim,n,order,N", [(2, 64, 2, 1024), (2, 32, 4, 1000), (3, 8, 4, 1000)])
+@pytest.mark.parametrize("dim,n,order,N", [(2, 64, 2, 1024), (2, 64, 2, 1100), (2, 32, 4, 1000),
+                                              (3, 8, 4, 1000)])
 def test_slices_in_passes(dim, n, order, N, precision):
     src, y, nu, z = problem(dim, n, order, N)
     s = solver_of(src, y, nu, 2e-2, precision)
