@@ -27,6 +27,7 @@
 #include <float.h>
 #include <math.h>
 #include <stdio.h>
+#include <stdlib.h>
 
 #include <algorithm>
 #include <atomic>
@@ -76,7 +77,6 @@ struct BInst {
 
 constexpr int BLAT_PREP = 512;      // threads of k_batch_lat_prep
 constexpr int BLAT_PREP_CTAS = 16;  // CTAs per problem over its target blocks
-
 // ---------------------------------------------------------------------------
 // kernels
 // ---------------------------------------------------------------------------
@@ -627,7 +627,8 @@ struct sdot_batch {
     std::vector<BInst> inst;
     std::vector<Lattice> lat;          // per problem: the points' lattice (coordinates and counts; host)
     std::vector<double> reach;         // per problem and dimension: the targets' distance from the origin
-    int64_t lat_tslice = 0;            // targets per unit of the lattice value sweep
+    std::vector<int> lat_group;        // per problem: the group whose slice sums are held together with its own
+    size_t sums_cap = size_t(4) << 30; // bytes of slice sums held at a time (SDOT_BATCH_SUMS_BYTES)
     int64_t total_q = 0, total_t = 0, total_part = 0, total_gp = 0;
 
     DevBuf<double> x, rho, jxw, w, y, nu, psi, grad, tpack, Lq, part, gpart, x0, g0, pdir, S, Y, rho_h, scal, alpha,
@@ -639,8 +640,12 @@ struct sdot_batch {
     DevBuf<double> lat_x, lat_sph, lat_top, lat_step, lat_ms, red;
     DevBuf<int> lat_q, lat_mem;
     DevBuf<int64_t> lat_off;
-    // unit counts of the lists on the device, and what they were made for
-    int nv = 0, ng = 0, nlv = 0, nlg = 0, nm = 0, nf = 0, lat_tiles = 0;
+    // unit counts of the lists on the device (lattice lists: by group, ends), and what they were made for
+    struct GroupEnds {
+        int value = 0, merge = 0, grad = 0;
+    };
+    int nv = 0, ng = 0, nf = 0, lat_tiles = 0;
+    std::vector<GroupEnds> lat_ends;
     bool units_ok = false;
     std::vector<int> units_act;
     DevBuf<BHist> dhist;
@@ -686,28 +691,6 @@ struct DevGuard {
     }
 };
 
-// The most tiles (over the tile sizes), and the most tile groups of the
-// gradient sweep, that problem i may use.
-struct LatMost {
-    int64_t tiles = 0;
-    int groups = 0;
-};
-LatMost lat_most(const sdot_batch *b, int i)
-{
-    LatMost m;
-    const Lattice &G = b->lat[i];
-    if (!G.ok) return m;
-    for (int k = 0; k < (b->dim == 2 ? 2 : 1); ++k) {
-        const int cap = b->dim == 2 ? LAT_CAPS2[k] : LAT_CAPS3[k];
-        int64_t t = 1;
-        for (int d = 0; d < b->dim; ++d) t *= (G.n[d] + cap - 1) / cap;
-        m.tiles = std::max(m.tiles, t);
-    }
-    const int gts = b->inst[i].gts;
-    m.groups = (int)((m.tiles + gts - 1) / gts);
-    return m;
-}
-
 // Gradient slices of every problem for the slice target b->shape[2] (at 8:
 // the single-problem dense path's count): target blocks of DENSE_B_THREADS *
 // TT, slices of at least 256 points, at most 64.  Sets nks, ntb, qslice and
@@ -727,7 +710,8 @@ int64_t plan_slices(sdot_batch *b)
         I.ntb = (int)tb;
         I.qslice = (P.nq + nks - 1) / nks;
         I.gp0 = gp0;
-        gp0 += (int64_t)std::max(nks, lat_most(b, (int)i).groups) * P.nt;
+        const int groups = b->lat[i].ok ? (lat_tile_range(b->lat[i].n, b->dim).most + I.gts - 1) / I.gts : 0;
+        gp0 += (int64_t)std::max(nks, groups) * P.nt;
     }
     b->total_gp = gp0;
     b->units_ok = false;
@@ -752,6 +736,121 @@ void plan_lattice(sdot_batch *b, int i)
     I.lat = 1;
 }
 
+// A problem's k-d blocks of targets: members and bounding spheres.
+struct TargetBlocks {
+    std::vector<int64_t> off;
+    std::vector<int> mem;
+    std::vector<double> sph;
+};
+
+// Units of the lattice sweeps (about eight per resident CTA over the whole
+// batch, of 4,096 points x tslice targets (value) and 64 targets x tslice / 64
+// tiles (gradient)), partial offsets, and the lattices' data and scratch on
+// the device.  Slice sums are held for groups of problems together, of up to
+// sums_cap bytes; a group's sweeps end before the next one's begin.  Where
+// there is no memory for the lattices' buffers, all problems run the point
+// sweeps.
+sdot_status upload_lattices(sdot_batch *b, const std::vector<TargetBlocks> &blk)
+{
+    const size_t np = b->probs.size();
+    const int D = b->dim;
+    std::vector<double> lx, lsph;
+    std::vector<int> lq, lmem;
+    std::vector<int64_t> loff;
+    std::vector<int64_t> ms0(np), sh0(np), sp0(np), x0(np), lq0(np), mem0(np), off0(np), sph0(np);
+    int64_t ms = 0, ms_most = 0, sh = 0, sp = 0, part0 = 0;
+    int group = 0;
+    double lpairs = 0.0;
+    for (size_t i = 0; i < np; ++i)
+        if (b->lat[i].ok) lpairs += (double)b->probs[i].nq * (double)b->probs[i].nt;
+    const int64_t tslice = std::min<int64_t>(
+        4096, std::max<int64_t>(128, (int64_t)(lpairs / ((double)LAT_TILE * b->sms * 2 * 8)) / 64 * 64));
+    b->lat_group.assign(np, 0);
+    for (size_t i = 0; i < np; ++i) {
+        BInst &I = b->inst[i];
+        const auto &P = b->probs[i];
+        const Lattice &G = b->lat[i];
+        const int64_t tiles = G.ok ? lat_tile_range(G.n, D).most : 0;
+        I.tslice = tslice;
+        I.nvs = (int)((P.nt + I.tslice - 1) / I.tslice);
+        I.gts = (int)(I.tslice / LAT_GT);
+        I.part0 = part0;
+        part0 += std::max<int64_t>(I.nvb, tiles * (LAT_TILE / LAT_THREADS));
+        if (!G.ok) continue;
+        const int64_t sums = tiles * I.nvs * LAT_TILE;
+        if (ms > 0 && (size_t)(ms + sums) * 8 > b->sums_cap) {
+            ms = 0;
+            ++group;
+        }
+        b->lat_group[i] = group;
+        ms0[i] = ms;
+        ms += sums;
+        ms_most = std::max(ms_most, ms);
+        sh0[i] = sh;
+        sh += 2 * tiles;
+        sp0[i] = sp;
+        sp += P.nt * D;
+        x0[i] = (int64_t)lx.size();
+        lx.insert(lx.end(), G.X.begin(), G.X.end());
+        lq0[i] = (int64_t)lq.size();
+        lq.insert(lq.end(), G.q.begin(), G.q.end());
+        mem0[i] = (int64_t)lmem.size();
+        lmem.insert(lmem.end(), blk[i].mem.begin(), blk[i].mem.end());
+        off0[i] = (int64_t)loff.size();
+        loff.insert(loff.end(), blk[i].off.begin(), blk[i].off.end());
+        sph0[i] = (int64_t)lsph.size();
+        lsph.insert(lsph.end(), blk[i].sph.begin(), blk[i].sph.end());
+    }
+    b->total_part = part0;
+    b->lat_ends.resize((size_t)group + 1);
+    if (lq.empty()) return SDOT_OK;
+    cudaError_t e = b->lat_x.alloc(lx.size());
+    if (e == cudaSuccess) e = b->lat_q.alloc(lq.size());
+    if (e == cudaSuccess) e = b->lat_mem.alloc(lmem.size());
+    if (e == cudaSuccess) e = b->lat_off.alloc(loff.size());
+    if (e == cudaSuccess) e = b->lat_sph.alloc(lsph.size());
+    if (e == cudaSuccess) e = b->lat_top.alloc(lsph.size() / 4);
+    if (e == cudaSuccess) e = b->lat_step.alloc(sp);
+    if (e == cudaSuccess) e = b->lat_ms.alloc(ms_most + sh);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        for (auto *v : {&b->lat_x, &b->lat_sph, &b->lat_top, &b->lat_step, &b->lat_ms}) v->release();
+        b->lat_q.release();
+        b->lat_mem.release();
+        b->lat_off.release();
+        b->lat.assign(np, Lattice());
+        return SDOT_OK;
+    }
+    BCK(e, "batch lattice");
+    BCK(cudaMemcpy(b->lat_x.p, lx.data(), lx.size() * 8, cudaMemcpyHostToDevice), "batch lattice");
+    BCK(cudaMemcpy(b->lat_q.p, lq.data(), lq.size() * sizeof(int), cudaMemcpyHostToDevice), "batch lattice");
+    BCK(cudaMemcpy(b->lat_mem.p, lmem.data(), lmem.size() * sizeof(int), cudaMemcpyHostToDevice), "batch lattice");
+    BCK(cudaMemcpy(b->lat_off.p, loff.data(), loff.size() * 8, cudaMemcpyHostToDevice), "batch lattice");
+    BCK(cudaMemcpy(b->lat_sph.p, lsph.data(), lsph.size() * 8, cudaMemcpyHostToDevice), "batch lattice");
+    for (size_t i = 0; i < np; ++i) {
+        BInst &I = b->inst[i];
+        Lattice &G = b->lat[i];
+        if (!G.ok) continue;
+        I.L.X = b->lat_x.p + x0[i];
+        I.L.q = b->lat_q.p + lq0[i];
+        for (int d = 0; d < 3; ++d) {
+            I.L.n[d] = G.n[d];
+            I.L.xo[d] = G.xo[d];
+        }
+        I.K.off = b->lat_off.p + off0[i];
+        I.K.mem = b->lat_mem.p + mem0[i];
+        I.K.sph = b->lat_sph.p + sph0[i];
+        I.K.top = b->lat_top.p + sph0[i] / 4;
+        I.K.n = (int)blk[i].off.size() - 1;
+        I.ms = b->lat_ms.p + ms0[i];
+        I.shift = b->lat_ms.p + ms_most + sh0[i];
+        I.step = b->lat_step.p + sp0[i];
+        std::vector<int>().swap(G.q);  // on the device from here on
+        plan_lattice(b, (int)i);
+    }
+    return SDOT_OK;
+}
+
 // Layout of every problem in the packed arrays and its launch shapes (the
 // single-problem dense path's: value blocks of DENSE_A_THREADS points,
 // gradient target blocks of DENSE_B_THREADS * TT and the same slice count).
@@ -760,7 +859,7 @@ sdot_status upload(sdot_batch *b)
     const int D = b->dim;
     const size_t np = b->probs.size();
     b->inst.assign(np, BInst{});
-    int64_t q0 = 0, t0 = 0, part0 = 0;
+    int64_t q0 = 0, t0 = 0;
     for (size_t i = 0; i < np; ++i) {
         const auto &P = b->probs[i];
         BInst &I = b->inst[i];
@@ -785,22 +884,15 @@ sdot_status upload(sdot_batch *b)
         I.t0 = t0;
         const int64_t per = DENSE_A_THREADS;
         I.nvb = (int)((P.nq + per - 1) / per);
-        I.part0 = part0;
         I.fp32 = 0;
         I.tol = P.prm.tolerance;
         q0 += P.nq;
         t0 += P.nt;
-        part0 += I.nvb;
     }
     b->total_q = q0;
     b->total_t = t0;
     // lattices: found per problem (threads over the problems), with k-d blocks of their targets
-    struct Blocks {
-        std::vector<int64_t> off;
-        std::vector<int> mem;
-        std::vector<double> sph;
-    };
-    std::vector<Blocks> blk(np);
+    std::vector<TargetBlocks> blk(np);
     b->lat.assign(np, Lattice());
     b->reach.assign(3 * np, 0.0);
     {
@@ -808,6 +900,7 @@ sdot_status upload(sdot_batch *b)
         auto one = [&](size_t i) {
             const auto &P = b->probs[i];
             find_lattice(b->hx.data() + b->inst[i].q0 * D, P.nq, D, b->lat[i]);
+            if (b->lat[i].ok && lat_tile_range(b->lat[i].n, D).most == 0) b->lat[i] = Lattice();
             if (!b->lat[i].ok) return;
             const double *y = b->hy.data() + b->inst[i].t0 * D;
             const std::vector<double> pts(y, y + P.nt * D);
@@ -841,85 +934,9 @@ sdot_status upload(sdot_batch *b)
         work();
         for (auto &t : pool) t.join();
     }
-    // units of the lattice sweeps: about eight per resident CTA over the whole batch, of 4,096 points x tslice
-    // targets (value) and 64 targets x tslice / 64 tiles (gradient)
-    double lpairs = 0.0;
-    for (size_t i = 0; i < np; ++i)
-        if (b->lat[i].ok) lpairs += (double)b->probs[i].nq * (double)b->probs[i].nt;
-    b->lat_tslice = std::min<int64_t>(
-        4096, std::max<int64_t>(128, (int64_t)(lpairs / ((double)LAT_TILE * b->sms * 2 * 8)) / 64 * 64));
-    std::vector<double> lx, lsph;
-    std::vector<int> lq, lmem;
-    std::vector<int64_t> loff;
-    int64_t ms = 0, sh = 0, sp = 0;
-    std::vector<int64_t> ms0(np), sh0(np), sp0(np), x0(np), lq0(np), mem0(np), off0(np), sph0(np);
-    part0 = 0;
-    for (size_t i = 0; i < np; ++i) {
-        BInst &I = b->inst[i];
-        const auto &P = b->probs[i];
-        const Lattice &G = b->lat[i];
-        I.tslice = b->lat_tslice;
-        I.nvs = (int)((P.nt + I.tslice - 1) / I.tslice);
-        I.gts = (int)std::max<int64_t>(1, b->lat_tslice / LAT_GT);
-        const LatMost m = lat_most(b, (int)i);
-        I.part0 = part0;
-        part0 += std::max<int64_t>(I.nvb, m.tiles * (LAT_TILE / LAT_THREADS));
-        if (!G.ok) continue;
-        ms0[i] = ms;
-        ms += m.tiles * I.nvs * LAT_TILE;
-        sh0[i] = sh;
-        sh += 2 * m.tiles;
-        sp0[i] = sp;
-        sp += P.nt * D;
-        x0[i] = (int64_t)lx.size();
-        lx.insert(lx.end(), G.X.begin(), G.X.end());
-        lq0[i] = (int64_t)lq.size();
-        lq.insert(lq.end(), G.q.begin(), G.q.end());
-        mem0[i] = (int64_t)lmem.size();
-        lmem.insert(lmem.end(), blk[i].mem.begin(), blk[i].mem.end());
-        off0[i] = (int64_t)loff.size();
-        loff.insert(loff.end(), blk[i].off.begin(), blk[i].off.end());
-        sph0[i] = (int64_t)lsph.size();
-        lsph.insert(lsph.end(), blk[i].sph.begin(), blk[i].sph.end());
-    }
-    b->total_part = part0;
+    const sdot_status s = upload_lattices(b, blk);
+    if (s != SDOT_OK) return s;
     const int64_t gp0 = plan_slices(b);
-    if (!lq.empty()) {
-        BCK(b->lat_x.alloc(lx.size()), "batch lattice");
-        BCK(b->lat_q.alloc(lq.size()), "batch lattice");
-        BCK(b->lat_mem.alloc(lmem.size()), "batch lattice");
-        BCK(b->lat_off.alloc(loff.size()), "batch lattice");
-        BCK(b->lat_sph.alloc(lsph.size()), "batch lattice");
-        BCK(b->lat_top.alloc(lsph.size() / 4), "batch lattice");
-        BCK(b->lat_step.alloc(sp), "batch lattice");
-        BCK(b->lat_ms.alloc(ms + sh), "batch lattice");
-        BCK(cudaMemcpy(b->lat_x.p, lx.data(), lx.size() * 8, cudaMemcpyHostToDevice), "batch lattice");
-        BCK(cudaMemcpy(b->lat_q.p, lq.data(), lq.size() * sizeof(int), cudaMemcpyHostToDevice), "batch lattice");
-        BCK(cudaMemcpy(b->lat_mem.p, lmem.data(), lmem.size() * sizeof(int), cudaMemcpyHostToDevice), "batch lattice");
-        BCK(cudaMemcpy(b->lat_off.p, loff.data(), loff.size() * 8, cudaMemcpyHostToDevice), "batch lattice");
-        BCK(cudaMemcpy(b->lat_sph.p, lsph.data(), lsph.size() * 8, cudaMemcpyHostToDevice), "batch lattice");
-        for (size_t i = 0; i < np; ++i) {
-            BInst &I = b->inst[i];
-            Lattice &G = b->lat[i];
-            if (!G.ok) continue;
-            I.L.X = b->lat_x.p + x0[i];
-            I.L.q = b->lat_q.p + lq0[i];
-            for (int d = 0; d < 3; ++d) {
-                I.L.n[d] = G.n[d];
-                I.L.xo[d] = G.xo[d];
-            }
-            I.K.off = b->lat_off.p + off0[i];
-            I.K.mem = b->lat_mem.p + mem0[i];
-            I.K.sph = b->lat_sph.p + sph0[i];
-            I.K.top = b->lat_top.p + sph0[i] / 4;
-            I.K.n = (int)blk[i].off.size() - 1;
-            I.ms = b->lat_ms.p + ms0[i];
-            I.shift = b->lat_ms.p + ms + sh0[i];
-            I.step = b->lat_step.p + sp0[i];
-            std::vector<int>().swap(G.q);  // on the device from here on
-            plan_lattice(b, (int)i);
-        }
-    }
     BCK(b->x.alloc(q0 * D), "batch alloc");
     BCK(b->rho.alloc(q0), "batch alloc");
     BCK(b->jxw.alloc(q0), "batch alloc");
@@ -935,7 +952,7 @@ sdot_status upload(sdot_batch *b)
     BCK(b->pdir.alloc(t0), "batch alloc");
     BCK(b->S.alloc(6 * t0), "batch alloc");
     BCK(b->Y.alloc(6 * t0), "batch alloc");
-    BCK(b->part.alloc(part0 * 4), "batch alloc");
+    BCK(b->part.alloc(b->total_part * 4), "batch alloc");
     BCK(b->gpart.alloc(gp0), "batch alloc");
     BCK(b->rho_h.alloc(np * 8), "batch alloc");
     BCK(b->scal.alloc(np * SC_COUNT), "batch alloc");
@@ -945,7 +962,7 @@ sdot_status upload(sdot_batch *b)
     BCK(b->act.alloc(np), "batch alloc");
     BCK(b->spare.alloc(np), "batch alloc");
     BCK(b->dhist.alloc(np), "batch alloc");
-    BCK(b->counter.alloc(4), "batch alloc");
+    BCK(b->counter.alloc(2 + 2 * b->lat_ends.size()), "batch alloc");
     BCK(b->red.alloc((size_t)(t0 / BFIN_THREADS + 2 * np + 1) * BRED), "batch alloc");
     std::vector<double> w(q0);
     for (int64_t q = 0; q < q0; ++q) w[q] = b->hrho[q] * b->hjxw[q];
@@ -969,24 +986,30 @@ void batch_sweeps(sdot_batch *b, int nact, int64_t maxnt)
     const dim3 pg((unsigned)std::min<int64_t>((maxnt + 255) / 256, 64), (unsigned)nact);
     const int lgrid = b->sms * 2;
     k_batch_prep<DIM><<<pg, 256, 0, st>>>(b->dinst.p, b->act.p, b->y.p, b->nu.p, b->psi.p, b->tpack.p);
-    if (b->nlv > 0) {
-        const size_t vs = sizeof(LatValueSmem<DIM>);
-        cudaFuncSetAttribute(k_batch_lat_value<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vs);
-        k_batch_lat_prep<DIM><<<dim3((unsigned)(BLAT_PREP_CTAS + b->lat_tiles), (unsigned)nact), BLAT_PREP, 0, st>>>(
-            b->dinst.p, b->act.p, b->y.p, b->psi.p);
-        k_batch_lat_value<DIM><<<std::min(b->nlv, lgrid), LAT_THREADS, vs, st>>>(b->dinst.p, b->lvunits.p, b->nlv,
-                                                                                 b->counter.p + 2, b->tpack.p);
-        k_batch_lat_merge<DIM><<<(unsigned)b->nm, LAT_THREADS, 0, st>>>(b->dinst.p, b->munits.p, b->tpack.p, b->rho.p,
-                                                                        b->jxw.p, b->Lq.p, b->part.p);
-    }
     if (b->nv > 0)
         k_batch_value<DIM><<<std::min(b->nv, b->sms * b->shape[0]), DENSE_A_THREADS, 0, st>>>(
             b->dinst.p, b->vunits.p, b->nv, b->counter.p, b->x.p, b->rho.p, b->jxw.p, b->tpack.p, b->Lq.p, b->part.p);
-    if (b->nlg > 0) {
-        const size_t gs = sizeof(LatGradSmem<DIM>);
+    if (b->lat_ends.back().value > 0) {
+        const size_t vs = sizeof(LatValueSmem<DIM>), gs = sizeof(LatGradSmem<DIM>);
+        cudaFuncSetAttribute(k_batch_lat_value<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vs);
         cudaFuncSetAttribute(k_batch_lat_grad<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gs);
-        k_batch_lat_grad<DIM><<<std::min(b->nlg, lgrid), LAT_THREADS, gs, st>>>(b->dinst.p, b->lgunits.p, b->nlg,
-                                                                                b->counter.p + 3, b->tpack.p, b->gpart.p);
+        k_batch_lat_prep<DIM><<<dim3((unsigned)(BLAT_PREP_CTAS + b->lat_tiles), (unsigned)nact), BLAT_PREP, 0, st>>>(
+            b->dinst.p, b->act.p, b->y.p, b->psi.p);
+        sdot_batch::GroupEnds from;
+        int *counter = b->counter.p + 2;
+        for (const auto &to : b->lat_ends) {  // the merge's weights stand in the slice sums until the gradient sweep
+            if (const int n = to.value - from.value) {
+                k_batch_lat_value<DIM><<<std::min(n, lgrid), LAT_THREADS, vs, st>>>(
+                    b->dinst.p, b->lvunits.p + from.value, n, counter, b->tpack.p);
+                k_batch_lat_merge<DIM><<<(unsigned)(to.merge - from.merge), LAT_THREADS, 0, st>>>(
+                    b->dinst.p, b->munits.p + from.merge, b->tpack.p, b->rho.p, b->jxw.p, b->Lq.p, b->part.p);
+            }
+            if (const int n = to.grad - from.grad)
+                k_batch_lat_grad<DIM><<<std::min(n, lgrid), LAT_THREADS, gs, st>>>(
+                    b->dinst.p, b->lgunits.p + from.grad, n, counter + 1, b->tpack.p, b->gpart.p);
+            from = to;
+            counter += 2;
+        }
     }
     if (b->ng > 0)
         k_batch_grad<DIM><<<std::min(b->ng, b->sms * b->shape[1]), DENSE_B_THREADS, 0, st>>>(
@@ -1014,23 +1037,28 @@ sdot_status batch_eval(sdot_batch *b, const std::vector<int> &act, double *ms)
         for (auto &o : order) {
             const int p = o.second;
             const BInst &I = b->inst[p];
-            if (I.lat) {
+            if (!I.lat)
+                for (int k = 0; k < I.nvb; ++k) vu.push_back(make_int2(p, k));
+            if (!I.lat_grad())
+                for (int k = 0; k < I.nks; ++k)
+                    for (int t = 0; t < I.ntb; ++t) gu.push_back(make_int4(p, t, k, 0));
+            for (int k = 0; k * (int64_t)BFIN_THREADS < I.a.nt; ++k) fu.push_back(make_int2(p, k));
+        }
+        for (size_t g = 0; g < b->lat_ends.size(); ++g) {
+            for (auto &o : order) {
+                const int p = o.second;
+                const BInst &I = b->inst[p];
+                if (!I.lat || b->lat_group[p] != (int)g) continue;
                 tiles = std::max(tiles, I.L.ntiles);
                 for (int k = 0; k < I.nvs; ++k)
                     for (int t = 0; t < I.L.ntiles; ++t) lv.push_back(make_int4(p, t, k, 0));
                 for (int k = 0; k < I.value_parts(); ++k) mu.push_back(make_int2(p, k));
-            } else {
-                for (int k = 0; k < I.nvb; ++k) vu.push_back(make_int2(p, k));
-            }
-            if (I.lat_grad()) {
+                if (!I.lat_grad()) continue;
                 const int nb = (int)((I.a.nt + LAT_GT - 1) / LAT_GT);
                 for (int k = 0; k < I.ngs; ++k)
                     for (int t = 0; t < nb; ++t) lg.push_back(make_int4(p, t, k, 0));
-            } else {
-                for (int k = 0; k < I.nks; ++k)
-                    for (int t = 0; t < I.ntb; ++t) gu.push_back(make_int4(p, t, k, 0));
             }
-            for (int k = 0; k * (int64_t)BFIN_THREADS < I.a.nt; ++k) fu.push_back(make_int2(p, k));
+            b->lat_ends[g] = {(int)lv.size(), (int)mu.size(), (int)lg.size()};
         }
         b->units_ok = false;
         auto put = [&](auto &buf, const auto &v) {
@@ -1047,15 +1075,12 @@ sdot_status batch_eval(sdot_batch *b, const std::vector<int> &act, double *ms)
         BCK(put(b->funits, fu), "batch units");
         b->nv = (int)vu.size();
         b->ng = (int)gu.size();
-        b->nlv = (int)lv.size();
-        b->nlg = (int)lg.size();
-        b->nm = (int)mu.size();
         b->nf = (int)fu.size();
         b->lat_tiles = tiles;
         b->units_act = act;
         b->units_ok = true;
     }
-    BCK(cudaMemsetAsync(b->counter.p, 0, 4 * sizeof(int), st), "batch counter");
+    BCK(cudaMemsetAsync(b->counter.p, 0, (2 + 2 * b->lat_ends.size()) * sizeof(int), st), "batch counter");
     cudaEventRecord(b->ev0, st);
     if (D == 2) batch_sweeps<2>(b, (int)act.size(), maxnt);
     else batch_sweeps<3>(b, (int)act.size(), maxnt);
@@ -1111,6 +1136,11 @@ sdot_status sdot_batch_create(sdot_batch **out, int device, int dim)
         cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess) {
         delete b;
         return SDOT_ECUDA;
+    }
+    // slice sums held at a time (bytes); above it the problems' lattice sweeps run in groups
+    if (const char *cap = getenv("SDOT_BATCH_SUMS_BYTES")) {
+        const long long v = atoll(cap);
+        if (v > 0) b->sums_cap = (size_t)v;
     }
     *out = b;
     return SDOT_OK;

@@ -165,45 +165,65 @@ constexpr double LAT_RUN_BITS = 230.0;
 
 constexpr int LAT_CAPS2[2] = {64, 32}, LAT_CAPS3[1] = {16};   // tile sizes (2D, 3D), the largest first
 
+// Tiles of cap points per dimension; false where their padding excludes the
+// size.  A tile's work goes by its padded size (64 or 32 points per dimension,
+// 16 in 3D); where that would be more than LAT_PAD times the points, the cell
+// sweeps (about four multiply-adds per pair against one here, plus a third for
+// the factors) are the faster ones.
+constexpr double LAT_PAD = 2.5;
+inline bool lat_tiles(const int *n, int dim, int cap, LatTiling &t)
+{
+    int64_t tiles = 1, nq = 1;
+    double padded = 1.0;
+    for (int d = 0; d < dim; ++d) {
+        t.nt[d] = (n[d] + cap - 1) / cap;
+        tiles *= t.nt[d];
+        nq *= n[d];
+        const int rest = n[d] - (t.nt[d] - 1) * cap;
+        padded *= (t.nt[d] - 1) * (double)cap + (dim == 2 && rest <= 32 ? 32 : cap);
+    }
+    if (padded > LAT_PAD * (double)nq || tiles > (1 << 20)) return false;
+    t.cap = cap;
+    t.ntiles = (int)tiles;
+    return true;
+}
+
 // Tile size for scaled exponents s = kappa / eps and targets within reach[d]
 // of the origin: the largest of 64 and 32 points per dimension (2D) or 16
-// (3D) whose factors span at most 2^(+-LAT_BITS).  A tile's work goes by its
-// padded size (64 or 32 points per dimension, 16 in 3D); where the padding
-// would make that more than LAT_PAD times the points, the cell sweeps (about
-// four multiply-adds per pair against one here, plus a third for the
-// factors) are the faster ones.
-constexpr double LAT_PAD = 2.5;
+// (3D) whose factors span at most 2^(+-LAT_BITS).
 inline LatTiling lat_tiling(const int *n, const int *xo, const double *X, int dim, double s, const double *reach)
 {
-    LatTiling best;
-    const int *caps = dim == 2 ? LAT_CAPS2 : LAT_CAPS3;
-    const int ncaps = dim == 2 ? 2 : 1;
-    int64_t nq = 1;
-    for (int d = 0; d < dim; ++d) nq *= n[d];
-    for (int k = 0; k < ncaps; ++k) {
-        const int cap = caps[k];
-        double span = 0.0, padded = 1.0;
+    for (int k = 0; k < (dim == 2 ? 2 : 1); ++k) {
+        const int cap = dim == 2 ? LAT_CAPS2[k] : LAT_CAPS3[k];
         LatTiling t;
-        t.cap = cap;
-        int64_t tiles = 1;
+        if (!lat_tiles(n, dim, cap, t)) continue;
         for (int d = 0; d < dim; ++d) {
-            t.nt[d] = (n[d] + cap - 1) / cap;
-            tiles *= t.nt[d];
             double h = 0.0;
             for (int i = 0; i < t.nt[d]; ++i) {
                 const int a = i * cap, b = std::min(n[d], a + cap) - 1;
                 h = std::max(h, 0.5 * (X[xo[d] + b] - X[xo[d] + a]));
             }
-            span += s * reach[d] * h / 16.0;
-            const int rest = n[d] - (t.nt[d] - 1) * cap;
-            padded *= (t.nt[d] - 1) * (double)cap + (dim == 2 && rest <= 32 ? 32 : cap);
+            t.span += s * reach[d] * h / 16.0;
         }
-        if (!(span <= LAT_BITS) || padded > LAT_PAD * (double)nq || tiles > (1 << 20)) continue;
-        t.ntiles = (int)tiles;
-        t.span = span;
-        return t;
+        if (t.span <= LAT_BITS) return t;
     }
-    return best;
+    return LatTiling();
+}
+
+// The fewest and the most tiles that lat_tiling may return at any s and reach (0: never any).
+struct LatTileRange {
+    int fewest = 0, most = 0;
+};
+inline LatTileRange lat_tile_range(const int *n, int dim)
+{
+    LatTileRange r;
+    for (int k = 0; k < (dim == 2 ? 2 : 1); ++k) {
+        LatTiling t;
+        if (!lat_tiles(n, dim, dim == 2 ? LAT_CAPS2[k] : LAT_CAPS3[k], t)) continue;
+        r.fewest = r.most == 0 ? t.ntiles : std::min(r.fewest, t.ntiles);
+        r.most = std::max(r.most, t.ntiles);
+    }
+    return r;
 }
 
 // Slices of n items (targets, tiles) over `units` independent work items so
