@@ -309,10 +309,12 @@ sdot_status sdot_conditioned_densities(sdot_ctx *ctx, const double *psi, double 
  * SemiDiscreteOT.cc:878-922, advanced together on one GPU) ----
  * A batch holds untruncated problems (tau <= 0, pointwise threshold) of one
  * dimension and uneven sizes, packed in device memory.  Every batched
- * evaluation runs all active problems in four launches (persistent sweeps
+ * evaluation runs all active problems in a few launches (persistent sweeps
  * over (problem, block) work units, largest first); each problem keeps its
  * own L-BFGS state, line search (deal.II rules, as sdot_solve) and
- * convergence control from its sdot_solver_params.  Sources use the
+ * convergence control from its sdot_solver_params.  A problem's evaluation
+ * does not depend on what else is in the batch, to the last bit (at one launch
+ * shape, below); it differs from sdot_evaluate's by rounding.  Sources use the
  * flattened quadrature layout of sdot_set_source without the cell structure
  * (the untruncated path never queries cells).  psi arrays concatenate the
  * problems in the order they were added, each in its caller order. */
@@ -357,7 +359,7 @@ sdot_status sdot_batch_problem_info(const sdot_batch *batch, int index, sdot_sol
  * and shape[1] are the persistent CTAs per SM of the value and gradient
  * sweeps, shape[2] the gradient sweep's slice target (each problem's points
  * are cut into slices until its (target block, slice) units number about
- * shape[2] per SM; 8 gives the single-problem path's slicing).  Default
+ * shape[2] per SM; 8 gives the single-problem point sweeps' slicing).  Default
  * {8, 8, 8}; each value in [1, 64].  The slicing changes only the order in
  * which each target's FP64 partial sums are added. */
 sdot_status sdot_batch_set_shape(sdot_batch *batch, const int *shape);

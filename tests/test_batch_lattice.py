@@ -77,3 +77,20 @@ def test_groups_of_problems(oracle_mod, monkeypatch, fp32, cap):
     if not fp32:
         check(oracle_mod, probs, vals, grads)
     b.close()
+
+
+@pytest.mark.parametrize("fp32", [False, True])
+@pytest.mark.parametrize("dim,n,order,N", [(2, 32, 2, 3000), (2, 16, 3, 700), (3, 8, 2, 2000), (2, 9, 2, 600)])
+def test_results_do_not_depend_on_the_companions(dim, n, order, N, fp32):
+    """One problem (on the lattice, and on the point sweeps) alone and in a batch with larger ones."""
+    one = problem(dim, n, order, N)
+    big = [problem(2, 128, 3, 16384), problem(2, 100, 3, 16000)] if dim == 2 else [problem(3, 32, 2, 20000)]
+    out = []
+    for probs in ([one], [one] + big, big + [one, problem(dim, n, order, 130)]):
+        b = batch_of(dim, probs)
+        vals, grads = b.evaluate([p[4] for p in probs], fp32=fp32)
+        k = [p is one for p in probs].index(True)
+        out.append((vals[k], grads[k]))
+        b.close()
+    for J, g in out[1:]:
+        assert J == out[0][0] and np.array_equal(g, out[0][1])
