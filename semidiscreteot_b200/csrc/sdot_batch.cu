@@ -1158,7 +1158,9 @@ void sdot_batch_destroy(sdot_batch *b)
         b->gpart.release(); b->x0.release(); b->g0.release(); b->pdir.release(); b->S.release(); b->Y.release();
         b->rho_h.release(); b->scal.release(); b->alpha.release(); b->outv.release(); b->dinst.release();
         b->act.release(); b->counter.release(); b->spare.release(); b->vunits.release(); b->gunits.release();
-        b->dhist.release();
+        b->dhist.release(); b->munits.release(); b->funits.release(); b->lvunits.release(); b->lgunits.release();
+        b->red.release(); b->lat_x.release(); b->lat_sph.release(); b->lat_top.release(); b->lat_step.release();
+        b->lat_ms.release(); b->lat_q.release(); b->lat_mem.release(); b->lat_off.release();
         cudaEventDestroy(b->ev0);
         cudaEventDestroy(b->ev1);
         cudaStreamDestroy(b->stream);
