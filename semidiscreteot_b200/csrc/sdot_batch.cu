@@ -33,6 +33,7 @@
 #include <atomic>
 #include <cmath>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <numeric>
 #include <tuple>
@@ -638,9 +639,8 @@ struct sdot_batch {
     DevBuf<int> act, counter, spare;
     DevBuf<int2> vunits, munits, funits;
     DevBuf<int4> gunits, lvunits, lgunits;
-    DevBuf<double> lat_x, lat_sph, lat_top, lat_step, lat_ms, red;
-    DevBuf<int> lat_q, lat_mem;
-    DevBuf<int64_t> lat_off;
+    DevBuf<double> lat_buf, red;       // lattices: coordinates, spheres, blocks, points; then the sweeps' scratch
+    DevBuf<double> arena;              // what the upload allocates, in one piece (each cudaMalloc costs up to 0.1 ms)
     // unit counts of the lists on the device (lattice lists: by group, ends), and what they were made for
     struct GroupEnds {
         int value = 0, merge = 0, grad = 0;
@@ -753,17 +753,24 @@ struct TargetBlocks {
 // points took 4.18 ms against 4.41, 16 problems 0.83 against 0.80, one of
 // 147,456 points x 16,384 targets 0.595 against 0.558.)  Slice sums are held
 // for groups of problems together, of up to sums_cap bytes; a group's sweeps
-// end before the next one's begin.  Where there is no memory for the lattices'
-// buffers, all problems run the point sweeps.
-sdot_status upload_lattices(sdot_batch *b, const std::vector<TargetBlocks> &blk)
+// end before the next one's begin.
+struct LatPlaces {
+    // places of a problem's data and scratch within their parts of the buffer
+    struct Place {
+        int64_t x = 0, sph = 0, off = 0, mem = 0, q = 0, ms = 0, shift = 0, step = 0;
+    };
+    std::vector<Place> at;
+    Place n;              // past the last problem
+    int64_t ms_most = 0;  // doubles of the largest group's sums
+};
+LatPlaces place_lattices(sdot_batch *b, const std::vector<TargetBlocks> &blk)
 {
     const size_t np = b->probs.size();
     const int D = b->dim;
-    std::vector<double> lx, lsph;
-    std::vector<int> lq, lmem;
-    std::vector<int64_t> loff;
-    std::vector<int64_t> ms0(np), sh0(np), sp0(np), x0(np), lq0(np), mem0(np), off0(np), sph0(np);
-    int64_t ms = 0, ms_most = 0, sh = 0, sp = 0, part0 = 0;
+    LatPlaces L;
+    L.at.resize(np);
+    LatPlaces::Place &n = L.n;
+    int64_t part0 = 0;
     int group = 0;
     b->lat_group.assign(np, 0);
     for (size_t i = 0; i < np; ++i) {
@@ -779,76 +786,76 @@ sdot_status upload_lattices(sdot_batch *b, const std::vector<TargetBlocks> &blk)
         part0 += std::max<int64_t>(I.nvb, tiles * (LAT_TILE / LAT_THREADS));
         if (!G.ok) continue;
         const int64_t sums = tiles * I.nvs * LAT_TILE;
-        if (ms > 0 && (size_t)(ms + sums) * 8 > b->sums_cap) {
-            ms = 0;
+        if (n.ms > 0 && (size_t)(n.ms + sums) * 8 > b->sums_cap) {
+            n.ms = 0;
             ++group;
         }
         b->lat_group[i] = group;
-        ms0[i] = ms;
-        ms += sums;
-        ms_most = std::max(ms_most, ms);
-        sh0[i] = sh;
-        sh += 2 * tiles;
-        sp0[i] = sp;
-        sp += P.nt * D;
-        x0[i] = (int64_t)lx.size();
-        lx.insert(lx.end(), G.X.begin(), G.X.end());
-        lq0[i] = (int64_t)lq.size();
-        lq.insert(lq.end(), G.q.begin(), G.q.end());
-        mem0[i] = (int64_t)lmem.size();
-        lmem.insert(lmem.end(), blk[i].mem.begin(), blk[i].mem.end());
-        off0[i] = (int64_t)loff.size();
-        loff.insert(loff.end(), blk[i].off.begin(), blk[i].off.end());
-        sph0[i] = (int64_t)lsph.size();
-        lsph.insert(lsph.end(), blk[i].sph.begin(), blk[i].sph.end());
+        L.at[i] = n;
+        n.x += (int64_t)G.X.size();
+        n.sph += (int64_t)blk[i].sph.size();
+        n.off += (int64_t)blk[i].off.size();
+        n.mem += (int64_t)blk[i].mem.size();
+        n.q += (int64_t)G.q.size();
+        n.ms += sums;
+        n.shift += 2 * tiles;
+        n.step += P.nt * D;
+        L.ms_most = std::max(L.ms_most, n.ms);
     }
     b->total_part = part0;
     b->lat_ends.resize((size_t)group + 1);
-    if (lq.empty()) return SDOT_OK;
-    cudaError_t e = b->lat_x.alloc(lx.size());
-    if (e == cudaSuccess) e = b->lat_q.alloc(lq.size());
-    if (e == cudaSuccess) e = b->lat_mem.alloc(lmem.size());
-    if (e == cudaSuccess) e = b->lat_off.alloc(loff.size());
-    if (e == cudaSuccess) e = b->lat_sph.alloc(lsph.size());
-    if (e == cudaSuccess) e = b->lat_top.alloc(lsph.size() / 4);
-    if (e == cudaSuccess) e = b->lat_step.alloc(sp);
-    if (e == cudaSuccess) e = b->lat_ms.alloc(ms_most + sh);
+    return L;
+}
+
+// The lattices' buffer; where there is no memory for it, all problems run the
+// point sweeps.
+sdot_status upload_lattices(sdot_batch *b, const std::vector<TargetBlocks> &blk, const LatPlaces &L)
+{
+    const size_t np = b->probs.size();
+    const auto &at = L.at;
+    const auto &n = L.n;
+    if (n.q == 0) return SDOT_OK;
+    // the parts, in doubles: coordinates, spheres, block ends, members, points | sums, shifts, steps, blocks' tops
+    // (the sums, whose weights the gradient sweep loads 16 bytes at a time, on a 256-byte boundary)
+    const int64_t sph = n.x, off = sph + n.sph, mem = off + n.off, q = mem + (n.mem + 1) / 2;
+    const int64_t data = (q + (n.q + 1) / 2 + 31) / 32 * 32;
+    const int64_t shift = data + L.ms_most, step = shift + n.shift, top = step + n.step;
+    const cudaError_t e = b->lat_buf.alloc((size_t)(top + n.sph / 4));
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
-        for (auto *v : {&b->lat_x, &b->lat_sph, &b->lat_top, &b->lat_step, &b->lat_ms}) v->release();
-        b->lat_q.release();
-        b->lat_mem.release();
-        b->lat_off.release();
         b->lat.assign(np, Lattice());
         return SDOT_OK;
     }
     BCK(e, "batch lattice");
-    BCK(cudaMemcpy(b->lat_x.p, lx.data(), lx.size() * 8, cudaMemcpyHostToDevice), "batch lattice");
-    BCK(cudaMemcpy(b->lat_q.p, lq.data(), lq.size() * sizeof(int), cudaMemcpyHostToDevice), "batch lattice");
-    BCK(cudaMemcpy(b->lat_mem.p, lmem.data(), lmem.size() * sizeof(int), cudaMemcpyHostToDevice), "batch lattice");
-    BCK(cudaMemcpy(b->lat_off.p, loff.data(), loff.size() * 8, cudaMemcpyHostToDevice), "batch lattice");
-    BCK(cudaMemcpy(b->lat_sph.p, lsph.data(), lsph.size() * 8, cudaMemcpyHostToDevice), "batch lattice");
+    const std::unique_ptr<double[]> host(new double[(size_t)data]);
     for (size_t i = 0; i < np; ++i) {
         BInst &I = b->inst[i];
         Lattice &G = b->lat[i];
         if (!G.ok) continue;
-        I.L.X = b->lat_x.p + x0[i];
-        I.L.q = b->lat_q.p + lq0[i];
-        for (int d = 0; d < 3; ++d) {
-            I.L.n[d] = G.n[d];
-            I.L.xo[d] = G.xo[d];
+        double *h = host.get(), *d = b->lat_buf.p;
+        std::copy(G.X.begin(), G.X.end(), h + at[i].x);
+        std::copy(blk[i].sph.begin(), blk[i].sph.end(), h + sph + at[i].sph);
+        std::copy(blk[i].off.begin(), blk[i].off.end(), reinterpret_cast<int64_t *>(h + off) + at[i].off);
+        std::copy(blk[i].mem.begin(), blk[i].mem.end(), reinterpret_cast<int *>(h + mem) + at[i].mem);
+        std::copy(G.q.begin(), G.q.end(), reinterpret_cast<int *>(h + q) + at[i].q);
+        I.L.X = d + at[i].x;
+        I.L.q = reinterpret_cast<int *>(d + q) + at[i].q;
+        for (int k = 0; k < 3; ++k) {
+            I.L.n[k] = G.n[k];
+            I.L.xo[k] = G.xo[k];
         }
-        I.K.off = b->lat_off.p + off0[i];
-        I.K.mem = b->lat_mem.p + mem0[i];
-        I.K.sph = b->lat_sph.p + sph0[i];
-        I.K.top = b->lat_top.p + sph0[i] / 4;
+        I.K.off = reinterpret_cast<int64_t *>(d + off) + at[i].off;
+        I.K.mem = reinterpret_cast<int *>(d + mem) + at[i].mem;
+        I.K.sph = d + sph + at[i].sph;
+        I.K.top = d + top + at[i].sph / 4;
         I.K.n = (int)blk[i].off.size() - 1;
-        I.ms = b->lat_ms.p + ms0[i];
-        I.shift = b->lat_ms.p + ms_most + sh0[i];
-        I.step = b->lat_step.p + sp0[i];
+        I.ms = d + data + at[i].ms;
+        I.shift = d + shift + at[i].shift;
+        I.step = d + step + at[i].step;
         std::vector<int>().swap(G.q);  // on the device from here on
         plan_lattice(b, (int)i);
     }
+    BCK(cudaMemcpy(b->lat_buf.p, host.get(), (size_t)data * 8, cudaMemcpyHostToDevice), "batch lattice");
     return SDOT_OK;
 }
 
@@ -904,14 +911,23 @@ sdot_status upload(sdot_batch *b)
             if (b->lat[i].ok && lat_tile_range(b->lat[i].n, D).most == 0) b->lat[i] = Lattice();
             if (!b->lat[i].ok) return;
             const double *y = b->hy.data() + b->inst[i].t0 * D;
-            const std::vector<double> pts(y, y + P.nt * D);
-            const std::vector<int64_t> ord = kd_order(pts, D, P.nt, TBLK_KD, blk[i].off);
-            blk[i].mem.assign(ord.begin(), ord.end());
-            for (size_t k = 0; k + 1 < blk[i].off.size(); ++k) {
-                const std::vector<int64_t> idx(ord.begin() + blk[i].off[k], ord.begin() + blk[i].off[k + 1]);
-                double sp[4];
-                sphere_of(pts.data(), idx, D, sp);
-                blk[i].sph.insert(blk[i].sph.end(), sp, sp + 4);
+            TargetBlocks &B = blk[i];
+            if (P.nt <= LAT_LIST) {  // the merge lists all targets: blocks in any order, their spheres are not read
+                B.mem.resize(P.nt);
+                std::iota(B.mem.begin(), B.mem.end(), 0);
+                for (int64_t k = 0; k < P.nt; k += TBLK_KD) B.off.push_back(k);
+                B.off.push_back(P.nt);
+                B.sph.assign(4 * (B.off.size() - 1), 0.0);
+            } else {
+                const std::vector<double> pts(y, y + P.nt * D);
+                const std::vector<int64_t> ord = kd_order(pts, D, P.nt, TBLK_KD, B.off);
+                B.mem.assign(ord.begin(), ord.end());
+                for (size_t k = 0; k + 1 < B.off.size(); ++k) {
+                    const std::vector<int64_t> idx(ord.begin() + B.off[k], ord.begin() + B.off[k + 1]);
+                    double sp[4];
+                    sphere_of(pts.data(), idx, D, sp);
+                    B.sph.insert(B.sph.end(), sp, sp + 4);
+                }
             }
             for (int64_t j = 0; j < P.nt; ++j)
                 for (int d = 0; d < D; ++d)
@@ -935,36 +951,60 @@ sdot_status upload(sdot_batch *b)
         work();
         for (auto &t : pool) t.join();
     }
-    const sdot_status s = upload_lattices(b, blk);
-    if (s != SDOT_OK) return s;
+    const LatPlaces places = place_lattices(b, blk);
     const int64_t gp0 = plan_slices(b);
-    BCK(b->x.alloc(q0 * D), "batch alloc");
-    BCK(b->rho.alloc(q0), "batch alloc");
-    BCK(b->jxw.alloc(q0), "batch alloc");
-    BCK(b->w.alloc(q0), "batch alloc");
-    BCK(b->Lq.alloc(q0), "batch alloc");
-    BCK(b->y.alloc(t0 * D), "batch alloc");
-    BCK(b->nu.alloc(t0), "batch alloc");
-    BCK(b->psi.alloc(t0), "batch alloc");
-    BCK(b->grad.alloc(t0), "batch alloc");
-    BCK(b->tpack.alloc(t0 * TPACK), "batch alloc");
-    BCK(b->x0.alloc(t0), "batch alloc");
-    BCK(b->g0.alloc(t0), "batch alloc");
-    BCK(b->pdir.alloc(t0), "batch alloc");
-    BCK(b->S.alloc(6 * t0), "batch alloc");
-    BCK(b->Y.alloc(6 * t0), "batch alloc");
-    BCK(b->part.alloc(b->total_part * 4), "batch alloc");
-    BCK(b->gpart.alloc(gp0), "batch alloc");
-    BCK(b->rho_h.alloc(np * 8), "batch alloc");
-    BCK(b->scal.alloc(np * SC_COUNT), "batch alloc");
-    BCK(b->alpha.alloc(np), "batch alloc");
-    BCK(b->outv.alloc(np), "batch alloc");
-    BCK(b->dinst.alloc(np), "batch alloc");
-    BCK(b->act.alloc(np), "batch alloc");
-    BCK(b->spare.alloc(np), "batch alloc");
-    BCK(b->dhist.alloc(np), "batch alloc");
-    BCK(b->counter.alloc(2 + 2 * b->lat_ends.size()), "batch alloc");
-    BCK(b->red.alloc((size_t)(t0 / BFIN_THREADS + 2 * np + 1) * BRED), "batch alloc");
+    {
+        struct Part {
+            void **p;
+            size_t *n;
+            bool *part;
+            size_t count, words;
+        };
+        std::vector<Part> parts;
+        size_t words = 0;
+        auto add = [&](auto &buf, size_t count) {
+            count = std::max<size_t>(count, 1);
+            parts.push_back({reinterpret_cast<void **>(&buf.p), &buf.n, &buf.part, count, words});
+            words += (count * sizeof(*buf.p) + 255) / 256 * 32;
+        };
+        add(b->x, q0 * D);
+        add(b->rho, q0);
+        add(b->jxw, q0);
+        add(b->w, q0);
+        add(b->Lq, q0);
+        add(b->y, t0 * D);
+        add(b->nu, t0);
+        add(b->psi, t0);
+        add(b->grad, t0);
+        add(b->tpack, t0 * TPACK);
+        add(b->x0, t0);
+        add(b->g0, t0);
+        add(b->pdir, t0);
+        add(b->S, 6 * t0);
+        add(b->Y, 6 * t0);
+        add(b->part, b->total_part * 4);
+        add(b->gpart, gp0);
+        add(b->rho_h, np * 8);
+        add(b->scal, np * SC_COUNT);
+        add(b->alpha, np);
+        add(b->outv, np);
+        add(b->dinst, np);
+        add(b->act, np);
+        add(b->spare, np);
+        add(b->dhist, np);
+        add(b->counter, 2 + 2 * b->lat_ends.size());
+        add(b->red, (size_t)(t0 / BFIN_THREADS + 2 * np + 1) * BRED);
+        for (auto &p : parts)  // (an upload that failed is made again)
+            if (*p.part) *p.p = nullptr, *p.n = 0;
+        BCK(b->arena.alloc(words), "batch alloc");
+        for (auto &p : parts) {
+            *p.p = b->arena.p + p.words;
+            *p.n = p.count;
+            *p.part = true;
+        }
+    }
+    const sdot_status s = upload_lattices(b, blk, places);
+    if (s != SDOT_OK) return s;
     std::vector<double> w(q0);
     for (int64_t q = 0; q < q0; ++q) w[q] = b->hrho[q] * b->hjxw[q];
     BCK(cudaMemcpy(b->x.p, b->hx.data(), q0 * D * 8, cudaMemcpyHostToDevice), "batch upload");
@@ -1159,8 +1199,7 @@ void sdot_batch_destroy(sdot_batch *b)
         b->rho_h.release(); b->scal.release(); b->alpha.release(); b->outv.release(); b->dinst.release();
         b->act.release(); b->counter.release(); b->spare.release(); b->vunits.release(); b->gunits.release();
         b->dhist.release(); b->munits.release(); b->funits.release(); b->lvunits.release(); b->lgunits.release();
-        b->red.release(); b->lat_x.release(); b->lat_sph.release(); b->lat_top.release(); b->lat_step.release();
-        b->lat_ms.release(); b->lat_q.release(); b->lat_mem.release(); b->lat_off.release();
+        b->red.release(); b->lat_buf.release(); b->arena.release();
         cudaEventDestroy(b->ev0);
         cudaEventDestroy(b->ev1);
         cudaStreamDestroy(b->stream);

@@ -95,14 +95,16 @@ template <class T>
 struct DevBuf {
     T *p = nullptr;
     size_t n = 0;
+    bool part = false;   // of another buffer's memory (batch upload), which frees it
     DevBuf() = default;
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
     ~DevBuf() { release(); }
     void release() {
-        if (p) cudaFree(p);
+        if (p && !part) cudaFree(p);
         p = nullptr;
         n = 0;
+        part = false;
     }
     cudaError_t alloc(size_t count) {
         if (count <= n && p) return cudaSuccess;
