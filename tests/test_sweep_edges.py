@@ -109,3 +109,25 @@ def test_covering_radius(oracle_mod, dim, n, N):
     s.setup_target(y, nu)
     assert s.compute_covering_radius() == oracle_of(oracle_mod, src, y, nu).covering_radius()
     s.close()
+
+
+@pytest.mark.parametrize("dim,n,order,N,eps", [(2, 16, 3, 200, 1e-3), (2, 12, 3, 100, 4e-4), (2, 48, 2, 800, 3e-4),
+                                               (3, 12, 2, 600, 2e-3), (3, 16, 2, 1500, 5e-4)])
+def test_truncated_fp64_gradient_relative(oracle_mod, dim, n, order, N, eps):
+    """FP64 gradient over tensor-product points, per target relative to its mass: exponents of up to 40 (natural
+    units) rounded eight times each here and in the oracle, 2 x 8 x 40 x 2^-53 = 7.1e-14, and nothing from the
+    exponentials, whose products are good to a few ulp."""
+    rng = np.random.default_rng(n + N)
+    src = structured_source(dim, n, order, nodal_density=lambda p: 1.0 + 0.5 * np.sin(3.0 * p[:, 0]))
+    y, nu = rng.random((N, dim)), rng.dirichlet(np.ones(N) * 5)
+    psi, g = 0.5 * eps * rng.standard_normal(N), np.zeros(N)
+    s = SotSolver(dim=dim, device=0, precision="fp64")
+    s.setup_source(src["x"], src["jxw"], src["density"], src["cell_offsets"], src["cell_centers"])
+    s.setup_target(y, nu)
+    s.configure(SolverParameters(epsilon=eps, tau=1e-12, use_log_sum_exp_trick=True))
+    s.evaluate_functional(psi, g)
+    s.close()
+    _, g0, _ = oracle_of(oracle_mod, src, y, nu).evaluate(
+        psi, oracle_mod.Params(epsilon=eps, tau=1e-12, use_log_sum_exp=True))
+    mass = g0 + nu
+    assert np.max((np.abs(g - g0) / mass)[mass > 1e-8]) <= 2 * 8 * 40 * 2.0 ** -53
