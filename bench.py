@@ -47,7 +47,11 @@ import numpy as np
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
-# Algorithmic FP64 flops per pair of the value sweep (FMA = 2): exponent
+# FP64 flops per pair of the lattice value sweep: one multiply-add of the
+# matrix product (the factors, one exponential per eight points and target, are
+# not counted).
+LATTICE_FLOPS_PER_PAIR = 2
+# Algorithmic FP64 flops per pair of the other value sweeps (FMA = 2): exponent
 # A + B.x (d FMA), max and shift (2), exp2 by 16-entry table and degree-5
 # polynomial (rint 3, polynomial 5 FMA, table product 1), accumulate (1 FMA).
 VALUE_FLOPS_PER_PAIR = {2: 22, 3: 24}
@@ -423,7 +427,9 @@ def measure_single(wl, precision, steps, warmup, local, clk, flush, e2e=True):
     _, kt = timed(True)
     pairs = solver.last_eval_info["n_pairs"]
     ms = float(np.mean(times))
+    truncated = wl["params"].tau > 0
     out = {"value": pairs / (ms * 1e-3), "ms_per_step": ms, "pairs_per_step": pairs, "kt": kt,
+           "sweeps": {} if truncated else solver.dense_sweeps(),
            "gpu_launches": int(sum(v["launches"] for v in kt.values()))}
     if e2e:
         hpsi = torch.zeros(N, dtype=torch.float64).pin_memory()
@@ -458,17 +464,25 @@ def roofline_of(m, wl, peaks, precision):
     tg = kt["gradient_sweep"]["ms"] / max(1, kt["gradient_sweep"]["launches"])
     pairs = m["pairs_per_step"]
     truncated = wl["params"].tau > 0
+    lattice = not truncated and m.get("sweeps", {}).get("tile", 0) > 0
     if tv >= tg or truncated:
-        ach = VALUE_FLOPS_PER_PAIR[dim] * pairs / (tv * 1e-3) / 1e12
+        flops = LATTICE_FLOPS_PER_PAIR if lattice else VALUE_FLOPS_PER_PAIR[dim]
+        ach = flops * pairs / (tv * 1e-3) / 1e12
         kname = ("k_fused (FP64 exp2 value sweep + FP32 ex2 gradient sweep, one kernel)" if truncated else
                  "dense FP64 value sweep: k_lat_value (points on a tensor lattice: per-dimension factors as FP64 "
-                 "matrix products) + k_lat_merge, or per tensor-grid cell or point; flops counted for the "
-                 "unfactored form")
+                 "matrix products; the products' flops) + k_lat_merge" if lattice else
+                 "dense FP64 value sweep per tensor-grid cell or point; flops counted for the unfactored form")
         return {"kernel": kname, "bound": "fp64", "achieved": ach, "peak": peaks["fp64_tflops"], "unit": "TFLOP/s",
                 "frac": ach / peaks["fp64_tflops"], "traffic": TRAFFIC_BYTES.get((wl["name"], precision)),
-                "flops_per_pair": VALUE_FLOPS_PER_PAIR[dim], "ms_per_launch": tv,
+                "flops_per_pair": flops, "ms_per_launch": tv,
                 "peak_source": "measured on this GPU by sdot_measure_peaks (FP64 FMA chains); "
                                "MEASURED_PEAKS.json has no FP64 figure"}
+    if m.get("sweeps", {}).get("lattice_gradient"):
+        ach = LATTICE_FLOPS_PER_PAIR * pairs / (tg * 1e-3) / 1e12
+        return {"kernel": "k_lat_grad (FP64 matrix products over lattice tiles; the products' flops)", "bound": "fp64",
+                "achieved": ach, "peak": peaks["fp64_tflops"], "unit": "TFLOP/s", "frac": ach / peaks["fp64_tflops"],
+                "traffic": TRAFFIC_BYTES.get((wl["name"], precision)), "flops_per_pair": LATTICE_FLOPS_PER_PAIR,
+                "ms_per_launch": tg, "peak_source": "measured on this GPU by sdot_measure_peaks (FP64 FMA chains)"}
     ach = pairs / (tg * 1e-3) / 1e9
     return {"kernel": "k_grad_dense_tensor / k_grad_dense (FP32 ex2 gradient sweep)" if precision != "fp64" else
             "k_grad_dense_tensor / k_grad_dense (FP64 exp2 gradient sweep)", "bound": "mufu", "achieved": ach,
@@ -614,7 +628,8 @@ def run_ours(args):
     if rank == 0:
         value = pairs / (t_ms * 1e-3)
         peaks = SotSolver.measure_peaks(local)
-        m = {"kt": kt, "pairs_per_step": lib.last_eval_info["n_pairs"]}
+        m = {"kt": kt, "pairs_per_step": lib.last_eval_info["n_pairs"],
+             "sweeps": {} if wl["params"].tau > 0 else lib.dense_sweeps()}
         line = {"metric": "LSE dual-gradient pairs/s", "value": value, "unit": "pairs/s", "n_gpus": world,
                 "steps": args.steps, "warmup": max(3, args.warmup), "ms_per_step": t_ms, "higher_is_better": True,
                 "scaling": "strong", "vs_baseline": None,

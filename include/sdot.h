@@ -39,7 +39,11 @@ typedef enum {
 /* Arithmetic of the two exponential sweeps.
  *   SDOT_PREC_FP64  : both sweeps in FP64 (value 1e-10 rel., gradient ~1e-14).
  *   SDOT_PREC_HYBRID: value sweep FP64, gradient sweep FP32 exp2 with FP64
- *                     accumulation (gradient error <= ~3e-6 * max nu_j).
+ *                     accumulation (gradient error about 3e-6 * max nu_j;
+ *                     untruncated sweeps round FP32 exponents of up to
+ *                     D^2 / (2 epsilon), D the largest distance of a point and
+ *                     a target, so at small epsilon an entry may be off by
+ *                     4 * 2^-24 * D^2 / (2 epsilon) of its target's mass).
  *   SDOT_PREC_MIXED : accepted and currently run as SDOT_PREC_HYBRID (an FP32
  *                     value sweep cannot meet the 1e-10 relative value bound,
  *                     so the value sweep stays FP64).                       */

@@ -397,7 +397,7 @@ struct BHist {
     int slot[HIST + 1];
 };
 
-// Two-loop recursion per problem (the single-problem k_two_loop, one CTA per
+// Two-loop recursion per problem (the directions of k_lbfgs_step, one CTA per
 // problem; history slots of problem p at S + (6 t0 + slot nt)), then
 // x0 = psi and g0 = g for the line search.  out[p] = g.p.
 __global__ void __launch_bounds__(1024)

@@ -8,16 +8,17 @@
 // Blocks.  Source cells and targets are ordered by k-d trees built at
 // set_source / set_target; a source block is a leaf of <= 8 warp units
 // (cell, q-group), a target block a leaf of <= 32 targets.  Each block has a
-// bounding sphere (FP64 and a conservative FP32 copy).
+// bounding sphere (FP64) and a conservative FP32 bounding box.
 //
 // Per evaluation:
 //   1. block-pair lists.  (b, t) is a pair iff the box of b's cell centres is
 //      within r of the box of t's targets (FP32, conservatively enlarged;
 //      super-blocks by their spheres).  With the blocks' spheres in place of
 //      their boxes a third more pairs were listed, staged and reduced.  The
-//      forward list (per b, t ascending) is filled from masks; the inverse list (per t, b ascending, with the
-//      pairs' forward positions) is its transpose, built on a second stream
-//      beside step 2, which does not need it.
+//      forward list (per b, t ascending) is filled from masks; the inverse list
+//      (per t, b ascending, with the pairs' forward positions) is its
+//      transpose, built on a second stream beside step 2, which does not need
+//      it.
 //   2. k_fused (CTA <-> source block, warp <-> unit):
 //      staging: the targets of the block's pairs, culled per target against
 //        the block sphere (|y - c_b| <= r + R_b), compacted in order;
