@@ -732,7 +732,7 @@ void plan_lattice(sdot_batch *b, int i)
     for (int d = 0; d < 3; ++d) I.L.nt[d] = t.nt[d];
     I.L.cap = t.cap;
     I.L.ntiles = t.ntiles;
-    lat_runs(G.period, G.step, b->dim, t.span, I.L);
+    lat_runs(G.period, G.step, b->dim, t, I.L);
     I.ngs = (t.ntiles + I.gts - 1) / I.gts;
     I.lat = 1;
 }

@@ -1126,7 +1126,7 @@ void dense_sweeps(const sdot_ctx *c, int *sweeps)
     const DenseShape d = dense_shape_of(c, c->prm.epsilon, c->precision == SDOT_PREC_FP64);
     const bool lat = d.lat.cap > 0;
     LatArgs L{};
-    if (lat) lat_runs(c->lat_period, c->lat_step, c->dim, d.lat.span, L);
+    if (lat) lat_runs(c->lat_period, c->lat_step, c->dim, d.lat, L);
     const int v[SDOT_DENSE_SWEEPS] = {d.lat.cap, d.lat.ntiles, lat && d.lat_grad, L.runs > 0, lat ? 0 : d.tm, d.nvs};
     std::copy(v, v + SDOT_DENSE_SWEEPS, sweeps);
 }
@@ -1149,7 +1149,7 @@ static LatArgs lat_args(const sdot_ctx *c, const LatTiling &t)
     }
     L.cap = t.cap;
     L.ntiles = t.ntiles;
-    lat_runs(c->lat_period, c->lat_step, c->dim, t.span, L);
+    lat_runs(c->lat_period, c->lat_step, c->dim, t, L);
     return L;
 }
 

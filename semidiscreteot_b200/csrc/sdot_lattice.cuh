@@ -23,13 +23,14 @@
 // The caller admits a tile size only when the factors of a tile span at most
 // 2^(+-LAT_BITS): every point's sum is then at least nu 2^-LAT_BITS relative
 // to M, and nothing leaves the FP64 range.  exp2_16_full clamps at 2^-1000.
-// With an exponential for each factor a clamped one is multiplied by the other
-// dimensions' only, at most 2^LAT_BITS: what it adds is 300 bits below the
-// least sum.  A run multiplies its clamped first factor by up to seven steps
-// too, as much as from one end of the tile to the other: with factors of
-// 2^(+-b) a clamped 2^-1000 grows to 2^(2 b - 1000) against a sum of 2^-b, so
-// runs are taken up to b = LAT_RUN_BITS only (310 bits apart), and factor by
-// factor beyond.
+// Only dimension 0's factors, which carry B0 - M, can be that small.  With an
+// exponential for each of them a clamped one is multiplied by the other
+// dimensions' only: with spans b_d, b in all, it adds at most 2^(b - b_0 - 1000)
+// to a sum of at least 2^-b, 300 bits below it.  A run multiplies its clamped
+// first factor by up to seven steps too, 2^g: runs are taken where
+// g + 2 b - b_0 still leaves LAT_CLAMP_LEFT bits (on a beam whose one run covers a
+// tile, g = 2 b_0 = 2 b, up to b = 233; on squares of 64^2-point tiles always),
+// and every factor has its own exponential otherwise.
 #pragma once
 
 #include "sdot_device.cuh"
@@ -88,13 +89,13 @@ struct LatDims {
     static constexpr int FS = FD + LAT_PAD_F;      // row of one target's factors in shared memory
 };
 
-// Run counts of a launch from the lattice's periods; span: the bits that the
-// factors of a tile span (host).
-inline void lat_runs(const int *period, const double *step, int dim, double span, LatArgs &L)
+// Run counts of a launch from the lattice's periods and its tiling (host).
+inline void lat_runs(const int *period, const double *step, int dim, const LatTiling &t, LatArgs &L)
 {
     const int T = dim == 2 ? 64 : 16;
     L.runs = 0;
-    if (!(span <= LAT_RUN_BITS)) return;
+    const double grow = std::min(2.0 * t.span0, t.slope0 * (LAT_RUN - 1) * step[0]);
+    if (!(grow + 2.0 * t.span - t.span0 <= 1000.0 - LAT_CLAMP_LEFT)) return;
     for (int d = 0; d < dim; ++d) {
         const int p = period[d];
         if (p <= 0) {

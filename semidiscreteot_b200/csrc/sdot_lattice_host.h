@@ -156,12 +156,14 @@ inline void find_lattice(const double *x, int64_t n, int dim, Lattice &L)
 // sweeps do not apply) and tile counts.
 struct LatTiling {
     int cap = 0, nt[3] = {1, 1, 1}, ntiles = 0;
-    double span = 0.0;   // the factors of a tile lie within 2^(+-span)
+    double span = 0.0, span0 = 0.0;   // the factors of a tile lie within 2^(+-span), dimension 0's within 2^(+-span0)
+    double slope0 = 0.0;              // bits per length of dimension 0's factors
 };
 
-// The largest span that the sweeps admit, and with factor runs (sdot_lattice.cuh says why).
+// The largest span that the sweeps admit, and the bits between a clamped term
+// and the least sum that they leave (sdot_lattice.cuh says why).
 constexpr double LAT_BITS = 350.0;
-constexpr double LAT_RUN_BITS = 230.0;
+constexpr double LAT_CLAMP_LEFT = 300.0;
 
 constexpr int LAT_CAPS2[2] = {64, 32}, LAT_CAPS3[1] = {16};   // tile sizes (2D, 3D), the largest first
 
@@ -204,7 +206,9 @@ inline LatTiling lat_tiling(const int *n, const int *xo, const double *X, int di
                 h = std::max(h, 0.5 * (X[xo[d] + b] - X[xo[d] + a]));
             }
             t.span += s * reach[d] * h / 16.0;
+            if (d == 0) t.span0 = t.span;
         }
+        t.slope0 = s * reach[0] / 16.0;
         if (t.span <= LAT_BITS) return t;
     }
     return LatTiling();

@@ -59,13 +59,16 @@ def check(s, want, psi, tol):
     assert abs(s.get_C_global() - st["C_global"]) <= 1e-10 * abs(st["C_global"])
 
 
-def beam(order=3):
+def beam(order=3, axis=0):
     """16 x 4 x 4 cells on 1 x 0.02 x 0.02 and targets at the two ends: with a period of 3 points one run of
-    factors covers a tile of 16 points."""
+    factors covers a tile of 16 points.  axis: the dimension that the beam lies along."""
     rng = np.random.default_rng(5)
     y = rng.random((40, 3)) * [0.02, 0.02, 0.02]
     y[20:, 0] += 0.98
-    return box_source((48 // order, 4, 4), order, (1.0, 0.02, 0.02)), y, rng.dirichlet(np.ones(40) * 5)
+    src = box_source((48 // order, 4, 4), order, (1.0, 0.02, 0.02))
+    turn = lambda a: np.ascontiguousarray(np.roll(a, axis, axis=1))
+    src["x"], src["cell_centers"] = turn(src["x"]), turn(src["cell_centers"])
+    return src, turn(y), rng.dirichlet(np.ones(40) * 5)
 
 
 BEAM_EPS = [3.2e-4, 3.25e-4, 3.3e-4, 3.4e-4, 3.45e-4, 3.6e-4, 4e-4, 4.5e-4, 4.8e-4, 5e-4, 5.2e-4, 5.5e-4, 6e-4]
@@ -80,6 +83,16 @@ def test_beam(oracle_mod, order, eps, precision):
     psi = np.zeros(len(nu))
     want = oracle_of(oracle_mod, src, y, nu, eps, psi)
     check(s, want, psi, tolerance(src, y, nu, eps, want, precision != "fp64"))
+    s.close()
+
+
+@pytest.mark.parametrize("axis", [1, 2])
+@pytest.mark.parametrize("eps", BEAM_EPS)
+def test_beam_along_another_axis(oracle_mod, axis, eps):
+    src, y, nu = beam(3, axis)
+    s = solver_of(src, y, nu, eps, "fp64")
+    psi = np.zeros(len(nu))
+    check(s, oracle_of(oracle_mod, src, y, nu, eps, psi), psi, 1e-12)
     s.close()
 
 

@@ -61,14 +61,14 @@ LATTICE = [
     (2, 56, 2, 1025, 1e-2, 64, 4, 1),     # more targets than are listed: the target blocks
     (2, 65, 3, 3000, 5e-3, 64, 16, 1),    # 195 points: fourth tiles of 3
     (2, 56, 2, 1100, 9e-4, 32, 16, 1),    # tiles of 32 (and 16) points
-    (2, 64, 2, 1500, 1.2e-3, 64, 4, 0),   # span beyond the runs'
+    (2, 64, 2, 1500, 1.2e-3, 64, 4, 1),   # factors of 300 bits
     (3, 8, 2, 64, 1e-2, 16, 1, 1),        # one full tile, one full block of targets
     (3, 7, 2, 9, 1e-2, 16, 1, 1),         # 14 points
     (3, 14, 2, 1300, 1e-2, 16, 8, 1),     # 28 points: second tiles of 12; target blocks
     (3, 18, 2, 1025, 1e-2, 16, 27, 1),    # 36 points: third tiles of 4
     (3, 10, 3, 1100, 2e-2, 16, 8, 1),     # 27-point cells: a period of 3
     (3, 10, 3, 65, 4e-3, 16, 8, 1),
-    (3, 10, 3, 65, 2e-3, 16, 8, 0),
+    (3, 10, 3, 65, 1.65e-3, 16, 8, 0),    # a run covers a tile, whose factors span 330 bits: one exponential each
 ]
 
 
