@@ -21,7 +21,7 @@ def solver_of(src, y, nu, eps, precision):
 
 @pytest.mark.parametrize("dim,n,order,N,tiles", [
     (2, 32, 2, 1024, 1), (2, 32, 2, 1025, 0),       # few points: only where all targets are listed
-    (2, 52, 2, 3001, 0), (2, 56, 2, 3001, 4), (2, 75, 2, 3001, 9), (2, 64, 3, 1025, 9),
+    (2, 48, 2, 3001, 0), (2, 52, 2, 3001, 4), (2, 75, 2, 3001, 9), (2, 64, 3, 1025, 9),
     (3, 8, 2, 1024, 1), (3, 8, 2, 1025, 0), (3, 13, 2, 1025, 0), (3, 14, 2, 1025, 8), (3, 16, 2, 1025, 8),
     (2, 11, 3, 33, 0), (3, 9, 2, 33, 0),            # 33 and 18 points per axis: more padding than points
 ])
