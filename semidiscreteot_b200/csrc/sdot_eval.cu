@@ -1098,9 +1098,10 @@ static DenseShape dense_shape_of(const sdot_ctx *c, double eps, bool fp64)
     // once it goes through their blocks in turn: few points are few CTAs with a long chain each.  Lattice against
     // cell sweeps, us per FP64 evaluation at eps = 1e-2, 1,025 / 3,001 / 10,538 targets: 2D 64^2 points 60 / 85 / 187
     // against 52 / 66 / 110, 96^2 58 / 76 / 153 against 60 / 84 / 175 (hybrid 66 / 86 / 168 against 62 / 84 / 164),
-    // 104^2 57 / 76 / 136 against 61 / 90 / 202 (66 / 86 / 157 against 64 / 90 / 188), 192^2 62 / 83 / 161 against 98 / 181 / 507; 3D 24^3 64 / 98 / 247
-    // against 66 / 97 / 208, 26^3 65 / 101 / 249 against 71 / 111 / 254 (hybrid 78 / 110 / 261 against 76 / 111 /
-    // 239), 28^3 63 / 102 / 234 against 76 / 120 / 287, 32^3 63 / 96 / 205 against 90 / 148 / 390.
+    // 104^2 57 / 76 / 136 against 61 / 90 / 202 (66 / 86 / 157 against 64 / 90 / 188), 192^2 62 / 83 / 161 against
+    // 98 / 181 / 507; 3D 24^3 64 / 98 / 247 against 66 / 97 / 208, 26^3 65 / 101 / 249 against 71 / 111 / 254 (hybrid
+    // 78 / 110 / 261 against 76 / 111 / 239), 28^3 63 / 102 / 234 against 76 / 120 / 287, 32^3 63 / 96 / 205 against
+    // 90 / 148 / 390.
     // (Batches have no such line: their other sweeps go by points without target slices, 1,468 us against 390 for
     // 16^3 points x 10,538 targets alone, and all problems' merges are one launch.)
     constexpr int64_t FEW_2D = 10000, FEW_3D = 18000;
